@@ -964,14 +964,14 @@ void phase1_pipelined(cdbg_engine* e, cdbg_seq_batch const* b, uint32_t k, uint3
 // hints; returns false (nothing launched that matters) when a file inflates
 // to more than its hint says, and the caller reads the files whole instead.
 // Phase 1 from the files with the device reader: the files' bytes as stored
-// go to the device; one warp per gzip file inflates it into the file's region
+// go to the device; one CTA per gzip file inflates it into the file's region
 // of HBM (inflate_streams), the FASTA records are cut in place
 // (fasta_compact), and the regions -- one sequence per file, records
 // separated by a byte that is not a base -- go through build_runs and
 // find_supers like the host reader's sequences, with the same runs.
 // Returns false, with nothing kept, when the files do not suit it (no gzip
 // file, or, with gpu_inflate = 0, one file holding so much of the input that
-// a warp per file is slower than the host threads) or when a stream goes
+// a CTA per file is slower than the host threads) or when a stream goes
 // back to the host reader.
 bool phase1_device_reader(cdbg_engine* e, std::vector<std::string> const& files, uint32_t threads, uint32_t k,
                           uint32_t m, uint32_t B, cdbg::run_table& rt_all, cdbg::super_list& sl_all, uint64_t* h2d,
@@ -995,10 +995,12 @@ bool phase1_device_reader(cdbg_engine* e, std::vector<std::string> const& files,
     }
     const uint64_t tot_in = ioff[nf], tot_out = ooff[nf];
     if (!any_gz) return false;
-    // a warp inflates a few tens of MB/s, a host thread several times that:
-    // the device reader wins while no file holds more than about 1/(6T) of
-    // the input
-    if (e->tune.gpu_inflate == 0 && (double)max_out * 6.0 * threads > (double)tot_out) return false;
+    // A CTA inflates ~170 MB/s and all files at once, T host threads ~T x 200
+    // MB/s together: the device reader wins while no file holds more than about
+    // 1/T of the input.  Phase 1 with the reading, device / host reader, gzip -1
+    // genomes: T = 16, 2.4 Mbp files: 12 files 20.2 / 16.5 ms, 16 files 21.3 /
+    // 24.9, 64 files 25.5 / 72; T = 4: 4 files 18.3 / 11.2, 6 files 18.6 / 21.3.
+    if (e->tune.gpu_inflate == 0 && (double)max_out * 1.25 * threads > (double)tot_out) return false;
     cudaStream_t st = e->st;
     char* h = (char*)e->h_in.ensure(tot_in + 64);
     cdbg::io::read_raw_files(files, threads, h, ioff.data());

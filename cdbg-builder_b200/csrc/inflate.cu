@@ -1,4 +1,4 @@
-// gzip (RFC 1952) / DEFLATE (RFC 1951) decoding on the device, one warp per
+// gzip (RFC 1952) / DEFLATE (RFC 1951) decoding on the device, one CTA per
 // file, and the FASTA record rules of the reference's reader (kseq, as used by
 // seq_reader.hpp:66 and restated by the host reader in host/io.cpp) applied
 // to the inflated bytes in place.
@@ -11,16 +11,26 @@
 // decides a result the host reader would decide differently: streams this
 // decoder does not accept go back to the host reader whole.
 //
-// Decoder layout (per warp): all 32 lanes run the same bit reader and table
-// lookups (identical values, broadcast shared-memory reads), so control flow
-// never diverges; lanes split the table construction and copies.  Output goes
-// through a 4 KiB ring in shared memory, written to HBM in aligned 1 KiB
-// chunks; match sources closer than the ring come from it, farther ones from
-// HBM (already written).  A literal/length lookup of 11 bits yields up to
-// three literals at once, or a whole match length; a distance lookup of 11
-// bits a whole distance (gzip -1 writes DNA as matches of about 4 bytes at a
-// few hundred bytes' distance, whose codes and extra bits fit the indexes);
-// codes longer than the tables fall back to a canonical decode by length.
+// Decoder layout (per CTA): warp 0 parses member and block headers, two warps
+// build the block's codes and all threads its lookup tables.
+// A block's symbols are decoded a window of IF_THREADS x WIN_LANE_BITS bits at
+// a time, a sub-window per thread.  Every thread but the first starts at a
+// guessed bit; a Huffman stream falls back into step with the true symbol
+// boundaries after a few symbols, and threads whose guess was wrong decode
+// again from their predecessor's exit until all agree (3 rounds for gzip -1
+// genomes, 5 for gzip -6).  The threads then write their symbols at their
+// output positions, one literal or match distance per output byte, and every
+// byte of the window finds its literal by following distances, independent of
+// the others; a source before the window is read from HBM.  A literal/length
+// lookup of 11 bits yields up to three literals at once, or a whole match
+// length; a distance lookup of 11 bits a whole distance (gzip -1 writes DNA as
+// matches of about 4 bytes at a few hundred bytes' distance, whose codes and
+// extra bits fit the indexes); codes longer than the tables fall back to a
+// canonical decode by length.
+//
+// Bound: the latency of one thread's dependent lookups, about 60 symbols per
+// window of 14 KB.  130 gzip -1 files of 2.4 MB (one per SM): 14.2 ms; symbol by
+// symbol with one warp per file 228 ms, windows of one warp per file 58.6 ms.
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -32,12 +42,21 @@ namespace cdbg {
 namespace {
 
 constexpr uint32_t FULL = 0xffffffffu;
-constexpr int LB_LIT = 11;               // literal/length table index bits
-constexpr int LB_DIST = 11;              // distance table index bits
-constexpr uint32_t IF_RING = 4096;       // shared-memory output window
-constexpr uint32_t IF_FLUSH = 1024;      // bytes per aligned write to HBM
-constexpr int IF_WARPS = 1;              // streams per CTA
-static_assert(IF_RING >= IF_FLUSH + 2 * 258, "match sources must be in the ring or already in HBM");
+constexpr int LB_LIT = 11;     // literal/length table index bits
+constexpr int LB_DIST = 11;    // distance table index bits
+constexpr int LB_CLEN = 7;     // code-length code table index bits (its longest code)
+constexpr int IF_THREADS = 256;
+constexpr int IF_WARPS = IF_THREADS / 32;
+// Bits decoded per thread and window: about a dozen symbols of genome data, so
+// most guesses are back in step by their sub-window's end; an odd number of
+// 32-bit words, so a warp's reads of the staged bits fall into different banks.
+constexpr uint32_t WIN_LANE_BITS = 160;
+constexpr int WIN_STAGE = 648;  // staged 64-bit words of input
+static_assert(IF_THREADS * WIN_LANE_BITS + 63 + 48 + 96 <= 64 * WIN_STAGE, "a window's bits and its last symbols fit");
+// Output bytes of a window, at most: a thread's symbols always fit (a match
+// takes at least 2 bits), so every window makes progress.
+constexpr uint32_t WIN_OUT = 24576;
+static_assert((WIN_LANE_BITS / 2 + 1) * 258 <= WIN_OUT, "one thread's symbols fit the window");
 
 // RFC 1951 3.2.5: length codes 257..285 and distance codes 0..29
 __constant__ uint16_t c_len_base[29] = {3,  4,  5,  6,  7,  8,  9,  10, 11,  13,  15,  17,  19,  23, 27,
@@ -60,8 +79,19 @@ struct code_aux {
     uint16_t sym[288];
 };
 
-struct __align__(16) warp_state {
-    uint8_t ring[IF_RING];
+// Header fields and the position, from the parsing warp to the CTA.
+struct block_ctl {
+    uint64_t bit;      // next bit of the stream
+    uint32_t status;   // stream_status
+    uint32_t type;     // block type, or BLK_DONE after the stream's last member
+    uint32_t last;     // the member's last block
+    uint32_t nlit, ndist;
+    uint32_t stored;   // bytes of a stored block
+    uint32_t member0;  // output position of the member's first byte
+};
+constexpr uint32_t BLK_DONE = 4;
+
+struct __align__(16) cta_state {
     // literal/length lookups (LB_LIT bits of input): bits 0-4 bits consumed,
     // bits 5-7 kind: 1-3 literals (bytes at bits 8, 16, 24), K_LEN a match
     // length (bits 8-16, extra bits that fit the index already added; bits
@@ -72,16 +102,31 @@ struct __align__(16) warp_state {
     // extra bits still to read, bits 9-24 distance (folded extra added),
     // bits 25-26 kind: 1 valid, 2 no valid distance, 0 decode by length
     uint32_t dist[1 << LB_DIST];
-    uint16_t one[1 << LB_LIT];  // one symbol per lookup, (length << 9) | symbol
-    code_aux la, da;
-    uint32_t hist[16];
+    union {
+        struct {  // while tables are built: one symbol per lookup, (length << 9) | symbol
+            uint16_t one_l[1 << LB_LIT];
+            uint16_t one_d[1 << LB_DIST];
+            uint16_t one_c[1 << LB_CLEN];
+        };
+        // window output: 0x8000 | literal byte, or match distance - 1
+        uint16_t ent[WIN_OUT];
+    };
+    uint64_t stage[WIN_STAGE];  // the window's input bits
+    code_aux la, da, ca;
+    uint32_t hist[2][16];
     uint8_t lens[320];
+    uint32_t exits[IF_THREADS];  // bit after each thread's symbols
+    uint32_t warp_sum[IF_WARPS];
+    uint32_t stop[2];
+    uint32_t total, end;  // of a window: bytes, bit after the last symbol
+    uint32_t ok[2];
+    block_ctl ctl;
 };
 
 constexpr uint32_t K_LEN = 4, K_END = 5, K_BAD = 6;
 
 // Little-endian bit reader over the input (RFC 1951 3.1.1: bits from the
-// least significant end of each byte).  All lanes hold the same state.  The
+// least significant end of each byte).  All lanes of the parsing warp hold the same state.  The
 // buffer above the `nb` valid bits holds either zeros or the input bits that
 // follow (a refill ORs the next eight bytes in place, so repeated bytes land
 // on identical bits); code that moves `ip` by hand clears it.
@@ -134,12 +179,12 @@ __device__ __forceinline__ uint32_t lanemask_lt_() {
     return m;
 }
 
-// Decoding tables of the code with lengths lens[0, n).  Returns false for an
-// over-subscribed set, and for an incomplete one unless it is a single code
-// of one bit or no code at all (with `strict`, for the code-length code, any
-// incomplete set) -- the sets zlib also refuses.  Warp-collective.
-__device__ bool build_code(uint8_t const* lens, int n, uint16_t* tab, int lb, code_aux& a, uint32_t* hist,
-                           int lane, bool strict) {
+// The canonical code with lengths lens[0, n) by length: counts, first codes and
+// symbols in order.  Returns false for an over-subscribed set, and for an
+// incomplete one unless it is a single code of one bit or no code at all (with
+// `strict`, for the code-length code, any incomplete set) -- the sets zlib also
+// refuses.  Warp-collective.
+__device__ bool build_aux(uint8_t const* lens, int n, code_aux& a, uint32_t* hist, int lane, bool strict) {
     if (lane < 16) hist[lane] = 0;
     __syncwarp();
     for (int s0 = 0; s0 < n; s0 += 32) {
@@ -170,7 +215,6 @@ __device__ bool build_code(uint8_t const* lens, int n, uint16_t* tab, int lb, co
     }
     ok = __shfl_sync(FULL, ok, 0);
     if (!ok) return false;
-    for (int i = lane; i < (1 << lb) / 2; i += 32) reinterpret_cast<uint32_t*>(tab)[i] = 0u;
     if (lane < 16) hist[lane] = 0;
     __syncwarp();
     for (int s0 = 0; s0 < n; s0 += 32) {
@@ -178,28 +222,23 @@ __device__ bool build_code(uint8_t const* lens, int n, uint16_t* tab, int lb, co
         const uint32_t l = s < n ? lens[s] : 0u;
         const uint32_t grp = __match_any_sync(FULL, l);
         const uint32_t before = l ? hist[l] : 0u;
-        const uint32_t rank = before + __popc(grp & lanemask_lt_());
+        const uint32_t rank = before + __popc(grp & ((1u << lane) - 1u));
         __syncwarp();
         if (l) {
             if (lane == __ffs(grp) - 1) hist[l] = before + __popc(grp);
             a.sym[a.base[l] + rank] = (uint16_t)s;
-            if (l <= (uint32_t)lb) {
-                const uint32_t rev = __brev(a.first[l] + rank) >> (32 - l);
-                const uint16_t e = (uint16_t)((l << 9) | (uint32_t)s);
-                for (uint32_t x = rev; x < (1u << lb); x += 1u << l) tab[x] = e;
-            }
         }
         __syncwarp();
     }
     return true;
 }
 
-// Canonical decode by length (codes longer than a table's index) of the
-// next bits `bb`: (bits used << 16) | symbol, or -1 for a bit string that is
-// no code.
-__device__ __noinline__ int decode_slow(uint64_t bb, code_aux const& a) {
+// Canonical decode of the next bits `bb` by length, codes of at most `maxlen`
+// bits: (bits used << 16) | symbol, or -1 for a bit string that starts with no
+// such code.
+__device__ __forceinline__ int decode_canonical(uint64_t bb, code_aux const& a, int maxlen) {
     uint32_t code = 0;
-    for (int len = 1; len < 16; ++len) {
+    for (int len = 1; len <= maxlen; ++len) {
         code = (code << 1) | ((uint32_t)bb & 1u);
         bb >>= 1;
         const uint32_t off = code - a.first[len];
@@ -207,32 +246,25 @@ __device__ __noinline__ int decode_slow(uint64_t bb, code_aux const& a) {
     }
     return -1;
 }
+__device__ __noinline__ int decode_slow(uint64_t bb, code_aux const& a) { return decode_canonical(bb, a, 15); }
 
-// One symbol from a one-symbol table (at least 15 bits buffered); -1 for a
-// bit string that is no code.
-__device__ __forceinline__ int decode_sym(bit_reader& br, uint16_t const* tab, int lb, code_aux const& a) {
-    const uint32_t e = tab[(uint32_t)br.bb & ((1u << lb) - 1u)];
-    const uint32_t l = e >> 9;
-    if (l) {
-        br.drop(l);
-        return (int)(e & 511u);
+// One-symbol lookups of `lb` index bits from thread t of `nt` on.
+__device__ __forceinline__ void fill_one(uint16_t* tab, int lb, code_aux const& a, uint32_t t, uint32_t nt) {
+    for (uint32_t x = t; x < (1u << lb); x += nt) {
+        const int r = decode_canonical(x, a, lb);
+        tab[x] = r < 0 ? (uint16_t)0 : (uint16_t)(((uint32_t)r >> 16 << 9) | ((uint32_t)r & 511u));
     }
-    const int r = decode_slow(br.bb, a);
-    if (r < 0) return -1;
-    br.drop((uint32_t)r >> 16);
-    return r & 0xffff;
 }
 
-// Literal/length lookups from the one-symbol table in w.one.  A literal whose
-// code leaves room in the index for the next code(s), when those are
-// literals too, yields two or three (the bits after a code are the index
-// shifted right by its length, upper bits zero, which select the same entry
-// for any code that fits); a length code whose extra bits fit in the index
-// comes with them added.  Warp-collective.
-__device__ void pack_litlen(warp_state& w, int lane) {
-    __syncwarp();
-    for (uint32_t x = (uint32_t)lane; x < (1u << LB_LIT); x += 32) {
-        const uint32_t e1 = w.one[x];
+// Literal/length lookups from the one-symbol table.  A literal whose code
+// leaves room in the index for the next code(s), when those are literals too,
+// yields two or three (the bits after a code are the index shifted right by
+// its length, upper bits zero, which select the same entry for any code that
+// fits); a length code whose extra bits fit in the index comes with them
+// added.
+__device__ __forceinline__ void pack_litlen(cta_state& w, uint32_t t) {
+    for (uint32_t x = t; x < (1u << LB_LIT); x += IF_THREADS) {
+        const uint32_t e1 = w.one_l[x];
         const uint32_t l1 = e1 >> 9, s1 = e1 & 511u;
         uint32_t out = 0;
         if (l1 == 0) {
@@ -240,13 +272,13 @@ __device__ void pack_litlen(warp_state& w, int lane) {
         } else if (s1 < 256) {
             uint32_t tot = l1, cnt = 1;
             out = s1 << 8;
-            const uint32_t e2 = w.one[x >> tot];
+            const uint32_t e2 = w.one_l[x >> tot];
             const uint32_t l2 = e2 >> 9, s2 = e2 & 511u;
             if (l2 && s2 < 256 && tot + l2 <= (uint32_t)LB_LIT) {
                 out |= s2 << 16;
                 ++cnt;
                 tot += l2;
-                const uint32_t e3 = w.one[x >> tot];
+                const uint32_t e3 = w.one_l[x >> tot];
                 const uint32_t l3 = e3 >> 9, s3 = e3 & 511u;
                 if (l3 && s3 < 256 && tot + l3 <= (uint32_t)LB_LIT) {
                     out |= s3 << 24;
@@ -271,14 +303,12 @@ __device__ void pack_litlen(warp_state& w, int lane) {
         }
         w.lit[x] = out;
     }
-    __syncwarp();
 }
 
-// Distance lookups from the one-symbol table in w.one.  Warp-collective.
-__device__ void pack_dist(warp_state& w, int lane) {
-    __syncwarp();
-    for (uint32_t x = (uint32_t)lane; x < (1u << LB_DIST); x += 32) {
-        const uint32_t e1 = w.one[x];
+// Distance lookups from the one-symbol table.
+__device__ __forceinline__ void pack_dist(cta_state& w, uint32_t t) {
+    for (uint32_t x = t; x < (1u << LB_DIST); x += IF_THREADS) {
+        const uint32_t e1 = w.one_d[x];
         const uint32_t l1 = e1 >> 9, s1 = e1 & 511u;
         uint32_t out = 0;
         if (l1 && s1 < 30) {
@@ -295,56 +325,244 @@ __device__ void pack_dist(warp_state& w, int lane) {
         }
         w.dist[x] = out;
     }
-    __syncwarp();
 }
 
-struct out_state {
-    uint8_t* o;      // region in HBM
-    uint32_t cap;    // (a stream of 4 GiB or more goes to the host reader)
-    uint32_t op;     // bytes produced
-    uint32_t fp;     // bytes written to HBM (a multiple of IF_FLUSH)
-};
-
-// Writes ring bytes [fp, fp + IF_FLUSH) to HBM (32 bytes per lane, aligned).
-__device__ __forceinline__ void flush_chunk(warp_state& w, out_state& os, int lane) {
-    __syncwarp();
-    const uint32_t r = os.fp & (IF_RING - 1);
-    uint4 const* src = reinterpret_cast<uint4 const*>(w.ring + r) + 2 * lane;
-    uint4* dst = reinterpret_cast<uint4*>(os.o + os.fp) + 2 * lane;
-    dst[0] = src[0];
-    dst[1] = src[1];
-    os.fp += IF_FLUSH;
-    __syncwarp();
-}
-
-// Copies L bytes from distance d back (d <= bytes produced in this member).
-// Lane i copies byte i of each 32-byte round.  Every source position lies
-// before the copy (an overlapping copy, d < L, reads position op - d +
-// (i mod d): the period repeats), so no lane reads what this copy writes; a
-// ring slot read here is written here only when the write lands a whole ring
-// later (d + L > IF_RING), and then each round's writes wait for all reads.
-// The common case -- at most 32 bytes, no overlap, source in the ring -- is
-// one round.
-__device__ __forceinline__ void copy_match(warp_state& w, out_state& os, uint32_t d, uint32_t L, int lane) {
-    __syncwarp();  // the bytes stored before are visible to every lane
-    const uint32_t i = (uint32_t)lane;
-    if (L <= 32 && d >= L && d + L <= IF_RING) {
-        if (i < L) w.ring[(os.op + i) & (IF_RING - 1)] = w.ring[(os.op - d + i) & (IF_RING - 1)];
-        os.op += L;
-        return;
-    }
-    const bool wrap = d + L > IF_RING;
-    for (uint32_t i0 = 0; i0 < L; i0 += 32) {
-        const uint32_t j = i0 + i;
-        uint8_t v = 0;
-        if (j < L) {
-            const uint32_t src = os.op - d + (d < L ? j % d : j);
-            v = d <= IF_RING ? w.ring[src & (IF_RING - 1)] : os.o[src];
+// One thread's symbols from staged bit `pos` until it reaches `limit`: the bit
+// after the last symbol in `pos`, the bytes they stand for in `out`.  Returns
+// LANE_MORE, LANE_END after an end-of-block symbol, or LANE_BAD at a bit
+// string that is no symbol (or past `bits_end`, the stream's last bit).  With
+// WRITE, the symbols' entries go to ent[o ..] and `back` is the bytes of this
+// member before the window: a distance past them is LANE_BAD.  A symbol takes
+// at most 48 bits, and the stage holds the bits that follow the window.
+enum : uint32_t { LANE_MORE = 0, LANE_END = 1, LANE_BAD = 2 };
+template <bool WRITE>
+__device__ __forceinline__ uint32_t lane_symbols(cta_state& w, uint32_t& pos, uint32_t limit, uint32_t bits_end,
+                                                 uint32_t& out, uint32_t o, uint32_t back) {
+    uint32_t const* sw = reinterpret_cast<uint32_t const*>(w.stage);
+    uint32_t p = pos, n = 0, st = LANE_MORE;
+    uint32_t wi = (p >> 5) + 2;
+    uint64_t bb = (((uint64_t)sw[wi - 1] << 32) | sw[wi - 2]) >> (p & 31);
+    uint32_t nb = 64 - (p & 31);
+    auto refill = [&]() {  // afterwards at least 33 bits
+        if (nb <= 32) {
+            bb |= (uint64_t)sw[wi++] << nb;
+            nb += 32;
         }
-        if (wrap) __syncwarp();
-        if (j < L) w.ring[(os.op + j) & (IF_RING - 1)] = v;
+    };
+    auto drop = [&](uint32_t c) {
+        bb >>= c;
+        nb -= c;
+        p += c;
+    };
+    while (p < limit) {
+        if (p > bits_end) {
+            st = LANE_BAD;
+            break;
+        }
+        refill();
+        const uint32_t e = w.lit[(uint32_t)bb & ((1u << LB_LIT) - 1u)];
+        const uint32_t kind = (e >> 5) & 7u;
+        uint32_t L;
+        if (kind - 1u < 3u) {  // one to three literals
+            if (WRITE) {
+                w.ent[o + n] = (uint16_t)(0x8000u | ((e >> 8) & 0xffu));
+                if (kind > 1) w.ent[o + n + 1] = (uint16_t)(0x8000u | ((e >> 16) & 0xffu));
+                if (kind > 2) w.ent[o + n + 2] = (uint16_t)(0x8000u | (e >> 24));
+            }
+            n += kind;
+            drop(e & 31u);
+            continue;
+        }
+        if (kind == K_LEN) {
+            drop(e & 31u);
+            const uint32_t x = (e >> 17) & 7u;
+            L = ((e >> 8) & 511u) + ((uint32_t)bb & ((1u << x) - 1u));
+            drop(x);
+        } else if (kind == K_END) {
+            drop(e & 31u);
+            st = LANE_END;
+            break;
+        } else if (kind == K_BAD) {
+            st = LANE_BAD;
+            break;
+        } else {
+            // a code longer than the index
+            const int r = decode_slow(bb, w.la);
+            if (r < 0) {
+                st = LANE_BAD;
+                break;
+            }
+            drop((uint32_t)r >> 16);
+            const uint32_t sym = (uint32_t)r & 0xffffu;
+            if (sym < 256) {
+                if (WRITE) w.ent[o + n] = (uint16_t)(0x8000u | sym);
+                ++n;
+                continue;
+            }
+            if (sym == 256) {
+                st = LANE_END;
+                break;
+            }
+            if (sym > 285) {
+                st = LANE_BAD;
+                break;
+            }
+            const uint32_t x = c_len_extra[sym - 257];
+            L = c_len_base[sym - 257] + ((uint32_t)bb & ((1u << x) - 1u));
+            drop(x);
+        }
+        refill();
+        const uint32_t de = w.dist[(uint32_t)bb & ((1u << LB_DIST) - 1u)];
+        const uint32_t dk = de >> 25;
+        uint32_t d, x;
+        if (dk == 1) {
+            drop(de & 31u);
+            d = (de >> 9) & 0xffffu;
+            x = (de >> 5) & 15u;
+        } else if (dk == 0) {
+            const int r = decode_slow(bb, w.da);
+            if (r < 0 || (r & 0xffff) >= 30) {
+                st = LANE_BAD;
+                break;
+            }
+            drop((uint32_t)r >> 16);
+            const uint32_t ds = (uint32_t)r & 0xffffu;
+            d = c_dist_base[ds];
+            x = c_dist_extra[ds];
+        } else {
+            st = LANE_BAD;
+            break;
+        }
+        d += (uint32_t)bb & ((1u << x) - 1u);
+        drop(x);
+        if (WRITE) {
+            if (d > back + o + n) {
+                st = LANE_BAD;
+                break;
+            }
+            for (uint32_t i = 0; i < L; ++i) w.ent[o + n + i] = (uint16_t)(d - 1);
+        }
+        n += L;
     }
-    os.op += L;
+    pos = p;
+    out = n;
+    return st;
+}
+
+// The next window of a block's symbols (up to IF_THREADS x WIN_LANE_BITS bits
+// from bit `bit`, moved past the symbols taken), written to o[op ..].
+// WIN_MORE: the block goes on; WIN_DONE: its end-of-block symbol was the last.
+// CTA-collective, with the same arguments.
+enum : uint32_t { WIN_MORE = 0, WIN_DONE = 1, WIN_BAD = 2, WIN_OVERFLOW = 3 };
+__device__ __forceinline__ uint32_t window_decode(cta_state& w, uint8_t const* in, uint64_t end, uint64_t& bit,
+                                                  uint8_t* o, uint32_t cap, uint32_t& op, uint32_t member0) {
+    const uint32_t t = threadIdx.x;
+    const int lane = t & 31, warp = t >> 5;
+    // input bits from the 8-byte word of the first bit on
+    const uint64_t a0 = (bit >> 6) * 8;
+    const uint32_t ph = (uint32_t)(bit & 63);
+    for (uint32_t i = t; i < (uint32_t)WIN_STAGE; i += IF_THREADS) {
+        const uint64_t a = a0 + 8ull * i;
+        w.stage[i] = a < end + 16 ? __ldg(reinterpret_cast<unsigned long long const*>(in + a)) : 0ull;
+    }
+    if (t < 2) w.stop[t] = IF_THREADS - 1;
+    __syncthreads();
+    // bits of the stream left from a0 on (a window past them is refused)
+    const uint64_t left = end > a0 ? (end - a0) * 8 : 0;
+    const uint32_t bits_end = left < 0xffffffffull ? (uint32_t)left : 0xffffffffu;
+    uint32_t start = ph + t * WIN_LANE_BITS;
+    const uint32_t limit = start + WIN_LANE_BITS;
+    uint32_t pos = start, n = 0;
+    uint32_t st = lane_symbols<false>(w, pos, limit, bits_end, n, 0, 0);
+    // Thread 0 started right; each round every thread up to the first that
+    // stopped takes its predecessor's exit as its start, so after r rounds
+    // threads 0..r are right whatever the guesses were: the loop ends by itself
+    // within IF_THREADS rounds.
+    uint32_t stop = 0;
+    for (int r = 0; r <= IF_THREADS; ++r) {
+        w.exits[t] = pos;
+        if (st != LANE_MORE) atomicMin(&w.stop[r & 1], t);
+        __syncthreads();
+        stop = w.stop[r & 1];
+        const uint32_t want = t ? w.exits[t - 1] : start;
+        const bool stale = t <= stop && want != start;
+        if (!__syncthreads_or(stale)) break;
+        if (t == 0) w.stop[r & 1] = IF_THREADS - 1;  // for the round after the next
+        if (stale) {
+            start = pos = want;
+            st = lane_symbols<false>(w, pos, limit, bits_end, n, 0, 0);
+        }
+    }
+    // output offsets; threads 0 .. take - 1 are right, complete and within
+    // the entry array (a prefix of the threads, by construction)
+    uint32_t incl = n;
+#pragma unroll
+    for (int s = 1; s < 32; s <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, incl, s);
+        if (lane >= s) incl += y;
+    }
+    if (lane == 31) w.warp_sum[warp] = incl;
+    __syncthreads();
+    for (int i = 0; i < warp; ++i) incl += w.warp_sum[i];
+    const uint32_t take = (uint32_t)__syncthreads_count(t <= stop && st != LANE_BAD && incl <= WIN_OUT);
+    if (take == 0) return WIN_BAD;  // thread 0's first symbol is none (its bytes always fit)
+    if (t == take - 1) {
+        w.total = incl;
+        w.end = pos;
+        w.ok[0] = st == LANE_END;
+    }
+    uint32_t wst = LANE_MORE;
+    if (t < take) {
+        uint32_t p = start, m;
+        wst = lane_symbols<true>(w, p, limit, bits_end, m, incl - n, op - member0);
+    }
+    if (__syncthreads_or(wst == LANE_BAD)) return WIN_BAD;  // a distance before the member's first byte
+    const uint32_t total = w.total;
+    const bool done = w.ok[0] != 0;
+    if ((uint64_t)op + total > cap) return WIN_OVERFLOW;
+    // Every byte follows its match distances back to a literal of the window
+    // or to a byte before it, which is in HBM; a thread takes the four bytes of
+    // an aligned output word.
+    const uint32_t ph4 = op & 3u;  // regions start 16-byte aligned
+    for (uint32_t g = t; 4 * g < total + ph4; g += IF_THREADS) {
+        uint32_t p[4], e[4];
+        const uint32_t j0 = 4 * g - ph4;  // (wraps below 0 in the first word)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            p[u] = j0 + u;
+            e[u] = p[u] < total ? w.ent[p[u]] : 0x8000u;
+        }
+        for (;;) {
+            bool more = false;
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                if (e[u] < 0x8000u && p[u] > e[u]) {  // distance e + 1 <= p: a byte of the window
+                    p[u] -= e[u] + 1;
+                    e[u] = w.ent[p[u]];
+                    more = true;
+                }
+            }
+            if (!more) break;
+        }
+        uint32_t v = 0;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            uint32_t b = e[u] & 0xffu;
+            if (e[u] < 0x8000u) b = o[op + p[u] - (e[u] + 1)];
+            v |= b << (8 * u);
+        }
+        if (j0 < total && j0 + 4 <= total) {
+            *reinterpret_cast<uint32_t*>(o + op + j0) = v;
+        } else {
+#pragma unroll
+            for (int u = 0; u < 4; ++u)
+                if (j0 + u < total) o[op + j0 + u] = (uint8_t)(v >> (8 * u));
+        }
+    }
+    op += total;
+    bit = a0 * 8 + w.end;
+    __syncthreads();  // the entries, the stage and the totals are reused; the bytes are visible to the CTA
+    return done ? WIN_DONE : WIN_MORE;
 }
 
 // gzip member header (RFC 1952 2.3.1) at a byte boundary.
@@ -380,275 +598,224 @@ __device__ bool read_member_header(bit_reader& br) {
     return !br.overrun();
 }
 
-__global__ void __launch_bounds__(IF_WARPS * 32) k_inflate(stream_set s) {
-    __shared__ warp_state W[IF_WARPS];
-    const int lane = threadIdx.x & 31, wi = threadIdx.x >> 5;
-    const uint32_t f = blockIdx.x * IF_WARPS + (uint32_t)wi;
-    if (f >= s.n) return;  // whole warp
-    warp_state& w = W[wi];
+// The next block header from bit ctl.bit on -- after the member header when
+// `member_start`, after the trailer checks of a member's last block and the
+// next member's header when `trailer` -- into ctl and the code lengths.  `op`
+// is the output position.  Warp-collective (the parsing warp).
+__device__ __forceinline__ void parse_block_header(cta_state& w, uint8_t const* in, uint64_t end, bool member_start,
+                                                   bool trailer, uint32_t op, int lane) {
+    block_ctl& c = w.ctl;
+    bit_reader br{in, 0, end, 0, 0};
+    br.seek(c.bit >> 3);
+    br.refill();
+    br.drop((uint32_t)(c.bit & 7));
+    uint32_t st = STREAM_OK, type = BLK_DONE, last = 0, nlit = 0, ndist = 0, stored = 0;
+    uint32_t member0 = c.member0;
+    __syncwarp();  // every lane has read ctl
+    do {
+        if (trailer) {
+            // trailer: CRC-32 (not checked here) and ISIZE = member size mod 2^32
+            br.align();
+            br.refill();
+            br.get(16);
+            br.get(16);
+            br.refill();
+            const uint32_t lo = br.get(16), isize = lo | (br.get(16) << 16);
+            if (br.overrun() || isize != op - member0) {
+                st = STREAM_BAD;
+                break;
+            }
+            const uint64_t p = br.pos();
+            if (p > br.end) {
+                st = STREAM_BAD;
+                break;
+            }
+            if (p == br.end) break;  // BLK_DONE
+            // another member follows (anything else fails its header check)
+            br.seek(p);
+        }
+        if (member_start || trailer) {
+            if (!read_member_header(br)) {
+                st = STREAM_BAD;
+                break;
+            }
+            member0 = op;
+        }
+        br.refill();
+        if (br.overrun()) {
+            st = STREAM_BAD;
+            break;
+        }
+        last = br.get(1);
+        type = br.get(2);
+        if (type == 0) {
+            // stored: LEN, NLEN at the next byte boundary, then LEN bytes
+            br.align();
+            stored = br.get(16);
+            const uint32_t nlen = br.get(16);
+            if ((stored ^ 0xffffu) != nlen || br.pos() + stored > br.end) st = STREAM_BAD;
+        } else if (type == 1) {
+            // fixed codes (RFC 1951 3.2.6); 32 distance codes of 5 bits
+            // (30 and 31 never valid) keep the set complete
+            for (int i = lane; i < 288 + 32; i += 32)
+                w.lens[i] = i < 144 ? 8 : i < 256 ? 9 : i < 280 ? 7 : i < 288 ? 8 : 5;
+            nlit = 288;
+            ndist = 32;
+        } else if (type == 2) {
+            // dynamic codes (RFC 1951 3.2.7)
+            nlit = br.get(5) + 257;
+            ndist = br.get(5) + 1;
+            const uint32_t hclen = br.get(4) + 4;
+            if (nlit > 286 || ndist > 30) {
+                st = STREAM_BAD;
+                break;
+            }
+            if (lane < 19) w.lens[lane] = 0;
+            __syncwarp();
+            for (uint32_t i = 0; i < hclen; ++i) {
+                br.refill();
+                const uint32_t v = br.get(3);
+                if (lane == 0) w.lens[c_clen_order[i]] = (uint8_t)v;
+            }
+            __syncwarp();
+            if (!build_aux(w.lens, 19, w.ca, w.hist[0], lane, true)) {
+                st = STREAM_BAD;
+                break;
+            }
+            __syncwarp();
+            fill_one(w.one_c, LB_CLEN, w.ca, (uint32_t)lane, 32);
+            __syncwarp();
+            const uint32_t total = nlit + ndist;
+            uint32_t n = 0, prev = 0;
+            while (n < total) {
+                br.refill();
+                if (br.overrun()) {
+                    st = STREAM_BAD;
+                    break;
+                }
+                const uint32_t e = w.one_c[(uint32_t)br.bb & ((1u << LB_CLEN) - 1u)];
+                if (e == 0) {  // no code of this bit string
+                    st = STREAM_BAD;
+                    break;
+                }
+                br.drop(e >> 9);
+                const uint32_t sym = e & 511u;
+                uint32_t rep = 1, val = sym;
+                if (sym >= 16) {
+                    if (sym == 16) {
+                        if (n == 0) {
+                            st = STREAM_BAD;
+                            break;
+                        }
+                        val = prev;
+                        rep = 3 + br.get(2);
+                    } else {
+                        val = 0;
+                        rep = sym == 17 ? 3 + br.get(3) : 11 + br.get(7);
+                    }
+                    if (n + rep > total) {
+                        st = STREAM_BAD;
+                        break;
+                    }
+                }
+                for (uint32_t j = (uint32_t)lane; j < rep; j += 32) w.lens[n + j] = (uint8_t)val;
+                prev = val;
+                n += rep;
+            }
+            __syncwarp();
+            if (st == STREAM_OK && w.lens[256] == 0) st = STREAM_BAD;
+        } else {
+            st = STREAM_BAD;
+        }
+    } while (false);
+    if (lane == 0) {
+        c.bit = br.ip * 8 - br.nb;
+        c.status = st;
+        c.type = type;
+        c.last = last;
+        c.nlit = nlit;
+        c.ndist = ndist;
+        c.stored = stored;
+        c.member0 = member0;
+    }
+}
+
+__global__ void __launch_bounds__(IF_THREADS) k_inflate(stream_set s) {
+    extern __shared__ __align__(16) unsigned char if_raw[];
+    cta_state& w = *reinterpret_cast<cta_state*>(if_raw);
+    const uint32_t f = blockIdx.x, t = threadIdx.x;
+    const int lane = t & 31, warp = t >> 5;
     const uint64_t cap64 = s.out_cap[f];
-    out_state os{s.out + s.out_off[f], (uint32_t)(cap64 < 0xfffff000ull ? cap64 : 0xfffff000ull), 0, 0};
-    uint32_t st = STREAM_OK;
+    const uint32_t cap = (uint32_t)(cap64 < 0xfffff000ull ? cap64 : 0xfffff000ull);  // (4 GiB: the host reader)
+    uint8_t* o = s.out + s.out_off[f];
+    const uint64_t in0 = s.in_off[f], end = in0 + s.in_len[f];
     if (!s.gz[f]) {
         // plain file: copied as is
-        const uint64_t n = s.in_len[f];
-        if (n > os.cap) {
+        const uint64_t n = end - in0;
+        uint32_t st = STREAM_OK;
+        if (n > cap)
             st = STREAM_OVERFLOW;
-        } else {
-            uint8_t const* src = s.in + s.in_off[f];
-            for (uint64_t i = (uint64_t)lane; i < n; i += 32) os.o[i] = src[i];
-            os.op = (uint32_t)n;
-        }
-        if (lane == 0) {
-            s.out_len[f] = os.op;
+        else
+            for (uint64_t i = t; i < n; i += IF_THREADS) o[i] = s.in[in0 + i];
+        if (t == 0) {
+            s.out_len[f] = st == STREAM_OK ? n : 0;
             s.status[f] = st;
         }
         return;
     }
-    bit_reader br{s.in, s.in_off[f], s.in_off[f] + s.in_len[f], 0, 0};
-    for (;;) {  // members
-        if (!read_member_header(br)) {
-            st = STREAM_BAD;
-            break;
-        }
-        const uint32_t member0 = os.op;
-        bool last = false;
-        while (!last && st == STREAM_OK) {  // blocks
-            br.refill();
-            if (br.overrun()) {
+    uint32_t op = 0, st = STREAM_OK;
+    uint64_t bit = in0 * 8;
+    bool member_start = true, trailer = false;
+    if (t == 0) w.ctl.member0 = 0;
+    for (;;) {  // blocks
+        if (t == 0) w.ctl.bit = bit;
+        __syncthreads();
+        if (warp == 0) parse_block_header(w, s.in, end, member_start, trailer, op, lane);
+        __syncthreads();
+        const block_ctl c = w.ctl;
+        st = c.status;
+        if (st != STREAM_OK || c.type == BLK_DONE) break;
+        member_start = false;
+        bit = c.bit;
+        if (c.type == 0) {
+            if ((uint64_t)op + c.stored > cap) {
+                st = STREAM_OVERFLOW;
+                break;
+            }
+            const uint64_t p = bit >> 3;
+            for (uint32_t i = t; i < c.stored; i += IF_THREADS) o[op + i] = s.in[p + i];
+            op += c.stored;
+            bit = (p + c.stored) * 8;
+            __syncthreads();  // every thread has read ctl
+        } else {
+            if (warp < 2) {
+                const bool lc = warp == 0;
+                const bool ok = build_aux(lc ? w.lens : w.lens + c.nlit, (int)(lc ? c.nlit : c.ndist),
+                                          lc ? w.la : w.da, w.hist[warp], lane, false);
+                if (lane == 0) w.ok[warp] = ok ? 1u : 0u;
+            }
+            __syncthreads();
+            if (!w.ok[0] || !w.ok[1]) {
                 st = STREAM_BAD;
                 break;
             }
-            last = br.get(1) != 0;
-            const uint32_t type = br.get(2);
-            if (type == 0) {
-                // stored: LEN, NLEN at the next byte boundary, then LEN bytes
-                br.align();
-                const uint32_t len = br.get(16), nlen = br.get(16);
-                if ((len ^ 0xffffu) != nlen) {
-                    st = STREAM_BAD;
-                    break;
-                }
-                if ((uint64_t)os.op + len > os.cap) {
-                    st = STREAM_OVERFLOW;
-                    break;
-                }
-                const uint64_t p = br.pos();
-                if (p + len > br.end) {
-                    st = STREAM_BAD;
-                    break;
-                }
-                for (uint32_t i0 = 0; i0 < len; i0 += 32) {
-                    if (os.op - os.fp >= IF_FLUSH) flush_chunk(w, os, lane);
-                    const uint32_t n = min(32u, len - i0);
-                    if ((uint32_t)lane < n) w.ring[(os.op + lane) & (IF_RING - 1)] = br.in[p + i0 + lane];
-                    os.op += n;
-                    __syncwarp();
-                }
-                br.seek(p + len);
-                continue;
-            }
-            if (type == 3) {
-                st = STREAM_BAD;
+            fill_one(w.one_l, LB_LIT, w.la, t, IF_THREADS);
+            fill_one(w.one_d, LB_DIST, w.da, t, IF_THREADS);
+            __syncthreads();
+            pack_litlen(w, t);
+            pack_dist(w, t);
+            __syncthreads();
+            uint32_t ws = WIN_MORE;
+            while (ws == WIN_MORE) ws = window_decode(w, s.in, end, bit, o, cap, op, c.member0);
+            if (ws != WIN_DONE) {
+                st = ws == WIN_OVERFLOW ? STREAM_OVERFLOW : STREAM_BAD;
                 break;
             }
-            if (type == 1) {
-                // fixed codes (RFC 1951 3.2.6); 32 distance codes of 5 bits
-                // (30 and 31 never valid) keep the set complete
-                for (int i = lane; i < 288 + 32; i += 32)
-                    w.lens[i] = i < 144 ? 8 : i < 256 ? 9 : i < 280 ? 7 : i < 288 ? 8 : 5;
-                __syncwarp();
-                build_code(w.lens, 288, w.one, LB_LIT, w.la, w.hist, lane, false);
-                pack_litlen(w, lane);
-                build_code(w.lens + 288, 32, w.one, LB_DIST, w.da, w.hist, lane, false);
-                pack_dist(w, lane);
-            } else {
-                // dynamic codes (RFC 1951 3.2.7)
-                const uint32_t hlit = br.get(5) + 257, hdist = br.get(5) + 1, hclen = br.get(4) + 4;
-                if (hlit > 286 || hdist > 30) {
-                    st = STREAM_BAD;
-                    break;
-                }
-                for (int i = lane; i < 19; i += 32) w.lens[i] = 0;
-                __syncwarp();
-                for (uint32_t i = 0; i < hclen; ++i) {
-                    br.refill();
-                    const uint32_t v = br.get(3);
-                    if (lane == 0) w.lens[c_clen_order[i]] = (uint8_t)v;
-                }
-                __syncwarp();
-                if (!build_code(w.lens, 19, w.one, LB_LIT, w.la, w.hist, lane, true)) {
-                    st = STREAM_BAD;
-                    break;
-                }
-                const uint32_t total = hlit + hdist;
-                uint32_t n = 0;
-                while (n < total) {
-                    br.refill();
-                    if (br.overrun()) {
-                        st = STREAM_BAD;
-                        break;
-                    }
-                    const int sym = decode_sym(br, w.one, LB_LIT, w.la);
-                    if (sym < 0) {
-                        st = STREAM_BAD;
-                        break;
-                    }
-                    if (sym < 16) {
-                        if (lane == 0) w.lens[n] = (uint8_t)sym;
-                        ++n;
-                    } else {
-                        uint32_t rep, val = 0;
-                        if (sym == 16) {
-                            if (n == 0) {
-                                st = STREAM_BAD;
-                                break;
-                            }
-                            val = w.lens[n - 1];
-                            rep = 3 + br.get(2);
-                        } else if (sym == 17) {
-                            rep = 3 + br.get(3);
-                        } else {
-                            rep = 11 + br.get(7);
-                        }
-                        if (n + rep > total) {
-                            st = STREAM_BAD;
-                            break;
-                        }
-                        for (uint32_t j = (uint32_t)lane; j < rep; j += 32) w.lens[n + j] = (uint8_t)val;
-                        n += rep;
-                    }
-                    __syncwarp();
-                }
-                if (st != STREAM_OK) break;
-                __syncwarp();
-                if (w.lens[256] == 0 || !build_code(w.lens, (int)hlit, w.one, LB_LIT, w.la, w.hist, lane, false)) {
-                    st = STREAM_BAD;
-                    break;
-                }
-                pack_litlen(w, lane);
-                if (!build_code(w.lens + hlit, (int)hdist, w.one, LB_DIST, w.da, w.hist, lane, false)) {
-                    st = STREAM_BAD;
-                    break;
-                }
-                pack_dist(w, lane);
-            }
-            // the block's symbols: after a refill at least 56 bits are
-            // buffered, enough for a whole match (15 + 5 + 15 + 13 bits)
-            for (;;) {
-                if (os.op - os.fp >= IF_FLUSH) flush_chunk(w, os, lane);
-                if (br.nb < 56) {
-                    br.refill();
-                    if (br.overrun()) {
-                        st = STREAM_BAD;
-                        break;
-                    }
-                }
-                const uint32_t e = w.lit[(uint32_t)br.bb & ((1u << LB_LIT) - 1u)];
-                const uint32_t kind = (e >> 5) & 7u;
-                if (kind - 1u < 3u) {  // one to three literals
-                    if ((uint64_t)os.op + kind > os.cap) {
-                        st = STREAM_OVERFLOW;
-                        break;
-                    }
-                    if ((uint32_t)lane < kind) w.ring[(os.op + lane) & (IF_RING - 1)] = (uint8_t)(e >> (8 + 8 * lane));
-                    os.op += kind;
-                    br.drop(e & 31u);
-                    continue;
-                }
-                uint32_t L;
-                if (kind == K_LEN) {
-                    br.drop(e & 31u);
-                    L = ((e >> 8) & 511u) + br.get((e >> 17) & 7u);
-                } else if (kind == K_END) {
-                    br.drop(e & 31u);
-                    break;
-                } else if (kind == K_BAD) {
-                    st = STREAM_BAD;
-                    break;
-                } else {
-                    // a code longer than the index
-                    const int r = decode_slow(br.bb, w.la);
-                    if (r < 0) {
-                        st = STREAM_BAD;
-                        break;
-                    }
-                    br.drop((uint32_t)r >> 16);
-                    const uint32_t sym = (uint32_t)r & 0xffffu;
-                    if (sym < 256) {
-                        if (os.op >= os.cap) {
-                            st = STREAM_OVERFLOW;
-                            break;
-                        }
-                        if (lane == 0) w.ring[os.op & (IF_RING - 1)] = (uint8_t)sym;
-                        ++os.op;
-                        continue;
-                    }
-                    if (sym == 256) break;
-                    if (sym > 285) {
-                        st = STREAM_BAD;
-                        break;
-                    }
-                    L = c_len_base[sym - 257] + br.get(c_len_extra[sym - 257]);
-                }
-                const uint32_t de = w.dist[(uint32_t)br.bb & ((1u << LB_DIST) - 1u)];
-                const uint32_t dk = de >> 25;
-                uint32_t d;
-                if (dk == 1) {
-                    br.drop(de & 31u);
-                    d = ((de >> 9) & 0xffffu) + br.get((de >> 5) & 15u);
-                } else if (dk == 0) {
-                    const int r = decode_slow(br.bb, w.da);
-                    if (r < 0 || (r & 0xffff) >= 30) {
-                        st = STREAM_BAD;
-                        break;
-                    }
-                    br.drop((uint32_t)r >> 16);
-                    const uint32_t ds = (uint32_t)r & 0xffffu;
-                    d = c_dist_base[ds] + br.get(c_dist_extra[ds]);
-                } else {
-                    st = STREAM_BAD;
-                    break;
-                }
-                if (d > os.op - member0) {
-                    st = STREAM_BAD;
-                    break;
-                }
-                if ((uint64_t)os.op + L > os.cap) {
-                    st = STREAM_OVERFLOW;
-                    break;
-                }
-                copy_match(w, os, d, L, lane);
-            }
         }
-        if (st != STREAM_OK) break;
-        // trailer: CRC-32 (not checked here) and ISIZE = member size mod 2^32
-        br.align();
-        br.refill();
-        br.get(16);
-        br.get(16);
-        br.refill();
-        const uint32_t isize = br.get(16) | (br.get(16) << 16);
-        if (br.overrun() || isize != os.op - member0) {
-            st = STREAM_BAD;
-            break;
-        }
-        const uint64_t p = br.pos();
-        if (p > br.end) {
-            st = STREAM_BAD;
-            break;
-        }
-        if (p == br.end) break;
-        // another member follows (anything else fails its header check)
-        br.seek(p);
+        trailer = c.last != 0;
     }
-    __syncwarp();
-    if (st == STREAM_OK) {
-        const uint32_t rest = os.op - os.fp;
-        for (uint32_t i = (uint32_t)lane; i < rest; i += 32) os.o[os.fp + i] = w.ring[(os.fp + i) & (IF_RING - 1)];
-    }
-    if (lane == 0) {
-        s.out_len[f] = st == STREAM_OK ? os.op : 0;
+    if (t == 0) {
+        s.out_len[f] = st == STREAM_OK ? op : 0;
         s.status[f] = st;
     }
 }
@@ -844,7 +1011,8 @@ __global__ void __launch_bounds__(FC_THREADS) k_fasta_compact(stream_set s, uint
 
 void inflate_streams(stream_set const& s, cudaStream_t st) {
     if (!s.n) return;
-    k_inflate<<<(s.n + IF_WARPS - 1) / IF_WARPS, IF_WARPS * 32, 0, st>>>(s);
+    CDBG_CUDA(cudaFuncSetAttribute(k_inflate, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(cta_state)));
+    k_inflate<<<s.n, IF_THREADS, sizeof(cta_state), st>>>(s);
     CDBG_CHECK_LAUNCH();
 }
 

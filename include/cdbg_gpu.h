@@ -78,7 +78,7 @@ typedef struct cdbg_tuning {
                                   default: one group per batch) */
     uint32_t radix_bits;       /* radix sort digit width: 8 or 11 (default 8) */
     uint32_t gpu_inflate;      /* input files of cdbg_gpu_build_files and
-                                  cdbg_gpu_phase1 read by the device (one warp
+                                  cdbg_gpu_phase1 read by the device (one CTA
                                   inflates each gzip file, FASTA records are
                                   cut on the device): 0 (default) when the
                                   work spreads over many files, 1 whenever
@@ -182,7 +182,7 @@ int cdbg_gpu_dump_supers(cdbg_engine* e, const cdbg_seq_batch* b, uint32_t k, ui
 
 /* Test aid (no counterpart in the reference): the device gzip decoder of the
  * device reader (gpu_inflate) on n gzip streams in host memory, inflated on
- * the device in one launch, one warp per stream.  outs[i] (host, out_caps[i]
+ * the device in one launch, one CTA per stream.  outs[i] (host, out_caps[i]
  * bytes) receives stream i's bytes and out_lens[i] their count when
  * status[i] is 0; status 1 = more than out_caps[i] bytes, 2 = not a stream
  * the decoder accepts (the host reader's zlib then decides). */
