@@ -627,7 +627,7 @@ def _per_unit(w):
         "k_minimizers": None,  # two units, see algorithmic_bytes
         # one (k-mer, record) read per occurrence + one table entry per distinct k-mer
         "k_insert": None,
-        "k_multi_pairs": ("occ", 4 + 4),          # occurrence slot read + pair written
+        "k_number": ("occ", 4 + w + 8),           # occurrence slot + its k-mer's table slot
         "k_ext_mask": ("distinct", w + 4 + 1),    # key + bucket read, mask written
         "k_links": ("distinct", w + 1 + 8 + 8),   # key + mask + recorded neighbours read, two links written
         "k_chain_paths": ("distinct", 8 + 1 + 1 + 4),  # links + flags + mask read, fragment element written

@@ -12,8 +12,8 @@
 //           occurrence index, in (record, index) order) by atomicMin.
 //  nodes    distinct k-mers are numbered in first-insertion order -- the
 //           iteration order of the reference's insertion-ordered map, which is
-//           its seed and class order -- by marking each k-mer's first
-//           occurrence in a bitmap over the batch's occurrences and scanning it.
+//           its seed and class order -- by one scan over the batch's
+//           occurrences: an occurrence is its k-mer's first when the slot says so.
 //  resolve  a primary k-mer owned by one record has that record's color set;
 //           one owned by several records gets the union of their sets
 //           (bucket_walker.hpp:360-428), built once per run of k-mers with the
@@ -146,8 +146,7 @@ __device__ __forceinline__ u128 key_cas(u128* a, u128 cmp, u128 val) {
 // One table slot: everything the load stage aggregates for a k-mer in 16
 // bytes (32 for 128-bit k-mers), two slots per 32-byte sector.
 //   rank  first insertion: the batch's lowest occurrence index of the k-mer
-//         (occurrences are in (record, index) order); after numbering, the
-//         k-mer's node index
+//         (occurrences are in (record, index) order)
 //   om    bits 0-3: side bits, primary, M_MULTI; bits 4-31: the first owning
 //         record (relative to the batch) + 1, 0 when none
 template <typename K>
@@ -299,16 +298,17 @@ struct occ_info {
     bool owned;
 };
 
-// Record holding occurrence o of the current block.  Every record has at least
-// one k-mer in practice, so the block's OCC_BLOCK occurrences fall within
-// OCC_BLOCK + 1 records starting at the record of its first occurrence: one
-// global binary search per block, then a search in shared memory.  Empty
-// records (len < k) can push an occurrence past the window; it then falls
-// back to the global search.
+// Records of a tile of WORDS x 32 consecutive occurrences (a multiple of
+// OCC_BLOCK, starting on one): the records that start in the tile mark their
+// first occurrence in a bitmap, and an occurrence's record is the one of the
+// nearest mark at or before it, or the tile's first record (r0).  One read of
+// the tile's record prefix instead of a search per occurrence; records without
+// k-mers mark nothing.
 constexpr int OCC_BLOCK = 256;
-struct occ_window {
-    uint64_t occ[OCC_BLOCK + 2];
-    uint64_t r0;
+template <int WORDS>
+struct tile_records {
+    uint32_t bits[WORDS];
+    uint32_t at[WORDS * 32];  // record of each mark, from r0
 };
 // blk_rec[b] = the record holding occurrence O0 + b * OCC_BLOCK, the first
 // occurrence of block b of the occurrence kernels (thread per record; a
@@ -322,30 +322,34 @@ __global__ void k_block_records(uint64_t const* __restrict__ occ, uint64_t R0, u
         blk_rec[b] = (uint32_t)(R0 + i);
 }
 
-__device__ __forceinline__ void load_occ_window(occ_window& w, uint64_t const* occ, uint64_t R0, uint64_t nrec,
-                                                uint32_t const* __restrict__ blk_rec, uint64_t blk) {
-    if (threadIdx.x == 0) w.r0 = blk_rec[blk];
+// Whole block; blk = the tile's first occurrence block.
+template <int WORDS>
+__device__ __forceinline__ uint32_t load_tile_records(tile_records<WORDS>& w, uint64_t const* __restrict__ occ,
+                                                      uint64_t R0, uint64_t nrec, uint64_t O0, uint64_t nblk,
+                                                      uint32_t const* __restrict__ blk_rec, uint64_t blk) {
+    static_assert(WORDS * 32 % OCC_BLOCK == 0, "whole occurrence blocks");
+    const uint64_t nb = blk + WORDS * 32 / OCC_BLOCK;
+    const uint32_t r0 = blk_rec[blk];
+    const uint32_t r1 = nb < nblk ? blk_rec[nb] : (uint32_t)(R0 + nrec - 1);
+    const uint64_t o0 = O0 + blk * OCC_BLOCK;
+    for (uint32_t i = threadIdx.x; i < (uint32_t)WORDS; i += blockDim.x) w.bits[i] = 0;
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < OCC_BLOCK + 2; i += blockDim.x) {
-        const uint64_t r = w.r0 + i;
-        w.occ[i] = (r <= R0 + nrec) ? occ[r] : ~0ull;
-    }
-    __syncthreads();
-}
-__device__ __forceinline__ uint64_t window_record(occ_window const& w, uint64_t const* occ, uint64_t R0,
-                                                  uint64_t nrec, uint64_t o) {
-    if (o < w.occ[OCC_BLOCK + 1]) {
-        uint32_t lo = 0, hi = OCC_BLOCK + 2;
-        while (lo < hi) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (w.occ[mid] <= o)
-                lo = mid + 1;
-            else
-                hi = mid;
+    for (uint32_t r = r0 + 1 + threadIdx.x; r <= r1; r += blockDim.x) {
+        const uint64_t x = occ[r] - o0;
+        if (x < (uint64_t)WORDS * 32 && occ[r + 1] - o0 > x) {
+            atomicOr(&w.bits[x >> 5], 1u << (x & 31));
+            w.at[x] = r - r0;
         }
-        return w.r0 + lo - 1;
     }
-    return R0 + upper_bound_u64(occ + R0, nrec + 1, o) - 1;
+    __syncthreads();
+    return r0;
+}
+// Record of occurrence `bit` of the tile's word `i`.
+template <int WORDS>
+__device__ __forceinline__ uint32_t tile_record(tile_records<WORDS> const& w, uint32_t r0, int i, uint32_t bit) {
+    uint32_t x = w.bits[i] & (0xffffffffu >> (31 - bit));
+    while (x == 0 && i > 0) x = w.bits[--i];
+    return x ? r0 + w.at[i * 32 + 31 - __clz(x)] : r0;
 }
 
 template <typename K>
@@ -401,18 +405,19 @@ __global__ void k_init_tables(uint64_t T, slot_t<K>* slots) {
     slots[i] = e;
 }
 
-// Occurrences t0 .. t0 + nocc - 1 of the batch (one bucket group's).
+// Occurrences t0 .. t1 - 1 of the batch (one bucket group's), one per thread
+// and one OCC_BLOCK per block.
 template <typename K>
-__global__ void __launch_bounds__(256) k_insert(rec_view R, tables<K> T, uint64_t R0, uint64_t nrec,
-                                                uint64_t O0, uint64_t t0, uint64_t nocc, uint32_t k,
-                                                uint32_t const* __restrict__ blk_rec,
+__global__ void __launch_bounds__(OCC_BLOCK) k_insert(rec_view R, tables<K> T, uint64_t R0, uint64_t nrec,
+                                                uint64_t O0, uint64_t t0, uint64_t t1, uint32_t k,
+                                                uint64_t nblk, uint32_t const* __restrict__ blk_rec,
                                                 uint32_t* __restrict__ occ_slot, uint32_t* err) {
-    __shared__ occ_window win;
-    // the window of the occurrence block holding this block's first occurrence
-    load_occ_window(win, R.occ, R0, nrec, blk_rec, (t0 + (uint64_t)blockIdx.x * blockDim.x) / OCC_BLOCK);
-    const uint64_t t = t0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= t0 + nocc) return;
-    const uint64_t rec = window_record(win, R.occ, R0, nrec, O0 + t);
+    __shared__ tile_records<OCC_BLOCK / 32> win;
+    const uint64_t blk = t0 / OCC_BLOCK + blockIdx.x;
+    const uint32_t r0 = load_tile_records(win, R.occ, R0, nrec, O0, nblk, blk_rec, blk);
+    const uint64_t t = blk * OCC_BLOCK + threadIdx.x;
+    if (t < t0 || t >= t1) return;
+    const uint64_t rec = tile_record(win, r0, threadIdx.x >> 5, threadIdx.x & 31);
     const occ_info<K> oi = decode_occ_r<K>(R, rec, O0 + t, k);
     const uint32_t tb = R.bucket[oi.r] - T.b0;
     const uint32_t mo = oi.contrib | (oi.owned ? M_PRIMARY : 0u);
@@ -433,7 +438,7 @@ __global__ void __launch_bounds__(256) k_insert(rec_view R, tables<K> T, uint64_
         occ_slot[t] = NONE32;
         return;
     }
-    // slot of this occurrence, bit 31 = owned (read by k_multi_pairs)
+    // slot of this occurrence, bit 31 = owned (read by k_number)
     occ_slot[t] = (uint32_t)s | (oi.owned ? 0x80000000u : 0u);
     if (claimed) return;
     // rank and om as read while probing (never newer than the slot): the
@@ -464,54 +469,102 @@ __global__ void __launch_bounds__(256) k_insert(rec_view R, tables<K> T, uint64_
     }
 }
 
-// Bit q of `bits` <- first occurrence of each distinct k-mer.
-template <typename K>
-__global__ void k_firstbits(uint64_t T, slot_t<K> const* __restrict__ slots, uint32_t* __restrict__ bits) {
-    uint64_t s = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= T || slots[s].key == kmer_ops<K>::empty()) return;
-    const uint32_t q = slots[s].rank;
-    atomicOr(&bits[q >> 5], 1u << (q & 31));
+// Occurrence words: for the 32 occurrences 32 i .. 32 i + 31 of the batch, x =
+// which of them are the first of their k-mer, y = the node index of the first
+// such one (the number of first occurrences before the word).  A k-mer's slot
+// keeps its first occurrence q (`rank`), so its node index is node_of(fw, q).
+__device__ __forceinline__ uint32_t node_of(uint2 const* __restrict__ fw, uint32_t q) {
+    const uint2 w = __ldg(fw + (q >> 5));
+    return w.y + __popc(w.x & ((1u << (q & 31)) - 1u));
 }
 
+__device__ __forceinline__ void slot_read(slot_t<uint64_t> const* e, uint64_t& key, uint32_t& rank, uint32_t& om) {
+    const ulonglong2 v = __ldg(reinterpret_cast<ulonglong2 const*>(e));
+    key = v.x;
+    rank = (uint32_t)v.y;
+    om = (uint32_t)(v.y >> 32);
+}
+__device__ __forceinline__ void slot_read(slot_t<u128> const* e, u128& key, uint32_t& rank, uint32_t& om) {
+    const ulonglong2 v = __ldg(reinterpret_cast<ulonglong2 const*>(e));
+    const uint2 ro = __ldg(reinterpret_cast<uint2 const*>(&e->rank));
+    key = ((u128)v.y << 64) | (u128)v.x;
+    rank = ro.x;
+    om = ro.y;
+}
 
-// Number the distinct k-mers of one bucket group in first-insertion order,
-// scanning its occurrences t0 .. t0 + nocc - 1: occurrence t is the first of
-// its k-mer iff bit t of `bits` is set, and its node index is *nbase plus the
-// number of first occurrences before it in the group.  Tiles of MN_ROUNDS x
-// 256 occurrences take indices in launch order and find their offset by
-// decoupled look-back; the last tile stores *nbase + the group's count in
-// *nnext (the next group's base).  The slot's rank field becomes the node
-// index, and the node arrays are written in node order; the bucket is the
-// slot's table (tab_off ascends over the group's buckets).
-constexpr int MN_ROUNDS = 8;
+// Node numbering and multi-record pairs of one bucket group, in one pass over
+// its occurrences t0 .. t1 - 1 (one slot read each):
+//   - occurrence t is the first of its k-mer iff the slot's rank is t; its node
+//     index is base[0] plus the number of first occurrences before it in the
+//     group (insertion order), and it writes the k-mer's node arrays;
+//   - an owned occurrence of a multi-record k-mer (M_PRIMARY and M_MULTI)
+//     emits the pair (first occurrence of the k-mer, record), in occurrence
+//     order from pair base[1] on: records ascend within a k-mer, so a stable
+//     sort by k-mer alone orders the pairs.
+// Tiles of NB_ROUNDS x 256 occurrences from ta (t0's occurrence block) take
+// indices in launch order and find both offsets by one decoupled look-back
+// (nodes in the low 31 bits, pairs above: a batch has fewer than 2^31
+// occurrences); the last tile stores both totals in next[].
+// Bound: random 16-byte slot reads (L2 sectors), all of a thread's in flight
+// together.  A scan of the table for first occurrences, node numbering that
+// stored the index back into the slot, and a separate pair pass took 14.5 ms of
+// a 200-genome k = 31 build (3.8e8 occurrences), this pass and the pair
+// conversion 5.2; 9.8 and 3.8 ms of a 60-genome k = 63 build.
+constexpr int NB_ROUNDS = 8;
 template <typename K>
-__global__ void __launch_bounds__(256) k_make_nodes(uint64_t t0, uint64_t nocc, uint32_t const* __restrict__ occ_slot,
-                                                    uint32_t const* __restrict__ bits, tables<K> TB, uint32_t nb,
-                                                    uint64_t R0, unsigned long long const* nbase,
-                                                    unsigned long long* nnext, uint32_t* tile_counter,
-                                                    unsigned long long* status, K* __restrict__ n_key,
-                                                    uint8_t* __restrict__ n_meta, uint32_t* __restrict__ n_rec,
-                                                    uint32_t* __restrict__ n_bucket, uint32_t* err) {
+__global__ void __launch_bounds__(256) k_number(uint64_t ta, uint64_t t0, uint64_t t1,
+                                                uint32_t const* __restrict__ occ_slot, tables<K> TB,
+                                                uint64_t const* __restrict__ occ, uint32_t const* __restrict__ rbucket,
+                                                uint64_t R0, uint64_t nrec, uint64_t O0, uint64_t nblk,
+                                                uint32_t const* __restrict__ blk_rec,
+                                                unsigned long long const* base, unsigned long long* next,
+                                                uint32_t* tile_counter, unsigned long long* status,
+                                                uint2* __restrict__ fw, K* __restrict__ n_key,
+                                                uint8_t* __restrict__ n_meta, uint32_t* __restrict__ n_rec,
+                                                uint32_t* __restrict__ n_bucket, uint32_t* __restrict__ pnode,
+                                                uint32_t* __restrict__ prec, uint32_t* err) {
     constexpr int NW = 256 / 32;
-    static_assert(MN_ROUNDS * NW == 64, "warp 0 scans two counts per lane");
+    constexpr int WORDS = NB_ROUNDS * NW;  // 32-occurrence words of a tile
+    static_assert(WORDS == 64, "warp 0 scans two counts per lane");
     __shared__ uint64_t s_tile;
-    __shared__ uint32_t wcnt[MN_ROUNDS * NW];
-    __shared__ unsigned long long s_base;
+    __shared__ uint32_t wfirst[WORDS], wmulti[WORDS], wcnt[WORDS];
+    __shared__ uint64_t s_node, s_pair;
+    __shared__ tile_records<WORDS> win;
     if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1u);
     __syncthreads();
     const uint64_t tile = s_tile;
-    const uint64_t ntiles = (nocc + MN_ROUNDS * 256 - 1) / (MN_ROUNDS * 256);
+    const uint64_t ntiles = (t1 - ta + WORDS * 32 - 1) / (WORDS * 32);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t rank[MN_ROUNDS], first = 0;
+    const uint64_t tt = ta + tile * (WORDS * 32) + threadIdx.x;  // round rr: tt + 256 rr
+    uint32_t sl[NB_ROUNDS];
 #pragma unroll
-    for (int rr = 0; rr < MN_ROUNDS; ++rr) {
-        const uint64_t l = (tile * MN_ROUNDS + rr) * 256 + threadIdx.x;
-        const uint64_t t = t0 + l;
-        const bool f = l < nocc && ((bits[t >> 5] >> (t & 31)) & 1u);
-        const uint32_t bal = __ballot_sync(0xffffffffu, f);
-        rank[rr] = __popc(bal & lanemask_lt());
+    for (int rr = 0; rr < NB_ROUNDS; ++rr) {
+        const uint64_t t = tt + 256u * rr;
+        sl[rr] = t >= t0 && t < t1 ? __ldg(occ_slot + t) : NONE32;
+    }
+    K key[NB_ROUNDS];
+    uint32_t rank[NB_ROUNDS], om[NB_ROUNDS];
+#pragma unroll
+    for (int rr = 0; rr < NB_ROUNDS; ++rr) {
+        rank[rr] = NONE32;
+        om[rr] = 0;
+        if (sl[rr] != NONE32) slot_read(TB.slots + ((sl[rr] & 0x7fffffffu) - TB.off0), key[rr], rank[rr], om[rr]);
+    }
+    const uint32_t r0 = load_tile_records(win, occ, R0, nrec, O0, nblk, blk_rec,
+                                          (ta + tile * (WORDS * 32)) / OCC_BLOCK);
+    uint32_t first = 0, multi = 0;
+#pragma unroll
+    for (int rr = 0; rr < NB_ROUNDS; ++rr) {
+        const bool f = rank[rr] == (uint32_t)(tt + 256u * rr);
+        const bool m = (sl[rr] >> 31) && sl[rr] != NONE32 && (om[rr] & (M_PRIMARY | M_MULTI)) == (M_PRIMARY | M_MULTI);
+        const uint32_t bf = __ballot_sync(0xffffffffu, f), bm = __ballot_sync(0xffffffffu, m);
         if (f) first |= 1u << rr;
-        if (lane == 0) wcnt[rr * NW + warp] = __popc(bal);
+        if (m) multi |= 1u << rr;
+        if (lane == 0) {
+            wfirst[rr * NW + warp] = bf;
+            wmulti[rr * NW + warp] = bm;
+            wcnt[rr * NW + warp] = __popc(bf) | (__popc(bm) << 16);
+        }
     }
     __syncthreads();
     if (warp == 0) {
@@ -527,59 +580,55 @@ __global__ void __launch_bounds__(256) k_make_nodes(uint64_t t0, uint64_t nocc, 
         wcnt[2 * lane] = ex;
         wcnt[2 * lane + 1] = ex + c0;
         uint64_t excl = 0;
-        const bool ok = prim::lookback_exclusive(status, tile, tot, excl);
+        const uint64_t both = (uint64_t)(tot & 0xffffu) | ((uint64_t)(tot >> 16) << 31);
+        const bool ok = prim::lookback_exclusive(status, tile, both, excl);
         if (lane == 0) {
             if (!ok) set_error(err, ERR_CHAIN_LIMIT);
-            s_base = *nbase + excl;
-            if (tile == ntiles - 1) *nnext = *nbase + excl + tot;
+            s_node = base[0] + (excl & 0x7fffffffu);
+            s_pair = base[1] + (excl >> 31);
+            if (tile == ntiles - 1) {
+                next[0] = s_node + (tot & 0xffffu);
+                next[1] = s_pair + (tot >> 16);
+            }
         }
     }
     __syncthreads();
-    const unsigned long long base = s_base;
-    // every round's slot loads go out before any store, so a thread keeps
-    // its MN_ROUNDS random slot reads in flight at once
-    uint32_t sl[MN_ROUNDS];
-#pragma unroll
-    for (int rr = 0; rr < MN_ROUNDS; ++rr) {
-        const uint64_t t = t0 + (tile * MN_ROUNDS + rr) * 256 + threadIdx.x;
-        sl[rr] = ((first >> rr) & 1u) ? __ldg(occ_slot + t) & 0x7fffffffu : 0u;
+    const uint64_t node0 = s_node, pair0 = s_pair;
+    if (threadIdx.x < WORDS) {
+        const uint64_t w = ((ta + tile * (WORDS * 32)) >> 5) + threadIdx.x;
+        if (w * 32 < t1) fw[w] = make_uint2(wfirst[threadIdx.x], (uint32_t)node0 + (wcnt[threadIdx.x] & 0xffffu));
     }
-    K key[MN_ROUNDS];
-    uint32_t om[MN_ROUNDS];
+    const uint32_t lt = lanemask_lt();
 #pragma unroll
-    for (int rr = 0; rr < MN_ROUNDS; ++rr) {
-        if ((first >> rr) & 1u) {
-            slot_t<K> const* e = TB.slots + (sl[rr] - TB.off0);
-            key[rr] = e->key;
-            om[rr] = e->om;
+    for (int rr = 0; rr < NB_ROUNDS; ++rr) {
+        const uint32_t i = rr * NW + warp;
+        const bool f = (first >> rr) & 1u, m = (multi >> rr) & 1u;
+        if (!f && !m) continue;
+        const uint32_t r = tile_record(win, r0, (int)i, (uint32_t)lane);
+        if (f) {
+            const uint64_t n = node0 + (wcnt[i] & 0xffffu) + __popc(wfirst[i] & lt);
+            n_key[n] = key[rr];
+            n_meta[n] = (uint8_t)(om[rr] & 7u);
+            uint32_t rec = NONE32;
+            if (om[rr] & M_PRIMARY) rec = (om[rr] & M_MULTI) ? MULTI_TAG : (uint32_t)(R0 + (om[rr] >> 4) - 1);
+            n_rec[n] = rec;
+            n_bucket[n] = rbucket[r];
         }
-    }
-#pragma unroll
-    for (int rr = 0; rr < MN_ROUNDS; ++rr) {
-        const bool f = (first >> rr) & 1u;
-        const uint32_t tb = warp_bucket_of(TB.tab_off, nb + 1, sl[rr], f);
-        if (!f) continue;
-        const uint64_t n = base + wcnt[rr * NW + warp] + rank[rr];
-        TB.slots[sl[rr] - TB.off0].rank = (uint32_t)n;
-        n_key[n] = key[rr];
-        n_meta[n] = (uint8_t)(om[rr] & 7u);
-        uint32_t rec = NONE32;
-        if (om[rr] & M_PRIMARY) rec = (om[rr] & M_MULTI) ? MULTI_TAG : (uint32_t)(R0 + (om[rr] >> 4) - 1);
-        n_rec[n] = rec;
-        n_bucket[n] = TB.b0 + tb;
+        if (m) {
+            const uint64_t at = pair0 + (wcnt[i] >> 16) + __popc(wmulti[i] & lt);
+            pnode[at] = rank[rr];
+            prec[at] = r;
+        }
     }
 }
 
-// Occurrences t0 .. t0 + nocc - 1: the slot index becomes the k-mer's node
-// index (bit 31, owned, kept), so later stages need no table.
-template <typename K>
-__global__ void k_occ_nodes(uint64_t t0, uint64_t nocc, uint32_t* __restrict__ occ_slot,
-                            slot_t<K> const* __restrict__ slots, uint64_t off0) {
-    const uint64_t t = t0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= t0 + nocc) return;
-    const uint32_t v = occ_slot[t];
-    if (v == NONE32) return;
-    occ_slot[t] = slots[(v & 0x7fffffffu) - off0].rank | (v & 0x80000000u);
+// Pairs [*pb, *pe) of one bucket group: first occurrences -> node indices.
+__global__ void k_pair_nodes(unsigned long long const* pb, unsigned long long const* pe,
+                             uint2 const* __restrict__ fw, uint32_t* __restrict__ pnode) {
+    const uint64_t e = *pe;
+    for (uint64_t i = *pb + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < e;
+         i += (uint64_t)gridDim.x * blockDim.x)
+        pnode[i] = node_of(fw, pnode[i]);
 }
 
 // Block-wide reservation of `want` consecutive entries of *cnt per thread,
@@ -611,107 +660,6 @@ __device__ __forceinline__ unsigned long long block_reserve(uint32_t want, unsig
     const unsigned long long r = s_base + s_warp[warp] + incl - want;
     __syncthreads();  // the shared words may be reused by the next call
     return r;
-}
-
-// (node, record) of the owned occurrences of multi-record k-mers, from the
-// slot each occurrence recorded at insert time, written in occurrence order
-// (records ascend within a node, so a stable sort by node alone orders the
-// pairs by (node, record)).  A block handles MP_ROUNDS consecutive
-// occurrence blocks of OCC_BLOCK (one per round); blocks take tile indices in
-// launch order and find their output offset by decoupled look-back; the grid
-// is exactly one block per tile.
-constexpr int MP_ROUNDS = 8;
-__global__ void __launch_bounds__(OCC_BLOCK)
-    k_multi_pairs(uint64_t const* __restrict__ occ, uint64_t R0, uint64_t nrec, uint64_t O0, uint64_t nocc,
-                  uint32_t const* __restrict__ blk_rec,
-                  uint32_t const* __restrict__ occ_slot, uint32_t const* __restrict__ slot_rank, uint32_t rank_stride,
-                  uint32_t const* __restrict__ n_rec, uint32_t* __restrict__ tile_counter,
-                  unsigned long long* __restrict__ status, unsigned long long* __restrict__ cnt,
-                  uint32_t* __restrict__ pnode, uint32_t* __restrict__ prec, uint64_t cap, uint32_t* err) {
-    constexpr int NW = OCC_BLOCK / 32;
-    static_assert(MP_ROUNDS * NW == 64, "warp 0 scans two counts per lane");
-    __shared__ uint64_t s_tile;
-    __shared__ uint32_t wcnt[MP_ROUNDS * NW];
-    __shared__ unsigned long long s_base;
-    if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1u);
-    __syncthreads();
-    const uint64_t tile = s_tile;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const uint64_t nblk = (nocc + OCC_BLOCK - 1) / OCC_BLOCK;
-    uint32_t node[MP_ROUNDS], rec[MP_ROUNDS], rank[MP_ROUNDS], emit = 0;
-#pragma unroll
-    for (int rr = 0; rr < MP_ROUNDS; ++rr) {
-        const uint64_t b = tile * MP_ROUNDS + rr;  // occurrence block
-        const uint64_t t = b * OCC_BLOCK + threadIdx.x;
-        bool e = false;
-        node[rr] = 0;
-        rec[rr] = 0;
-        if (t < nocc) {
-            const uint32_t v = occ_slot[t];
-            if (v != NONE32 && (v & 0x80000000u)) {
-                uint32_t n;
-                bool multi;
-                if (slot_rank) {
-                    // the slot's node index and owner bits in one load: a
-                    // multi-record k-mer has both M_PRIMARY and M_MULTI (the
-                    // MULTI_TAG k_make_nodes writes to n_rec)
-                    const uint2 ro = __ldg(reinterpret_cast<uint2 const*>(
-                        slot_rank + (uint64_t)(v & 0x7fffffffu) * rank_stride));
-                    n = ro.x;
-                    multi = (ro.y & (M_PRIMARY | M_MULTI)) == (M_PRIMARY | M_MULTI);
-                } else {
-                    n = v & 0x7fffffffu;
-                    multi = n_rec[n] == MULTI_TAG;
-                }
-                if (multi) {
-                    // the record lies between this occurrence block's first record
-                    // and the next one's (a few dozen records): search only there
-                    const uint64_t rlo = blk_rec[b];
-                    const uint64_t rhi = (b + 1 < nblk) ? blk_rec[b + 1] : R0 + nrec - 1;
-                    node[rr] = n;
-                    rec[rr] = (uint32_t)(rlo + upper_bound_u64(occ + rlo, rhi - rlo + 1, O0 + t) - 1);
-                    e = true;
-                }
-            }
-        }
-        const uint32_t bal = __ballot_sync(0xffffffffu, e);
-        rank[rr] = __popc(bal & lanemask_lt());
-        if (e) emit |= 1u << rr;
-        if (lane == 0) wcnt[rr * NW + warp] = __popc(bal);
-    }
-    __syncthreads();
-    if (warp == 0) {
-        // exclusive prefix of the (round, warp) counts in position order
-        const uint32_t c0 = wcnt[2 * lane], c1 = wcnt[2 * lane + 1];
-        uint32_t x = c0 + c1;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x += y;
-        }
-        const uint32_t tot = __shfl_sync(0xffffffffu, x, 31);
-        const uint32_t ex = x - c0 - c1;
-        wcnt[2 * lane] = ex;
-        wcnt[2 * lane + 1] = ex + c0;
-        uint64_t excl = 0;
-        const bool ok = prim::lookback_exclusive(status, tile, tot, excl);
-        if (lane == 0) {
-            if (!ok) set_error(err, ERR_CHAIN_LIMIT);
-            if (tot) atomicAdd(cnt, (unsigned long long)tot);
-            s_base = excl;
-        }
-    }
-    __syncthreads();
-    const unsigned long long base = s_base;
-#pragma unroll
-    for (int rr = 0; rr < MP_ROUNDS; ++rr) {
-        if (!((emit >> rr) & 1u)) continue;
-        const unsigned long long at = base + wcnt[rr * NW + warp] + rank[rr];
-        if (at < cap) {
-            pnode[at] = node[rr];
-            prec[at] = rec[rr];
-        }
-    }
 }
 
 // First of each run of equal (node, record) pairs (a record may own a k-mer
@@ -1674,10 +1622,9 @@ __global__ void k_node_cid(uint64_t D, uint32_t const* __restrict__ n_rec, uint3
 }
 
 // ---- extension masks and clean links -------------------------------------
-// Node index of k-mer x, NONE32 when absent.  The tables are read-only once
-// the nodes are numbered, so the probes go through the read-only path, and a
-// 64-bit-key slot's probe load brings its rank (the node index) along.
-// Probes from slot s on: node index of x, or NONE32.
+// The tables are read-only once they are filled, so the probes go through the
+// read-only path, and a 64-bit-key slot's probe load brings its rank along.
+// Probes from slot s on: first occurrence of x, or NONE32.
 template <typename K>
 __device__ __forceinline__ uint32_t node_probe(slot_t<K> const* t, uint32_t cap, uint32_t s, K x) {
     const K EMPTY = kmer_ops<K>::empty();
@@ -1712,6 +1659,7 @@ template <typename K>
 __global__ void __launch_bounds__(256, 8) k_ext_mask(unsigned long long const* nb, unsigned long long const* ne,
                                                      tables<K> T, K const* __restrict__ n_key,
                                                      uint32_t const* __restrict__ n_bucket, uint32_t k,
+                                                     uint2 const* __restrict__ fw,
                                                      uint8_t* __restrict__ n_mask, uint32_t* __restrict__ link) {
     const uint64_t n = *nb + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= *ne) return;
@@ -1746,8 +1694,8 @@ __global__ void __launch_bounds__(256, 8) k_ext_mask(unsigned long long const* n
         }
     }
     n_mask[n] = (uint8_t)out;
-    link[2 * n] = __popc(out >> 4) == 1 ? left : NONE32;
-    link[2 * n + 1] = __popc(out & 0xfu) == 1 ? right : NONE32;
+    link[2 * n] = __popc(out >> 4) == 1 ? node_of(fw, left) : NONE32;
+    link[2 * n + 1] = __popc(out & 0xfu) == 1 ? node_of(fw, right) : NONE32;
 }
 
 __device__ __forceinline__ uint32_t fwd_nib(uint32_t m, bool rc) { return (rc ? (m >> 4) : m) & 0xfu; }
@@ -2280,7 +2228,10 @@ __global__ void k_add_offsets(uint64_t n, uint64_t const* __restrict__ src, uint
     if (i < n) dst[i] = src[i] + add;
 }
 __global__ void k_set_u64(uint64_t* p, uint64_t v) { *p = v; }
-__global__ void k_copy_u64(unsigned long long const* src, unsigned long long* dst) { *dst = *src; }
+__global__ void k_copy_u64x2(unsigned long long const* src, unsigned long long* dst) {
+    dst[0] = src[0];
+    dst[1] = src[1];
+}
 __global__ void k_used_flags(uint64_t n, uint32_t const* __restrict__ first, uint32_t* __restrict__ keep) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) keep[i] = first[i] != NONE32 ? 1u : 0u;
@@ -2417,14 +2368,12 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     CDBG_CUDA(cudaMemcpyAsync(d_toff, toff.data(), 8ull * (nb + 1), cudaMemcpyHostToDevice, st));
     CDBG_CUDA(cudaMemcpyAsync(d_tcap, tcap.data(), 8ull * nb, cudaMemcpyHostToDevice, st));
     slot_t<K>* slots = A.alloc<slot_t<K>>(Tmax + 1);
-    // record of each occurrence block's first occurrence (k_insert, k_multi_pairs)
+    // record of each occurrence block's first occurrence (k_insert, k_number)
     const uint64_t nblk = ceil_div(nocc, (uint64_t)OCC_BLOCK);
     uint32_t* blk_rec = A.alloc<uint32_t>(nblk + 1);
     k_block_records<<<grid(nrec, 256), 256, 0, st>>>(R.occ, R0, nrec, O0, nblk, blk_rec);
     CDBG_CHECK_LAUNCH();
-    const uint64_t nwb = ceil_div(nocc, 32);
-    uint32_t* bits = A.alloc<uint32_t>(nwb);
-    CDBG_CUDA(cudaMemsetAsync(bits, 0, 4 * nwb, st));
+    uint2* fw = A.alloc<uint2>(ceil_div(nocc, 32) + 1);  // first occurrences, by word (node_of)
     // node arrays, sized for the worst case (every occurrence a distinct
     // k-mer): the groups number their nodes on the device, without a host
     // round trip per group
@@ -2434,23 +2383,29 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     uint32_t* n_bucket = A.alloc<uint32_t>(nocc);
     uint8_t* n_mask = A.alloc<uint8_t>(nocc);
     uint32_t* link = A.alloc<uint32_t>(2 * nocc);
+    // (node, record) pairs of multi-record k-mers: at most one per occurrence
+    uint32_t* pnode = A.alloc<uint32_t>(nocc);
+    uint32_t* prec = A.alloc<uint32_t>(nocc);
     // look-back state of every group's numbering, zeroed once
+    constexpr uint64_t NB_TILE = (uint64_t)NB_ROUNDS * 256;
     std::vector<uint64_t> gtile(ng + 1, 0);
-    for (size_t g = 0; g < ng; ++g)
-        gtile[g + 1] = gtile[g] + ceil_div(bocc[b0 + gb[g + 1]] - bocc[b0 + gb[g]], (uint64_t)MN_ROUNDS * 256);
-    unsigned long long* mn_status = A.alloc<unsigned long long>(gtile[ng] + 1);
-    uint32_t* mn_counter = A.alloc<uint32_t>(ng + 1);
-    unsigned long long* ncnt = A.alloc<unsigned long long>(2);  // node bases, alternating by group
-    CDBG_CUDA(cudaMemsetAsync(mn_status, 0, 8 * (gtile[ng] + 1), st));
-    CDBG_CUDA(cudaMemsetAsync(mn_counter, 0, 4 * (ng + 1), st));
-    CDBG_CUDA(cudaMemsetAsync(ncnt, 0, 16, st));
+    for (size_t g = 0; g < ng; ++g) {
+        const uint64_t t0 = bocc[b0 + gb[g]] - O0, t1 = bocc[b0 + gb[g + 1]] - O0;
+        gtile[g + 1] = gtile[g] + (t1 > t0 ? ceil_div(t1 - t0 / OCC_BLOCK * OCC_BLOCK, NB_TILE) : 0);
+    }
+    // zeroed together: look-back status, the node and pair counts so far
+    // (alternating by group), tile counters
+    unsigned long long* nb_status = A.alloc<unsigned long long>(gtile[ng] + 4 + (ng + 1) / 2 + 1);
+    unsigned long long* ncnt = nb_status + gtile[ng];
+    uint32_t* nb_counter = reinterpret_cast<uint32_t*>(ncnt + 4);
+    CDBG_CUDA(cudaMemsetAsync(nb_status, 0, 8 * (gtile[ng] + 4 + (ng + 1) / 2 + 1), st));
     for (size_t g = 0; g < ng; ++g) {
         const uint32_t g0 = gb[g], g1 = gb[g + 1];
         const uint64_t t0 = bocc[b0 + g0] - O0, tn = bocc[b0 + g1] - bocc[b0 + g0];
         const uint64_t Tg = toff[g1] - toff[g0];
         if (tn == 0) {
-            // no occurrence: the next group starts from the same node count
-            k_copy_u64<<<1, 1, 0, st>>>(ncnt + (g & 1), ncnt + ((g + 1) & 1));
+            // no occurrence: the next group starts from the same counts
+            k_copy_u64x2<<<1, 1, 0, st>>>(ncnt + 2 * (g & 1), ncnt + 2 * ((g + 1) & 1));
             CDBG_CHECK_LAUNCH();
             continue;
         }
@@ -2467,26 +2422,29 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         CDBG_CHECK_LAUNCH();
         {
             CDBG_PROF("k_insert", st);
-            k_insert<K><<<grid(tn, 256), 256, 0, st>>>(R, TG, R0, nrec, O0, t0, tn, k, blk_rec, occ_slot, d_err);
+            k_insert<K><<<(unsigned)(ceil_div(t0 + tn, OCC_BLOCK) - t0 / OCC_BLOCK), OCC_BLOCK, 0, st>>>(
+                R, TG, R0, nrec, O0, t0, t0 + tn, k, nblk, blk_rec, occ_slot, d_err);
+        }
+        CDBG_CHECK_LAUNCH();
+        unsigned long long* nbase = ncnt + 2 * (g & 1);
+        unsigned long long* nnext = ncnt + 2 * ((g + 1) & 1);
+        {
+            CDBG_PROF("k_number", st);
+            k_number<K><<<(unsigned)(gtile[g + 1] - gtile[g]), 256, 0, st>>>(
+                t0 / OCC_BLOCK * OCC_BLOCK, t0, t0 + tn, occ_slot, TG, R.occ, R.bucket, R0, nrec, O0, nblk, blk_rec,
+                nbase, nnext, nb_counter + g, nb_status + gtile[g], fw, n_key, n_meta, n_rec, n_bucket, pnode, prec,
+                d_err);
         }
         CDBG_CHECK_LAUNCH();
         {
-            CDBG_PROF("k_firstbits", st);
-            k_firstbits<K><<<grid(Tg, 256), 256, 0, st>>>(Tg, slots, bits);
-        }
-        CDBG_CHECK_LAUNCH();
-        unsigned long long* nbase = ncnt + (g & 1);
-        unsigned long long* nnext = ncnt + ((g + 1) & 1);
-        {
-            CDBG_PROF("k_make_nodes", st);
-            k_make_nodes<K><<<(unsigned)(gtile[g + 1] - gtile[g]), 256, 0, st>>>(
-                t0, tn, occ_slot, bits, TG, g1 - g0, R0, nbase, nnext, mn_counter + g, mn_status + gtile[g],
-                n_key, n_meta, n_rec, n_bucket, d_err);
+            CDBG_PROF("k_pair_nodes", st);
+            k_pair_nodes<<<(unsigned)std::min<uint64_t>(grid(tn, 256), 148 * 16), 256, 0, st>>>(nbase + 1, nnext + 1,
+                                                                                               fw, pnode);
         }
         CDBG_CHECK_LAUNCH();
         {
             CDBG_PROF("k_ext_mask", st);
-            k_ext_mask<K><<<grid(tn, 256), 256, 0, st>>>(nbase, nnext, TG, n_key, n_bucket, k, n_mask, link);
+            k_ext_mask<K><<<grid(tn, 256), 256, 0, st>>>(nbase, nnext, TG, n_key, n_bucket, k, fw, n_mask, link);
         }
         CDBG_CHECK_LAUNCH();
         {
@@ -2494,43 +2452,13 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
             k_links<K><<<grid(tn, 256), 256, 0, st>>>(nbase, nnext, TG, n_key, n_bucket, n_mask, k, link);
         }
         CDBG_CHECK_LAUNCH();
-        if (ng > 1) {
-            // the next group reuses this group's table memory: occurrences
-            // keep their node index instead of their slot
-            {
-                CDBG_PROF("k_occ_nodes", st);
-                k_occ_nodes<K><<<grid(tn, 256), 256, 0, st>>>(t0, tn, occ_slot, slots, toff[g0]);
-            }
-            CDBG_CHECK_LAUNCH();
-        }
     }
-    const uint64_t D = read_dev(ncnt + (ng & 1), st);
+    uint64_t counts[2];  // nodes, pairs
+    read_small(counts, ncnt + 2 * (ng & 1), 16, st);
+    const uint64_t D = counts[0], npairs = counts[1];
     if (D >= (1ull << 31)) throw std::runtime_error("too many distinct k-mers in one bucket batch");
     check_device_error_word(d_err, st, "k-mer table insert");
-    // ---- multi-record k-mers: (node, record) pairs in one pass, at most one
-    // per occurrence
-    unsigned long long* cnt = A.alloc<unsigned long long>(1);
-    uint32_t* tile_counter = A.alloc<uint32_t>(1);
-    const uint64_t mp_tiles = ceil_div(nblk, (uint64_t)MP_ROUNDS);
-    unsigned long long* status = A.alloc<unsigned long long>(mp_tiles);
-    uint32_t* pnode = A.alloc<uint32_t>(nocc);
-    uint32_t* prec = A.alloc<uint32_t>(nocc);
-    CDBG_CUDA(cudaMemsetAsync(cnt, 0, 8, st));
-    CDBG_CUDA(cudaMemsetAsync(tile_counter, 0, 4, st));
-    CDBG_CUDA(cudaMemsetAsync(status, 0, 8 * mp_tiles, st));
-    {
-        CDBG_PROF("k_multi_pairs", st);
-        // one group: the table is still whole, and an occurrence's slot holds
-        // its node index (rank field); several: occ_slot holds node indices
-        uint32_t const* rankp = ng == 1 ? reinterpret_cast<uint32_t const*>(
-                                              reinterpret_cast<char const*>(slots) + offsetof(slot_t<K>, rank))
-                                        : nullptr;
-        k_multi_pairs<<<(unsigned)mp_tiles, OCC_BLOCK, 0, st>>>(R.occ, R0, nrec, O0, nocc, blk_rec, occ_slot,
-                                                            rankp, (uint32_t)(sizeof(slot_t<K>) / 4), n_rec,
-                                                            tile_counter, status, cnt, pnode, prec, nocc, d_err);
-    }
-    CDBG_CHECK_LAUNCH();
-    const uint64_t npairs = read_dev(cnt, st);
+    // ---- multi-record k-mers, from their (node, record) pairs
     uint64_t M = 0;
     uint32_t* mnode = nullptr;
     uint64_t* moff = nullptr;

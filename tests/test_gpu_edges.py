@@ -1,0 +1,64 @@
+"""GPU: builds at the sizes where a kernel's tiling can go wrong, against the
+CPU oracle: k-mer occurrences on the edges of the occurrence blocks (256) and
+tiles (2048), records spanning many tiles (homopolymers, short tandem repeats),
+tables processed in bucket groups.  Fragments and color sets are exact."""
+import os
+
+import numpy as np
+import pytest
+
+from cdbg_gpu import native
+
+pytestmark = pytest.mark.gpu
+
+
+def _dna(rng, n):
+    return rng.choice(np.frombuffer(b"ACGT", dtype=np.uint8), size=n).tobytes()
+
+
+def _check(oracle, engine, tmp_path, genomes, k, B):
+    """genomes: one list of sequences per color."""
+    files = []
+    for g, seqs in enumerate(genomes):
+        p = os.path.join(str(tmp_path), "g%d.fa" % g)
+        with open(p, "wb") as f:
+            f.write(b"".join(b">s%d\n%s\n" % (i, s) for i, s in enumerate(seqs)))
+        files.append(p)
+    lst = os.path.join(str(tmp_path), "files.txt")
+    with open(lst, "w") as f:
+        f.write("".join(p + "\n" for p in files))
+    bd, od = os.path.join(str(tmp_path), "b"), os.path.join(str(tmp_path), "o")
+    os.makedirs(bd)
+    oracle.phase1(lst, k, B, bucket_dir=bd)
+    oracle.phase2(bd, B, k, len(genomes), od)
+    flat = [(s, g) for g, seqs in enumerate(genomes) for s in seqs]
+    r = engine.build(native.host_batch([s for s, _ in flat], [g for _, g in flat]), k, B, len(genomes))
+    frag, cs = os.path.join(str(tmp_path), "f.bin"), os.path.join(str(tmp_path), "c.sets")
+    want = open(os.path.join(od, "frag_unitigs.bin"), "rb").read()
+    assert native.result_frag_bytes(r) == want
+    engine.build_files(files, k, B, frag, cs)
+    assert open(frag, "rb").read() == want
+    assert open(cs, "rb").read() == open(os.path.join(od, "out.color_sets"), "rb").read()
+
+
+@pytest.mark.parametrize("k", [31, 63])
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 2047, 2048, 2049, 6143])
+def test_occurrence_tile_edges(oracle, engine, tmp_path, k, n):
+    rng = np.random.default_rng(n + k)
+    s = _dna(rng, n + k - 1)
+    t = bytearray(s)
+    t[len(t) // 2] = ord("A") if t[len(t) // 2] != ord("A") else ord("C")
+    _check(oracle, engine, tmp_path, [[s], [bytes(t), s[: k + 3]]], k, 1)
+
+
+@pytest.mark.parametrize("group_mb", [0, 1])
+@pytest.mark.parametrize("k", [31, 63])
+def test_long_records_and_groups(oracle, tmp_path, k, group_mb):
+    rng = np.random.default_rng(7 + k)
+    a, b = _dna(rng, 30_000), _dna(rng, 20_011)
+    g0 = [a, b"A" * 5000, b[:300] + b"AC" * 2600 + b[300:]]
+    g1 = [a[:9000] + b"T" * 4097 + a[9000:], b]
+    g2 = [b"G" * (k + 255), a[100:131 + k], (b[:211] * 30)[:5200]]
+    with native.Engine(0) as e:
+        e.set_tuning(table_group_mb=group_mb)
+        _check(oracle, e, tmp_path, [g0, g1, g2], k, 37)
