@@ -52,6 +52,8 @@ struct kmer_ops<uint64_t> {
     static __host__ __device__ __forceinline__ K empty() { return ~K(0); }
     static __host__ __device__ __forceinline__ uint64_t hash(K x) { return mix64(x); }
     static __host__ __device__ __forceinline__ uint32_t low2(K x) { return (uint32_t)(x & 3); }
+    // lane `src`'s x (the whole warp calls it)
+    static __device__ __forceinline__ K shfl(K x, int src) { return __shfl_sync(0xffffffffu, x, src); }
     // k-mer whose bases are the k bases of `x` read LSB-first (base i at bits
     // 2i): forward value and reverse-complement value.
     static __device__ __forceinline__ void from_lsb(uint64_t x, uint32_t k, K& fwd, K& rc) {
@@ -87,6 +89,11 @@ struct kmer_ops<u128> {
         return mix64(lo) ^ (mix64(hi + 0x9e3779b97f4a7c15ULL) << 1);
     }
     static __host__ __device__ __forceinline__ uint32_t low2(K x) { return (uint32_t)(x & 3); }
+    static __device__ __forceinline__ K shfl(K x, int src) {
+        const uint64_t lo = __shfl_sync(0xffffffffu, (uint64_t)x, src);
+        const uint64_t hi = __shfl_sync(0xffffffffu, (uint64_t)(x >> 64), src);
+        return ((K)hi << 64) | (K)lo;
+    }
     static __device__ __forceinline__ void load(uint64_t const* __restrict__ words, uint64_t pos,
                                                 uint32_t k, K& fwd, K& rc) {
         const uint64_t a = stream_bits64(words, pos);

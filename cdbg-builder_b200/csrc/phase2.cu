@@ -42,6 +42,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdlib>
+#include <cstring>
 #include <vector>
 
 #include "device_kmer.cuh"
@@ -168,99 +169,114 @@ static_assert(sizeof(slot_t<uint64_t>) == 16, "slot layout");
 static_assert(sizeof(slot_t<u128>) == 32, "slot layout");
 constexpr uint64_t MAX_BATCH_RECORDS = (1ull << 28) - 2;  // owner field of `om`
 
-// First slot of key x in a table of `cap` slots (cap < 2^32): the key folded
-// to 64 bits, an odd-constant multiply, and its top 32 bits scaled to the
-// capacity.  Table positions decide no output (nodes are numbered by first
-// occurrence, not by slot), only probe lengths.
-__device__ __forceinline__ uint32_t slot_of(uint64_t x, uint32_t cap) {
-    const uint64_t h = (x ^ (x >> 31)) * 0x9e3779b97f4a7c15ULL;
-    return (uint32_t)(((h >> 32) * (uint64_t)cap) >> 32);
+// Probing is linear.  64-bit-key slots go by pairs of neighbours (a sector): from
+// pair slot_home(x, cap / 2) on, both slots read by one 32-byte load and taken in
+// order, until x or an empty slot.  A probe is a dependent read, and a warp waits
+// for its longest: at the load of a 200-genome build (1/3) single slots take 1.24
+// steps found / 1.58 absent and 3.6 for the slowest of 32, pairs 1.04 / 1.1 and 2
+// (k_insert of that build 10.0 -> 9.6 ms).  128-bit-key slots fill a sector each
+// and go one by one from slot_home(x, cap): pairs read two sectors where one
+// mostly decides (neighbour lookups 86 -> 100 us per million k-mers).
+// The hash: the key folded to 64 bits, an odd-constant multiply, and its top 32
+// bits scaled to the number of homes (< 2^32).  Table positions decide no output
+// (nodes are numbered by first occurrence, not by slot), only probe lengths.
+__device__ __forceinline__ uint32_t slot_hash(uint64_t x) {
+    return (uint32_t)(((x ^ (x >> 31)) * 0x9e3779b97f4a7c15ULL) >> 32);
 }
-__device__ __forceinline__ uint32_t slot_of(u128 x, uint32_t cap) {
-    const uint64_t f = (uint64_t)x ^ ((uint64_t)(x >> 64) * 0xc2b2ae3d27d4eb4fULL);
-    return slot_of(f, cap);
+__device__ __forceinline__ uint32_t slot_hash(u128 x) {
+    return slot_hash((uint64_t)((uint64_t)x ^ ((uint64_t)(x >> 64) * 0xc2b2ae3d27d4eb4fULL)));
 }
-
-// A 64-bit-key slot's key and (rank | om << 32) in one 16-byte load that
-// bypasses L1.
-__device__ __forceinline__ void slot_load(slot_t<uint64_t> const* e, uint64_t& key, uint64_t& ro) {
-    asm volatile("ld.volatile.global.v2.u64 {%0, %1}, [%2];" : "=l"(key), "=l"(ro) : "l"(e) : "memory");
-}
-
-// Insert-or-find; returns the slot (absolute) or NONE64 when the region is
-// full.  `ro` receives the slot's (rank | om << 32) as read while probing: a
-// value the slot held, so possibly older than the current one (rank only
-// falls and om only gains bits, which the caller's updates rely on).
-// `slots` holds the slots from absolute index off0 on (the tables of the
-// bucket group being processed); returned indices are absolute.
 template <typename K>
-__device__ __forceinline__ uint64_t table_upsert(slot_t<K>* slots, uint64_t off0, uint64_t off, uint64_t cap, K x,
-                                                 uint64_t& ro) {
-    const K EMPTY = kmer_ops<K>::empty();
-    const uint32_t cap32 = (uint32_t)cap;
-    uint32_t s = slot_of(x, cap32);
-    for (uint32_t i = 0; i < cap32; ++i) {
-        slot_t<K>* e = &slots[off + s - off0];
-        if constexpr (sizeof(K) == 8) {
-            uint64_t cur, v;
-            slot_load(e, cur, v);
-            if (cur == x) {
-                ro = v;
-                return off + s;
-            }
-            if (cur == EMPTY) {
-                const K old = (K)atomicCAS((unsigned long long*)&e->key, (unsigned long long)EMPTY,
-                                           (unsigned long long)x);
-                if (old == EMPTY || old == x) {
-                    ro = v;
-                    return off + s;
-                }
-            }
-        } else {
-            const K old = key_cas(&e->key, EMPTY, x);  // atomic 128-bit read-or-claim
-            if (old == EMPTY || old == x) {
-                ro = *(volatile uint64_t const*)&e->rank;
-                return off + s;
-            }
-        }
-        s = s + 1 == cap32 ? 0u : s + 1;
-    }
-    return ~0ull;
+__device__ __forceinline__ uint32_t slot_home(K x, uint32_t homes) {
+    return __umulhi(slot_hash(x), homes);
 }
 
-// 64-bit-key tables: insert-or-find like table_upsert, but an empty slot is
-// claimed together with the payload a new k-mer gets -- its rank and om --
-// in one 128-bit compare-and-swap of the whole slot (key, rank, om), so the
-// occurrence that creates a k-mer needs no further atomics.  `claimed` tells
-// whether this call wrote the payload; otherwise `ro` is the slot's (rank |
-// om << 32) as read (the caller's updates as in table_upsert).
+// Keys and (rank | om << 32) of a pair of 64-bit-key slots in one 32-byte load
+// past L1.
+__device__ __forceinline__ void pair_load(slot_t<uint64_t> const* e, uint64_t& k0, uint64_t& v0, uint64_t& k1,
+                                          uint64_t& v1) {
+    asm volatile("ld.relaxed.gpu.global.v4.u64 {%0, %1, %2, %3}, [%4];"
+                 : "=l"(k0), "=l"(v0), "=l"(k1), "=l"(v1)
+                 : "l"(e)
+                 : "memory");
+}
+// A 128-bit key, whole.
+__device__ __forceinline__ u128 key_load(u128 const* e) {
+    uint64_t lo, hi;
+    asm volatile("{\n\t.reg .b128 d;\n\tld.relaxed.gpu.global.b128 d, [%2];\n\tmov.b128 {%0, %1}, d;\n\t}"
+                 : "=l"(lo), "=l"(hi)
+                 : "l"(e)
+                 : "memory");
+    return ((u128)hi << 64) | (u128)lo;
+}
+
+// Insert-or-find of x by the occurrence whose payload is `payload` (rank | om <<
+// 32, what the slot of a new k-mer gets); returns the slot (absolute) or ~0 when
+// the region is full.  `claimed` tells whether this call stored the payload;
+// otherwise `ro` receives the slot's (rank | om << 32) as read while probing: a
+// value the slot held, so possibly older than the current one (rank only falls
+// and om only gains bits, which the caller's updates rely on).  `slots` holds
+// the slots from absolute index off0 on (the tables of the bucket group being
+// processed); returned indices are absolute.
+// A 64-bit key is claimed together with its payload in one 128-bit
+// compare-and-swap of the whole slot.
 __device__ __forceinline__ uint64_t table_claim(slot_t<uint64_t>* slots, uint64_t off0, uint64_t off, uint64_t cap,
                                                 uint64_t x, uint64_t payload, uint64_t& ro, bool& claimed) {
     const uint64_t EMPTY = kmer_ops<uint64_t>::empty();
+    const uint32_t pairs = (uint32_t)(cap / 2);
+    uint32_t p = slot_home(x, pairs);
+    claimed = false;
+    for (uint32_t i = 0; i < pairs; ++i) {
+        slot_t<uint64_t>* e = &slots[off + 2 * (uint64_t)p - off0];
+        uint64_t key[2], v[2];
+        pair_load(e, key[0], v[0], key[1], v[1]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            if (key[j] == EMPTY) {
+                const u128 old = key_cas(reinterpret_cast<u128*>(e + j), ((u128)v[j] << 64) | (u128)EMPTY,
+                                         ((u128)payload << 64) | (u128)x);
+                key[j] = (uint64_t)old;
+                if (key[j] == EMPTY && (uint64_t)(old >> 64) == v[j]) {
+                    claimed = true;
+                    return off + 2 * (uint64_t)p + j;
+                }
+                v[j] = (uint64_t)(old >> 64);
+            }
+            if (key[j] == x) {
+                ro = v[j];
+                return off + 2 * (uint64_t)p + j;
+            }
+        }
+        p = p + 1 == pairs ? 0u : p + 1;
+    }
+    return ~0ull;
+}
+// A 128-bit key is claimed first and its payload stored by a second
+// compare-and-swap of (rank, om), which fails only against another occurrence
+// of the same k-mer.
+__device__ __forceinline__ uint64_t table_claim(slot_t<u128>* slots, uint64_t off0, uint64_t off, uint64_t cap,
+                                                u128 x, uint64_t payload, uint64_t& ro, bool& claimed) {
+    const u128 EMPTY = kmer_ops<u128>::empty();
     const uint32_t cap32 = (uint32_t)cap;
-    uint32_t s = slot_of(x, cap32);
+    uint32_t p = slot_home(x, cap32);
     claimed = false;
     for (uint32_t i = 0; i < cap32; ++i) {
-        slot_t<uint64_t>* e = &slots[off + s - off0];
-        uint64_t cur, v;
-        slot_load(e, cur, v);
-        if (cur == x) {
-            ro = v;
-            return off + s;
-        }
-        if (cur == EMPTY) {
-            const u128 old = key_cas(reinterpret_cast<u128*>(e), ((u128)v << 64) | (u128)EMPTY,
-                                     ((u128)payload << 64) | (u128)x);
-            if ((uint64_t)old == EMPTY && (uint64_t)(old >> 64) == v) {
-                claimed = true;
-                return off + s;
-            }
-            if ((uint64_t)old == x) {
-                ro = (uint64_t)(old >> 64);
-                return off + s;
+        slot_t<u128>* e = &slots[off + p - off0];
+        u128 key = key_load(&e->key);
+        if (key == EMPTY) {
+            key = key_cas(&e->key, EMPTY, x);
+            if (key == EMPTY) {
+                const unsigned long long was = (unsigned long long)NONE32;
+                ro = atomicCAS(reinterpret_cast<unsigned long long*>(&e->rank), was, payload);
+                claimed = ro == was;
+                return off + p;
             }
         }
-        s = s + 1 == cap32 ? 0u : s + 1;
+        if (key == x) {
+            ro = *(volatile uint64_t const*)&e->rank;
+            return off + p;
+        }
+        p = p + 1 == cap32 ? 0u : p + 1;
     }
     return ~0ull;
 }
@@ -408,7 +424,7 @@ __global__ void k_init_tables(uint64_t T, slot_t<K>* slots) {
 // Occurrences t0 .. t1 - 1 of the batch (one bucket group's), one per thread
 // and one OCC_BLOCK per block.
 template <typename K>
-__global__ void __launch_bounds__(OCC_BLOCK) k_insert(rec_view R, tables<K> T, uint64_t R0, uint64_t nrec,
+__global__ void __launch_bounds__(OCC_BLOCK, 8) k_insert(rec_view R, tables<K> T, uint64_t R0, uint64_t nrec,
                                                 uint64_t O0, uint64_t t0, uint64_t t1, uint32_t k,
                                                 uint64_t nblk, uint32_t const* __restrict__ blk_rec,
                                                 uint32_t* __restrict__ occ_slot, uint32_t* err) {
@@ -424,15 +440,10 @@ __global__ void __launch_bounds__(OCC_BLOCK) k_insert(rec_view R, tables<K> T, u
     const uint32_t own = (uint32_t)(oi.r - R0 + 1) << 4;
     uint64_t ro = 0;
     bool claimed = false;
-    uint64_t s;
-    if constexpr (sizeof(K) == 8) {
-        // a new k-mer's slot: rank t, and om as the updates below would leave it
-        const uint32_t om0 = oi.owned ? (own | mo) : mo;
-        s = table_claim(T.slots, T.off0, T.tab_off[tb], T.tab_cap[tb], oi.can,
-                        (uint64_t)(uint32_t)t | ((uint64_t)om0 << 32), ro, claimed);
-    } else {
-        s = table_upsert<K>(T.slots, T.off0, T.tab_off[tb], T.tab_cap[tb], oi.can, ro);
-    }
+    // a new k-mer's slot: rank t, and om as the updates below would leave it
+    const uint32_t om0 = oi.owned ? (own | mo) : mo;
+    const uint64_t s = table_claim(T.slots, T.off0, T.tab_off[tb], T.tab_cap[tb], oi.can,
+                                   (uint64_t)(uint32_t)t | ((uint64_t)om0 << 32), ro, claimed);
     if (s == ~0ull) {
         set_error(err, ERR_TABLE_FULL);
         occ_slot[t] = NONE32;
@@ -514,15 +525,14 @@ constexpr int NB_ROUNDS = 8;
 template <typename K>
 __global__ void __launch_bounds__(256) k_number(uint64_t ta, uint64_t t0, uint64_t t1,
                                                 uint32_t const* __restrict__ occ_slot, tables<K> TB,
-                                                uint64_t const* __restrict__ occ, uint32_t const* __restrict__ rbucket,
-                                                uint64_t R0, uint64_t nrec, uint64_t O0, uint64_t nblk,
-                                                uint32_t const* __restrict__ blk_rec,
+                                                uint64_t const* __restrict__ occ, uint64_t R0, uint64_t nrec,
+                                                uint64_t O0, uint64_t nblk, uint32_t const* __restrict__ blk_rec,
                                                 unsigned long long const* base, unsigned long long* next,
                                                 uint32_t* tile_counter, unsigned long long* status,
                                                 uint2* __restrict__ fw, K* __restrict__ n_key,
                                                 uint8_t* __restrict__ n_meta, uint32_t* __restrict__ n_rec,
-                                                uint32_t* __restrict__ n_bucket, uint32_t* __restrict__ pnode,
-                                                uint32_t* __restrict__ prec, uint32_t* err) {
+                                                uint32_t* __restrict__ pnode, uint32_t* __restrict__ prec,
+                                                uint32_t* err) {
     constexpr int NW = 256 / 32;
     constexpr int WORDS = NB_ROUNDS * NW;  // 32-occurrence words of a tile
     static_assert(WORDS == 64, "warp 0 scans two counts per lane");
@@ -603,8 +613,6 @@ __global__ void __launch_bounds__(256) k_number(uint64_t ta, uint64_t t0, uint64
     for (int rr = 0; rr < NB_ROUNDS; ++rr) {
         const uint32_t i = rr * NW + warp;
         const bool f = (first >> rr) & 1u, m = (multi >> rr) & 1u;
-        if (!f && !m) continue;
-        const uint32_t r = tile_record(win, r0, (int)i, (uint32_t)lane);
         if (f) {
             const uint64_t n = node0 + (wcnt[i] & 0xffffu) + __popc(wfirst[i] & lt);
             n_key[n] = key[rr];
@@ -612,12 +620,11 @@ __global__ void __launch_bounds__(256) k_number(uint64_t ta, uint64_t t0, uint64
             uint32_t rec = NONE32;
             if (om[rr] & M_PRIMARY) rec = (om[rr] & M_MULTI) ? MULTI_TAG : (uint32_t)(R0 + (om[rr] >> 4) - 1);
             n_rec[n] = rec;
-            n_bucket[n] = rbucket[r];
         }
         if (m) {
             const uint64_t at = pair0 + (wcnt[i] >> 16) + __popc(wmulti[i] & lt);
             pnode[at] = rank[rr];
-            prec[at] = r;
+            prec[at] = tile_record(win, r0, (int)i, (uint32_t)lane);
         }
     }
 }
@@ -1623,79 +1630,267 @@ __global__ void k_node_cid(uint64_t D, uint32_t const* __restrict__ n_rec, uint3
 
 // ---- extension masks and clean links -------------------------------------
 // The tables are read-only once they are filled, so the probes go through the
-// read-only path, and a 64-bit-key slot's probe load brings its rank along.
-// Probes from slot s on: first occurrence of x, or NONE32.
-template <typename K>
-__device__ __forceinline__ uint32_t node_probe(slot_t<K> const* t, uint32_t cap, uint32_t s, K x) {
-    const K EMPTY = kmer_ops<K>::empty();
+// read-only path.  First occurrence of x, or NONE32 when absent.
+__device__ __forceinline__ uint32_t node_probe(slot_t<uint64_t> const* t, uint32_t cap, uint64_t x) {
+    const uint64_t EMPTY = kmer_ops<uint64_t>::empty();
+    const uint32_t pairs = cap / 2;
+    uint32_t p = slot_home(x, pairs);
+    for (uint32_t i = 0; i < pairs; ++i) {
+        uint64_t k0, v0, k1, v1;
+        asm volatile("ld.global.nc.v4.u64 {%0, %1, %2, %3}, [%4];"
+                     : "=l"(k0), "=l"(v0), "=l"(k1), "=l"(v1)
+                     : "l"(t + 2 * (uint64_t)p));
+        if (k0 == x) return (uint32_t)v0;
+        if (k1 == x) return (uint32_t)v1;
+        if (k0 == EMPTY || k1 == EMPTY) return NONE32;
+        p = p + 1 == pairs ? 0u : p + 1;
+    }
+    return NONE32;
+}
+__device__ __forceinline__ uint32_t node_probe(slot_t<u128> const* t, uint32_t cap, u128 x) {
+    const u128 EMPTY = kmer_ops<u128>::empty();
+    uint32_t p = slot_home(x, cap);
     for (uint32_t i = 0; i < cap; ++i) {
-        slot_t<K> const* e = &t[s];
-        if constexpr (sizeof(K) == 8) {
-            const ulonglong2 v = __ldg(reinterpret_cast<ulonglong2 const*>(e));
-            if (v.x == x) return (uint32_t)v.y;
-            if (v.x == EMPTY) return NONE32;
-        } else {
-            const ulonglong2 kv = __ldg(reinterpret_cast<ulonglong2 const*>(e));
-            const K cur = ((u128)kv.y << 64) | (u128)kv.x;
-            if (cur == x) return __ldg(&e->rank);
-            if (cur == EMPTY) return NONE32;
-        }
-        s = s + 1 == cap ? 0u : s + 1;
+        slot_t<u128> const* e = t + p;
+        const ulonglong2 v = __ldg(reinterpret_cast<ulonglong2 const*>(e));
+        const u128 key = ((u128)v.y << 64) | (u128)v.x;
+        if (key == x) return __ldg(&e->rank);
+        if (key == EMPTY) return NONE32;
+        p = p + 1 == cap ? 0u : p + 1;
     }
     return NONE32;
 }
 
-template <typename K>
-__device__ __forceinline__ uint32_t node_lookup(tables<K> const& T, uint32_t tb, K x) {
-    const uint32_t cap = (uint32_t)T.tab_cap[tb];
-    return node_probe<K>(T.slots + (T.tab_off[tb] - T.off0), cap, slot_of(x, cap), x);
+// One bucket of k_ext_mask / k_ext_flat: blocks from `block` on share its
+// occurrences [ba, bb) (batch-relative) evenly, a block taking the k-mers first
+// inserted by its share.  An item past the last holds the grid's size.
+struct ext_item {
+    uint32_t bucket, block, ba, bb;
+};
+struct ext_share {
+    uint32_t bucket, oa, ob, ba, bb;
+};
+// The calling block's share: 32-way search over the n items (whole warps call).
+__device__ __forceinline__ ext_share find_share(ext_item const* __restrict__ items, uint32_t n) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t lo = 0, hi = n;  // the item is in [lo, hi)
+    while (hi - lo > 1) {
+        const uint32_t step = (hi - lo + 31) / 32;
+        const uint32_t i = lo + lane * step;
+        const bool le = i < hi && items[i].block <= blockIdx.x;
+        const uint32_t m = __ballot_sync(0xffffffffu, le);  // a prefix of the lanes, lane 0 among them
+        const uint32_t at = 31 - __clz(m);
+        const uint32_t l = lo + at * step;
+        hi = min(l + step, hi);
+        lo = l;
+    }
+    const ext_item it = items[lo];
+    const uint32_t parts = items[lo + 1].block - it.block, c = blockIdx.x - it.block;
+    const uint64_t len = it.bb - it.ba;
+    return ext_share{it.bucket, it.ba + (uint32_t)(len * c / parts), it.ba + (uint32_t)(len * (c + 1) / parts), it.ba,
+                     it.bb};
 }
-
-// Nodes [*nb, *ne) (one bucket group's, numbered on the device).
-// Also records, per side, the node of the neighbour when it is the side's
-// only one (link[2n] left, link[2n + 1] right, NONE32 otherwise): k_links
-// then needs no probe.
+// Filter hash of a k-mer from v = x ^ revcomp(x), the same for both strands (no
+// canonical form needed, and a neighbour's v is one XOR away from its node's).
+// Bases i and k - 1 - i of v are equal, so its low half says it all.
+__device__ __forceinline__ uint32_t strand_hash(uint64_t v) {
+    const uint32_t a = (uint32_t)v;
+    return (a ^ (a >> 15)) * 0x9e3779b1u;
+}
+__device__ __forceinline__ uint32_t strand_hash(u128 v) {
+    const uint32_t a = (uint32_t)v, b = (uint32_t)((uint64_t)v >> 32);
+    return ((a ^ (a >> 15)) * 0x85ebca6bu ^ b) * 0x9e3779b1u;
+}
+// Threads of a block: two blocks per SM, with 32 registers a thread (64 for
+// 128-bit k-mers).  FLAT_OCC: occurrences of a k_ext_flat block, for four or two
+// rounds of its threads: fewer leave threads idle, more put the tables of too many
+// buckets in flight for L2 (k = 31: 57 / 54 / 50 / 56 / 88 us per million k-mers
+// at 256 / 512 / 1024 / 2048 / 4096; k = 63: 98 / 93 / 98 / 120 / 156).
 template <typename K>
-__global__ void __launch_bounds__(256, 8) k_ext_mask(unsigned long long const* nb, unsigned long long const* ne,
-                                                     tables<K> T, K const* __restrict__ n_key,
-                                                     uint32_t const* __restrict__ n_bucket, uint32_t k,
-                                                     uint2 const* __restrict__ fw,
-                                                     uint8_t* __restrict__ n_mask, uint32_t* __restrict__ link) {
-    const uint64_t n = *nb + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= *ne) return;
+struct ext_cfg {
+    static constexpr int THREADS = sizeof(K) == 8 ? 1024 : 512;
+    static constexpr uint32_t FLAT_OCC = sizeof(K) == 8 ? 1024 : 512;
+};
+constexpr uint32_t EXT_FILTER_WORDS = 102 * 1024 / 4;
+// Buckets of more occurrences go to k_ext_flat: their keys fill the filter.  us
+// per million k-mers by distinct k-mers per bucket, k_ext_mask / k_ext_flat: k =
+// 31: 63 K 28.8 / 50, 111 K 36 / 50, 189 K (about 2^18 occurrences) 54 / 50, 473 K
+// 133 / 50; k = 63: 77 K 52 / 92, 139 K 66 / 93, 348 K 148 / 94.
+constexpr uint32_t EXT_FILTER_OCC = 1u << 18;
+constexpr uint32_t EXT_ITEM_OCC = 16384;  // least occurrences worth reading the bucket's keys again
+
+// Extension masks: which of a node's 8 possible neighbours are nodes of its
+// bucket, and per side the neighbour's node when it is the side's only one
+// (link[2n] left, link[2n + 1] right, NONE32 otherwise), so k_links needs no
+// probe.  A neighbour is first compared with the nodes before and after (nodes
+// are in insertion order: most neighbours along a record are there), then
+// looked up in a bitmap of the bucket's keys in shared memory, two bits of one
+// word per key, and only what passes is probed in the table, a warp's lookups packed over its
+// lanes.
+// Bound: instruction issue (70% of the ALU pipe), then the table's random sectors.
+// 200 genomes, k = 31: 13.4 -> 7.4 ms, 60 genomes, k = 63: 11.6 -> 5.9 ms against
+// all 8 neighbours probed; with one filter bit per key 8.9 / 6.1.
+template <typename K>
+__global__ void __launch_bounds__(ext_cfg<K>::THREADS, 2)
+    k_ext_mask(ext_item const* __restrict__ items, uint32_t nitems, uint32_t t1, unsigned long long const* ne,
+               tables<K> T, K const* __restrict__ n_key, uint32_t k, uint2 const* __restrict__ fw, uint8_t* __restrict__ n_mask,
+               uint32_t* __restrict__ link) {
     typedef kmer_ops<K> ops;
-    const K can = n_key[n];
-    const K msk = ops::mask(k);
-    const K rev = ops::revcomp(can, k);
-    const uint32_t tb = n_bucket[n] - T.b0;
-    const uint32_t cap = (uint32_t)T.tab_cap[tb];
-    slot_t<K> const* t = T.slots + (T.tab_off[tb] - T.off0);
+    constexpr uint32_t THREADS = ext_cfg<K>::THREADS;
+    extern __shared__ __align__(16) uint32_t ext_filter[];
+    __shared__ uint8_t queue[THREADS / 32][256];
+    const ext_share it = find_share(items, nitems);
+    auto nodes_before = [&](uint32_t o) { return o < t1 ? node_of(fw, o) : (uint32_t)*ne; };
+    const uint32_t na = nodes_before(it.oa), nz = nodes_before(it.ob);
+    if (na == nz) return;
+    const uint32_t ba = nodes_before(it.ba), bb = nodes_before(it.bb);
+    const uint32_t words = min(EXT_FILTER_WORDS, ((bb - ba) / 2 + 4) & ~3u);  // 16 bits per key if they fit
+    for (uint32_t i = threadIdx.x; i < words / 4; i += THREADS)
+        reinterpret_cast<uint4*>(ext_filter)[i] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
+    for (uint32_t n = ba + threadIdx.x; n < bb; n += THREADS) {
+        const K x = n_key[n];
+        const uint32_t h = strand_hash((K)(x ^ ops::revcomp(x, k)));
+        atomicOr(&ext_filter[__umulhi(h, words)], (1u << (h & 31)) | (1u << ((h >> 5) & 31)));
+    }
+    __syncthreads();
+    const K msk = ops::mask(k), msk1 = msk >> 2;
     const uint32_t top = 2 * (k - 1);
-    uint32_t out = 0, right = NONE32, left = NONE32;
-    // appending nt to x prepends 3 - nt to revcomp(x): (rc(x) >> 2) | (3 - nt) << 2(k-1)
+    const uint32_t cap = (uint32_t)T.tab_cap[it.bucket];
+    slot_t<K> const* t = T.slots + (T.tab_off[it.bucket] - T.off0);
+    const int lane = threadIdx.x & 31;
+    uint8_t* const wq = queue[threadIdx.x >> 5];
+    constexpr uint32_t NODE_TAG = 0x80000000u;
+    for (uint32_t n0 = na + (threadIdx.x & ~31u); n0 < nz; n0 += THREADS) {
+        const uint32_t n = n0 + lane;
+        const bool on = n < nz;
+        const K can = on ? n_key[n] : (K)0;
+        const K rev = ops::revcomp(can, k);
+        uint32_t out = 0, need = 0;
+        uint32_t side[2] = {NONE32, NONE32};  // right, left: NODE_TAG | node, or first occurrence
+        // neighbour c: base c & 3 appended to the k-mer (c < 4) or to its
+        // reverse complement; appending nt to x prepends 3 - nt to revcomp(x).
+        // A node y is neighbour c of this one in one of four ways: y or
+        // revcomp(y) starts with the k-mer's last k - 1 bases, or the same for
+        // the k-mer's reverse complement.
+        auto adjacent = [&](K y, uint32_t m) {
+            const K hi = y >> 2, lo = y & msk1;
+            const uint32_t first = ops::low2(y >> top), last = ops::low2(y);
+            auto hit = [&](uint32_t c) {
+                out |= 1u << c;
+                side[c >> 2] = NODE_TAG | m;
+            };
+            if (hi == (can & msk1)) hit(last);
+            if (lo == (rev >> 2)) hit(3u - first);
+            if (hi == (rev & msk1)) hit(4u + last);
+            if (lo == (can >> 2)) hit(7u - first);
+        };
+        if (on && n > ba) adjacent(n_key[n - 1], n - 1);
+        if (on && n + 1 < bb) adjacent(n_key[n + 1], n + 1);
+        {
+            const K vr = ((can << 2) & msk) ^ (rev >> 2), vl = ((rev << 2) & msk) ^ (can >> 2);
 #pragma unroll
-    for (uint32_t nt = 0; nt < 4; ++nt) {
-        const K hi = (K)(3u - nt) << top;
-        const K f = ((can << 2) | (K)nt) & msk;
-        const K fr = (rev >> 2) | hi;
-        const K cf = f <= fr ? f : fr;
-        const uint32_t a = node_probe<K>(t, cap, slot_of(cf, cap), cf);
-        if (a != NONE32) {
-            out |= 1u << nt;
-            right = a;
+            for (uint32_t c = 0; c < 8; ++c) {
+                const K v = (c < 4 ? vr : vl) ^ (K)(c & 3u) ^ ((K)(3u - (c & 3u)) << top);
+                const uint32_t h = strand_hash(v), w = ext_filter[__umulhi(h, words)];
+                need |= ((w >> (h & 31)) & (w >> ((h >> 5) & 31)) & 1u) << c;
+            }
         }
-        const K r = ((rev << 2) | (K)nt) & msk;
-        const K rr = (can >> 2) | hi;
-        const K cr = r <= rr ? r : rr;
-        const uint32_t b = node_probe<K>(t, cap, slot_of(cr, cap), cr);
-        if (b != NONE32) {
-            out |= 1u << (4 + nt);
-            left = b;
+        need = on ? need & ~out : 0u;
+        // the warp's lookups, laid end to end over its lanes: entry = the
+        // node's lane and c
+        const uint32_t cnt = __popc(need);
+        uint32_t total;
+        const uint32_t at = warp_excl_scan32(cnt, total);
+        __syncwarp();
+        {
+            uint32_t m = need;
+            for (uint32_t i = at; m; ++i, m &= m - 1) wq[i] = (uint8_t)((lane << 3) | (__ffs(m) - 1));
+        }
+        __syncwarp();
+        uint32_t next = at;
+        for (uint32_t q0 = 0; q0 < total; q0 += 32) {
+            const uint32_t e = q0 + lane < total ? wq[q0 + lane] : 0u;
+            const int src = (int)(e >> 3);
+            const uint32_t c = e & 7u, nt = c & 3u;
+            const K cs = ops::shfl(can, src), rs = ops::shfl(rev, src);
+            uint32_t got = NONE32;
+            if (q0 + lane < total) {
+                const K x = c < 4 ? cs : rs, y = c < 4 ? rs : cs;
+                const K f = ((x << 2) | (K)nt) & msk, r = (y >> 2) | ((K)(3u - nt) << top);
+                const K z = f <= r ? f : r;
+                got = node_probe(t, cap, z);
+            }
+            // each node's lane takes its answers
+            for (;;) {
+                const bool mine = need != 0 && next < q0 + 32;
+                if (!__any_sync(0xffffffffu, mine)) break;
+                const uint32_t v = __shfl_sync(0xffffffffu, got, (int)(next & 31));
+                if (mine) {
+                    const uint32_t cc = __ffs(need) - 1;
+                    need &= need - 1;
+                    ++next;
+                    if (v != NONE32) {
+                        out |= 1u << cc;
+                        side[cc >> 2] = v;
+                    }
+                }
+            }
+        }
+        if (on) {
+            n_mask[n] = (uint8_t)out;
+            auto node = [&](uint32_t v) { return (v & NODE_TAG) ? v & ~NODE_TAG : node_of(fw, v); };
+            uint2 l;
+            l.x = __popc(out >> 4) == 1 ? node(side[1]) : NONE32;
+            l.y = __popc(out & 0xfu) == 1 ? node(side[0]) : NONE32;
+            reinterpret_cast<uint2*>(link)[n] = l;
         }
     }
-    n_mask[n] = (uint8_t)out;
-    link[2 * n] = __popc(out >> 4) == 1 ? node_of(fw, left) : NONE32;
-    link[2 * n + 1] = __popc(out & 0xfu) == 1 ? node_of(fw, right) : NONE32;
+}
+
+// The same without a filter, for buckets of more keys than one is good for:
+// small blocks in bucket order, so the buckets in flight stay in L2.
+template <typename K>
+__global__ void __launch_bounds__(256, 8)
+    k_ext_flat(ext_item const* __restrict__ items, uint32_t nitems, uint32_t t1, unsigned long long const* ne,
+               tables<K> T, K const* __restrict__ n_key, uint32_t k, uint2 const* __restrict__ fw,
+               uint8_t* __restrict__ n_mask, uint32_t* __restrict__ link) {
+    typedef kmer_ops<K> ops;
+    const ext_share it = find_share(items, nitems);
+    auto nodes_before = [&](uint32_t o) { return o < t1 ? node_of(fw, o) : (uint32_t)*ne; };
+    const uint32_t na = nodes_before(it.oa), nz = nodes_before(it.ob);
+    const K msk = ops::mask(k);
+    const uint32_t top = 2 * (k - 1);
+    const uint32_t cap = (uint32_t)T.tab_cap[it.bucket];
+    slot_t<K> const* t = T.slots + (T.tab_off[it.bucket] - T.off0);
+    for (uint32_t n = na + threadIdx.x; n < nz; n += 256) {
+        const K can = n_key[n];
+        const K rev = ops::revcomp(can, k);
+        uint32_t out = 0, right = NONE32, left = NONE32;
+#pragma unroll
+        for (uint32_t nt = 0; nt < 4; ++nt) {
+            const K hi = (K)(3u - nt) << top;
+            const K f = ((can << 2) | (K)nt) & msk;
+            const K fr = (rev >> 2) | hi;
+            const uint32_t a = node_probe(t, cap, f <= fr ? f : fr);
+            if (a != NONE32) {
+                out |= 1u << nt;
+                right = a;
+            }
+            const K r = ((rev << 2) | (K)nt) & msk;
+            const K rr = (can >> 2) | hi;
+            const uint32_t b = node_probe(t, cap, r <= rr ? r : rr);
+            if (b != NONE32) {
+                out |= 1u << (4 + nt);
+                left = b;
+            }
+        }
+        n_mask[n] = (uint8_t)out;
+        uint2 l;
+        l.x = __popc(out >> 4) == 1 ? node_of(fw, left) : NONE32;
+        l.y = __popc(out & 0xfu) == 1 ? node_of(fw, right) : NONE32;
+        reinterpret_cast<uint2*>(link)[n] = l;
+    }
 }
 
 __device__ __forceinline__ uint32_t fwd_nib(uint32_t m, bool rc) { return (rc ? (m >> 4) : m) & 0xfu; }
@@ -1706,9 +1901,8 @@ __device__ __forceinline__ uint32_t back_nib(uint32_t m, bool rc) { return (rc ?
 // sides' only neighbours as k_ext_mask found them.
 template <typename K>
 __global__ void __launch_bounds__(256, 8) k_links(unsigned long long const* nb, unsigned long long const* ne,
-                                                  tables<K> T, K const* __restrict__ n_key,
-                                                  uint32_t const* __restrict__ n_bucket,
-                                                  uint8_t const* __restrict__ n_mask, uint32_t k,
+                                                  K const* __restrict__ n_key, uint8_t const* __restrict__ n_mask,
+                                                  uint32_t k,
                                                   uint32_t* __restrict__ link) {
     const uint64_t n = *nb + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (n >= *ne) return;
@@ -2346,7 +2540,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         // slots per occurrence q/4 > 1 (distinct <= occurrences): the default
         // 2 keeps the load factor <= 1/2 for short unsuccessful probes in the
         // neighbour lookups
-        const uint64_t cap = o ? std::max<uint64_t>(64, (o * q + 3) / 4 + 16) : 0;
+        const uint64_t cap = o ? std::max<uint64_t>(64, (o * q / 4 + 17) & ~uint64_t(1)) : 0;  // whole pairs
         toff[b] = T;
         tcap[b] = cap;
         T += cap;
@@ -2363,10 +2557,38 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     uint64_t Tmax = 0;
     for (size_t g = 0; g < ng; ++g) Tmax = std::max<uint64_t>(Tmax, toff[gb[g + 1]] - toff[gb[g]]);
     uint32_t* occ_slot = A.alloc<uint32_t>(nocc);
-    uint64_t* d_toff = A.alloc<uint64_t>(nb + 1);
-    uint64_t* d_tcap = A.alloc<uint64_t>(nb);
-    CDBG_CUDA(cudaMemcpyAsync(d_toff, toff.data(), 8ull * (nb + 1), cudaMemcpyHostToDevice, st));
-    CDBG_CUDA(cudaMemcpyAsync(d_tcap, tcap.data(), 8ull * nb, cudaMemcpyHostToDevice, st));
+    // the buckets of k_ext_mask and of k_ext_flat, per group, with their blocks.
+    // A k_ext_mask bucket is split so that there are about four blocks per
+    // resident one (the last ones leave few SMs idle), but into no smaller parts
+    // than are worth reading the bucket's keys again for its filter.
+    std::vector<ext_item> items;
+    std::vector<uint32_t> gitem(2 * ng + 1, 0), gblocks(2 * ng, 0);
+    {
+        const uint64_t share = std::max<uint64_t>(EXT_ITEM_OCC, nocc / (148 * 8));
+        for (size_t g = 0; g < 2 * ng; ++g) {  // group g / 2, flat when odd
+            uint32_t blocks = 0;
+            for (uint32_t b = gb[g / 2]; b < gb[g / 2 + 1]; ++b) {
+                const uint64_t ba = bocc[b0 + b] - O0, n = bocc[b0 + b + 1] - O0 - ba;
+                if (n == 0 || (n > EXT_FILTER_OCC) != (g & 1)) continue;
+                items.push_back(ext_item{b - gb[g / 2], blocks, (uint32_t)ba, (uint32_t)(ba + n)});
+                blocks += (uint32_t)((g & 1) ? ceil_div(n, (uint64_t)ext_cfg<K>::FLAT_OCC) : n > share + share / 2 ? ceil_div(n, share) : 1);
+            }
+            items.push_back(ext_item{0, blocks, 0, 0});
+            gblocks[g] = blocks;
+            gitem[g + 1] = (uint32_t)items.size();
+        }
+    }
+    // one upload: table offsets, capacities, items
+    const size_t items_at = 8 * (2 * (size_t)nb + 1), up_bytes = items_at + items.size() * sizeof(ext_item);
+    std::vector<uint8_t> up(up_bytes);
+    std::memcpy(up.data(), toff.data(), 8 * ((size_t)nb + 1));
+    std::memcpy(up.data() + 8 * ((size_t)nb + 1), tcap.data(), 8 * (size_t)nb);
+    std::memcpy(up.data() + items_at, items.data(), items.size() * sizeof(ext_item));
+    uint8_t* d_up = A.alloc<uint8_t>(up_bytes);
+    CDBG_CUDA(cudaMemcpyAsync(d_up, up.data(), up_bytes, cudaMemcpyHostToDevice, st));
+    uint64_t const* d_toff = reinterpret_cast<uint64_t const*>(d_up);
+    uint64_t const* d_tcap = d_toff + nb + 1;
+    ext_item const* d_items = reinterpret_cast<ext_item const*>(d_up + items_at);
     slot_t<K>* slots = A.alloc<slot_t<K>>(Tmax + 1);
     // record of each occurrence block's first occurrence (k_insert, k_number)
     const uint64_t nblk = ceil_div(nocc, (uint64_t)OCC_BLOCK);
@@ -2380,7 +2602,6 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     K* n_key = A.alloc<K>(nocc);
     uint8_t* n_meta = A.alloc<uint8_t>(nocc);
     uint32_t* n_rec = A.alloc<uint32_t>(nocc);
-    uint32_t* n_bucket = A.alloc<uint32_t>(nocc);
     uint8_t* n_mask = A.alloc<uint8_t>(nocc);
     uint32_t* link = A.alloc<uint32_t>(2 * nocc);
     // (node, record) pairs of multi-record k-mers: at most one per occurrence
@@ -2431,9 +2652,8 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         {
             CDBG_PROF("k_number", st);
             k_number<K><<<(unsigned)(gtile[g + 1] - gtile[g]), 256, 0, st>>>(
-                t0 / OCC_BLOCK * OCC_BLOCK, t0, t0 + tn, occ_slot, TG, R.occ, R.bucket, R0, nrec, O0, nblk, blk_rec,
-                nbase, nnext, nb_counter + g, nb_status + gtile[g], fw, n_key, n_meta, n_rec, n_bucket, pnode, prec,
-                d_err);
+                t0 / OCC_BLOCK * OCC_BLOCK, t0, t0 + tn, occ_slot, TG, R.occ, R0, nrec, O0, nblk, blk_rec, nbase,
+                nnext, nb_counter + g, nb_status + gtile[g], fw, n_key, n_meta, n_rec, pnode, prec, d_err);
         }
         CDBG_CHECK_LAUNCH();
         {
@@ -2444,12 +2664,21 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         CDBG_CHECK_LAUNCH();
         {
             CDBG_PROF("k_ext_mask", st);
-            k_ext_mask<K><<<grid(tn, 256), 256, 0, st>>>(nbase, nnext, TG, n_key, n_bucket, k, fw, n_mask, link);
+            constexpr int smem = EXT_FILTER_WORDS * 4;
+            CDBG_CUDA(cudaFuncSetAttribute(k_ext_mask<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            if (gblocks[2 * g])
+                k_ext_mask<K><<<gblocks[2 * g], ext_cfg<K>::THREADS, smem, st>>>(
+                    d_items + gitem[2 * g], gitem[2 * g + 1] - gitem[2 * g] - 1, (uint32_t)(t0 + tn), nnext, TG, n_key, k,
+                    fw, n_mask, link);
+            if (gblocks[2 * g + 1])
+                k_ext_flat<K><<<gblocks[2 * g + 1], 256, 0, st>>>(
+                    d_items + gitem[2 * g + 1], gitem[2 * g + 2] - gitem[2 * g + 1] - 1, (uint32_t)(t0 + tn), nnext, TG,
+                    n_key, k, fw, n_mask, link);
         }
         CDBG_CHECK_LAUNCH();
         {
             CDBG_PROF("k_links", st);
-            k_links<K><<<grid(tn, 256), 256, 0, st>>>(nbase, nnext, TG, n_key, n_bucket, n_mask, k, link);
+            k_links<K><<<grid(tn, 256), 256, 0, st>>>(nbase, nnext, n_key, n_mask, k, link);
         }
         CDBG_CHECK_LAUNCH();
     }

@@ -62,3 +62,17 @@ def test_long_records_and_groups(oracle, tmp_path, k, group_mb):
     with native.Engine(0) as e:
         e.set_tuning(table_group_mb=group_mb)
         _check(oracle, e, tmp_path, [g0, g1, g2], k, 37)
+
+
+@pytest.mark.parametrize("k", [21, 31, 63])
+@pytest.mark.parametrize("buckets,n", [(1, 300_000), (1, 250_000), (3, 900_000), (64, 200_000)])
+def test_neighbour_lookups_by_bucket_size(oracle, engine, tmp_path, k, buckets, n):
+    """Extension masks with the presence filter (buckets of up to 2^18
+    occurrences), split buckets among them, and without; branches, repeats and
+    self-neighbours."""
+    rng = np.random.default_rng(n + k + buckets)
+    a = _dna(rng, n)
+    b = bytearray(a[: n // 3])
+    for i in rng.integers(0, len(b), len(b) // 60).tolist():
+        b[i] = b"ACGT"[int(rng.integers(0, 4))]
+    _check(oracle, engine, tmp_path, [[a, b"A" * (2 * k), b"ACGT" * k], [bytes(b), a[-2 * k:] + a[:2 * k]]], k, buckets)
