@@ -120,8 +120,11 @@ struct call_scope {
     cdbg::kernel_profiler* prev_prof;
     cdbg::host_mailbox* prev_mailbox;
     int prev_bits;
+    uint32_t* prev_err;
     explicit call_scope(cdbg_engine* en)
-        : e(en), prev_prof(cdbg::g_prof), prev_mailbox(cdbg::g_mailbox), prev_bits(cdbg::g_radix_bits) {
+        : e(en), prev_prof(cdbg::g_prof), prev_mailbox(cdbg::g_mailbox), prev_bits(cdbg::g_radix_bits),
+          prev_err(cdbg::g_dev_err) {
+        cdbg::g_dev_err = e->d_err;
         cdbg::g_prof = &e->prof;
         cdbg::g_mailbox = &e->mailbox;
         cdbg::g_radix_bits = e->tune.radix_bits == 11 ? 11 : 8;
@@ -131,6 +134,7 @@ struct call_scope {
         cdbg::g_prof = prev_prof;  // calls nest (the autotuner builds through the public entry)
         cdbg::g_mailbox = prev_mailbox;
         cdbg::g_radix_bits = prev_bits;
+        cdbg::g_dev_err = prev_err;
     }
 };
 
@@ -209,6 +213,7 @@ std::atomic<uint64_t> g_launches{0};
 void set_last_error(std::string const& msg) { g_last_error = msg; }
 thread_local kernel_profiler* g_prof = nullptr;
 thread_local host_mailbox* g_mailbox = nullptr;
+thread_local uint32_t* g_dev_err = nullptr;
 thread_local int g_radix_bits = 8;
 
 void check_device_error(cdbg_engine* e, char const* stage) {
@@ -284,6 +289,7 @@ int cdbg_engine_create(int device, cdbg_engine** out) {
         CDBG_CUDA(cudaMemset(e->d_err, 0, 16));
         e->mailbox.bytes = size_t(256) << 10;
         CDBG_CUDA(cudaHostAlloc(&e->mailbox.h, e->mailbox.bytes, cudaHostAllocMapped));
+        std::memset(e->mailbox.h, 0, cdbg::MAIL_DATA);
         CDBG_CUDA(cudaHostGetDevicePointer(&e->mailbox.d, e->mailbox.h, 0));
         *out = e;
         return 0;

@@ -158,33 +158,96 @@ struct host_mailbox {
     void* h = nullptr;  // host address
     void* d = nullptr;  // device address of the same pages
     size_t bytes = 0;
+    uint32_t seq = 0;   // number of the last delivery
 };
 extern thread_local host_mailbox* g_mailbox;
 // Radix digit width of the sorts run by this host thread's current engine
 // call (8 or 11 bits; a performance knob, cdbg_tuning.radix_bits).
 extern thread_local int g_radix_bits;
+// Device error word of this host thread's current engine call.
+extern thread_local uint32_t* g_dev_err;
 
 namespace {
-__global__ void k_mail_bytes(uint8_t const* __restrict__ src, uint8_t* __restrict__ dst, uint64_t n) {
-    if (((uintptr_t)src & 7) == 0 && (n & 7) == 0) {
-        for (uint64_t i = threadIdx.x; i < n / 8; i += blockDim.x)
-            reinterpret_cast<uint64_t*>(dst)[i] = reinterpret_cast<uint64_t const*>(src)[i];
-    } else {
-        for (uint64_t i = threadIdx.x; i < n; i += blockDim.x) dst[i] = src[i];
+constexpr size_t MAIL_DATA = 64;  // mailbox: the delivery number, then the data
+constexpr int MAIL_MAX = 6;       // values of one delivery
+struct mail_set {
+    uint8_t const* src[MAIL_MAX];
+    uint32_t n[MAIL_MAX];
+    uint32_t at[MAIL_MAX];  // offset in the mailbox's data
+    uint32_t count;
+};
+__global__ void k_mail(mail_set m, uint8_t* __restrict__ box, uint32_t seq) {
+    uint8_t* data = box + MAIL_DATA;
+    for (uint32_t j = 0; j < m.count; ++j) {
+        uint8_t const* src = m.src[j];
+        uint8_t* dst = data + m.at[j];
+        if (((uintptr_t)src & 7) == 0 && (m.n[j] & 7) == 0) {
+            for (uint32_t i = threadIdx.x; i < m.n[j] / 8; i += blockDim.x)
+                reinterpret_cast<uint64_t*>(dst)[i] = reinterpret_cast<uint64_t const*>(src)[i];
+        } else {
+            for (uint32_t i = threadIdx.x; i < m.n[j]; i += blockDim.x) dst[i] = src[i];
+        }
     }
+    __threadfence_system();
+    __syncthreads();
+    if (threadIdx.x == 0) *(volatile uint32_t*)box = seq;
 }
 
-inline void read_small(void* host_dst, void const* dev_src, size_t n, cudaStream_t st) {
-    host_mailbox* mb = g_mailbox;
-    if (mb && mb->h && n <= mb->bytes) {
-        k_mail_bytes<<<1, 256, 0, st>>>(static_cast<uint8_t const*>(dev_src), static_cast<uint8_t*>(mb->d), n);
-        CDBG_CHECK_LAUNCH();
-        CDBG_CUDA(cudaStreamSynchronize(st));
-        std::memcpy(host_dst, mb->h, n);
-    } else {
-        CDBG_CUDA(cudaMemcpyAsync(host_dst, dev_src, n, cudaMemcpyDeviceToHost, st));
-        CDBG_CUDA(cudaStreamSynchronize(st));
+// Device values the host waits for together: add() them, then wait().
+class mail_reader {
+public:
+    explicit mail_reader(cudaStream_t st) : m_st(st) { m_set.count = 0; }
+    template <typename T>
+    mail_reader& add(T* host_dst, void const* dev_src, size_t bytes = sizeof(T)) {
+        if (m_set.count == MAIL_MAX) throw std::runtime_error("mail_reader: too many values");
+        m_dst[m_set.count] = host_dst;
+        m_set.src[m_set.count] = static_cast<uint8_t const*>(dev_src);
+        m_set.n[m_set.count] = (uint32_t)bytes;
+        m_set.at[m_set.count] = (uint32_t)m_used;
+        m_used += (bytes + 15) & ~size_t(15);
+        ++m_set.count;
+        return *this;
     }
+    void wait() {
+        host_mailbox* mb = g_mailbox;
+        if (!mb || !mb->h || MAIL_DATA + m_used > mb->bytes) {
+            for (uint32_t j = 0; j < m_set.count; ++j)
+                CDBG_CUDA(cudaMemcpyAsync(m_dst[j], m_set.src[j], m_set.n[j], cudaMemcpyDeviceToHost, m_st));
+            CDBG_CUDA(cudaStreamSynchronize(m_st));
+            return;
+        }
+        const uint32_t seq = ++mb->seq;
+        k_mail<<<1, m_used > 512 ? 256 : 32, 0, m_st>>>(m_set, static_cast<uint8_t*>(mb->d), seq);
+        CDBG_CHECK_LAUNCH();
+        // Short waits watch the delivery number; longer ones (and errors) go
+        // to the driver, whose wake-up costs microseconds.
+        volatile uint32_t const* flag = static_cast<volatile uint32_t const*>(mb->h);
+        bool got = false;
+        for (int spin = 0; spin < 20000 && !got; ++spin) {
+            got = *flag == seq;
+#if defined(__x86_64__)
+            if (!got) __builtin_ia32_pause();
+#endif
+        }
+        if (!got) CDBG_CUDA(cudaStreamSynchronize(m_st));
+        std::atomic_thread_fence(std::memory_order_acquire);
+        for (uint32_t j = 0; j < m_set.count; ++j)
+            std::memcpy(m_dst[j], static_cast<uint8_t const*>(mb->h) + MAIL_DATA + m_set.at[j], m_set.n[j]);
+        m_set.count = 0;
+        m_used = 0;
+    }
+
+private:
+    cudaStream_t m_st;
+    mail_set m_set;
+    void* m_dst[MAIL_MAX];
+    size_t m_used = 0;
+};
+
+inline void read_small(void* host_dst, void const* dev_src, size_t n, cudaStream_t st) {
+    mail_reader r(st);
+    r.add(static_cast<uint8_t*>(host_dst), dev_src, n);
+    r.wait();
 }
 }  // namespace
 

@@ -2,8 +2,8 @@
 // stable LSD radix sort of (key, value) pairs, u32 or u64 keys.
 //
 // Radix sort: one fused histogram pass computes the digit histograms of every
-// requested pass in a single read of the keys; passes whose digit is constant
-// over all keys are skipped.  Each executed pass is ONE kernel (k_rs_onesweep):
+// requested pass in a single read of the keys; passes of large sorts whose digit
+// is constant over all keys are skipped.  Each executed pass is ONE kernel (k_rs_onesweep):
 // tiles rank their keys stably with warp match-any, find their global digit
 // offsets by a decoupled look-back per digit, stage the tile in shared memory
 // in digit order and write each digit's run contiguously.
@@ -24,7 +24,7 @@ namespace prim {
 namespace {
 
 constexpr int SCAN_THREADS = 256;
-constexpr int SCAN_ITEMS = 8;
+constexpr int SCAN_ITEMS = 16;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
 
 template <typename U>
@@ -57,100 +57,6 @@ __device__ __forceinline__ U block_exclusive_scan(U v, U* smem_warp, U& total) {
     total = smem_warp[NW];
     __syncthreads();
     return r;
-}
-
-// Tile sums: thread t adds elements t, t + 256, ... of the tile (coalesced).
-template <typename T, typename U>
-__global__ void __launch_bounds__(SCAN_THREADS) k_tile_sums(T const* __restrict__ in, uint64_t n,
-                                                            U* __restrict__ sums) {
-    __shared__ U sw[SCAN_THREADS / 32 + 1];
-    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
-    U s = 0;
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; ++i) {
-        const uint64_t j = base + (uint64_t)i * SCAN_THREADS + threadIdx.x;
-        if (j < n) s += (U)in[j];
-    }
-    U tot;
-    block_exclusive_scan<U, SCAN_THREADS>(s, sw, tot);
-    if (threadIdx.x == 0) sums[blockIdx.x] = tot;
-}
-
-// Shared-memory index of tile element j, padded so that a thread reading its
-// SCAN_ITEMS consecutive elements meets no bank conflict (4- and 8-byte types).
-template <typename V>
-__device__ __forceinline__ uint32_t scan_pad(uint32_t j) {
-    return j + (j >> (sizeof(V) == 8 ? 4 : 5));
-}
-
-// Tile scan: coalesced loads and stores through shared memory; each thread
-// scans SCAN_ITEMS consecutive elements.
-template <typename T, typename U>
-__global__ void __launch_bounds__(SCAN_THREADS) k_tile_scan(T const* __restrict__ in, uint64_t n,
-                                                            U const* __restrict__ offs,
-                                                            U* __restrict__ out, U* total_out) {
-    __shared__ U sw[SCAN_THREADS / 32 + 1];
-    __shared__ T sin[SCAN_TILE + SCAN_TILE / 16];
-    __shared__ U sout[SCAN_TILE + SCAN_TILE / 16];
-    const uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; ++i) {
-        const uint32_t j = (uint32_t)i * SCAN_THREADS + threadIdx.x;
-        sin[scan_pad<T>(j)] = (base + j < n) ? in[base + j] : T(0);
-    }
-    __syncthreads();
-    T v[SCAN_ITEMS];
-    U s = 0;
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; ++i) {
-        v[i] = sin[scan_pad<T>(threadIdx.x * SCAN_ITEMS + i)];
-        s += (U)v[i];
-    }
-    U tot;
-    U p = block_exclusive_scan<U, SCAN_THREADS>(s, sw, tot);
-    p += offs ? offs[blockIdx.x] : U(0);
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; ++i) {
-        sout[scan_pad<U>(threadIdx.x * SCAN_ITEMS + i)] = p;
-        p += (U)v[i];
-    }
-    if (total_out && blockIdx.x == gridDim.x - 1 && threadIdx.x == SCAN_THREADS - 1) *total_out = p;
-    __syncthreads();
-#pragma unroll
-    for (int i = 0; i < SCAN_ITEMS; ++i) {
-        const uint32_t j = (uint32_t)i * SCAN_THREADS + threadIdx.x;
-        if (base + j < n) out[base + j] = sout[scan_pad<U>(j)];
-    }
-}
-
-// out[i] = sum(in[0..i)), in place allowed (out == in when T == U).  When
-// total_dev is given the grand total is written there (device memory).
-template <typename T, typename U>
-void exclusive_scan(T const* in, U* out, uint64_t n, dev_arena& A, cudaStream_t st,
-                    U* total_dev = nullptr) {
-    if (n == 0) {
-        if (total_dev) CDBG_CUDA(cudaMemsetAsync(total_dev, 0, sizeof(U), st));
-        return;
-    }
-    const uint64_t tiles = ceil_div(n, SCAN_TILE);
-    auto m = A.mark();
-    U* offs = nullptr;
-    if (tiles > 1) {
-        U* sums = A.alloc<U>(tiles);
-        {
-            CDBG_PROF("k_tile_sums", st);
-            k_tile_sums<T, U><<<(unsigned)tiles, SCAN_THREADS, 0, st>>>(in, n, sums);
-        }
-        CDBG_CHECK_LAUNCH();
-        exclusive_scan<U, U>(sums, sums, tiles, A, st, (U*)nullptr);
-        offs = sums;
-    }
-    {
-        CDBG_PROF("k_tile_scan", st);
-        k_tile_scan<T, U><<<(unsigned)tiles, SCAN_THREADS, 0, st>>>(in, n, offs, out, total_dev);
-    }
-    CDBG_CHECK_LAUNCH();
-    A.release(m);
 }
 
 // ------------------------------------------------------------ ordered output
@@ -203,6 +109,129 @@ __device__ __forceinline__ bool lookback_exclusive(unsigned long long* status, u
     return ok;
 }
 
+// ------------------------------------------------------------------ scan
+// Shared-memory index of tile element j, padded so that a thread reading its
+// consecutive elements meets no bank conflict (4- and 8-byte types).
+template <typename V>
+__device__ __forceinline__ uint32_t scan_pad(uint32_t j) {
+    return j + (j >> (sizeof(V) == 8 ? 4 : 5));
+}
+
+// One tile of the scan, [base, base + THREADS * ITEMS) of n: coalesced loads and
+// stores through shared memory, each thread scanning ITEMS consecutive elements.
+// `before(tot)` turns the tile's total into the sum of everything before it
+// (called by the whole block); returns the inclusive sum of the tile's end to
+// the last thread.
+template <typename T, typename U, int THREADS, int ITEMS, typename Before>
+__device__ __forceinline__ U scan_tile(T const* __restrict__ in, uint64_t n, uint64_t base, U* __restrict__ out,
+                                       U* buf, U* sw, Before const& before) {
+    // the inputs go through the same buffer as the outputs (a T is no wider)
+    static_assert(sizeof(T) <= sizeof(U), "inputs are staged in the output buffer");
+    T* sin = reinterpret_cast<T*>(buf);
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t j = (uint32_t)i * THREADS + threadIdx.x;
+        sin[scan_pad<T>(j)] = (base + j < n) ? in[base + j] : T(0);
+    }
+    __syncthreads();
+    T v[ITEMS];
+    U s = 0;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        v[i] = sin[scan_pad<T>(threadIdx.x * ITEMS + i)];
+        s += (U)v[i];
+    }
+    U tot;
+    U p = block_exclusive_scan<U, THREADS>(s, sw, tot);  // (its barriers separate the reads from the writes below)
+    p += before(tot);
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        buf[scan_pad<U>(threadIdx.x * ITEMS + i)] = p;
+        p += (U)v[i];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t j = (uint32_t)i * THREADS + threadIdx.x;
+        if (base + j < n) out[base + j] = buf[scan_pad<U>(j)];
+    }
+    return p;
+}
+
+// n <= SCAN_ONE elements by one block, in one launch.
+constexpr int SCAN_ONE_THREADS = 512;
+constexpr int SCAN_ONE_ITEMS = 8;
+constexpr uint64_t SCAN_ONE = SCAN_ONE_THREADS * SCAN_ONE_ITEMS;
+template <typename T, typename U>
+__global__ void __launch_bounds__(SCAN_ONE_THREADS) k_scan_one(T const* __restrict__ in, uint64_t n,
+                                                               U* __restrict__ out, U* total_out) {
+    __shared__ U sw[SCAN_ONE_THREADS / 32 + 1];
+    __shared__ U buf[SCAN_ONE + SCAN_ONE / 16];
+    const U p = scan_tile<T, U, SCAN_ONE_THREADS, SCAN_ONE_ITEMS>(in, n, 0, out, buf, sw, [](U) { return U(0); });
+    if (total_out && threadIdx.x == SCAN_ONE_THREADS - 1) *total_out = p;
+}
+
+// More in one pass over the data: tiles take their indices in launch order and
+// find the sum before them by decoupled look-back.
+// Bound: HBM (one read and one write; tile sums, their scan and the tiles again
+// read the input twice: 3.5 -> 2.9 ms of a 200-genome build, three launches
+// where this takes one and a memset).
+template <typename T, typename U>
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan(T const* __restrict__ in, uint64_t n, U* __restrict__ out,
+                                                       uint32_t* tile_counter, unsigned long long* status,
+                                                       U* total_out, uint32_t* err) {
+    __shared__ U sw[SCAN_THREADS / 32 + 1];
+    __shared__ U buf[SCAN_TILE + SCAN_TILE / 16];
+    __shared__ uint64_t s_tile, s_excl;
+    if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1u);
+    __syncthreads();
+    const uint64_t tile = s_tile;
+    const U p = scan_tile<T, U, SCAN_THREADS, SCAN_ITEMS>(in, n, tile * SCAN_TILE, out, buf, sw, [&](U tot) {
+        if (threadIdx.x < 32) {
+            uint64_t excl = 0;
+            const bool ok = lookback_exclusive(status, tile, (uint64_t)tot, excl);
+            if (threadIdx.x == 0) {
+                if (!ok) set_error(err, ERR_CHAIN_LIMIT);
+                s_excl = excl;
+            }
+        }
+        __syncthreads();
+        return (U)s_excl;
+    });
+    if (total_out && tile == gridDim.x - 1 && threadIdx.x == SCAN_THREADS - 1) *total_out = p;
+}
+
+// out[i] = sum(in[0..i)), in place allowed (out == in when T == U).  When
+// total_dev is given the grand total is written there (device memory).  Sums
+// stay below 2^62.
+template <typename T, typename U>
+void exclusive_scan(T const* in, U* out, uint64_t n, dev_arena& A, cudaStream_t st,
+                    U* total_dev = nullptr) {
+    if (n == 0) {
+        if (total_dev) CDBG_CUDA(cudaMemsetAsync(total_dev, 0, sizeof(U), st));
+        return;
+    }
+    if (n <= SCAN_ONE) {
+        {
+            CDBG_PROF("k_scan_one", st);
+            k_scan_one<T, U><<<1, SCAN_ONE_THREADS, 0, st>>>(in, n, out, total_dev);
+        }
+        CDBG_CHECK_LAUNCH();
+        return;
+    }
+    const uint64_t tiles = ceil_div(n, SCAN_TILE);
+    auto m = A.mark();
+    unsigned long long* status = A.alloc<unsigned long long>(tiles + 1);  // and the tile counter
+    CDBG_CUDA(cudaMemsetAsync(status, 0, 8 * (tiles + 1), st));
+    {
+        CDBG_PROF_BYTES("k_scan", st, n * (sizeof(T) + sizeof(U)));
+        k_scan<T, U><<<(unsigned)tiles, SCAN_THREADS, 0, st>>>(in, n, out, reinterpret_cast<uint32_t*>(status + tiles),
+                                                               status, total_dev, g_dev_err);
+    }
+    CDBG_CHECK_LAUNCH();
+    A.release(m);
+}
+
 // ------------------------------------------------------------------ radix sort
 constexpr int RS_THREADS = 256;
 constexpr int RS_BITS = 8;
@@ -234,7 +263,7 @@ struct rs_smem {
     uint32_t wcnt[RS_WARPS][BINS];  // per-warp digit counts, then prefixes
     uint32_t dstart[BINS];          // tile-local start of each digit
     uint64_t gbase[BINS];           // global start of each digit for this tile
-    uint32_t sw[RS_WARPS + 1];
+    uint64_t sw[RS_WARPS + 1];
     uint32_t tile;
 };
 
@@ -244,7 +273,7 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
                                                             K* __restrict__ keys_out, V* __restrict__ vals_out,
                                                             uint64_t n, int shift, uint32_t* tile_counter,
                                                             unsigned long long* status,
-                                                            unsigned long long const* __restrict__ digit_start,
+                                                            unsigned long long const* __restrict__ hist,
                                                             uint32_t epoch, uint32_t* err) {
     using S = rs_smem<BITS, ITEMS, K, V>;
     constexpr int BINS = S::BINS, TILE = S::TILE, DPT = (BINS + RS_THREADS - 1) / RS_THREADS;
@@ -328,19 +357,25 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
             const unsigned long long ep = (unsigned long long)epoch << 58;
             *(volatile unsigned long long*)&status[tile * BINS + d] = RS_INC | ep | ((excl + cnt[j]) & RS_VALMASK);
         }
-        sm.gbase[d] = digit_start[d] + excl;
+        sm.gbase[d] = excl;
     }
-    // tile-local digit starts (exclusive scan of the counts over digits)
+    // digit starts (exclusive scans over digits): tile-local ones of the counts,
+    // global ones of the pass's histogram
     {
         // thread t owns digits t, t + RS_THREADS, ...: one block scan per
-        // column keeps the starts in digit order
-        uint32_t carry = 0;
+        // column keeps the starts in digit order.  Both scans at once: a tile's
+        // counts add up to at most TILE, the histogram to n < 2^48.
+        uint64_t carry = 0;
 #pragma unroll
         for (int j = 0; j < DPT; ++j) {
-            uint32_t tot;
-            const uint32_t ex = block_exclusive_scan<uint32_t, RS_THREADS>(cnt[j], sm.sw, tot);
             const int d = threadIdx.x + j * RS_THREADS;
-            if (d < BINS) sm.dstart[d] = carry + ex;
+            const uint64_t both = d < BINS ? ((uint64_t)__ldg(hist + d) << 16) | cnt[j] : 0;
+            uint64_t tot;
+            const uint64_t ex = carry + block_exclusive_scan<uint64_t, RS_THREADS>(both, sm.sw, tot);
+            if (d < BINS) {
+                sm.dstart[d] = (uint32_t)(ex & 0xffffu);
+                sm.gbase[d] += ex >> 16;
+            }
             carry += tot;
         }
     }
@@ -367,18 +402,108 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
     }
 }
 
-// Exclusive scan of each pass's digit histogram: starts[p][d].
-template <int BITS>
-__global__ void k_rs_digit_starts(unsigned long long const* __restrict__ hist, int npasses,
-                                  unsigned long long* __restrict__ starts) {
-    constexpr int BINS = 1 << BITS;
-    const int p = blockIdx.x;
-    if (p >= npasses || threadIdx.x != 0) return;
-    unsigned long long run = 0;
-    for (int d = 0; d < BINS; ++d) {
-        starts[(size_t)p * BINS + d] = run;
-        run += hist[(size_t)p * BINS + d];
+// Up to RS_SMALL pairs: the whole LSD sort by one block in shared memory, in one
+// launch, 8-bit digits whatever the tuning says.  Ranks as k_rs_onesweep's; a
+// pass whose digit is the same in every key is skipped.
+// Bound: latency, about 2 us a pass; a memset, a histogram and one launch per
+// pass take about 5 us each at these sizes.
+constexpr int RSS_THREADS = 1024;
+constexpr int RSS_ITEMS = 8;
+constexpr int RSS_WARPS = RSS_THREADS / 32;
+constexpr uint32_t RS_SMALL = RSS_THREADS * RSS_ITEMS;
+template <typename K, typename V>
+struct rss_smem {
+    K sk[RS_SMALL];
+    V sv[RS_SMALL];
+    uint16_t wcnt[RSS_WARPS][RS_BINS];  // per-warp digit counts, then prefixes
+    uint32_t dstart[RS_BINS];
+    uint32_t sw[RSS_WARPS + 1];
+};
+template <typename K, typename V>
+__global__ void __launch_bounds__(RSS_THREADS) k_rs_small(K* __restrict__ keys, V* __restrict__ vals, uint32_t n,
+                                                          int begin_bit, int end_bit) {
+    extern __shared__ __align__(16) unsigned char rs_raw[];
+    rss_smem<K, V>& sm = *reinterpret_cast<rss_smem<K, V>*>(rs_raw);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t p0 = (uint32_t)warp * (RSS_ITEMS * 32) + lane;
+    K k[RSS_ITEMS];
+    V v[RSS_ITEMS];
+#pragma unroll
+    for (int r = 0; r < RSS_ITEMS; ++r) {
+        const uint32_t p = p0 + 32u * r;
+        k[r] = p < n ? keys[p] : ~K(0);
+        v[r] = p < n ? vals[p] : V(0);
     }
+    for (int shift = begin_bit; shift < end_bit; shift += RS_BITS) {
+        const uint32_t mask = end_bit - shift < RS_BITS ? (1u << (end_bit - shift)) - 1u : RS_BINS - 1u;
+        for (int i = threadIdx.x; i < RSS_WARPS * RS_BINS / 2; i += RSS_THREADS)
+            reinterpret_cast<uint32_t*>(&sm.wcnt[0][0])[i] = 0;
+        __syncthreads();
+        uint32_t rk[RSS_ITEMS];
+#pragma unroll
+        for (int r = 0; r < RSS_ITEMS; ++r) {
+            const bool ok = p0 + 32u * r < n;
+            const uint32_t d = ok ? (uint32_t)(k[r] >> shift) & mask : (uint32_t)RS_BINS;
+            const uint32_t peers = __match_any_sync(0xffffffffu, d);
+            const int leader = __ffs(peers) - 1;
+            uint32_t old = 0;
+            if (ok && lane == leader) {
+                old = sm.wcnt[warp][d];
+                sm.wcnt[warp][d] = (uint16_t)(old + __popc(peers));
+            }
+            rk[r] = __shfl_sync(0xffffffffu, old, leader) + __popc(peers & lanemask_lt());
+        }
+        __syncthreads();
+        uint32_t cnt = 0;
+        if (threadIdx.x < RS_BINS) {
+#pragma unroll 8
+            for (int w = 0; w < RSS_WARPS; ++w) {
+                const uint32_t c = sm.wcnt[w][threadIdx.x];
+                sm.wcnt[w][threadIdx.x] = (uint16_t)cnt;
+                cnt += c;
+            }
+        }
+        uint32_t tot;
+        const uint32_t ex = block_exclusive_scan<uint32_t, RSS_THREADS>(cnt, sm.sw, tot);
+        if (threadIdx.x < RS_BINS) sm.dstart[threadIdx.x] = ex;
+        if (__syncthreads_or(cnt == n)) continue;  // one digit for all
+#pragma unroll
+        for (int r = 0; r < RSS_ITEMS; ++r) {
+            if (p0 + 32u * r < n) {
+                const uint32_t d = (uint32_t)(k[r] >> shift) & mask;
+                const uint32_t at = sm.dstart[d] + sm.wcnt[warp][d] + rk[r];
+                sm.sk[at] = k[r];
+                sm.sv[at] = v[r];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int r = 0; r < RSS_ITEMS; ++r) {
+            const uint32_t p = p0 + 32u * r;
+            if (p < n) {
+                k[r] = sm.sk[p];
+                v[r] = sm.sv[p];
+            }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < RSS_ITEMS; ++r) {
+        const uint32_t p = p0 + 32u * r;
+        if (p < n) {
+            keys[p] = k[r];
+            vals[p] = v[r];
+        }
+    }
+}
+template <typename V, typename K>
+void radix_sort_small(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit, cudaStream_t st) {
+    CDBG_CUDA(cudaFuncSetAttribute(k_rs_small<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   (int)sizeof(rss_smem<K, V>)));
+    {
+        CDBG_PROF("k_rs_small", st);
+        k_rs_small<K, V><<<1, RSS_THREADS, sizeof(rss_smem<K, V>), st>>>(keys, vals, (uint32_t)n, begin_bit, end_bit);
+    }
+    CDBG_CHECK_LAUNCH();
 }
 
 // Histograms of all passes with BITS-bit digits, in one read.  hist is
@@ -403,6 +528,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_histograms_w(K const* __restr
     }
 }
 
+constexpr uint64_t RS_HOST_CHECK = 1ull << 20;
 template <int BITS, typename V, typename K>
 int radix_sort_pairs_w(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit, dev_arena& A,
                        cudaStream_t st, uint32_t* err) {
@@ -410,12 +536,19 @@ int radix_sort_pairs_w(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit,
     constexpr int ITEMS = 16;
     using S = rs_smem<BITS, ITEMS, K, V>;
     constexpr int TILE = S::TILE;
+    static_assert(TILE < (1 << 16), "a tile's counts are scanned in 16 bits");
     const int npasses = (end_bit - begin_bit + BITS - 1) / BITS;
     if (npasses > 15) throw std::runtime_error("radix sort: too many passes");
     auto m = A.mark();
-    unsigned long long* hist = A.alloc<unsigned long long>((size_t)npasses * BINS);
-    unsigned long long* starts = A.alloc<unsigned long long>((size_t)npasses * BINS);
-    CDBG_CUDA(cudaMemsetAsync(hist, 0, sizeof(unsigned long long) * npasses * BINS, st));
+    const uint64_t ntiles = ceil_div(n, (uint64_t)TILE);
+    K* k2 = A.alloc<K>(n);
+    V* v2 = A.alloc<V>(n);
+    // zeroed together: look-back status, histograms, tile counters
+    const size_t words = ntiles * BINS + (size_t)npasses * BINS + (npasses + 1) / 2;
+    unsigned long long* status = A.alloc<unsigned long long>(words);
+    unsigned long long* hist = status + ntiles * BINS;
+    uint32_t* counters = reinterpret_cast<uint32_t*>(hist + (size_t)npasses * BINS);
+    CDBG_CUDA(cudaMemsetAsync(status, 0, 8 * words, st));
     {
         uint64_t blocks = ceil_div(n, (uint64_t)RS_THREADS * 16);
         if (blocks > 148 * 8) blocks = 148 * 8;
@@ -428,19 +561,15 @@ int radix_sort_pairs_w(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit,
             k_rs_histograms_w<BITS, K><<<(unsigned)blocks, RS_THREADS, hs, st>>>(keys, n, begin_bit, npasses, hist);
         }
         CDBG_CHECK_LAUNCH();
-        k_rs_digit_starts<BITS><<<npasses, 32, 0, st>>>(hist, npasses, starts);
-        CDBG_CHECK_LAUNCH();
     }
-    std::vector<unsigned long long> h((size_t)npasses * BINS);
-    read_small(h.data(), hist, h.size() * 8, st);
-
-    const uint64_t ntiles = ceil_div(n, (uint64_t)TILE);
-    K* k2 = A.alloc<K>(n);
-    V* v2 = A.alloc<V>(n);
-    unsigned long long* status = A.alloc<unsigned long long>(ntiles * BINS);
-    uint32_t* counters = A.alloc<uint32_t>(npasses);
-    CDBG_CUDA(cudaMemsetAsync(status, 0, sizeof(unsigned long long) * ntiles * BINS, st));
-    CDBG_CUDA(cudaMemsetAsync(counters, 0, sizeof(uint32_t) * npasses, st));
+    // A pass whose digit is the same in every key is skipped, which needs the
+    // histograms on the host.  Below RS_HOST_CHECK pairs a pass costs no more
+    // than that wait (about 10 us), and every pass runs.
+    std::vector<unsigned long long> h;
+    if (n >= RS_HOST_CHECK) {
+        h.resize((size_t)npasses * BINS);
+        read_small(h.data(), hist, h.size() * 8, st);
+    }
     CDBG_CUDA(cudaFuncSetAttribute(k_rs_onesweep<BITS, ITEMS, K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)sizeof(S)));
     K *kin = keys, *kout = k2;
@@ -448,7 +577,7 @@ int radix_sort_pairs_w(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit,
     int ran = 0;
     for (int p = 0; p < npasses; ++p) {
         bool trivial = false;
-        for (int d = 0; d < BINS; ++d)
+        for (int d = 0; d < BINS && !h.empty(); ++d)
             if (h[(size_t)p * BINS + d] == n) trivial = true;
         if (trivial) continue;
         const int shift = begin_bit + p * BITS;
@@ -456,7 +585,7 @@ int radix_sort_pairs_w(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit,
             // one read and one write of every (key, value) pair
             CDBG_PROF_BYTES("k_rs_onesweep", st, 2.0 * n * (sizeof(K) + sizeof(V)));
             k_rs_onesweep<BITS, ITEMS, K, V><<<(unsigned)ntiles, RS_THREADS, sizeof(S), st>>>(
-                kin, vin, kout, vout, n, shift, counters + p, status, starts + (size_t)p * BINS, (uint32_t)(p + 1),
+                kin, vin, kout, vout, n, shift, counters + p, status, hist + (size_t)p * BINS, (uint32_t)(p + 1),
                 err);
         }
         CDBG_CHECK_LAUNCH();
@@ -476,14 +605,17 @@ int radix_sort_pairs_w(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit,
 // 11-bit digits (g_radix_bits: the engine's tuning; 11 bits take 3 passes
 // where 8 bits take 4, with 8x the counters and look-back state per tile).
 // Results end in (keys, vals); the arena provides the ping-pong buffers.
-// Needs a host synchronize (to read the digit histograms); returns the number
-// of passes run.  A look-back that gives up sets *err.
+// Returns the number of passes run.  A look-back that gives up sets *err.
 template <typename V, typename K = uint64_t>
 int radix_sort_pairs(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit, dev_arena& A, cudaStream_t st,
                      uint32_t* err) {
     static_assert(sizeof(K) == 4 || sizeof(K) == 8, "u32 or u64 keys");
     if (end_bit > 8 * (int)sizeof(K)) end_bit = 8 * (int)sizeof(K);
     if (n <= 1 || end_bit <= begin_bit) return 0;
+    if (n <= RS_SMALL) {
+        radix_sort_small<V, K>(keys, vals, n, begin_bit, end_bit, st);
+        return 1;
+    }
     if (g_radix_bits == 11) return radix_sort_pairs_w<11, V, K>(keys, vals, n, begin_bit, end_bit, A, st, err);
     return radix_sort_pairs_w<RS_BITS, V, K>(keys, vals, n, begin_bit, end_bit, A, st, err);
 }
@@ -602,6 +734,10 @@ template <typename V>
 void sort_pairs_u64_exact(uint64_t* keys, V* vals, uint64_t n, dev_arena& A, cudaStream_t st, uint32_t* err) {
     if (n <= 1) return;
     if (n >= (1ull << 32)) throw std::runtime_error("sort_pairs_u64_exact: n >= 2^32");
+    if (n <= RS_SMALL) {  // all 64 bits in the one launch
+        radix_sort_small<V, uint64_t>(keys, vals, n, 0, 64, st);
+        return;
+    }
     radix_sort_pairs<V, uint64_t>(keys, vals, n, 32, 64, A, st, err);
     auto m = A.mark();
     const uint64_t cap = n / 8 + 1024;
