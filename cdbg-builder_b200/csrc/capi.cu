@@ -513,7 +513,7 @@ int cdbg_gpu_dump_supers(cdbg_engine* e, const cdbg_seq_batch* b, uint32_t k, ui
         apply_limit(e);
         cdbg::seq_input in = stage_batch(e, b, nullptr);
         cdbg::run_table rt;
-        cdbg::build_runs(in, k, e->A, e->st, rt, e->A);
+        cdbg::build_runs(in, k, e->A, e->st, rt, e->A, e->tune.minimizer_tile);
         cdbg::super_list sl;
         cdbg::find_supers(rt, k, m, num_buckets, e->A, e->st, sl, e->d_err, e->tune.minimizer_tile);
         cdbg::check_device_error(e, "super-k-mers");
@@ -637,7 +637,7 @@ int cdbg_gpu_phase1(cdbg_engine* e, const cdbg_phase1_args* a, cdbg_phase1_stats
                 cdbg_seq_batch b{hb.seq.data(), hb.seq.size(), hb.off.data(), hb.color.data(),
                                  (uint32_t)hb.color.size(), 0};
                 cdbg::seq_input in = stage_batch(e, &b, nullptr);
-                cdbg::build_runs(in, k, e->A, e->st, rt, e->P);
+                cdbg::build_runs(in, k, e->A, e->st, rt, e->P, e->tune.minimizer_tile);
                 cdbg::find_supers(rt, k, m, a->num_buckets, e->A, e->st, sl, e->d_err, e->tune.minimizer_tile,
                                   packed);
                 CDBG_CUDA(cudaStreamSynchronize(e->st));
@@ -930,7 +930,7 @@ void phase1_pipelined(cdbg_engine* e, cdbg_seq_batch const* b, uint32_t k, uint3
         in.seq_color = d_color + cut[i];
         in.num_seqs = ns;
         cdbg::run_table rt;
-        cdbg::build_runs(in, k, e->A, st, rt, e->P, words, base, cap);
+        cdbg::build_runs(in, k, e->A, st, rt, e->P, e->tune.minimizer_tile, words, base, cap);
         if (rt.n == 0) continue;
         base = rt.nwords - 8;
         n_kmers += rt.n_kmers;
@@ -1064,7 +1064,7 @@ bool phase1_device_reader(cdbg_engine* e, std::vector<std::string> const& files,
     const uint64_t cap = tot_out / 32 + tot_out / std::max<uint32_t>(k, 1) + 128;
     uint64_t* words = e->P.alloc<uint64_t>(cap);
     cdbg::run_table rt;
-    cdbg::build_runs(in, k, e->A, st, rt, e->P, words, 0, cap);
+    cdbg::build_runs(in, k, e->A, st, rt, e->P, e->tune.minimizer_tile, words, 0, cap);
     if (rt.n == 0) {  // nothing to build from: the host reader's path handles it
         e->A.release(ma);
         e->P.release(mp);
@@ -1194,7 +1194,7 @@ bool phase1_from_files(cdbg_engine* e, std::vector<std::string> const& files, ui
         in.seq_color = d_col;
         in.num_seqs = ns;
         cdbg::run_table rt;
-        cdbg::build_runs(in, k, e->A, st, rt, e->P, words, base, cap);
+        cdbg::build_runs(in, k, e->A, st, rt, e->P, e->tune.minimizer_tile, words, base, cap);
         if (rt.n == 0) continue;
         base = rt.nwords - 8;
         n_kmers += rt.n_kmers;
@@ -1295,7 +1295,6 @@ int build_core(cdbg_engine* e, const cdbg_build_params* p, phase1_fn const& phas
         cdbg::build_records(rt, sl, k, p->num_buckets, e->A, e->st, rs, e->d_err, e->P);
         e->last_rs = rs;  // for cdbg_engine_record_bytes (lives in P until the next call)
         e->have_rs = true;
-        cdbg::check_device_error(e, "phase 1");
         const uint64_t n_kmers = rt.n_kmers, n_supers = sl.n, n_bases = rt.n_bases;
         e->A.reset();  // phase-1 scratch (staged input, super-k-mers, sort buffers)
         CDBG_CUDA(cudaEventRecord(ev[1], e->st));
@@ -1419,7 +1418,7 @@ int cdbg_gpu_build(cdbg_engine* e, const cdbg_seq_batch* b, const cdbg_build_par
             phase1_pipelined(e, b, k, m, p->num_buckets, 4, rt, sl, h2d);
         } else {
             cdbg::seq_input in = stage_batch(e, b, h2d);
-            cdbg::build_runs(in, k, e->A, e->st, rt, e->P);
+            cdbg::build_runs(in, k, e->A, e->st, rt, e->P, e->tune.minimizer_tile);
             cdbg::find_supers(rt, k, m, p->num_buckets, e->A, e->st, sl, e->d_err, e->tune.minimizer_tile, packed);
         }
         return true;

@@ -195,62 +195,121 @@ __global__ void __launch_bounds__(EV_THREADS)
     ev_write(E, St, p0, s_excl + ex, cap, events);
 }
 
-// Pair events into runs; keep[i] = len >= k.
+// Pair events into runs.  size[i] = (1 << 32) + stream words of a run of at
+// least k bases, tiles[i] its minimizer tiles of tt (k-1)-mers, both 0 for a
+// shorter one; acc[0..1] += k-mers and bases of the runs kept.
 __global__ void k_runs_from_events(uint64_t const* __restrict__ ev, uint64_t nruns,
                                    uint64_t const* __restrict__ seq_off, uint32_t num_seqs,
-                                   uint32_t const* __restrict__ seq_color, uint32_t k,
+                                   uint32_t const* __restrict__ seq_color, uint32_t k, uint32_t tt,
                                    uint64_t* __restrict__ src, uint32_t* __restrict__ len,
-                                   uint32_t* __restrict__ color, uint32_t* __restrict__ keep,
-                                   uint32_t* err) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nruns) return;
-    const uint64_t a = ev[2 * i] >> 1, b = ev[2 * i + 1] >> 1;
-    const uint64_t l = b - a;
-    if (l >= 0xffffffffull) set_error(err, ERR_FIELD_OVERFLOW);
-    src[i] = a;
-    len[i] = (uint32_t)l;
-    uint32_t s = upper_bound_u64(seq_off, num_seqs + 1, a) - 1;
-    color[i] = seq_color[s];
-    keep[i] = l >= k ? 1u : 0u;
+                                   uint32_t* __restrict__ color, uint64_t* __restrict__ size,
+                                   uint64_t* __restrict__ tiles, unsigned long long* __restrict__ acc, uint32_t* err) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned long long kmers = 0, bases = 0;
+    if (i < nruns) {
+        const uint64_t a = ev[2 * i] >> 1, b = ev[2 * i + 1] >> 1;
+        const uint64_t l = b - a;
+        if (l >= 0xffffffffull) set_error(err, ERR_FIELD_OVERFLOW);
+        src[i] = a;
+        len[i] = (uint32_t)l;
+        const uint32_t s = upper_bound_u64(seq_off, num_seqs + 1, a) - 1;
+        color[i] = seq_color[s];
+        const bool keep = l >= k;
+        size[i] = keep ? (1ull << 32) + (l + 31) / 32 : 0;
+        tiles[i] = keep ? (l - k + 2 + tt - 1) / tt : 0;
+        kmers = keep ? l - k + 1 : 0;
+        bases = keep ? l : 0;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+        kmers += __shfl_down_sync(0xffffffffu, kmers, o);
+        bases += __shfl_down_sync(0xffffffffu, bases, o);
+    }
+    if ((threadIdx.x & 31) == 0 && bases) {
+        atomicAdd(acc, kmers);
+        atomicAdd(acc + 1, bases);
+    }
 }
 
-__global__ void k_runs_compact(uint64_t nruns, uint32_t const* __restrict__ keep,
-                               uint64_t const* __restrict__ kpos, uint64_t const* __restrict__ src,
-                               uint32_t const* __restrict__ len, uint32_t const* __restrict__ color,
+// Runs of at least k bases in order: pos[i] and tpos[i] are the exclusive sums of
+// size and tiles (their totals at nruns).  Stream offsets start at word `base`.
+__global__ void k_runs_compact(uint64_t nruns, uint64_t const* __restrict__ size, uint64_t const* __restrict__ pos,
+                               uint64_t const* __restrict__ tpos, uint64_t const* __restrict__ src,
+                               uint32_t const* __restrict__ len, uint32_t const* __restrict__ color, uint64_t base,
                                uint64_t* __restrict__ osrc, uint32_t* __restrict__ olen,
-                               uint32_t* __restrict__ ocolor, uint64_t* __restrict__ padded) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nruns || !keep[i]) return;
-    const uint64_t o = kpos[i];
+                               uint32_t* __restrict__ ocolor, uint64_t* __restrict__ soff,
+                               uint64_t* __restrict__ tstart) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i > nruns || (i < nruns && !size[i])) return;
+    const uint64_t o = pos[i] >> 32;
+    soff[o] = ((pos[i] & 0xffffffffu) + base) * 32;
+    tstart[o] = tpos[i];
+    if (i == nruns) return;
     osrc[o] = src[i];
     olen[o] = len[i];
     ocolor[o] = color[i];
-    padded[o] = ((uint64_t)len[i] + 31) & ~uint64_t(31);
 }
 
-// One 64-bit stream word per thread.
-__global__ void k_pack(uint8_t const* __restrict__ ascii, uint32_t nruns,
-                       uint64_t const* __restrict__ soff, uint64_t const* __restrict__ src,
-                       uint32_t const* __restrict__ len, uint64_t nwords_data,
-                       uint64_t* __restrict__ words) {
-    uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= nwords_data) return;
-    const uint64_t pos = w * 32;
-    const uint32_t r = upper_bound_u64(soff, nruns, pos) - 1;
+// 2-bit codes of four ACGT bytes (either case), byte i at bits 2i: bits 1-2 of
+// A, C, G, T are 0, 1, 3, 2.
+__device__ __forceinline__ uint32_t pack4(uint32_t w) {
+    uint32_t x = (w >> 1) & 0x03030303u;
+    x ^= (x >> 1) & 0x01010101u;
+    return (x | (x >> 6) | (x >> 12) | (x >> 18)) & 0xffu;
+}
+
+// One 64-bit stream word (32 bases) per thread.  soff is in bases from word
+// `base` on.  The words of a warp mostly belong to one run: its first active lane
+// searches, the others take its run or search themselves.  The 32 bytes come from
+// three aligned 16-byte loads where those lie inside the input.
+// Bound: HBM.  One search and 32 byte loads per word took 1.04 ms for 0.97 Gbases
+// (1.2 TB/s), this 0.44 ms (2.8 TB/s).
+__global__ void k_pack(uint8_t const* __restrict__ ascii, uint64_t nbytes, uint32_t nruns,
+                       uint64_t const* __restrict__ soff, uint64_t base, uint64_t const* __restrict__ src,
+                       uint32_t const* __restrict__ len, uint64_t nwords_data, uint64_t* __restrict__ words) {
+    const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    const bool on = w < nwords_data;
+    const uint64_t pos = (w + base) * 32;
+    const uint32_t am = __ballot_sync(0xffffffffu, on);
+    if (!on) return;
+    const int leader = __ffs(am) - 1;
+    uint32_t r = 0;
+    if ((int)(threadIdx.x & 31) == leader) r = upper_bound_u64(soff, nruns, pos) - 1;
+    r = __shfl_sync(am, r, leader);
+    if (soff[r + 1] <= pos) r = upper_bound_u64(soff, nruns, pos) - 1;
     const uint64_t j = pos - soff[r];
     const uint32_t L = len[r];
     uint64_t out = 0;
     if (j < L) {
         const uint32_t n = (L - j) < 32 ? (uint32_t)(L - j) : 32u;
-        uint8_t const* p = ascii + src[r] + j;
-        for (uint32_t i = 0; i < n; ++i) out |= (uint64_t)(nuc_code(p[i]) & 3u) << (2 * i);
+        const uint64_t a = src[r] + j;
+        const uint64_t a16 = a & ~uint64_t(15);
+        if (a16 + 48 <= nbytes && ((reinterpret_cast<uintptr_t>(ascii) & 15) == 0)) {
+            uint4 const* q = reinterpret_cast<uint4 const*>(ascii + a16);
+            const uint4 x = __ldg(q), y = __ldg(q + 1), z = __ldg(q + 2);
+            const uint32_t v[12] = {x.x, x.y, x.z, x.w, y.x, y.y, y.z, y.w, z.x, z.y, z.z, z.w};
+            // codes of all 48 bytes, then the 32 bases from byte a - a16 on
+            uint64_t lo = 0;
+            uint32_t hi = 0;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) lo |= (uint64_t)pack4(v[i]) << (8 * i);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) hi |= pack4(v[8 + i]) << (8 * i);
+            const uint32_t s = 2 * (uint32_t)(a - a16);
+            out = s ? (lo >> s) | ((uint64_t)hi << (64 - s)) : lo;
+            if (n < 32) out &= (uint64_t(1) << (2 * n)) - 1;
+        } else {
+            uint8_t const* p = ascii + a;
+            for (uint32_t i = 0; i < n; ++i) out |= (uint64_t)(nuc_code(p[i]) & 3u) << (2 * i);
+        }
     }
     words[w] = out;
 }
 
 // ------------------------------------------------------------ minimizer tile
 constexpr int MZ_THREADS = 256;
-constexpr int MZ_TT = 2048;  // default (k-1)-mers per tile
+constexpr int MZ_TT = 2048;
+constexpr uint32_t MZ_DEFAULT_TILE = 4096;  // (k-1)-mers per tile when the caller says 0
 
 __device__ __forceinline__ uint32_t smem_u32(void const* p) {
     return (uint32_t)__cvta_generic_to_shared(p);
@@ -691,32 +750,6 @@ size_t mz_smem() {
     return b;
 }
 
-__global__ void k_run_tiles(uint32_t nruns, uint32_t const* __restrict__ len, uint32_t k, uint32_t tt,
-                            uint64_t* __restrict__ ntiles) {
-    uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= nruns) return;
-    const uint64_t nk1 = (uint64_t)len[r] - k + 2;
-    ntiles[r] = (nk1 + tt - 1) / tt;
-}
-
-__global__ void k_run_kmers(uint32_t nruns, uint32_t const* __restrict__ len, uint32_t k,
-                            unsigned long long* __restrict__ acc) {
-    uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long v = 0, b = 0;
-    if (r < nruns) {
-        v = (unsigned long long)len[r] - k + 1;
-        b = len[r];
-    }
-    for (int o = 16; o; o >>= 1) {
-        v += __shfl_down_sync(0xffffffffu, v, o);
-        b += __shfl_down_sync(0xffffffffu, b, o);
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicAdd(acc, v);
-        atomicAdd(acc + 1, b);
-    }
-}
-
 // Super-k-mer fields from the cut list (bucket_ingester.hpp:80-126).
 struct super_fields {
     uint64_t start, key;
@@ -801,102 +834,164 @@ __device__ __forceinline__ bool same_bases(uint64_t const* __restrict__ words, u
     return true;
 }
 
-// Super-k-mer fields in key order (one gather per field), so the grouping and
-// record passes below read them sequentially.
-__global__ void k_permute_supers(uint64_t n, uint32_t const* __restrict__ idx, uint64_t const* __restrict__ start,
-                                 uint32_t const* __restrict__ len, uint32_t const* __restrict__ color,
-                                 uint32_t const* __restrict__ flags, uint64_t* __restrict__ p_start,
-                                 uint32_t* __restrict__ p_len, uint32_t* __restrict__ p_color,
-                                 uint32_t* __restrict__ p_flags) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const uint32_t i = idx[p];
-    p_start[p] = start[i];
-    p_len[p] = len[i];
-    p_color[p] = color[i];
-    p_flags[p] = flags[i];
-}
-
-__global__ void k_permute_packed(uint64_t n, uint32_t const* __restrict__ idx, uint4 const* __restrict__ packed,
-                                 uint64_t* __restrict__ p_start, uint32_t* __restrict__ p_len,
-                                 uint32_t* __restrict__ p_color, uint32_t* __restrict__ p_flags) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const uint4 v = packed[idx[p]];
-    p_start[p] = ((uint64_t)v.y << 32) | v.x;
-    p_len[p] = v.z;
-    p_color[p] = v.w >> 4;
-    p_flags[p] = v.w & 0xfu;
-}
-
-// head[p]: position p starts a new record (key, length or bases differ from
-// p - 1); ckeep[p]: p adds a color to its record (the first of each color).
-__global__ void k_group_heads_sorted(uint64_t n, uint64_t const* __restrict__ key,
-                                     uint64_t const* __restrict__ start, uint32_t const* __restrict__ len,
-                                     uint32_t const* __restrict__ color, uint64_t const* __restrict__ words,
-                                     uint32_t* __restrict__ head, uint32_t* __restrict__ ckeep) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    bool h = true;
-    if (p > 0) {
-        h = !(key[p] == key[p - 1] && len[p] == len[p - 1] && same_bases(words, start[p], start[p - 1], len[p]));
-        ckeep[p] = (h || color[p] != color[p - 1]) ? 1u : 0u;
+// Super-k-mers in input order as k_records gathers them: packed (16 bytes, one
+// sector each), or one array per field (colors of 2^28 and more).
+struct super_fields_view {
+    uint4 const* packed;
+    uint64_t const* start;
+    uint32_t const* len;
+    uint32_t const* color;
+    uint32_t const* flags;
+};
+__device__ __forceinline__ void super_get(super_fields_view const& v, uint32_t i, uint64_t& start, uint32_t& len,
+                                          uint32_t& color, uint32_t& flags) {
+    if (v.packed) {
+        const uint4 x = __ldg(v.packed + i);
+        start = ((uint64_t)x.y << 32) | x.x;
+        len = x.z;
+        color = x.w >> 4;
+        flags = x.w & 0xfu;
     } else {
-        ckeep[p] = 1u;
+        start = v.start[i];
+        len = v.len[i];
+        color = v.color[i];
+        flags = v.flags[i];
     }
-    head[p] = h ? 1u : 0u;
 }
 
-__global__ void k_records_fill_sorted(uint64_t n, uint32_t const* __restrict__ head,
-                                      uint64_t const* __restrict__ rid_ex, uint32_t const* __restrict__ ckeep,
-                                      uint64_t const* __restrict__ cpos, uint64_t const* __restrict__ key,
-                                      uint32_t bb, uint64_t const* __restrict__ start,
-                                      uint32_t const* __restrict__ len, uint32_t const* __restrict__ color,
-                                      uint32_t const* __restrict__ flags, uint64_t* __restrict__ r_start,
-                                      uint32_t* __restrict__ r_len, uint32_t* __restrict__ r_flags,
-                                      uint64_t* __restrict__ r_coloff, uint32_t* __restrict__ colors,
-                                      uint32_t* __restrict__ r_bucket) {
-    uint64_t p = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const uint64_t rid = rid_ex[p] + head[p] - 1;  // inclusive count - 1
-    if (head[p]) {
-        r_start[rid] = start[p];
-        r_len[rid] = len[p];
-        r_coloff[rid] = cpos[p];
-        r_bucket[rid] = bb ? (uint32_t)(key[p] >> (64 - bb)) : 0u;
+// Records from the super-k-mers in key order, in one pass: position p starts a
+// record when its key, length or bases differ from p - 1's, and adds a color
+// when it starts a record or its color differs from p - 1's (colors ascend
+// within a record); both outputs take their offsets from a decoupled look-back
+// over tiles of RC_ROUNDS x 256 positions.  A record's flags are the AND over its
+// copies: ANDed within a warp first, one atomic per record and warp (r_flags
+// starts all ones).  A record that starts a bucket fills the starts of the empty
+// buckets before it.  tot[0..1] = records, colors.
+// Bound: the random 16-byte gather.  A gather into key order, a grouping pass,
+// two scans and a fill pass took 6.9 ms of a 200-genome build (1.0e8
+// super-k-mers), this 4.8.
+constexpr int RC_ROUNDS = 4;
+__global__ void __launch_bounds__(256)
+    k_records(uint64_t n, uint64_t ntiles, uint32_t const* __restrict__ idx, uint64_t const* __restrict__ key,
+              super_fields_view sv, uint64_t const* __restrict__ words, uint32_t bb, uint32_t B,
+              uint32_t* tile_counter, unsigned long long* status_r, unsigned long long* status_c,
+              uint64_t* __restrict__ r_start, uint32_t* __restrict__ r_len, uint32_t* r_flags,
+              uint64_t* __restrict__ r_coloff, uint32_t* __restrict__ colors, uint64_t* __restrict__ bucket_start,
+              unsigned long long* __restrict__ tot, uint32_t* err) {
+    constexpr int NW = 256 / 32, TILE = RC_ROUNDS * 256;
+    static_assert(RC_ROUNDS * NW == 32, "warp 0 scans one count per lane");
+    // position base + j of the tile at j + 1, its predecessor at 0
+    __shared__ uint64_t s_key[TILE + 1], s_start[TILE + 1];
+    __shared__ uint32_t s_len[TILE + 1], s_color[TILE + 1];
+    __shared__ uint32_t whead[RC_ROUNDS * NW], wcol[RC_ROUNDS * NW], wcnt[RC_ROUNDS * NW];
+    __shared__ uint64_t s_tile, s_r, s_c;
+    if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1u);
+    __syncthreads();
+    const uint64_t tile = s_tile, base = tile * TILE;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t kk[RC_ROUNDS], start[RC_ROUNDS];
+    uint32_t len[RC_ROUNDS], color[RC_ROUNDS], flags[RC_ROUNDS];
+#pragma unroll
+    for (int rr = 0; rr < RC_ROUNDS; ++rr) {
+        const uint64_t p = base + 256u * rr + threadIdx.x;
+        flags[rr] = 0xfu;
+        if (p < n) {
+            kk[rr] = key[p];
+            super_get(sv, idx[p], start[rr], len[rr], color[rr], flags[rr]);
+            const uint32_t j = 256u * rr + threadIdx.x + 1;
+            s_key[j] = kk[rr];
+            s_start[j] = start[rr];
+            s_len[j] = len[rr];
+            s_color[j] = color[rr];
+        }
     }
-    const uint32_t f = flags[p];
-    if (f != 0xfu) atomicAnd(&r_flags[rid], f);  // AND over the record's copies (starts at 0xf)
-    if (ckeep[p]) colors[cpos[p]] = color[p];
+    if (threadIdx.x == 0 && base > 0) {
+        uint64_t st;
+        uint32_t l, c, f;
+        super_get(sv, idx[base - 1], st, l, c, f);
+        s_key[0] = key[base - 1];
+        s_start[0] = st;
+        s_len[0] = l;
+        s_color[0] = c;
+    }
+    __syncthreads();
+    uint32_t head = 0, ckeep = 0;
+#pragma unroll
+    for (int rr = 0; rr < RC_ROUNDS; ++rr) {
+        const uint64_t p = base + 256u * rr + threadIdx.x;
+        bool h = false, c = false;
+        if (p < n) {
+            const uint32_t j = 256u * rr + threadIdx.x;
+            h = p == 0 || !(kk[rr] == s_key[j] && len[rr] == s_len[j] &&
+                            same_bases(words, start[rr], s_start[j], len[rr]));
+            c = h || color[rr] != s_color[j];
+        }
+        const uint32_t bh = __ballot_sync(0xffffffffu, h), bc = __ballot_sync(0xffffffffu, c);
+        head |= (uint32_t)h << rr;
+        ckeep |= (uint32_t)c << rr;
+        if (lane == 0) {
+            whead[rr * NW + warp] = bh;
+            wcol[rr * NW + warp] = bc;
+            wcnt[rr * NW + warp] = __popc(bh) | (__popc(bc) << 16);
+        }
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t c = wcnt[lane];
+        const uint32_t x = prim::warp_inclusive_scan(c);
+        const uint32_t t = __shfl_sync(0xffffffffu, x, 31);
+        wcnt[lane] = x - c;
+        uint64_t er = 0, ec = 0;
+        const bool ok_r = prim::lookback_exclusive(status_r, tile, t & 0xffffu, er);
+        const bool ok_c = prim::lookback_exclusive(status_c, tile, t >> 16, ec);
+        if (lane == 0) {
+            if (!ok_r || !ok_c) set_error(err, ERR_CHAIN_LIMIT);
+            s_r = er;
+            s_c = ec;
+            if (tile == ntiles - 1) {
+                tot[0] = er + (t & 0xffffu);
+                tot[1] = ec + (t >> 16);
+            }
+        }
+    }
+    __syncthreads();
+    const uint64_t r0 = s_r, c0 = s_c;
+    const uint32_t lt = lanemask_lt();
+#pragma unroll
+    for (int rr = 0; rr < RC_ROUNDS; ++rr) {
+        const uint64_t p = base + 256u * rr + threadIdx.x;
+        const uint32_t i = rr * NW + warp, j = 256u * rr + threadIdx.x;
+        const bool h = (head >> rr) & 1u, c = (ckeep >> rr) & 1u;
+        // the record holding p (its heads up to and including p, less one)
+        const uint64_t rid = r0 + (wcnt[i] & 0xffffu) + __popc(whead[i] & lt) + (h ? 1 : 0) - 1;
+        const uint64_t cat = c0 + (wcnt[i] >> 16) + __popc(wcol[i] & lt);
+        if (h) {
+            r_start[rid] = start[rr];
+            r_len[rid] = len[rr];
+            r_coloff[rid] = cat;
+            const uint32_t b = bb ? (uint32_t)(kk[rr] >> (64 - bb)) : 0u;
+            const uint32_t from = p == 0 ? 0u : (bb ? (uint32_t)(s_key[j] >> (64 - bb)) : 0u) + 1;
+            for (uint32_t x = from; x <= b; ++x) bucket_start[x] = rid;
+        }
+        if (c) colors[cat] = color[rr];
+        // flags: AND over the lanes of the same record, by the first of them.
+        // The lanes of a record are those up to the next head.
+        const uint32_t after = whead[i] & ~(lt | (1u << lane));  // heads after this lane
+        const int last = after ? __ffs(after) - 2 : 31;          // last lane of this lane's record
+        uint32_t f = flags[rr];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t of = __shfl_down_sync(0xffffffffu, f, o);
+            if (lane + o <= last) f &= of;
+        }
+        if (p < n && (h || lane == 0) && f != 0xfu) atomicAnd(&r_flags[rid], f);
+        if (p == n - 1) {
+            r_coloff[rid + 1] = cat + (c ? 1 : 0);
+            for (uint32_t x = (bb ? (uint32_t)(kk[rr] >> (64 - bb)) : 0u) + 1; x <= B; ++x) bucket_start[x] = rid + 1;
+        }
+    }
 }
 
-// bucket_start[b] = first record of bucket b (records are in bucket order):
-// each record that starts a bucket fills the starts of the empty buckets
-// before it; the last record fills the rest with n.
-__global__ void k_bucket_bounds(uint64_t n, uint32_t const* __restrict__ rb, uint32_t B,
-                                uint64_t* __restrict__ bucket_start) {
-    uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n) return;
-    const uint32_t b = rb[r];
-    const uint32_t prev = r ? rb[r - 1] + 1 : 0;
-    for (uint32_t x = prev; x <= b; ++x) bucket_start[x] = r;
-    if (r == n - 1)
-        for (uint32_t x = b + 1; x <= B; ++x) bucket_start[x] = n;
-}
-
-__global__ void k_add_u64(uint64_t* p, uint64_t n, uint64_t v) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] += v;
-}
-
-__global__ void k_fill_u32(uint32_t* p, uint64_t n, uint32_t v) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = v;
-}
-__global__ void k_iota_u32(uint32_t* p, uint64_t n) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = (uint32_t)i;
-}
 __global__ void k_set_last_u64(uint64_t* p, uint64_t idx, uint64_t const* v) { p[idx] = *v; }
 
 // ------------------------------------------------------------ serialization
@@ -1048,45 +1143,41 @@ T read_dev(T const* p, cudaStream_t st) {
 
 // ----------------------------------------------------------------- host side
 void build_runs(seq_input const& in, uint32_t k, dev_arena& A, cudaStream_t st, run_table& rt,
-                dev_arena& out, uint64_t* words_out, uint64_t word_base, uint64_t words_cap) {
+                dev_arena& out, uint32_t tile, uint64_t* words_out, uint64_t word_base, uint64_t words_cap) {
     rt = run_table();
+    rt.tile = tile ? tile : MZ_DEFAULT_TILE;
     const uint64_t npos = in.nbytes + 1;
     const uint64_t tiles = ceil_div(npos, EV_TILE);
-    uint32_t* tcount = A.alloc<uint32_t>(tiles);
-    uint64_t* toff = A.alloc<uint64_t>(tiles + 1);
-    // bit p of `starts`: a sequence starts at p (or p = nbytes)
-    const uint64_t nsw = (in.nbytes >> 5) + 2;
-    uint32_t* starts = A.alloc<uint32_t>(nsw);
-    CDBG_CUDA(cudaMemsetAsync(starts, 0, 4 * nsw, st));
+    // zeroed together: sequence-start bitmap (bit p: a sequence starts at p, or p
+    // = nbytes), look-back status, tile counter, and the counts the host reads
+    const uint64_t nsw = ((in.nbytes >> 5) + 2 + 1) / 2;  // in 8-byte words
+    enum { C_EVENTS, C_RUNS, C_TILES, C_KMERS, C_BASES, C_ERR, C_COUNTER, NCOUNTS };
+    unsigned long long* zero = A.alloc<unsigned long long>(NCOUNTS + tiles + nsw);
+    unsigned long long* counts = zero;
+    unsigned long long* status = zero + NCOUNTS;
+    uint32_t* starts = reinterpret_cast<uint32_t*>(status + tiles);
+    uint32_t* err = reinterpret_cast<uint32_t*>(counts + C_ERR);
+    CDBG_CUDA(cudaMemsetAsync(zero, 0, 8 * (NCOUNTS + tiles + nsw), st));
     k_seq_starts<<<grid((uint64_t)in.num_seqs + 1, 256), 256, 0, st>>>(in.seq_off, in.num_seqs, starts);
     CDBG_CHECK_LAUNCH();
     // one pass into room for a run every 64 bases (two events each); input
     // with more runs than that takes the two passes
-    uint64_t ev_cap = in.nbytes / 32 + 1024;
+    const uint64_t ev_cap = in.nbytes / 32 + 1024;
     uint64_t* ev = A.alloc<uint64_t>(ev_cap);
-    uint64_t nev = 0;
     {
-        uint32_t* counter = A.alloc<uint32_t>(1);
-        unsigned long long* status = A.alloc<unsigned long long>(tiles);
-        unsigned long long* total = A.alloc<unsigned long long>(1);
-        uint32_t* lerr = A.alloc<uint32_t>(1);
-        CDBG_CUDA(cudaMemsetAsync(counter, 0, 4, st));
-        CDBG_CUDA(cudaMemsetAsync(status, 0, 8 * tiles, st));
-        CDBG_CUDA(cudaMemsetAsync(lerr, 0, 4, st));
-        {
-            CDBG_PROF("k_run_events", st);
-            k_run_events_1p<<<(unsigned)tiles, EV_THREADS, 0, st>>>(in.ascii, in.nbytes, starts, tiles, counter,
-                                                                   status, ev, ev_cap, total, lerr);
-        }
-        CDBG_CHECK_LAUNCH();
-        uint64_t got[2] = {0, 0};
-        read_small(&got[0], total, 8, st);
-        uint32_t le = 0;
-        read_small(&le, lerr, 4, st);
-        if (le) throw std::runtime_error("run events: look-back wait limit reached");
-        nev = got[0];
+        CDBG_PROF("k_run_events", st);
+        k_run_events_1p<<<(unsigned)tiles, EV_THREADS, 0, st>>>(in.ascii, in.nbytes, starts, tiles,
+                                                               reinterpret_cast<uint32_t*>(counts + C_COUNTER), status,
+                                                               ev, ev_cap, counts + C_EVENTS, err);
     }
+    CDBG_CHECK_LAUNCH();
+    uint64_t h[NCOUNTS];
+    read_small(h, counts, sizeof(h), st);
+    if ((uint32_t)h[C_ERR]) throw std::runtime_error("run events: look-back wait limit reached");
+    uint64_t nev = h[C_EVENTS];
     if (nev > ev_cap) {
+        uint32_t* tcount = A.alloc<uint32_t>(tiles);
+        uint64_t* toff = A.alloc<uint64_t>(tiles + 1);
         {
             CDBG_PROF("k_run_events", st);
             k_run_events<false><<<(unsigned)tiles, EV_THREADS, 0, st>>>(in.ascii, in.nbytes, starts, tcount,
@@ -1105,33 +1196,38 @@ void build_runs(seq_input const& in, uint32_t k, dev_arena& A, cudaStream_t st, 
     }
     const uint64_t nraw = nev / 2;
     if (nraw == 0) return;
+    if (nraw >= 0xffffffffull) throw std::runtime_error("too many ACGT runs");
     uint64_t* src = A.alloc<uint64_t>(nraw);
     uint32_t* len = A.alloc<uint32_t>(nraw);
     uint32_t* color = A.alloc<uint32_t>(nraw);
-    uint32_t* keep = A.alloc<uint32_t>(nraw);
-    uint64_t* kpos = A.alloc<uint64_t>(nraw + 1);
-    uint32_t* err = A.alloc<uint32_t>(1);
-    CDBG_CUDA(cudaMemsetAsync(err, 0, 4, st));
-    k_runs_from_events<<<grid(nraw, 256), 256, 0, st>>>(ev, nraw, in.seq_off, in.num_seqs,
-                                                         in.seq_color, k, src, len, color, keep, err);
+    uint64_t* size = A.alloc<uint64_t>(nraw);
+    uint64_t* ntl = A.alloc<uint64_t>(nraw);
+    uint64_t* pos = A.alloc<uint64_t>(nraw + 1);
+    uint64_t* tpos = A.alloc<uint64_t>(nraw + 1);
+    rt.src = A.alloc<uint64_t>(nraw);
+    rt.len = A.alloc<uint32_t>(nraw);
+    rt.color = A.alloc<uint32_t>(nraw);
+    rt.soff = A.alloc<uint64_t>(nraw + 1);
+    rt.tstart = A.alloc<uint64_t>(nraw + 1);
+    k_runs_from_events<<<grid(nraw, 256), 256, 0, st>>>(ev, nraw, in.seq_off, in.num_seqs, in.seq_color, k, rt.tile,
+                                                         src, len, color, size, ntl, counts + C_KMERS, err);
     CDBG_CHECK_LAUNCH();
-    prim::exclusive_scan<uint32_t, uint64_t>(keep, kpos, nraw, A, st, kpos + nraw);
-    const uint64_t nruns = read_dev(kpos + nraw, st);
-    if (read_dev(err, st) != 0) throw std::runtime_error("run length exceeds 2^32 bases");
+    // (runs in the high 32 bits, stream words in the low: an input on the device
+    // has fewer than 2^32 words of 32 bases)
+    prim::exclusive_scan<uint64_t, uint64_t>(size, pos, nraw, A, st, pos + nraw);
+    prim::exclusive_scan<uint64_t, uint64_t>(ntl, tpos, nraw, A, st, tpos + nraw);
+    k_runs_compact<<<grid(nraw + 1, 256), 256, 0, st>>>(nraw, size, pos, tpos, src, len, color, word_base, rt.src,
+                                                         rt.len, rt.color, rt.soff, rt.tstart);
+    CDBG_CHECK_LAUNCH();
+    uint64_t total = 0;
+    mail_reader(st).add(h, counts, sizeof(h)).add(&total, pos + nraw).add(&rt.ntiles, tpos + nraw).wait();
+    if ((uint32_t)h[C_ERR]) throw std::runtime_error("run length exceeds 2^32 bases");
+    const uint64_t nruns = total >> 32;
     if (nruns == 0) return;
-    if (nruns >= 0xffffffffull) throw std::runtime_error("too many ACGT runs");
     rt.n = (uint32_t)nruns;
-    rt.src = A.alloc<uint64_t>(nruns);
-    rt.len = A.alloc<uint32_t>(nruns);
-    rt.color = A.alloc<uint32_t>(nruns);
-    uint64_t* padded = A.alloc<uint64_t>(nruns);
-    rt.soff = A.alloc<uint64_t>(nruns + 1);
-    k_runs_compact<<<grid(nraw, 256), 256, 0, st>>>(nraw, keep, kpos, src, len, color, rt.src, rt.len,
-                                                     rt.color, padded);
-    CDBG_CHECK_LAUNCH();
-    prim::exclusive_scan<uint64_t, uint64_t>(padded, rt.soff, nruns, A, st, rt.soff + nruns);
-    const uint64_t total = read_dev(rt.soff + nruns, st);
-    const uint64_t nwd = total / 32;
+    rt.n_kmers = h[C_KMERS];
+    rt.n_bases = h[C_BASES];
+    const uint64_t nwd = total & 0xffffffffu;
     uint64_t* dst;
     if (words_out) {
         // this batch's runs go at word `word_base` of a shared stream
@@ -1147,23 +1243,12 @@ void build_runs(seq_input const& in, uint32_t k, dev_arena& A, cudaStream_t st, 
     CDBG_CUDA(cudaMemsetAsync(dst + nwd, 0, 8 * 8, st));
     if (nwd) {
         {
-            CDBG_PROF("k_pack", st);
-            k_pack<<<grid(nwd, 256), 256, 0, st>>>(in.ascii, rt.n, rt.soff, rt.src, rt.len, nwd, dst);
+            CDBG_PROF_BYTES("k_pack", st, 40.0 * nwd);
+            k_pack<<<grid(nwd, 256), 256, 0, st>>>(in.ascii, in.nbytes, rt.n, rt.soff, word_base, rt.src, rt.len, nwd,
+                                                    dst);
         }
         CDBG_CHECK_LAUNCH();
     }
-    if (words_out && word_base) {
-        k_add_u64<<<grid(nruns + 1, 256), 256, 0, st>>>(rt.soff, nruns + 1, word_base * 32);
-        CDBG_CHECK_LAUNCH();
-    }
-    unsigned long long* acc = A.alloc<unsigned long long>(2);
-    CDBG_CUDA(cudaMemsetAsync(acc, 0, 16, st));
-    k_run_kmers<<<grid(nruns, 256), 256, 0, st>>>(rt.n, rt.len, k, acc);
-    CDBG_CHECK_LAUNCH();
-    unsigned long long h[2];
-    read_small(h, acc, 16, st);
-    rt.n_kmers = h[0];
-    rt.n_bases = h[1];
 }
 
 template <int TT>
@@ -1176,7 +1261,7 @@ void find_supers(run_table const& rt, uint32_t k, uint32_t m, uint32_t B, dev_ar
         find_supers_tt<1024>(rt, k, m, B, A, st, out, d_err, packed);
     else if (tile == 2048)
         find_supers_tt<2048>(rt, k, m, B, A, st, out, d_err, packed);
-    else if (tile == 4096 || tile == 0)
+    else if (tile == MZ_DEFAULT_TILE || tile == 0)
         find_supers_tt<4096>(rt, k, m, B, A, st, out, d_err, packed);
     else
         throw std::runtime_error("minimizer tile must be 1024, 2048 or 4096");
@@ -1189,12 +1274,9 @@ void find_supers_tt(run_table const& rt, uint32_t k, uint32_t m, uint32_t B, dev
     if (rt.n == 0) return;
     if (k < 2 || m >= k || k - m > 62 || m > 32)
         throw std::runtime_error("unsupported k/m combination");
-    uint64_t* ntl = A.alloc<uint64_t>(rt.n);
-    uint64_t* tstart = A.alloc<uint64_t>(rt.n + 1);
-    k_run_tiles<<<grid(rt.n, 256), 256, 0, st>>>(rt.n, rt.len, k, TT, ntl);
-    CDBG_CHECK_LAUNCH();
-    prim::exclusive_scan<uint64_t, uint64_t>(ntl, tstart, rt.n, A, st, tstart + rt.n);
-    const uint64_t ntiles = read_dev(tstart + rt.n, st);
+    if (rt.tile != TT) throw std::runtime_error("runs tiled for another minimizer tile");
+    uint64_t const* tstart = rt.tstart;
+    const uint64_t ntiles = rt.ntiles;
     // one pass with a capacity of 1/4 of the (k-1)-mers (about 2.5x the
     // density of random sequence); the exact two-pass path if it overflows
     const uint64_t npos = rt.n_kmers + rt.n;
@@ -1202,10 +1284,9 @@ void find_supers_tt(run_table const& rt, uint32_t k, uint32_t m, uint32_t B, dev
     uint64_t* minv = A.alloc<uint64_t>(cap);
     uint32_t* run = A.alloc<uint32_t>(cap);
     uint32_t* aa = A.alloc<uint32_t>(cap);
-    unsigned long long* status = A.alloc<unsigned long long>(ntiles);
-    uint32_t* counter = A.alloc<uint32_t>(1);
-    CDBG_CUDA(cudaMemsetAsync(status, 0, 8 * ntiles, st));
-    CDBG_CUDA(cudaMemsetAsync(counter, 0, 4, st));
+    unsigned long long* status = A.alloc<unsigned long long>(ntiles + 1);  // and the tile counter
+    uint32_t* counter = reinterpret_cast<uint32_t*>(status + ntiles);
+    CDBG_CUDA(cudaMemsetAsync(status, 0, 8 * (ntiles + 1), st));
     {
         CDBG_PROF("k_minimizers", st);
         // the register-window form for the two windows of the default m
@@ -1320,6 +1401,16 @@ void keep_bucket_range(super_list& sl, uint32_t B, uint32_t lo, uint32_t hi, dev
     sl = o;
 }
 
+namespace {
+// Throws when the device error word is set (and clears it).
+void phase1_error(uint32_t* d_err, cudaStream_t st) {
+    const uint32_t e = read_dev(d_err, st);
+    if (!e) return;
+    CDBG_CUDA(cudaMemsetAsync(d_err, 0, 4, st));
+    throw std::runtime_error("device error " + std::to_string(e) + " in phase 1");
+}
+}  // namespace
+
 void build_records(run_table const& rt, super_list& sl, uint32_t k, uint32_t B, dev_arena& A,
                    cudaStream_t st, record_set& rs, uint32_t* d_err, dev_arena& out) {
     (void)k;
@@ -1335,66 +1426,57 @@ void build_records(run_table const& rt, super_list& sl, uint32_t k, uint32_t B, 
         CDBG_CUDA(cudaMemsetAsync(rs.bucket_start, 0, 8 * (B + 1), st));
         rs.col_off = out.alloc<uint64_t>(1);
         CDBG_CUDA(cudaMemsetAsync(rs.col_off, 0, 8, st));
+        phase1_error(d_err, st);
         return;
     }
     uint32_t* idx = A.alloc<uint32_t>(n);
-    k_iota_u32<<<grid(n, 256), 256, 0, st>>>(idx, n);
-    CDBG_CHECK_LAUNCH();
-    // sort a copy of the keys (the super list keeps its input order)
-    uint64_t* skey = A.alloc<uint64_t>(n);
-    CDBG_CUDA(cudaMemcpyAsync(skey, sl.key, n * 8, cudaMemcpyDeviceToDevice, st));
-    prim::sort_pairs_u64_exact<uint32_t>(skey, idx, n, A, st, d_err);
-    uint64_t* p_start = A.alloc<uint64_t>(n);
-    uint32_t* p_len = A.alloc<uint32_t>(n);
-    uint32_t* p_color = A.alloc<uint32_t>(n);
-    uint32_t* p_flags = A.alloc<uint32_t>(n);
-    {
-        CDBG_PROF("k_permute_supers", st);
-        if (sl.packed)
-            k_permute_packed<<<grid(n, 256), 256, 0, st>>>(n, idx, sl.packed, p_start, p_len, p_color, p_flags);
-        else
-            k_permute_supers<<<grid(n, 256), 256, 0, st>>>(n, idx, sl.start, sl.len, sl.color, sl.flags, p_start,
-                                                            p_len, p_color, p_flags);
-    }
-    CDBG_CHECK_LAUNCH();
-    uint32_t* head = A.alloc<uint32_t>(n);
-    uint32_t* ckeep = A.alloc<uint32_t>(n);
-    {
-        CDBG_PROF("k_group_heads", st);
-        k_group_heads_sorted<<<grid(n, 256), 256, 0, st>>>(n, skey, p_start, p_len, p_color, rt.words, head, ckeep);
-    }
-    CDBG_CHECK_LAUNCH();
-    uint64_t* rid = A.alloc<uint64_t>(n + 1);
-    uint64_t* cpos = A.alloc<uint64_t>(n + 1);
-    prim::exclusive_scan<uint32_t, uint64_t>(head, rid, n, A, st, rid + n);
-    prim::exclusive_scan<uint32_t, uint64_t>(ckeep, cpos, n, A, st, cpos + n);
-    uint64_t tot[2];
-    read_small(&tot[0], rid + n, 8, st);
-    read_small(&tot[1], cpos + n, 8, st);
-    const uint64_t nr = tot[0], nc = tot[1];
-    rs.n = nr;
-    rs.ncolors = nc;
-    rs.start = out.alloc<uint64_t>(nr);
-    rs.len = out.alloc<uint32_t>(nr);
-    rs.flags = out.alloc<uint32_t>(nr);
-    rs.col_off = out.alloc<uint64_t>(nr + 1);
-    rs.colors = out.alloc<uint32_t>(nc);
-    uint32_t* rb = A.alloc<uint32_t>(nr);
-    k_fill_u32<<<grid(nr, 256), 256, 0, st>>>(rs.flags, nr, 0xfu);
-    CDBG_CHECK_LAUNCH();
+    // (the super-k-mers stay in input order, their keys are sorted in place)
+    prim::sort_pairs_u64_exact<uint32_t>(sl.key, idx, n, A, st, d_err, true);
+    // the record arrays, sized for every super-k-mer a record of its own: where
+    // the result goes when that is little memory, else scratch they are copied
+    // from once their number is known
+    const bool direct = n <= (1u << 20);
+    dev_arena& W = direct ? out : A;
+    rs.start = W.alloc<uint64_t>(n);
+    rs.len = W.alloc<uint32_t>(n);
+    rs.flags = W.alloc<uint32_t>(n);
+    rs.col_off = W.alloc<uint64_t>(n + 1);
+    rs.colors = W.alloc<uint32_t>(n);
+    CDBG_CUDA(cudaMemsetAsync(rs.flags, 0xff, 4 * n, st));
+    const uint64_t ntiles = ceil_div(n, (uint64_t)RC_ROUNDS * 256);
+    unsigned long long* status = A.alloc<unsigned long long>(2 * ntiles + 3);  // two look-backs, totals, tile counter
+    unsigned long long* tot = status + 2 * ntiles;
+    CDBG_CUDA(cudaMemsetAsync(status, 0, 8 * (2 * ntiles + 3), st));
     uint32_t bb = 0;
     while ((1ull << bb) < B) ++bb;
     {
-        CDBG_PROF("k_records_fill", st);
-        k_records_fill_sorted<<<grid(n, 256), 256, 0, st>>>(n, head, rid, ckeep, cpos, skey, bb, p_start, p_len,
-                                                             p_color, p_flags, rs.start, rs.len, rs.flags,
-                                                             rs.col_off, rs.colors, rb);
+        CDBG_PROF("k_records", st);
+        super_fields_view sv{sl.packed, sl.start, sl.len, sl.color, sl.flags};
+        k_records<<<(unsigned)ntiles, 256, 0, st>>>(n, ntiles, idx, sl.key, sv, rt.words, bb, B,
+                                                    reinterpret_cast<uint32_t*>(tot + 2), status, status + ntiles,
+                                                    rs.start, rs.len, rs.flags, rs.col_off, rs.colors,
+                                                    rs.bucket_start, tot, d_err);
     }
     CDBG_CHECK_LAUNCH();
-    k_set_last_u64<<<1, 1, 0, st>>>(rs.col_off, nr, cpos + n);
-    CDBG_CHECK_LAUNCH();
-    k_bucket_bounds<<<grid(nr, 256), 256, 0, st>>>(nr, rb, B, rs.bucket_start);
-    CDBG_CHECK_LAUNCH();
+    uint64_t t[2];
+    uint32_t derr = 0;
+    mail_reader(st).add(t, tot, 16).add(&derr, d_err, 4).wait();
+    if (derr) phase1_error(d_err, st);
+    rs.n = t[0];
+    rs.ncolors = t[1];
+    if (!direct) {
+        auto keep = [&](auto*& p, uint64_t count) {
+            using T = std::remove_pointer_t<std::remove_reference_t<decltype(p)>>;
+            T* q = out.alloc<T>(count);
+            CDBG_CUDA(cudaMemcpyAsync(q, p, count * sizeof(T), cudaMemcpyDeviceToDevice, st));
+            p = q;
+        };
+        keep(rs.start, rs.n);
+        keep(rs.len, rs.n);
+        keep(rs.flags, rs.n);
+        keep(rs.col_off, rs.n + 1);
+        keep(rs.colors, rs.ncolors);
+    }
 }
 
 // Serialized size of every record summed into *sum (the uncompressed bytes

@@ -29,6 +29,10 @@ struct run_table {
     uint64_t nwords = 0;
     uint64_t n_kmers = 0;      // sum over runs of (len - k + 1)
     uint64_t n_bases = 0;      // sum over runs of len
+    // minimizer tiles of `tile` (k-1)-mers: the runs' first ones, n + 1 entries
+    uint64_t* tstart = nullptr;
+    uint64_t ntiles = 0;
+    uint32_t tile = 0;
 };
 
 // Super-k-mer records grouped by bucket (device).  Record bases live in a
@@ -53,11 +57,13 @@ struct phase1_stats {
 };
 
 // Runs + packing: ASCII -> 2-bit stream of ACGT runs >= k.
+// `tile` = (k-1)-mers per minimizer tile: 1024, 2048 or 4096 (0 = 4096), the same
+// for find_supers on these runs.
 // The 2-bit stream (rt.words) comes from `out`, everything else from A.  With
 // `words_out`, the runs are packed at word `word_base` of that stream instead
 // (capacity `words_cap` words) and rt.soff / rt.words / rt.nwords refer to it.
 void build_runs(seq_input const& in, uint32_t k, dev_arena& A, cudaStream_t st, run_table& rt, dev_arena& out,
-                uint64_t* words_out = nullptr, uint64_t word_base = 0, uint64_t words_cap = 0);
+                uint32_t tile = 0, uint64_t* words_out = nullptr, uint64_t word_base = 0, uint64_t words_cap = 0);
 
 // Super-k-mer occurrences of every run (for parity tests): arrays in input
 // order, allocated from the arena.  Returns the count.
@@ -72,7 +78,7 @@ struct super_list {
     // packed form (start, len, color << 4 | flags) instead of the arrays above
     uint4* packed = nullptr;
 };
-// `tile` = (k-1)-mers per minimizer tile: 1024 or 2048 (0 = 2048).  With
+// `tile` as given to build_runs.  With
 // `packed` (for build_records; colors must be < 2^28) only `key` and
 // `packed` are filled.
 void find_supers(run_table const& rt, uint32_t k, uint32_t m, uint32_t B, dev_arena& A,

@@ -1368,11 +1368,6 @@ __global__ void k_assign_new(uint64_t nnew, uint32_t const* __restrict__ rcand, 
     if (j < nnew) cid[rcand[j]] = (uint32_t)(base + j);
 }
 
-__global__ void k_iota32(uint64_t n, uint32_t* __restrict__ p) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = (uint32_t)i;
-}
-
 // Set comparison split by length.  A set of at most SHORT_SET words is
 // compared by its own lane, eight loads in flight at a time; a longer one by
 // the whole warp, lanes reading consecutive words (one coalesced line per
@@ -2845,9 +2840,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         uint64_t* skey = A.alloc<uint64_t>(nc);
         uint32_t* sidx = A.alloc<uint32_t>(nc);
         CDBG_CUDA(cudaMemcpyAsync(skey, cv.hash, 8 * nc, cudaMemcpyDeviceToDevice, st));
-        k_iota32<<<grid(nc, 256), 256, 0, st>>>(nc, sidx);
-        CDBG_CHECK_LAUNCH();
-        prim::sort_pairs_u64_exact<uint32_t>(skey, sidx, nc, A, st, d_err);
+        prim::sort_pairs_u64_exact<uint32_t>(skey, sidx, nc, A, st, d_err, true);
         uint32_t* head = A.alloc<uint32_t>(nc);
         uint64_t* hpos = A.alloc<uint64_t>(nc + 1);
         k_run_heads<<<grid(nc, 256), 256, 0, st>>>(nc, skey, head);

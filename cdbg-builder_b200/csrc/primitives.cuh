@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
         const uint32_t pos = (uint32_t)warp * (ITEMS * 32) + (uint32_t)r * 32 + lane;
         const bool ok = pos < tile_n;
         k[r] = ok ? keys_in[base + pos] : ~K(0);
-        v[r] = ok ? vals_in[base + pos] : V(0);
+        v[r] = !ok ? V(0) : vals_in ? vals_in[base + pos] : (V)(base + pos);
     }
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
@@ -421,7 +421,7 @@ struct rss_smem {
 };
 template <typename K, typename V>
 __global__ void __launch_bounds__(RSS_THREADS) k_rs_small(K* __restrict__ keys, V* __restrict__ vals, uint32_t n,
-                                                          int begin_bit, int end_bit) {
+                                                          int begin_bit, int end_bit, bool iota) {
     extern __shared__ __align__(16) unsigned char rs_raw[];
     rss_smem<K, V>& sm = *reinterpret_cast<rss_smem<K, V>*>(rs_raw);
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(RSS_THREADS) k_rs_small(K* __restrict__ keys, 
     for (int r = 0; r < RSS_ITEMS; ++r) {
         const uint32_t p = p0 + 32u * r;
         k[r] = p < n ? keys[p] : ~K(0);
-        v[r] = p < n ? vals[p] : V(0);
+        v[r] = p >= n ? V(0) : iota ? (V)p : vals[p];
     }
     for (int shift = begin_bit; shift < end_bit; shift += RS_BITS) {
         const uint32_t mask = end_bit - shift < RS_BITS ? (1u << (end_bit - shift)) - 1u : RS_BINS - 1u;
@@ -496,12 +496,13 @@ __global__ void __launch_bounds__(RSS_THREADS) k_rs_small(K* __restrict__ keys, 
     }
 }
 template <typename V, typename K>
-void radix_sort_small(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit, cudaStream_t st) {
+void radix_sort_small(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit, cudaStream_t st, bool iota) {
     CDBG_CUDA(cudaFuncSetAttribute(k_rs_small<K, V>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                    (int)sizeof(rss_smem<K, V>)));
     {
         CDBG_PROF("k_rs_small", st);
-        k_rs_small<K, V><<<1, RSS_THREADS, sizeof(rss_smem<K, V>), st>>>(keys, vals, (uint32_t)n, begin_bit, end_bit);
+        k_rs_small<K, V><<<1, RSS_THREADS, sizeof(rss_smem<K, V>), st>>>(keys, vals, (uint32_t)n, begin_bit, end_bit,
+                                                                          iota);
     }
     CDBG_CHECK_LAUNCH();
 }
@@ -529,9 +530,14 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_histograms_w(K const* __restr
 }
 
 constexpr uint64_t RS_HOST_CHECK = 1ull << 20;
+template <typename V>
+__global__ void k_iota(V* __restrict__ vals, uint64_t n) {
+    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) vals[i] = (V)i;
+}
 template <int BITS, typename V, typename K>
 int radix_sort_pairs_w(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit, dev_arena& A,
-                       cudaStream_t st, uint32_t* err) {
+                       cudaStream_t st, uint32_t* err, bool iota) {
     constexpr int BINS = 1 << BITS;
     constexpr int ITEMS = 16;
     using S = rs_smem<BITS, ITEMS, K, V>;
@@ -585,13 +591,17 @@ int radix_sort_pairs_w(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit,
             // one read and one write of every (key, value) pair
             CDBG_PROF_BYTES("k_rs_onesweep", st, 2.0 * n * (sizeof(K) + sizeof(V)));
             k_rs_onesweep<BITS, ITEMS, K, V><<<(unsigned)ntiles, RS_THREADS, sizeof(S), st>>>(
-                kin, vin, kout, vout, n, shift, counters + p, status, hist + (size_t)p * BINS, (uint32_t)(p + 1),
+                kin, iota && ran == 0 ? nullptr : vin, kout, vout, n, shift, counters + p, status, hist + (size_t)p * BINS, (uint32_t)(p + 1),
                 err);
         }
         CDBG_CHECK_LAUNCH();
         std::swap(kin, kout);
         std::swap(vin, vout);
         ++ran;
+    }
+    if (iota && ran == 0) {
+        k_iota<V><<<(unsigned)ceil_div(n, 256), 256, 0, st>>>(vals, n);
+        CDBG_CHECK_LAUNCH();
     }
     if (kin != keys) {
         CDBG_CUDA(cudaMemcpyAsync(keys, kin, n * sizeof(K), cudaMemcpyDeviceToDevice, st));
@@ -605,19 +615,20 @@ int radix_sort_pairs_w(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit,
 // 11-bit digits (g_radix_bits: the engine's tuning; 11 bits take 3 passes
 // where 8 bits take 4, with 8x the counters and look-back state per tile).
 // Results end in (keys, vals); the arena provides the ping-pong buffers.
+// With `iota`, the values on entry are 0, 1, .. n - 1 whatever `vals` holds.
 // Returns the number of passes run.  A look-back that gives up sets *err.
 template <typename V, typename K = uint64_t>
 int radix_sort_pairs(K* keys, V* vals, uint64_t n, int begin_bit, int end_bit, dev_arena& A, cudaStream_t st,
-                     uint32_t* err) {
+                     uint32_t* err, bool iota = false) {
     static_assert(sizeof(K) == 4 || sizeof(K) == 8, "u32 or u64 keys");
     if (end_bit > 8 * (int)sizeof(K)) end_bit = 8 * (int)sizeof(K);
-    if (n <= 1 || end_bit <= begin_bit) return 0;
+    if (!iota && (n <= 1 || end_bit <= begin_bit)) return 0;
     if (n <= RS_SMALL) {
-        radix_sort_small<V, K>(keys, vals, n, begin_bit, end_bit, st);
+        radix_sort_small<V, K>(keys, vals, n, begin_bit, end_bit, st, iota);
         return 1;
     }
-    if (g_radix_bits == 11) return radix_sort_pairs_w<11, V, K>(keys, vals, n, begin_bit, end_bit, A, st, err);
-    return radix_sort_pairs_w<RS_BITS, V, K>(keys, vals, n, begin_bit, end_bit, A, st, err);
+    if (g_radix_bits == 11) return radix_sort_pairs_w<11, V, K>(keys, vals, n, begin_bit, end_bit, A, st, err, iota);
+    return radix_sort_pairs_w<RS_BITS, V, K>(keys, vals, n, begin_bit, end_bit, A, st, err, iota);
 }
 
 // ----------------------------------------- exact 64-bit order, 32-bit passes
@@ -729,16 +740,17 @@ __global__ void k_hi_scatter(uint64_t* __restrict__ keys, V* __restrict__ vals, 
 // 8-pass LSD sort -- in 4 passes over the top 32 bits: keys that tie on those
 // bits but differ below them (rare when the top bits are a hash) are found
 // afterwards, and only their runs are sorted again on (run, low 32 bits).
-// n < 2^32.
+// n < 2^32; `iota` as in radix_sort_pairs.
 template <typename V>
-void sort_pairs_u64_exact(uint64_t* keys, V* vals, uint64_t n, dev_arena& A, cudaStream_t st, uint32_t* err) {
-    if (n <= 1) return;
+void sort_pairs_u64_exact(uint64_t* keys, V* vals, uint64_t n, dev_arena& A, cudaStream_t st, uint32_t* err,
+                          bool iota = false) {
+    if (n == 0 || (n == 1 && !iota)) return;
     if (n >= (1ull << 32)) throw std::runtime_error("sort_pairs_u64_exact: n >= 2^32");
     if (n <= RS_SMALL) {  // all 64 bits in the one launch
-        radix_sort_small<V, uint64_t>(keys, vals, n, 0, 64, st);
+        radix_sort_small<V, uint64_t>(keys, vals, n, 0, 64, st, iota);
         return;
     }
-    radix_sort_pairs<V, uint64_t>(keys, vals, n, 32, 64, A, st, err);
+    radix_sort_pairs<V, uint64_t>(keys, vals, n, 32, 64, A, st, err, iota);
     auto m = A.mark();
     const uint64_t cap = n / 8 + 1024;
     uint32_t* list = A.alloc<uint32_t>(cap);

@@ -76,3 +76,27 @@ def test_neighbour_lookups_by_bucket_size(oracle, engine, tmp_path, k, buckets, 
     for i in rng.integers(0, len(b), len(b) // 60).tolist():
         b[i] = b"ACGT"[int(rng.integers(0, 4))]
     _check(oracle, engine, tmp_path, [[a, b"A" * (2 * k), b"ACGT" * k], [bytes(b), a[-2 * k:] + a[:2 * k]]], k, buckets)
+
+
+@pytest.mark.parametrize("shift", [0, 1, 7, 16])
+@pytest.mark.parametrize("tail", [0, 1, 15, 31, 47])
+def test_device_input_alignment(oracle, engine, tmp_path, shift, tail):
+    """Sequences in HBM at any byte offset, ending at any distance from an
+    aligned address, in either case, with runs of other characters."""
+    import torch
+    k, B = 31, 16
+    rng = np.random.default_rng(shift * 50 + tail)
+    s = [_dna(rng, 4000 + tail), _dna(rng, 31).lower(), b"ACGTN" + _dna(rng, 333) + b"-" * 40 + _dna(rng, 64), b"NN",
+         _dna(rng, 97)]
+    data = np.frombuffer(b"".join(s), dtype=np.uint8)
+    off = np.zeros(len(s) + 1, dtype=np.int64)
+    off[1:] = np.cumsum([len(x) for x in s])
+    buf = torch.empty(shift + len(data), dtype=torch.uint8, device="cuda")
+    buf[shift:] = torch.from_numpy(data.copy())
+    d_off, d_col = torch.from_numpy(off).cuda(), torch.tensor([0, 0, 1, 1, 1], dtype=torch.int32).cuda()
+    torch.cuda.synchronize()
+    b = native.SeqBatch(buf.data_ptr() + shift, len(data), d_off.data_ptr(), d_col.data_ptr(), len(s), 1)
+    want = engine.build(native.host_batch(s, [0, 0, 1, 1, 1]), k, B, 2)
+    want = native.result_frag_bytes(want)
+    assert native.result_frag_bytes(engine.build(b, k, B, 2)) == want
+    _check(oracle, engine, tmp_path, [s[:2], s[2:]], k, B)
