@@ -287,7 +287,7 @@ int cdbg_engine_create(int device, cdbg_engine** out) {
         e->P.set_stream(e->st);
         CDBG_CUDA(cudaMalloc(&e->d_err, 16));
         CDBG_CUDA(cudaMemset(e->d_err, 0, 16));
-        e->mailbox.bytes = size_t(256) << 10;
+        e->mailbox.bytes = size_t(512) << 10;
         CDBG_CUDA(cudaHostAlloc(&e->mailbox.h, e->mailbox.bytes, cudaHostAllocMapped));
         std::memset(e->mailbox.h, 0, cdbg::MAIL_DATA);
         CDBG_CUDA(cudaHostGetDevicePointer(&e->mailbox.d, e->mailbox.h, 0));

@@ -669,75 +669,96 @@ __device__ __forceinline__ unsigned long long block_reserve(uint32_t want, unsig
     return r;
 }
 
-// First of each run of equal (node, record) pairs (a record may own a k-mer
-// at two positions).
-__global__ void k_unique_pairs(uint64_t n, uint32_t const* __restrict__ pn, uint32_t const* __restrict__ pr,
-                               uint32_t* __restrict__ keep) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) keep[i] = (i == 0 || pn[i] != pn[i - 1] || pr[i] != pr[i - 1]) ? 1u : 0u;
-}
+// Look-back state of one ordered selection (prim::ordered_select), zeroed.
+struct select_ws {
+    unsigned long long* status;
+    unsigned long long* total;
+    uint32_t* counter;
+    uint64_t ntiles;
+};
 
-// Kept pairs as (node << 32 | record).
-__global__ void k_compact_pairs(uint64_t n, uint32_t const* __restrict__ pn, uint32_t const* __restrict__ pr,
-                                uint32_t const* __restrict__ keep, uint64_t const* __restrict__ pos,
-                                uint64_t* __restrict__ out) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && keep[i]) out[pos[i]] = ((uint64_t)pn[i] << 32) | pr[i];
-}
-
-__global__ void k_node_heads(uint64_t n, uint64_t const* __restrict__ a, uint32_t* __restrict__ head) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) head[i] = (i == 0 || (a[i] >> 32) != (a[i - 1] >> 32)) ? 1u : 0u;
-}
-
-// Multi-record nodes: m-th head -> node id, record range [moff[m], moff[m+1]).
-__global__ void k_multi_index(uint64_t n, uint64_t const* __restrict__ a, uint32_t const* __restrict__ head,
-                              uint64_t const* __restrict__ hpos, uint32_t* __restrict__ mnode,
-                              uint64_t* __restrict__ moff, uint32_t* __restrict__ n_rec) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n || !head[i]) return;
-    const uint64_t m = hpos[i];
-    const uint32_t node = (uint32_t)(a[i] >> 32);
-    mnode[m] = node;
-    moff[m] = i;
-    n_rec[node] = MULTI_TAG | (uint32_t)m;
+// Multi-record nodes from the (node, record) pairs in node order, in one pass:
+// each pair once (a record may own a k-mer at two positions: equal pairs are
+// neighbours) into urec, and the m-th node with its record range [moff[m],
+// moff[m + 1]).
+__global__ void __launch_bounds__(256) k_multi_index(uint64_t n, uint32_t const* __restrict__ pn,
+                                                     uint32_t const* __restrict__ pr, select_ws wk, select_ws wh,
+                                                     uint32_t* __restrict__ urec, uint32_t* __restrict__ mnode,
+                                                     uint64_t* __restrict__ moff, uint32_t* __restrict__ n_rec,
+                                                     uint32_t* err) {
+    __shared__ prim::ordered_select keep, head;
+    const uint64_t tile = prim::select_tile(keep, wk.counter);
+    uint32_t node[prim::SEL_ROUNDS], rec[prim::SEL_ROUNDS], sk = 0, sh = 0;
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t i = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        if (i >= n) continue;
+        node[r] = pn[i];
+        rec[r] = pr[i];
+        const bool h = i == 0 || pn[i - 1] != node[r];
+        if (h) sh |= 1u << r;
+        if (h || pr[i - 1] != rec[r]) sk |= 1u << r;
+    }
+    prim::select_rank(keep, sk, tile, wk.ntiles, wk.status, wk.total, err);
+    prim::select_rank(head, sh, tile, wk.ntiles, wh.status, wh.total, err);
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t i = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        const uint64_t o = prim::select_pos(keep, r), m = prim::select_pos(head, r);
+        if ((sk >> r) & 1u) urec[o] = rec[r];
+        if ((sh >> r) & 1u) {
+            mnode[m] = node[r];
+            moff[m] = o;
+            n_rec[node[r]] = MULTI_TAG | (uint32_t)m;
+        }
+        if (i == n - 1) moff[m + ((sh >> r) & 1u)] = o + ((sk >> r) & 1u);
+    }
 }
 
 // Multi-record nodes in node order whose owning-record list equals the
 // previous one's (the k-mers of a stretch shared by the same records) share
-// one union: ghead[m] = 1 starts a new group.
-__global__ void k_multi_same(uint64_t M, uint64_t const* __restrict__ moff, uint64_t const* __restrict__ upairs,
-                             uint32_t* __restrict__ ghead) {
-    uint64_t m = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    bool same = false;
-    if (m > 0) {
-        const uint64_t a0 = moff[m - 1], a1 = moff[m], b1 = moff[m + 1];
-        if (a1 - a0 == b1 - a1) {
-            same = true;
-            for (uint64_t i = 0; i < a1 - a0; ++i)
-                if ((uint32_t)upairs[a0 + i] != (uint32_t)upairs[a1 + i]) {
-                    same = false;
-                    break;
-                }
+// one union: group g has its first node and its record range, every multi
+// node its group.
+__global__ void __launch_bounds__(256) k_multi_groups(uint64_t M, uint64_t const* __restrict__ moff,
+                                                      uint32_t const* __restrict__ urec,
+                                                      uint32_t const* __restrict__ mnode, select_ws ws,
+                                                      uint32_t* __restrict__ gnode, uint64_t* __restrict__ gbeg,
+                                                      uint64_t* __restrict__ gend, uint32_t* __restrict__ mgrp,
+                                                      uint32_t* err) {
+    __shared__ prim::ordered_select head;
+    const uint64_t tile = prim::select_tile(head, ws.counter);
+    uint32_t sel = 0;
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t m = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        if (m >= M) continue;
+        bool same = false;
+        if (m > 0) {
+            const uint64_t a0 = moff[m - 1], a1 = moff[m], b1 = moff[m + 1];
+            if (a1 - a0 == b1 - a1) {
+                same = true;
+                for (uint64_t i = 0; i < a1 - a0; ++i)
+                    if (urec[a0 + i] != urec[a1 + i]) {
+                        same = false;
+                        break;
+                    }
+            }
         }
+        if (!same) sel |= 1u << r;
     }
-    ghead[m] = same ? 0u : 1u;
-}
-
-// Group g (of its head node m): node, record range; every multi node's group.
-__global__ void k_multi_groups(uint64_t M, uint32_t const* __restrict__ ghead, uint64_t const* __restrict__ gpos,
-                               uint32_t const* __restrict__ mnode, uint64_t const* __restrict__ moff,
-                               uint32_t* __restrict__ gnode, uint64_t* __restrict__ gbeg, uint64_t* __restrict__ gend,
-                               uint32_t* __restrict__ mgrp) {
-    uint64_t m = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    const uint64_t g = gpos[m] + ghead[m] - 1;
-    mgrp[m] = (uint32_t)g;
-    if (ghead[m]) {
-        gnode[g] = mnode[m];
-        gbeg[g] = moff[m];
-        gend[g] = moff[m + 1];
+    prim::select_rank(head, sel, tile, ws.ntiles, ws.status, ws.total, err);
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t m = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        if (m >= M) continue;
+        const bool h = (sel >> r) & 1u;
+        const uint64_t g = prim::select_pos(head, r) + (h ? 1 : 0) - 1;
+        mgrp[m] = (uint32_t)g;
+        if (h) {
+            gnode[g] = mnode[m];
+            gbeg[g] = moff[m];
+            gend[g] = moff[m + 1];
+        }
     }
 }
 
@@ -802,7 +823,7 @@ __device__ __forceinline__ void warp_or_list(uint32_t* bm, uint32_t const* __res
 // pass 1: write the ascending list at pool[poff[m]].
 template <bool WRITE>
 __global__ void k_union(uint64_t M, uint64_t const* __restrict__ mbeg, uint64_t const* __restrict__ mend,
-                        uint64_t const* __restrict__ upairs,
+                        uint32_t const* __restrict__ urec,
                         uint64_t const* __restrict__ col_off, uint32_t const* __restrict__ colors,
                         uint32_t C, uint32_t* __restrict__ msize, uint64_t* __restrict__ mhash,
                         uint64_t const* __restrict__ poff, uint32_t* __restrict__ pool) {
@@ -815,7 +836,7 @@ __global__ void k_union(uint64_t M, uint64_t const* __restrict__ mbeg, uint64_t 
     for (uint32_t w = lane; w < nw; w += 32) bm[w] = 0;
     __syncwarp();
     for (uint64_t p = mbeg[m]; p < mend[m]; ++p) {
-        const uint32_t r = (uint32_t)(upairs[p] & 0xffffffffu);
+        const uint32_t r = urec[p];
         warp_or_list(bm, colors, col_off[r], col_off[r + 1], nw, lane);
     }
     __syncwarp();
@@ -851,11 +872,11 @@ __global__ void k_union(uint64_t M, uint64_t const* __restrict__ mbeg, uint64_t 
 
 // ---- multi-record unions as bitmaps -----------------------------------------
 // Records with at least `heavy` colors get a bitmap.
-__global__ void k_heavy_flags(uint64_t nu, uint64_t const* __restrict__ upairs, uint64_t const* __restrict__ col_off,
+__global__ void k_heavy_flags(uint64_t nu, uint32_t const* __restrict__ urec, uint64_t const* __restrict__ col_off,
                               uint32_t R0, uint32_t heavy, uint32_t* __restrict__ flag) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= nu) return;
-    const uint32_t r = (uint32_t)(upairs[i] & 0xffffffffu);
+    const uint32_t r = urec[i];
     if (col_off[r + 1] - col_off[r] >= heavy) flag[r - R0] = 1u;
 }
 
@@ -893,7 +914,7 @@ __global__ void k_heavy_bitmaps(uint64_t nrec, uint32_t const* __restrict__ flag
 template <int WPL>
 __global__ void __launch_bounds__(256) k_union_bm(
     uint64_t M, uint64_t const* __restrict__ mbeg, uint64_t const* __restrict__ mend,
-    uint64_t const* __restrict__ upairs, uint64_t const* __restrict__ col_off, uint32_t const* __restrict__ colors,
+    uint32_t const* __restrict__ urec, uint64_t const* __restrict__ col_off, uint32_t const* __restrict__ colors,
     uint32_t R0, uint32_t const* __restrict__ hflag, uint64_t const* __restrict__ hpos,
     uint32_t const* __restrict__ rbits, uint32_t nw, uint32_t* __restrict__ mbits, uint32_t* __restrict__ msize,
     uint64_t* __restrict__ mhash) {
@@ -913,8 +934,8 @@ __global__ void __launch_bounds__(256) k_union_bm(
         bool heavy = false, light = false;
         uint64_t src = 0, c0 = 0, c1 = 0;
         if (p < pend) {
-            const uint32_t r = (uint32_t)(upairs[p] & 0xffffffffu);
-            heavy = hflag[r - R0] != 0;
+            const uint32_t r = urec[p];
+            heavy = hflag && hflag[r - R0] != 0;
             light = !heavy;
             if (heavy) {
                 src = hpos[r - R0] * (uint64_t)nw;
@@ -1007,16 +1028,31 @@ struct cand_view {
     uint64_t* hash;
 };
 
-__global__ void k_cand_records(uint64_t nrec, uint32_t R0, uint32_t const* __restrict__ rec_first,
-                               uint32_t const* __restrict__ keep, uint64_t const* __restrict__ pos,
-                               uint64_t const* __restrict__ rhash, cand_view cv, uint32_t* __restrict__ rec_cand) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nrec || !keep[i]) return;
-    const uint64_t c = pos[i];
-    cv.kind_id[c] = R0 + (uint32_t)i;
-    cv.first[c] = rec_first[i];
-    cv.hash[c] = rhash[R0 + i];
-    rec_cand[i] = (uint32_t)c;
+// Records that are some k-mer's color set (rec_first set), in record order.
+__global__ void __launch_bounds__(256) k_cand_records(uint64_t nrec, uint32_t R0,
+                                                      uint32_t const* __restrict__ rec_first, select_ws ws,
+                                                      uint64_t const* __restrict__ rhash, cand_view cv,
+                                                      uint32_t* __restrict__ rec_cand, uint32_t* err) {
+    __shared__ prim::ordered_select used;
+    const uint64_t tile = prim::select_tile(used, ws.counter);
+    uint32_t first[prim::SEL_ROUNDS], sel = 0;
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t i = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        first[r] = i < nrec ? rec_first[i] : NONE32;
+        if (first[r] != NONE32) sel |= 1u << r;
+    }
+    prim::select_rank(used, sel, tile, ws.ntiles, ws.status, ws.total, err);
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        if (!((sel >> r) & 1u)) continue;
+        const uint64_t i = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        const uint64_t c = prim::select_pos(used, r);
+        cv.kind_id[c] = R0 + (uint32_t)i;
+        cv.first[c] = first[r];
+        cv.hash[c] = rhash[R0 + i];
+        rec_cand[i] = (uint32_t)c;
+    }
 }
 
 __global__ void k_cand_multi(uint64_t M, uint64_t base, uint32_t const* __restrict__ mnode,
@@ -1344,21 +1380,30 @@ __global__ void k_dict_lookup(uint64_t nc, cand_view cv, uint64_t const* __restr
     cid[c] = res;
 }
 
-__global__ void k_new_flags(uint64_t nc, uint32_t const* __restrict__ cid, uint32_t* __restrict__ flag) {
-    uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < nc) flag[c] = cid[c] == NONE32 ? 1u : 0u;
-}
-
-__global__ void k_run_heads(uint64_t n, uint64_t const* __restrict__ key, uint32_t* __restrict__ head) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) head[i] = (i == 0 || key[i] != key[i - 1]) ? 1u : 0u;
-}
-
-// run_start[run id] = position of the run's head
-__global__ void k_run_starts(uint64_t n, uint32_t const* __restrict__ head, uint64_t const* __restrict__ hpos,
-                             uint64_t* __restrict__ run_start) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n && head[i]) run_start[hpos[i]] = i;
+// Runs of equal hashes in the sorted candidates: run[i] of every position, the
+// runs' starts, and rep_first set to none for every candidate.
+__global__ void __launch_bounds__(256) k_hash_runs(uint64_t n, uint64_t const* __restrict__ key, select_ws ws,
+                                                   uint32_t* __restrict__ run, uint32_t* __restrict__ run_start,
+                                                   uint32_t* __restrict__ rep_first, uint32_t* err) {
+    __shared__ prim::ordered_select head;
+    const uint64_t tile = prim::select_tile(head, ws.counter);
+    uint32_t sel = 0;
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t i = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        if (i < n && (i == 0 || key[i] != key[i - 1])) sel |= 1u << r;
+    }
+    prim::select_rank(head, sel, tile, ws.ntiles, ws.status, ws.total, err);
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t i = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        if (i >= n) continue;
+        const bool h = (sel >> r) & 1u;
+        const uint32_t q = (uint32_t)(prim::select_pos(head, r) + (h ? 1 : 0) - 1);
+        run[i] = q;
+        if (h) run_start[q] = (uint32_t)i;
+        rep_first[i] = NONE32;
+    }
 }
 
 // New class j (in first-appearance order) = candidate rcand[j]; cid base+j.
@@ -1463,9 +1508,9 @@ __device__ __forceinline__ bool warp_sets_equal(cand_set const& a, cand_set cons
 // its own pair of sets; short pairs are compared by the lane, long ones by
 // the warp in turn.  The grid covers n in whole blocks of 256 threads.
 __global__ void __launch_bounds__(256) k_member_match_raw(
-    uint64_t n, uint32_t const* __restrict__ head, uint64_t const* __restrict__ hpos,
-    uint64_t const* __restrict__ run_start, uint32_t const* __restrict__ nidx, cand_view cv, list_src L,
-    uint32_t* __restrict__ rep, uint32_t* __restrict__ rep_first, uint32_t* __restrict__ collided) {
+    uint64_t n, uint32_t const* __restrict__ run_of, uint32_t const* __restrict__ run_start,
+    uint32_t const* __restrict__ nidx, cand_view cv, list_src L, uint32_t* __restrict__ rep,
+    uint32_t* __restrict__ rep_first, uint32_t* __restrict__ collided, uint32_t* __restrict__ any) {
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int lane = threadIdx.x & 31;
     int need = 0;  // 0: decided, 1: lane compares, 2: warp compares
@@ -1474,7 +1519,7 @@ __global__ void __launch_bounds__(256) k_member_match_raw(
     uint32_t c = 0, h = 0;
     cand_set sc{nullptr, nullptr, 0}, sh{nullptr, nullptr, 0};
     if (i < n) {
-        run = hpos[i] + head[i] - 1;
+        run = run_of[i];
         c = nidx[i];
         h = nidx[run_start[run]];
         if (c == h) {
@@ -1499,6 +1544,7 @@ __global__ void __launch_bounds__(256) k_member_match_raw(
         } else {
             rep[c] = c;
             collided[run] = 1;
+            *any = 1;
         }
     }
     // rep_first[h] = min first appearance over the head and its equal
@@ -1518,7 +1564,7 @@ __global__ void __launch_bounds__(256) k_member_match_raw(
 }
 
 __global__ void k_group_collided_raw(uint64_t nruns, uint32_t const* __restrict__ collided,
-                                     uint64_t const* __restrict__ run_start, uint64_t n,
+                                     uint32_t const* __restrict__ run_start, uint64_t n,
                                      uint32_t const* __restrict__ nidx, cand_view cv, list_src L,
                                      uint32_t* __restrict__ rep, uint32_t* __restrict__ rep_first) {
     uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1546,31 +1592,52 @@ __global__ void k_group_collided_raw(uint64_t nruns, uint32_t const* __restrict_
     }
 }
 
-__global__ void k_rep_flags(uint64_t nc, uint32_t const* __restrict__ rep, uint32_t* __restrict__ is_rep) {
-    uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c < nc) is_rep[c] = rep[c] == (uint32_t)c ? 1u : 0u;
-}
-
-// Compact the representatives into their own candidate view.
-__global__ void k_rep_compact(uint64_t nc, uint32_t const* __restrict__ is_rep, uint64_t const* __restrict__ pos,
-                              cand_view cv, uint32_t const* __restrict__ rep_first, cand_view rv,
-                              uint32_t* __restrict__ rep_index) {
-    uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= nc || !is_rep[c]) return;
-    const uint64_t p = pos[c];
-    rv.kind_id[p] = cv.kind_id[c];
-    rv.first[p] = rep_first[c];
-    rv.hash[p] = cv.hash[c];
-    rep_index[c] = (uint32_t)p;
+// The representatives into their own candidate view, in candidate order.
+__global__ void __launch_bounds__(256) k_rep_compact(uint64_t nc, uint32_t const* __restrict__ rep, select_ws ws,
+                                                     cand_view cv, uint32_t const* __restrict__ rep_first,
+                                                     cand_view rv, uint32_t* __restrict__ rep_index, uint32_t* err) {
+    __shared__ prim::ordered_select is_rep;
+    const uint64_t tile = prim::select_tile(is_rep, ws.counter);
+    uint32_t sel = 0;
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t c = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        if (c < nc && rep[c] == (uint32_t)c) sel |= 1u << r;
+    }
+    prim::select_rank(is_rep, sel, tile, ws.ntiles, ws.status, ws.total, err);
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        if (!((sel >> r) & 1u)) continue;
+        const uint64_t c = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        const uint64_t p = prim::select_pos(is_rep, r);
+        rv.kind_id[p] = cv.kind_id[c];
+        rv.first[p] = rep_first[c];
+        rv.hash[p] = cv.hash[c];
+        rep_index[c] = (uint32_t)p;
+    }
 }
 
 // New representatives (not in the dictionary): keys = first appearance.
-__global__ void k_new_reps(uint64_t nr, uint32_t const* __restrict__ rcid, uint64_t const* __restrict__ npos,
-                           cand_view rv, uint64_t* __restrict__ key, uint32_t* __restrict__ idx) {
-    uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= nr || rcid[j] != NONE32) return;
-    key[npos[j]] = rv.first[j];
-    idx[npos[j]] = (uint32_t)j;
+__global__ void __launch_bounds__(256) k_new_reps(uint64_t nr, uint32_t const* __restrict__ rcid, select_ws ws,
+                                                  cand_view rv, uint32_t* __restrict__ key,
+                                                  uint32_t* __restrict__ idx, uint32_t* err) {
+    __shared__ prim::ordered_select is_new;
+    const uint64_t tile = prim::select_tile(is_new, ws.counter);
+    uint32_t sel = 0;
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t j = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        if (j < nr && rcid[j] == NONE32) sel |= 1u << r;
+    }
+    prim::select_rank(is_new, sel, tile, ws.ntiles, ws.status, ws.total, err);
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        if (!((sel >> r) & 1u)) continue;
+        const uint64_t j = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        const uint64_t p = prim::select_pos(is_new, r);
+        key[p] = rv.first[j];
+        idx[p] = (uint32_t)j;
+    }
 }
 
 __global__ void k_cand_cid(uint64_t nc, uint32_t const* __restrict__ rep, uint32_t const* __restrict__ rep_index,
@@ -2172,9 +2239,12 @@ __global__ void __launch_bounds__(256) k_chain_ends(chain_ws W, uint32_t* __rest
 // Each end walks to the other end; the end with the smaller node index leads
 // and reserves the chain's slots [c0, c0 + L).  heads[h] = (node | rc << 31,
 // L, c0 low, c0 high).
-__global__ void __launch_bounds__(256) k_chain_lead(chain_ws W, uint32_t const* __restrict__ ends, uint64_t nends,
+__global__ void __launch_bounds__(256) k_chain_lead(chain_ws W, uint32_t const* __restrict__ ends,
+                                                    unsigned long long const* __restrict__ pends,
                                                     uint4* __restrict__ heads, unsigned long long* __restrict__ nheads,
                                                     uint32_t* err) {
+    const uint64_t nends = *pends;  // (the grid may be larger)
+    if ((uint64_t)blockIdx.x * blockDim.x >= nends) return;
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t c = 0, L = 0;
     bool rc = false, lead = false;
@@ -2208,9 +2278,10 @@ __global__ void __launch_bounds__(256) k_chain_lead(chain_ws W, uint32_t const* 
 }
 
 // One thread per path chain: lay the chain out at c0 and replay the seed loop.
-__global__ void __launch_bounds__(128) k_chain_paths(chain_ws W, uint4 const* __restrict__ heads, uint64_t nheads) {
+__global__ void __launch_bounds__(128) k_chain_paths(chain_ws W, uint4 const* __restrict__ heads,
+                                                     unsigned long long const* __restrict__ nheads) {
     const uint64_t h = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= nheads) return;
+    if (h >= *nheads) return;
     const uint4 hd = heads[h];
     uint32_t cc = hd.x & 0x7fffffffu;
     bool r = (hd.x >> 31) != 0;
@@ -2273,23 +2344,37 @@ __global__ void k_chain_cycles(chain_ws W, uint32_t* err) {
 __device__ __forceinline__ uint32_t frag_cid(uint32_t const* n_cid, uint32_t node) { return n_cid[node]; }
 
 // Seed nodes in node order (= fragment order): seed_of[f] = node of fragment f.
-__global__ void k_seed_flags(uint64_t D, uint32_t const* __restrict__ seed_len, uint32_t* __restrict__ is_seed) {
-    uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n < D) is_seed[n] = seed_len[n] ? 1u : 0u;
-}
-__global__ void k_seed_list(uint64_t D, uint32_t const* __restrict__ is_seed, uint64_t const* __restrict__ fpos,
-                            uint32_t* __restrict__ seed_of) {
-    uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n < D && is_seed[n]) seed_of[fpos[n]] = (uint32_t)n;
+__global__ void __launch_bounds__(256) k_seed_list(uint64_t D, uint32_t const* __restrict__ seed_len, select_ws ws,
+                                                   uint32_t* __restrict__ seed_of, uint32_t* err) {
+    __shared__ prim::ordered_select seeds;
+    const uint64_t tile = prim::select_tile(seeds, ws.counter);
+    uint32_t sel = 0;
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t n = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        if (n < D && seed_len[n]) sel |= 1u << r;
+    }
+    prim::select_rank(seeds, sel, tile, ws.ntiles, ws.status, ws.total, err);
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r)
+        if ((sel >> r) & 1u)
+            seed_of[prim::select_pos(seeds, r)] = (uint32_t)(tile * prim::SEL_TILE + 256u * r + threadIdx.x);
 }
 
 // Thread per fragment: serialized size (frag_unitig_writer::write_batch layout).
-__global__ void k_frag_sizes(uint64_t F, uint32_t const* __restrict__ seed_of, uint32_t const* __restrict__ seed_start,
-                             uint32_t const* __restrict__ seed_len, uint32_t const* __restrict__ fe,
-                             uint32_t const* __restrict__ n_cid, uint32_t k, uint64_t* __restrict__ sz,
-                             unsigned long long* __restrict__ seq_total) {
-    uint64_t f = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint64_t seq = 0;
+// and, by decoupled look-back over blocks, its offset: off[f], off[F] the total.
+__global__ void __launch_bounds__(256) k_frag_sizes(uint64_t F, uint32_t const* __restrict__ seed_of,
+                                                    uint32_t const* __restrict__ seed_start,
+                                                    uint32_t const* __restrict__ seed_len,
+                                                    uint32_t const* __restrict__ fe,
+                                                    uint32_t const* __restrict__ n_cid, uint32_t k, select_ws ws,
+                                                    uint64_t* __restrict__ off,
+                                                    unsigned long long* __restrict__ seq_total, uint32_t* err) {
+    __shared__ uint64_t sw[256 / 32 + 1], s_tile, s_base;
+    if (threadIdx.x == 0) s_tile = atomicAdd(ws.counter, 1u);
+    __syncthreads();
+    const uint64_t tile = s_tile, f = tile * 256 + threadIdx.x;
+    uint64_t seq = 0, size = 0;
     if (f < F) {
         const uint32_t n = seed_of[f];
         const uint32_t len = seed_len[n], a = seed_start[n];
@@ -2300,8 +2385,21 @@ __global__ void k_frag_sizes(uint64_t F, uint32_t const* __restrict__ seed_of, u
             prev = c;
         }
         seq = (uint64_t)k + len - 1;
-        sz[f] = 1 + 4 + 12ull * runs + 4 + seq;
+        size = 1 + 4 + 12ull * runs + 4 + seq;
     }
+    uint64_t tot;
+    const uint64_t ex = prim::block_exclusive_scan<uint64_t, 256>(size, sw, tot);
+    if (threadIdx.x < 32) {
+        uint64_t excl = 0;
+        const bool ok = prim::lookback_exclusive(ws.status, tile, tot, excl);
+        if (threadIdx.x == 0) {
+            if (!ok) set_error(err, ERR_CHAIN_LIMIT);
+            s_base = excl;
+        }
+    }
+    __syncthreads();
+    if (f < F) off[f] = s_base + ex;
+    if (f == F - 1) off[F] = *ws.total = s_base + ex + size;
     seq = prim::warp_inclusive_scan(seq);
     if ((threadIdx.x & 31) == 31 && seq) atomicAdd(seq_total, (unsigned long long)seq);
 }
@@ -2374,19 +2472,19 @@ __global__ void __launch_bounds__(FW_THREADS)
     k_frag_write(uint64_t F, uint32_t const* __restrict__ seed_of, uint32_t const* __restrict__ seed_start,
                  uint32_t const* __restrict__ seed_len, uint8_t const* __restrict__ seed_open,
                  uint32_t const* __restrict__ fe, uint32_t const* __restrict__ n_cid, K const* __restrict__ n_key,
-                 uint32_t k, uint64_t const* __restrict__ off, uint8_t* __restrict__ out) {
+                 uint32_t k, uint64_t const* __restrict__ off, uint64_t base, uint8_t* __restrict__ out) {
     __shared__ __align__(16) uint8_t buf[FW_BYTES];
     const uint64_t f0 = (uint64_t)blockIdx.x * FW_THREADS;
     const uint64_t f1 = (f0 + FW_THREADS < F) ? f0 + FW_THREADS : F;
-    const uint64_t g0 = off[f0], g1 = off[f1];
+    const uint64_t g0 = base + off[f0], g1 = base + off[f1];  // out is 16-byte aligned, out + base need not be
     const uint32_t phase = (uint32_t)(g0 & 15);
     const uint64_t f = f0 + threadIdx.x;
     if (g1 - g0 + phase > (uint64_t)FW_BYTES) {  // block-uniform
-        if (f < F) emit_fragment<K>(out + off[f], seed_of[f], seed_start, seed_len, seed_open, fe, n_cid, n_key, k);
+        if (f < F) emit_fragment<K>(out + base + off[f], seed_of[f], seed_start, seed_len, seed_open, fe, n_cid, n_key, k);
         return;
     }
     if (f < F)
-        emit_fragment<K>(buf + phase + (off[f] - g0), seed_of[f], seed_start, seed_len, seed_open, fe, n_cid, n_key,
+        emit_fragment<K>(buf + phase + (base + off[f] - g0), seed_of[f], seed_start, seed_len, seed_open, fe, n_cid, n_key,
                          k);
     __syncthreads();
     const uint64_t a0 = (g0 + 15) & ~uint64_t(15);  // first aligned byte inside the range
@@ -2405,25 +2503,14 @@ __global__ void __launch_bounds__(FW_THREADS)
 
 // ---------------------------------------------------------------------------
 // ---- small helpers ----------------------------------------------------------
-__global__ void k_count_flags(uint64_t n, uint32_t const* __restrict__ f, unsigned long long* __restrict__ c) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    uint32_t v = (i < n) ? f[i] : 0u;
-    const uint32_t b = __ballot_sync(0xffffffffu, v != 0);
-    if ((threadIdx.x & 31) == 0 && b) atomicAdd(c, (unsigned long long)__popc(b));
-}
 __global__ void k_add_offsets(uint64_t n, uint64_t const* __restrict__ src, uint64_t add,
                               uint64_t* __restrict__ dst) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) dst[i] = src[i] + add;
 }
-__global__ void k_set_u64(uint64_t* p, uint64_t v) { *p = v; }
 __global__ void k_copy_u64x2(unsigned long long const* src, unsigned long long* dst) {
     dst[0] = src[0];
     dst[1] = src[1];
-}
-__global__ void k_used_flags(uint64_t n, uint32_t const* __restrict__ first, uint32_t* __restrict__ keep) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) keep[i] = first[i] != NONE32 ? 1u : 0u;
 }
 
 void add_offsets(uint64_t const* src, uint64_t n, uint64_t add, uint64_t* dst, cudaStream_t st) {
@@ -2472,6 +2559,7 @@ struct class_dict {
     dvec<uint64_t>& slot_hash;
     dvec<uint32_t>& slot_cid;
     uint64_t n = 0, nbits = 0, total_integers = 0, mask = 0;
+    uint64_t tabled = 0;  // classes in the table: the first batch needs none, later ones add the rest
 
     explicit class_dict(phase2_state& S)
         : cls_hash(S.cls_hash), bit_off(S.bit_off), words(S.words), slot_hash(S.slot_hash), slot_cid(S.slot_cid) {}
@@ -2488,12 +2576,12 @@ struct class_dict {
         cls_hash.n = 0;
     }
     dict_view view() const { return dict_view{slot_hash.p, slot_cid.p, mask, bit_off.p, words.p}; }
-    // Make room for n classes (load <= 1/2); classes [first_new, n) still need
-    // inserting.  A resized table is rebuilt from every class hash.
-    void ensure_table(uint64_t first_new, cudaStream_t st, uint32_t* d_err) {
+    // Every class in the table (load <= 1/2), before a lookup.  A resized table is
+    // rebuilt from every class hash.
+    void ensure_table(cudaStream_t st, uint32_t* d_err) {
         uint64_t cap = 1024;
         while (cap < 2 * n) cap <<= 1;
-        uint64_t from = first_new;
+        uint64_t from = tabled;
         if (!slot_hash.p || cap - 1 > mask) {
             slot_hash.reserve(cap, st);
             slot_cid.reserve(cap, st);
@@ -2506,6 +2594,35 @@ struct class_dict {
                                                               d_err);
             CDBG_CHECK_LAUNCH();
         }
+        tabled = n;
+    }
+};
+
+// A block of zeroed device words handed out piece by piece.
+struct zero_block {
+    unsigned long long* p;
+    uint64_t used = 0, cap;
+    zero_block(uint64_t words, dev_arena& A, cudaStream_t st) : cap(words) {
+        p = A.alloc<unsigned long long>(words);
+        CDBG_CUDA(cudaMemsetAsync(p, 0, 8 * words, st));
+    }
+    template <typename T>
+    T* take(uint64_t count) {
+        T* r = reinterpret_cast<T*>(p + used);
+        used += (count * sizeof(T) + 7) / 8;
+        if (used > cap) throw std::runtime_error("zero_block: block too small");
+        return r;
+    }
+    static uint64_t tiles(uint64_t n, uint64_t tile) { return std::max<uint64_t>(1, ceil_div(n, tile)); }
+    // words of an ordered selection over n elements
+    static uint64_t select_words(uint64_t n, uint64_t tile = prim::SEL_TILE) { return tiles(n, tile) + 2; }
+    select_ws select(uint64_t n, uint64_t tile = prim::SEL_TILE) {
+        select_ws w;
+        w.ntiles = tiles(n, tile);
+        w.status = take<unsigned long long>(w.ntiles);
+        w.total = take<unsigned long long>(1);
+        w.counter = take<uint32_t>(1);
+        return w;
     }
 };
 
@@ -2678,15 +2795,21 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         CDBG_CHECK_LAUNCH();
     }
     uint64_t counts[2];  // nodes, pairs
-    read_small(counts, ncnt + 2 * (ng & 1), 16, st);
+    uint32_t derr = 0;
+    mail_reader(st).add(counts, ncnt + 2 * (ng & 1), 16).add(&derr, d_err).wait();
     const uint64_t D = counts[0], npairs = counts[1];
     if (D >= (1ull << 31)) throw std::runtime_error("too many distinct k-mers in one bucket batch");
-    check_device_error_word(d_err, st, "k-mer table insert");
+    if (derr) check_device_error_word(d_err, st, "k-mer table insert");
+    // zeroed together: selections over the pairs, records, nodes and fragments,
+    // heavy-record flags, the chains' seed lengths and covered flags, counts
+    zero_block Z(3 * zero_block::select_words(npairs) + zero_block::select_words(nrec) + zero_block::select_words(D) +
+                     zero_block::select_words(D, 256) + nrec / 2 + D / 2 + D / 8 + 16,
+                 A, st);
     // ---- multi-record k-mers, from their (node, record) pairs
     uint64_t M = 0;
     uint32_t* mnode = nullptr;
     uint64_t* moff = nullptr;
-    uint64_t* upairs = nullptr;
+    uint32_t* urec = nullptr;
     uint32_t* msize = nullptr;
     uint64_t* mhash = nullptr;
     uint64_t* poff = nullptr;
@@ -2697,61 +2820,87 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     uint64_t* gbeg = nullptr;    // record range of each group
     uint64_t* gend = nullptr;
     uint32_t* mgrp = nullptr;    // group of each multi node
+    uint64_t nu = 0;
     if (npairs) {
         // stable by node (records already ascend within a node): the node bits only
         const int node_bits = D > 1 ? 64 - __builtin_clzll(D - 1) : 1;
         prim::radix_sort_pairs<uint32_t, uint32_t>(pnode, prec, npairs, 0, node_bits, A, st, d_err);
-        uint32_t* keep = A.alloc<uint32_t>(npairs);
-        uint64_t* kpos = A.alloc<uint64_t>(npairs + 1);
-        k_unique_pairs<<<grid(npairs, 256), 256, 0, st>>>(npairs, pnode, prec, keep);
-        CDBG_CHECK_LAUNCH();
-        prim::exclusive_scan<uint32_t, uint64_t>(keep, kpos, npairs, A, st, kpos + npairs);
-        const uint64_t nu = read_dev(kpos + npairs, st);
-        upairs = A.alloc<uint64_t>(nu);
-        k_compact_pairs<<<grid(npairs, 256), 256, 0, st>>>(npairs, pnode, prec, keep, kpos, upairs);
-        CDBG_CHECK_LAUNCH();
-        uint32_t* head = A.alloc<uint32_t>(nu);
-        uint64_t* hpos = A.alloc<uint64_t>(nu + 1);
-        k_node_heads<<<grid(nu, 256), 256, 0, st>>>(nu, upairs, head);
-        CDBG_CHECK_LAUNCH();
-        prim::exclusive_scan<uint32_t, uint64_t>(head, hpos, nu, A, st, hpos + nu);
-        M = read_dev(hpos + nu, st);
-        mnode = A.alloc<uint32_t>(M);
-        moff = A.alloc<uint64_t>(M + 1);
-        k_multi_index<<<grid(nu, 256), 256, 0, st>>>(nu, upairs, head, hpos, mnode, moff, n_rec);
-        CDBG_CHECK_LAUNCH();
-        k_set_u64<<<1, 1, 0, st>>>(moff + M, nu);
-        CDBG_CHECK_LAUNCH();
-        // one union per run of multi nodes with the same owning records
+        // (arrays sized for the pairs when those are few, else for the counts)
+        select_ws wk = Z.select(npairs), wh = Z.select(npairs);
+        urec = A.alloc<uint32_t>(npairs);
+        mnode = A.alloc<uint32_t>(npairs);
+        moff = A.alloc<uint64_t>(npairs + 1);
         {
-            uint32_t* ghead = A.alloc<uint32_t>(M);
-            uint64_t* gpos = A.alloc<uint64_t>(M + 1);
-            k_multi_same<<<grid(M, 256), 256, 0, st>>>(M, moff, upairs, ghead);
-            CDBG_CHECK_LAUNCH();
-            prim::exclusive_scan<uint32_t, uint64_t>(ghead, gpos, M, A, st, gpos + M);
-            G = read_dev(gpos + M, st);
-            gnode = A.alloc<uint32_t>(G);
-            gbeg = A.alloc<uint64_t>(G);
-            gend = A.alloc<uint64_t>(G);
-            mgrp = A.alloc<uint32_t>(M);
-            k_multi_groups<<<grid(M, 256), 256, 0, st>>>(M, ghead, gpos, mnode, moff, gnode, gbeg, gend, mgrp);
-            CDBG_CHECK_LAUNCH();
+            CDBG_PROF("k_multi_index", st);
+            k_multi_index<<<(unsigned)wk.ntiles, 256, 0, st>>>(npairs, pnode, prec, wk, wh, urec, mnode, moff, n_rec,
+                                                               d_err);
         }
+        CDBG_CHECK_LAUNCH();
+        mail_reader(st).add(&nu, wk.total).add(&M, wh.total).wait();
+        // one union per run of multi nodes with the same owning records
+        gnode = A.alloc<uint32_t>(M);
+        gbeg = A.alloc<uint64_t>(M);
+        gend = A.alloc<uint64_t>(M);
+        mgrp = A.alloc<uint32_t>(M);
+    }
+    // ---- counts the host needs next: union groups, heavy records (with a
+    // bitmap: unions of at least that many colors), records used as color sets
+    const uint32_t nw = (C + 31) / 32;
+    const uint32_t heavy = std::max<uint32_t>(1, p.heavy_colors);
+    const bool may_heavy = M && p.union_bitmaps && C >= heavy;
+    uint32_t* hflag = nullptr;
+    uint64_t* hpos = nullptr;
+    select_ws wg{}, wr = Z.select(nrec);
+    if (M) {
+        wg = Z.select(M);
+        {
+            CDBG_PROF("k_multi_groups", st);
+            k_multi_groups<<<(unsigned)wg.ntiles, 256, 0, st>>>(M, moff, urec, mnode, wg, gnode, gbeg, gend, mgrp,
+                                                                d_err);
+        }
+        CDBG_CHECK_LAUNCH();
+    }
+    if (may_heavy) {
+        hflag = Z.take<uint32_t>(nrec);
+        hpos = A.alloc<uint64_t>(nrec + 1);
+        k_heavy_flags<<<grid(nu, 256), 256, 0, st>>>(nu, urec, R.col_off, (uint32_t)R0, heavy, hflag);
+        CDBG_CHECK_LAUNCH();
+        prim::exclusive_scan<uint32_t, uint64_t>(hflag, hpos, nrec, A, st, hpos + nrec);
+    }
+    uint32_t* rec_first = A.alloc<uint32_t>(nrec);
+    CDBG_CUDA(cudaMemsetAsync(rec_first, 0xff, 4 * nrec, st));
+    {
+        CDBG_PROF("k_rec_first", st);
+        k_rec_first<<<grid(D, 256), 256, 0, st>>>(D, n_rec, (uint32_t)R0, rec_first);
+    }
+    CDBG_CHECK_LAUNCH();
+    // candidates: used records, then union groups
+    cand_view cv;
+    cv.kind_id = A.alloc<uint32_t>(nrec + M + 1);
+    cv.first = A.alloc<uint32_t>(nrec + M + 1);
+    cv.hash = A.alloc<uint64_t>(nrec + M + 1);
+    uint32_t* rec_cand = A.alloc<uint32_t>(nrec);
+    {
+        CDBG_PROF("k_cand_records", st);
+        k_cand_records<<<(unsigned)wr.ntiles, 256, 0, st>>>(nrec, (uint32_t)R0, rec_first, wr, d_rhash, cv, rec_cand,
+                                                            d_err);
+    }
+    CDBG_CHECK_LAUNCH();
+    uint64_t nrc = 0, nheavy = 0;
+    {
+        mail_reader mr(st);
+        mr.add(&nrc, wr.total);
+        if (M) mr.add(&G, wg.total);
+        if (may_heavy) mr.add(&nheavy, hpos + nrec);
+        mr.wait();
+    }
+    if (M) {
         msize = A.alloc<uint32_t>(G);
         mhash = A.alloc<uint64_t>(G);
-        const uint32_t nw = (C + 31) / 32;
         int wpb = (int)std::max<uint64_t>(1, std::min<uint64_t>(8, (96 * 1024) / (4ull * nw)));
         const size_t shm = (size_t)wpb * nw * 4;
         if (p.union_bitmaps) {
-            // heavy records (>= 64 colors) used by multi-record nodes get a bitmap once
-            uint32_t* hflag = A.alloc<uint32_t>(nrec);
-            uint64_t* hpos = A.alloc<uint64_t>(nrec + 1);
-            CDBG_CUDA(cudaMemsetAsync(hflag, 0, 4 * nrec, st));
-            k_heavy_flags<<<grid(nu, 256), 256, 0, st>>>(nu, upairs, R.col_off, (uint32_t)R0,
-                                                          std::max<uint32_t>(1, p.heavy_colors), hflag);
-            CDBG_CHECK_LAUNCH();
-            prim::exclusive_scan<uint32_t, uint64_t>(hflag, hpos, nrec, A, st, hpos + nrec);
-            const uint64_t nheavy = read_dev(hpos + nrec, st);
+            // heavy records used by multi-record nodes get a bitmap once
             uint32_t* rbits = A.alloc<uint32_t>(nheavy * nw + 1);
             if (shm > 48 * 1024)
                 CDBG_CUDA(cudaFuncSetAttribute(k_heavy_bitmaps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
@@ -2767,7 +2916,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
                 auto launch = [&](auto kern) {
                     if (shm > 48 * 1024)
                         CDBG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-                    kern<<<grid(G, wpb), wpb * 32, shm, st>>>(G, gbeg, gend, upairs, R.col_off, R.colors, (uint32_t)R0,
+                    kern<<<grid(G, wpb), wpb * 32, shm, st>>>(G, gbeg, gend, urec, R.col_off, R.colors, (uint32_t)R0,
                                                               hflag, hpos, rbits, nw, mbits, msize, mhash);
                 };
                 if (nw <= 32)
@@ -2789,7 +2938,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
             }
             {
                 CDBG_PROF("k_union", st);
-                k_union<false><<<grid(G, wpb), wpb * 32, shm, st>>>(G, gbeg, gend, upairs, R.col_off, R.colors, C,
+                k_union<false><<<grid(G, wpb), wpb * 32, shm, st>>>(G, gbeg, gend, urec, R.col_off, R.colors, C,
                                                                      msize, mhash, nullptr, nullptr);
             }
             CDBG_CHECK_LAUNCH();
@@ -2799,41 +2948,21 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
             pool = A.alloc<uint32_t>(ptot + 1);
             {
                 CDBG_PROF("k_union", st);
-                k_union<true><<<grid(G, wpb), wpb * 32, shm, st>>>(G, gbeg, gend, upairs, R.col_off, R.colors, C,
+                k_union<true><<<grid(G, wpb), wpb * 32, shm, st>>>(G, gbeg, gend, urec, R.col_off, R.colors, C,
                                                                     msize, mhash, poff, pool);
             }
             CDBG_CHECK_LAUNCH();
         }
     }
     out.n_multi += M;
-    // ---- candidates: used records, then multi nodes
-    uint32_t* rec_first = A.alloc<uint32_t>(nrec);
-    CDBG_CUDA(cudaMemsetAsync(rec_first, 0xff, 4 * nrec, st));
-    {
-        CDBG_PROF("k_rec_first", st);
-        k_rec_first<<<grid(D, 256), 256, 0, st>>>(D, n_rec, (uint32_t)R0, rec_first);
-    }
-    CDBG_CHECK_LAUNCH();
-    uint32_t* rkeep = A.alloc<uint32_t>(nrec);
-    uint64_t* rpos = A.alloc<uint64_t>(nrec + 1);
-    k_used_flags<<<grid(nrec, 256), 256, 0, st>>>(nrec, rec_first, rkeep);
-    CDBG_CHECK_LAUNCH();
-    prim::exclusive_scan<uint32_t, uint64_t>(rkeep, rpos, nrec, A, st, rpos + nrec);
-    const uint64_t nrc = read_dev(rpos + nrec, st);
     const uint64_t nc = nrc + G;
-    cand_view cv;
-    cv.kind_id = A.alloc<uint32_t>(nc + 1);
-    cv.first = A.alloc<uint32_t>(nc + 1);
-    cv.hash = A.alloc<uint64_t>(nc + 1);
-    uint32_t* rec_cand = A.alloc<uint32_t>(nrec);
-    k_cand_records<<<grid(nrec, 256), 256, 0, st>>>(nrec, (uint32_t)R0, rec_first, rkeep, rpos, d_rhash, cv, rec_cand);
-    CDBG_CHECK_LAUNCH();
     if (G) {
         k_cand_multi<<<grid(G, 256), 256, 0, st>>>(G, nrc, gnode, mhash, cv);
         CDBG_CHECK_LAUNCH();
     }
-    list_src L{R.col_off, R.colors, poff, pool, msize, mbits, (C + 31) / 32};
+    list_src L{R.col_off, R.colors, poff, pool, msize, mbits, nw};
     uint32_t* cid = A.alloc<uint32_t>(nc + 1);
+    unsigned long long* ints = Z.take<unsigned long long>(1);  // colors in the new classes
     if (nc) {
         // 1. group candidates with equal color sets (sort by set hash, then
         //    compare raw lists inside equal-hash runs)
@@ -2841,52 +2970,50 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         uint32_t* sidx = A.alloc<uint32_t>(nc);
         CDBG_CUDA(cudaMemcpyAsync(skey, cv.hash, 8 * nc, cudaMemcpyDeviceToDevice, st));
         prim::sort_pairs_u64_exact<uint32_t>(skey, sidx, nc, A, st, d_err, true);
-        uint32_t* head = A.alloc<uint32_t>(nc);
-        uint64_t* hpos = A.alloc<uint64_t>(nc + 1);
-        k_run_heads<<<grid(nc, 256), 256, 0, st>>>(nc, skey, head);
-        CDBG_CHECK_LAUNCH();
-        prim::exclusive_scan<uint32_t, uint64_t>(head, hpos, nc, A, st, hpos + nc);
-        const uint64_t nruns = read_dev(hpos + nc, st);
-        uint64_t* run_start = A.alloc<uint64_t>(nruns + 1);
-        k_run_starts<<<grid(nc, 256), 256, 0, st>>>(nc, head, hpos, run_start);
-        CDBG_CHECK_LAUNCH();
+        // zeroed together: selections of runs, representatives (twice) and new
+        // ones, the runs' collision flags, counts
+        zero_block Y(4 * zero_block::select_words(nc) + nc / 2 + 8, A, st);
+        uint32_t* run = A.alloc<uint32_t>(nc);
+        uint32_t* run_start = A.alloc<uint32_t>(nc);
         uint32_t* rep = A.alloc<uint32_t>(nc);
         uint32_t* rep_first = A.alloc<uint32_t>(nc);
-        uint32_t* collided = A.alloc<uint32_t>(nruns + 1);
-        CDBG_CUDA(cudaMemsetAsync(rep_first, 0xff, 4 * nc, st));
-        CDBG_CUDA(cudaMemsetAsync(collided, 0, 4 * (nruns + 1), st));
+        select_ws wq = Y.select(nc), wp = Y.select(nc), wp2 = Y.select(nc), wn = Y.select(nc);
+        uint32_t* collided = Y.take<uint32_t>(nc);
+        uint32_t* any_collided = Y.take<uint32_t>(1);
+        {
+            CDBG_PROF("k_hash_runs", st);
+            k_hash_runs<<<(unsigned)wq.ntiles, 256, 0, st>>>(nc, skey, wq, run, run_start, rep_first, d_err);
+        }
+        CDBG_CHECK_LAUNCH();
         {
             CDBG_PROF("k_member_match", st);
-            k_member_match_raw<<<grid(nc, 256), 256, 0, st>>>(nc, head, hpos, run_start, sidx, cv, L, rep, rep_first,
-                                                               collided);
+            k_member_match_raw<<<grid(nc, 256), 256, 0, st>>>(nc, run, run_start, sidx, cv, L, rep, rep_first, collided,
+                                                               any_collided);
         }
         CDBG_CHECK_LAUNCH();
-        {
-            unsigned long long* ncol = A.alloc<unsigned long long>(1);
-            CDBG_CUDA(cudaMemsetAsync(ncol, 0, 8, st));
-            k_count_flags<<<grid(nruns, 256), 256, 0, st>>>(nruns, collided, ncol);
-            CDBG_CHECK_LAUNCH();
-            if (read_dev(ncol, st)) {
-                k_group_collided_raw<<<grid(nruns, 128), 128, 0, st>>>(nruns, collided, run_start, nc, sidx, cv, L,
-                                                                       rep, rep_first);
-                CDBG_CHECK_LAUNCH();
-            }
-        }
         // 2. representatives: compact, encode, look up in the dictionary
-        uint32_t* is_rep = A.alloc<uint32_t>(nc);
-        uint64_t* rpos = A.alloc<uint64_t>(nc + 1);
-        k_rep_flags<<<grid(nc, 256), 256, 0, st>>>(nc, rep, is_rep);
-        CDBG_CHECK_LAUNCH();
-        prim::exclusive_scan<uint32_t, uint64_t>(is_rep, rpos, nc, A, st, rpos + nc);
-        const uint64_t nr = read_dev(rpos + nc, st);
         cand_view rv;
-        rv.kind_id = A.alloc<uint32_t>(nr + 1);
-        rv.first = A.alloc<uint32_t>(nr + 1);
-        rv.hash = A.alloc<uint64_t>(nr + 1);
+        rv.kind_id = A.alloc<uint32_t>(nc + 1);
+        rv.first = A.alloc<uint32_t>(nc + 1);
+        rv.hash = A.alloc<uint64_t>(nc + 1);
         uint32_t* rep_index = A.alloc<uint32_t>(nc);
-        k_rep_compact<<<grid(nc, 256), 256, 0, st>>>(nc, is_rep, rpos, cv, rep_first, rv, rep_index);
-        CDBG_CHECK_LAUNCH();
-        const uint32_t nw = (C + 31) / 32;
+        auto compact_reps = [&](select_ws w) {
+            CDBG_PROF("k_rep_compact", st);
+            k_rep_compact<<<(unsigned)w.ntiles, 256, 0, st>>>(nc, rep, w, cv, rep_first, rv, rep_index, d_err);
+            CDBG_CHECK_LAUNCH();
+        };
+        compact_reps(wp);
+        uint64_t nr = 0, nruns = 0;
+        uint32_t any = 0;
+        mail_reader(st).add(&nr, wp.total).add(&nruns, wq.total).add(&any, any_collided).wait();
+        if (any) {
+            // equal hashes of different sets: those runs grouped exactly
+            k_group_collided_raw<<<grid(nruns, 128), 128, 0, st>>>(nruns, collided, run_start, nc, sidx, cv, L, rep,
+                                                                   rep_first);
+            CDBG_CHECK_LAUNCH();
+            compact_reps(wp2);
+            nr = read_dev(wp2.total, st);
+        }
         int wpb = (int)std::max<uint64_t>(1, std::min<uint64_t>(8, (96 * 1024) / (4ull * nw)));
         const size_t shm = (size_t)wpb * nw * 4;
         if (shm > 48 * 1024) {
@@ -2910,37 +3037,43 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
             k_encode<true><<<grid(ceil_div(nr, 32), wpb), wpb * 32, shm, st>>>(nr, rv, L, C, nullptr, cb, cw);
         }
         CDBG_CHECK_LAUNCH();
+        // 3. new classes in order of first appearance.  An empty dictionary (the
+        // first batch) holds none of them.
         uint32_t* rcid = A.alloc<uint32_t>(nr + 1);
-        {
-            CDBG_PROF("k_dict_lookup", st);
-            k_dict_lookup<<<grid(nr, 256), 256, 0, st>>>(nr, rv, cw, cb, dict.view(), rcid);
-        }
-        CDBG_CHECK_LAUNCH();
-        // 3. new classes in order of first appearance
-        uint32_t* nflag = A.alloc<uint32_t>(nr);
-        uint64_t* npos = A.alloc<uint64_t>(nr + 1);
-        k_new_flags<<<grid(nr, 256), 256, 0, st>>>(nr, rcid, nflag);
-        CDBG_CHECK_LAUNCH();
-        prim::exclusive_scan<uint32_t, uint64_t>(nflag, npos, nr, A, st, npos + nr);
-        const uint64_t nnew = read_dev(npos + nr, st);
-        if (nnew) {
-            uint64_t* rkey = A.alloc<uint64_t>(nnew);
-            uint32_t* rcand = A.alloc<uint32_t>(nnew);
-            k_new_reps<<<grid(nr, 256), 256, 0, st>>>(nr, rcid, npos, rv, rkey, rcand);
+        const bool all_new = dict.n == 0;
+        uint64_t nnew = nr;
+        uint32_t* rkey = rv.first;
+        uint32_t* rcand = A.alloc<uint32_t>(nr);
+        if (!all_new) {
+            dict.ensure_table(st, d_err);
+            {
+                CDBG_PROF("k_dict_lookup", st);
+                k_dict_lookup<<<grid(nr, 256), 256, 0, st>>>(nr, rv, cw, cb, dict.view(), rcid);
+            }
             CDBG_CHECK_LAUNCH();
-            prim::radix_sort_pairs<uint32_t>(rkey, rcand, nnew, 0, 32, A, st, d_err);
+            rkey = A.alloc<uint32_t>(nr);
+            {
+                CDBG_PROF("k_new_reps", st);
+                k_new_reps<<<(unsigned)zero_block::tiles(nr, prim::SEL_TILE), 256, 0, st>>>(
+                    nr, rcid, select_ws{wn.status, wn.total, wn.counter, zero_block::tiles(nr, prim::SEL_TILE)}, rv, rkey,
+                    rcand, d_err);
+            }
+            CDBG_CHECK_LAUNCH();
+            nnew = read_dev(wn.total, st);
+        }
+        if (nnew) {
+            const int node_bits = D > 1 ? 64 - __builtin_clzll(D - 1) : 1;
+            prim::radix_sort_pairs<uint32_t, uint32_t>(rkey, rcand, nnew, 0, node_bits, A, st, d_err, all_new);
             const uint64_t base = dict.n;
             k_assign_new<<<grid(nnew, 256), 256, 0, st>>>(nnew, rcand, base, rcid);
             CDBG_CHECK_LAUNCH();
             uint64_t* nbits = A.alloc<uint64_t>(nnew);
             uint64_t* nh = A.alloc<uint64_t>(nnew);
             uint64_t* boff = A.alloc<uint64_t>(nnew + 1);
-            unsigned long long* ints = A.alloc<unsigned long long>(1);
-            CDBG_CUDA(cudaMemsetAsync(ints, 0, 8, st));
             k_new_sizes<<<grid(nnew, 256), 256, 0, st>>>(nnew, rcand, rv, L, cb, nbits, nh, ints);
             CDBG_CHECK_LAUNCH();
             prim::exclusive_scan<uint64_t, uint64_t>(nbits, boff, nnew, A, st, boff + nnew);
-            const uint64_t badd = read_dev(boff + nnew, st);
+            const uint64_t badd = all_new ? ctot : read_dev(boff + nnew, st);
             add_offsets(boff, nnew + 1, dict.nbits, boff, st);  // absolute bit offsets
             if (p.copy_st && (dict.bit_off.cap < base + nnew + 1 ||
                               dict.words.cap < (dict.nbits + badd + 63) / 64 + 4)) {
@@ -2958,13 +3091,11 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
                 k_append_bits<<<grid(nnew, 8), 256, 0, st>>>(nnew, rcand, cw, cb, boff, dict.words.p);
             }
             CDBG_CHECK_LAUNCH();
-            dict.total_integers += read_dev(ints, st);
             dict.n = base + nnew;
             dict.cls_hash.n = dict.n;
             dict.bit_off.n = dict.n + 1;
             dict.nbits += badd;
             dict.words.n = (dict.nbits + 63) / 64;
-            dict.ensure_table(base, st, d_err);
         }
         // 4. every candidate takes its representative's class id
         k_cand_cid<<<grid(nc, 256), 256, 0, st>>>(nc, rep, rep_index, rcid, cid);
@@ -2988,34 +3119,33 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     W.ch_vis = A.alloc<uint8_t>(D);
     W.fe = A.alloc<uint32_t>(D);
     W.seed_start = A.alloc<uint32_t>(D);
-    W.seed_len = A.alloc<uint32_t>(D);
+    W.seed_len = Z.take<uint32_t>(D);
     W.seed_open = A.alloc<uint8_t>(D);
-    W.covered = A.alloc<uint8_t>(D);
-    W.cursor = A.alloc<unsigned long long>(1);
+    W.covered = Z.take<uint8_t>(D);
+    W.cursor = Z.take<unsigned long long>(1);
     W.D = D;
-    CDBG_CUDA(cudaMemsetAsync(W.seed_len, 0, 4 * D, st));
-    CDBG_CUDA(cudaMemsetAsync(W.covered, 0, D, st));
-    CDBG_CUDA(cudaMemsetAsync(W.cursor, 0, 8, st));
     {
         uint32_t* ends = A.alloc<uint32_t>(D);
-        unsigned long long* cnt2 = A.alloc<unsigned long long>(2);
-        CDBG_CUDA(cudaMemsetAsync(cnt2, 0, 16, st));
+        unsigned long long* cnt2 = Z.take<unsigned long long>(2);
         {
             CDBG_PROF("k_chain_ends", st);
             k_chain_ends<<<grid(D, 256), 256, 0, st>>>(W, ends, cnt2);
         }
         CDBG_CHECK_LAUNCH();
-        const uint64_t nends = read_dev(cnt2, st);
+        // grids and the heads sized for D ends when that is cheaper than the waits
+        // for their number (about 10 us each)
+        const bool wait = D > (1ull << 21);
+        const uint64_t nends = wait ? read_dev(cnt2, st) : D;
         uint4* heads = A.alloc<uint4>(nends + 1);
         if (nends) {
             CDBG_PROF("k_chain_lead", st);
-            k_chain_lead<<<grid(nends, 256), 256, 0, st>>>(W, ends, nends, heads, cnt2 + 1, d_err);
+            k_chain_lead<<<grid(nends, 256), 256, 0, st>>>(W, ends, cnt2, heads, cnt2 + 1, d_err);
         }
         CDBG_CHECK_LAUNCH();
-        const uint64_t nheads = read_dev(cnt2 + 1, st);
+        const uint64_t nheads = wait ? read_dev(cnt2 + 1, st) : nends;
         if (nheads) {
             CDBG_PROF("k_chain_paths", st);
-            k_chain_paths<<<grid(nheads, 128), 128, 0, st>>>(W, heads, nheads);
+            k_chain_paths<<<grid(nheads, 128), 128, 0, st>>>(W, heads, cnt2 + 1);
         }
         CDBG_CHECK_LAUNCH();
     }
@@ -3025,35 +3155,47 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     }
     CDBG_CHECK_LAUNCH();
     // ---- fragments, in seed order
-    uint32_t* is_seed = A.alloc<uint32_t>(D);
-    uint64_t* fpos = A.alloc<uint64_t>(D + 1);
-    k_seed_flags<<<grid(D, 256), 256, 0, st>>>(D, W.seed_len, is_seed);
-    CDBG_CHECK_LAUNCH();
-    prim::exclusive_scan<uint32_t, uint64_t>(is_seed, fpos, D, A, st, fpos + D);
-    const uint64_t nfr = read_dev(fpos + D, st);
-    check_device_error_word(d_err, st, "unitig walk");
-    uint32_t* seed_of = A.alloc<uint32_t>(nfr + 1);
-    k_seed_list<<<grid(D, 256), 256, 0, st>>>(D, is_seed, fpos, seed_of);
-    CDBG_CHECK_LAUNCH();
-    uint64_t* fsz = A.alloc<uint64_t>(nfr + 1);
-    uint64_t* foff = A.alloc<uint64_t>(nfr + 1);
-    unsigned long long* seqt = A.alloc<unsigned long long>(1);
-    CDBG_CUDA(cudaMemsetAsync(seqt, 0, 8, st));
-    if (nfr) {
-        CDBG_PROF("k_frag_sizes", st);
-        k_frag_sizes<<<grid(nfr, 256), 256, 0, st>>>(nfr, seed_of, W.seed_start, W.seed_len, W.fe, n_cid, k, fsz, seqt);
+    uint32_t* seed_of = A.alloc<uint32_t>(D);
+    select_ws wseed = Z.select(D), wfrag = Z.select(D, 256);
+    {
+        CDBG_PROF("k_seed_list", st);
+        k_seed_list<<<(unsigned)wseed.ntiles, 256, 0, st>>>(D, W.seed_len, wseed, seed_of, d_err);
     }
     CDBG_CHECK_LAUNCH();
-    prim::exclusive_scan<uint64_t, uint64_t>(fsz, foff, nfr, A, st, foff + nfr);
-    const uint64_t fbytes = read_dev(foff + nfr, st);
-    uint8_t* fb = A.alloc<uint8_t>(fbytes + 8);
+    uint64_t nfr = 0;
+    mail_reader(st).add(&nfr, wseed.total).add(&derr, d_err).wait();
+    if (derr) check_device_error_word(d_err, st, "unitig walk");
+    uint64_t* foff = A.alloc<uint64_t>(nfr + 1);
+    unsigned long long* seqt = Z.take<unsigned long long>(1);
+    if (nfr) {
+        CDBG_PROF("k_frag_sizes", st);
+        k_frag_sizes<<<grid(nfr, 256), 256, 0, st>>>(nfr, seed_of, W.seed_start, W.seed_len, W.fe, n_cid, k, wfrag, foff,
+                                                     seqt, d_err);
+    }
+    CDBG_CHECK_LAUNCH();
+    uint64_t fbytes = 0, seq_total = 0, new_ints = 0;
+    mail_reader(st).add(&fbytes, wfrag.total).add(&seq_total, seqt).add(&new_ints, ints).wait();
+    dict.total_integers += new_ints;
+    const uint64_t frag_old = dfrag.n;
+    uint8_t* fb = nullptr;  // the fragments: scratch on their way to the host, or where the output stays
+    if (p.to_host) {
+        fb = A.alloc<uint8_t>(fbytes + 16);
+    } else {
+        if (p.copy_st && dfrag.n + fbytes + 16 > dfrag.cap) {
+            // growing frees the old buffer: after the host copies that read it
+            CDBG_CUDA(cudaEventRecord(p.copy_ev, p.copy_st));
+            CDBG_CUDA(cudaStreamWaitEvent(st, p.copy_ev, 0));
+        }
+        dfrag.reserve(dfrag.n + fbytes + 16, st);
+        fb = dfrag.p;
+    }
     if (nfr) {
         CDBG_PROF("k_frag_write", st);
         k_frag_write<K><<<grid(nfr, FW_THREADS), FW_THREADS, 0, st>>>(nfr, seed_of, W.seed_start, W.seed_len,
-                                                                       W.seed_open, W.fe, n_cid, n_key, k, foff, fb);
+                                                                       W.seed_open, W.fe, n_cid, n_key, k, foff,
+                                                                       p.to_host ? 0 : frag_old, fb);
     }
     CDBG_CHECK_LAUNCH();
-    const uint64_t seq_total = read_dev(seqt, st);
     out.n_fragments += nfr;
     out.total_seq_bytes += seq_total;
     out.n_occ += nocc;
@@ -3063,14 +3205,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         out.frag.resize(o + fbytes);
         CDBG_CUDA(cudaMemcpyAsync(out.frag.data() + o, fb, fbytes, cudaMemcpyDeviceToHost, st));
     } else {
-        const uint64_t old_n = dfrag.n;
-        if (p.copy_st && dfrag.n + fbytes + 8 > dfrag.cap) {
-            // growing frees the old buffer: after the host copies that read it
-            CDBG_CUDA(cudaEventRecord(p.copy_ev, p.copy_st));
-            CDBG_CUDA(cudaStreamWaitEvent(st, p.copy_ev, 0));
-        }
-        dfrag.reserve(dfrag.n + fbytes + 8, st);
-        CDBG_CUDA(cudaMemcpyAsync(dfrag.p + dfrag.n, fb, fbytes, cudaMemcpyDeviceToDevice, st));
+        const uint64_t old_n = frag_old;
         dfrag.n += fbytes;
         if (p.keep_frag_offsets && nfr) {
             dfoff.reserve(dfoff.n + nfr + 1, st);
@@ -3108,7 +3243,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
             out.offs_host_copied = dict.n;
         }
     }
-    CDBG_CUDA(cudaStreamSynchronize(st));
+    if (p.to_host) CDBG_CUDA(cudaStreamSynchronize(st));
     out.frag_nbytes += fbytes;
     check_device_error_word(d_err, st, "phase-2 batch");
     A.release(mark);
@@ -3143,8 +3278,10 @@ void run_all(record_set const& rs, phase2_params const& p, dev_arena& A, cudaStr
     k_gather_u64<<<grid(B + 1, 256), 256, 0, st>>>(B + 1, occ, rs.bucket_start, d_bocc);
     CDBG_CHECK_LAUNCH();
     std::vector<uint64_t> bocc(B + 1), hbstart(B + 1);
-    read_small(bocc.data(), d_bocc, 8ull * (B + 1), st);
-    read_small(hbstart.data(), rs.bucket_start, 8ull * (B + 1), st);
+    mail_reader(st)
+        .add(bocc.data(), d_bocc, 8ull * (B + 1))
+        .add(hbstart.data(), rs.bucket_start, 8ull * (B + 1))
+        .wait();
     uint64_t budget = p.batch_occ;
     if (budget == 0) {
         int dev = 0;
@@ -3163,6 +3300,7 @@ void run_all(record_set const& rs, phase2_params const& p, dev_arena& A, cudaStr
         dict.nbits = S.nbits;
         dict.total_integers = S.total_integers;
         dict.mask = S.mask;
+        dict.tabled = S.tabled;
     } else {
         dict.init(st);
     }
@@ -3188,6 +3326,7 @@ void run_all(record_set const& rs, phase2_params const& p, dev_arena& A, cudaStr
     S.nbits = dict.nbits;
     S.total_integers = dict.total_integers;
     S.mask = dict.mask;
+    S.tabled = dict.tabled;
     out.n_classes = dict.n;
     out.nbits = dict.nbits;
     out.total_integers = dict.total_integers;

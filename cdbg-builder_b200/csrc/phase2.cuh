@@ -25,6 +25,7 @@ struct phase2_state {
     dvec<uint64_t> frag_off;   // their record offsets (phase2_params::keep_frag_offsets)
     // dictionary size, kept so that a later call can continue it
     uint64_t n = 0, nbits = 0, total_integers = 0, mask = 0;
+    uint64_t tabled = 0;  // classes in the hash table
     // Order later frees on `st` (after a stream switch).
     void set_stream(cudaStream_t st) {
         cls_hash.st_last = bit_off.st_last = words.st_last = slot_hash.st_last = st;

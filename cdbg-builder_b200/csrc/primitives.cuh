@@ -109,6 +109,53 @@ __device__ __forceinline__ bool lookback_exclusive(unsigned long long* status, u
     return ok;
 }
 
+// Positions of the selected elements of a tile of SEL_TILE = 4 rounds x 256
+// threads among all selected ones, in element order: element tile * SEL_TILE +
+// round * 256 + thread.  Every thread of the 256 calls all three.
+constexpr int SEL_ROUNDS = 4;
+constexpr int SEL_TILE = SEL_ROUNDS * 256;
+struct ordered_select {
+    uint32_t bal[32];   // selected lanes of (round, warp)
+    uint32_t cnt[32];   // selected before (round, warp) in the tile
+    uint64_t tile, base;
+};
+__device__ __forceinline__ uint64_t select_tile(ordered_select& s, uint32_t* tile_counter) {
+    if (threadIdx.x == 0) s.tile = atomicAdd(tile_counter, 1u);
+    __syncthreads();
+    return s.tile;
+}
+// Bit r of `sel`: this thread's element of round r is selected.  The last tile
+// stores the total.
+__device__ __forceinline__ void select_rank(ordered_select& s, uint32_t sel, uint64_t tile, uint64_t ntiles,
+                                            unsigned long long* status, unsigned long long* total, uint32_t* err) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int r = 0; r < SEL_ROUNDS; ++r) {
+        const uint32_t b = __ballot_sync(0xffffffffu, (sel >> r) & 1u);
+        if (lane == 0) s.bal[r * 8 + warp] = b;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const uint32_t c = __popc(s.bal[lane]);
+        const uint32_t x = warp_inclusive_scan(c);
+        const uint32_t tot = __shfl_sync(0xffffffffu, x, 31);
+        s.cnt[lane] = x - c;
+        uint64_t excl = 0;
+        const bool ok = lookback_exclusive(status, tile, tot, excl);
+        if (lane == 0) {
+            if (!ok) set_error(err, ERR_CHAIN_LIMIT);
+            s.base = excl;
+            if (tile == ntiles - 1) *total = excl + tot;
+        }
+    }
+    __syncthreads();
+}
+// Selected elements before this thread's element of round r.
+__device__ __forceinline__ uint64_t select_pos(ordered_select const& s, int r) {
+    const int i = r * 8 + (int)(threadIdx.x >> 5);
+    return s.base + s.cnt[i] + __popc(s.bal[i] & lanemask_lt());
+}
+
 // ------------------------------------------------------------------ scan
 // Shared-memory index of tile element j, padded so that a thread reading its
 // consecutive elements meets no bank conflict (4- and 8-byte types).
