@@ -879,11 +879,12 @@ __global__ void __launch_bounds__(256)
               uint64_t* __restrict__ r_coloff, uint32_t* __restrict__ colors, uint64_t* __restrict__ bucket_start,
               unsigned long long* __restrict__ tot, uint32_t* err) {
     constexpr int NW = 256 / 32, TILE = RC_ROUNDS * 256;
-    static_assert(RC_ROUNDS * NW == 32, "warp 0 scans one count per lane");
+    static_assert(RC_ROUNDS * NW == 32, "a warp scans one count per lane");
     // position base + j of the tile at j + 1, its predecessor at 0
     __shared__ uint64_t s_key[TILE + 1], s_start[TILE + 1];
     __shared__ uint32_t s_len[TILE + 1], s_color[TILE + 1];
     __shared__ uint32_t whead[RC_ROUNDS * NW], wcol[RC_ROUNDS * NW], wcnt[RC_ROUNDS * NW];
+    __shared__ uint32_t brec[RC_ROUNDS * NW], bcol[RC_ROUNDS * NW];  // records, colors before (round, warp)
     __shared__ uint64_t s_tile, s_r, s_c;
     if (threadIdx.x == 0) s_tile = atomicAdd(tile_counter, 1u);
     __syncthreads();
@@ -936,22 +937,17 @@ __global__ void __launch_bounds__(256)
         }
     }
     __syncthreads();
-    if (warp == 0) {
-        const uint32_t c = wcnt[lane];
+    if (warp < 2) {  // warp 0: records, warp 1: colors
+        const uint32_t c = (wcnt[lane] >> (16 * warp)) & 0xffffu;
         const uint32_t x = prim::warp_inclusive_scan(c);
         const uint32_t t = __shfl_sync(0xffffffffu, x, 31);
-        wcnt[lane] = x - c;
-        uint64_t er = 0, ec = 0;
-        const bool ok_r = prim::lookback_exclusive(status_r, tile, t & 0xffffu, er);
-        const bool ok_c = prim::lookback_exclusive(status_c, tile, t >> 16, ec);
+        (warp == 0 ? brec : bcol)[lane] = x - c;
+        uint64_t excl = 0;
+        const bool ok = prim::lookback_exclusive(warp == 0 ? status_r : status_c, tile, t, excl);
         if (lane == 0) {
-            if (!ok_r || !ok_c) set_error(err, ERR_CHAIN_LIMIT);
-            s_r = er;
-            s_c = ec;
-            if (tile == ntiles - 1) {
-                tot[0] = er + (t & 0xffffu);
-                tot[1] = ec + (t >> 16);
-            }
+            if (!ok) set_error(err, ERR_CHAIN_LIMIT);
+            (warp == 0 ? s_r : s_c) = excl;
+            if (tile == ntiles - 1) tot[warp] = excl + t;
         }
     }
     __syncthreads();
@@ -963,8 +959,8 @@ __global__ void __launch_bounds__(256)
         const uint32_t i = rr * NW + warp, j = 256u * rr + threadIdx.x;
         const bool h = (head >> rr) & 1u, c = (ckeep >> rr) & 1u;
         // the record holding p (its heads up to and including p, less one)
-        const uint64_t rid = r0 + (wcnt[i] & 0xffffu) + __popc(whead[i] & lt) + (h ? 1 : 0) - 1;
-        const uint64_t cat = c0 + (wcnt[i] >> 16) + __popc(wcol[i] & lt);
+        const uint64_t rid = r0 + brec[i] + __popc(whead[i] & lt) + (h ? 1 : 0) - 1;
+        const uint64_t cat = c0 + bcol[i] + __popc(wcol[i] & lt);
         if (h) {
             r_start[rid] = start[rr];
             r_len[rid] = len[rr];

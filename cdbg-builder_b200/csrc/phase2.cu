@@ -699,8 +699,14 @@ __global__ void __launch_bounds__(256) k_multi_index(uint64_t n, uint32_t const*
         if (h) sh |= 1u << r;
         if (h || pr[i - 1] != rec[r]) sk |= 1u << r;
     }
-    prim::select_rank(keep, sk, tile, wk.ntiles, wk.status, wk.total, err);
-    prim::select_rank(head, sh, tile, wk.ntiles, wh.status, wh.total, err);
+    prim::select_put(keep, sk);
+    prim::select_put(head, sh);
+    __syncthreads();
+    if (threadIdx.x < 32)
+        prim::select_scan(keep, tile, wk.ntiles, wk.status, wk.total, err);
+    else if (threadIdx.x < 64)
+        prim::select_scan(head, tile, wk.ntiles, wh.status, wh.total, err);
+    __syncthreads();
 #pragma unroll
     for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
         const uint64_t i = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
@@ -1960,53 +1966,51 @@ __device__ __forceinline__ uint32_t back_nib(uint32_t m, bool rc) { return (rc ?
 
 // link[2n] = L port, link[2n+1] = R port: (node << 1) | rc of the state
 // reached, NONE32 when the step is not clean.  On entry link holds the
-// sides' only neighbours as k_ext_mask found them.
+// sides' only neighbours as k_ext_mask found them.  Nodes with at most one
+// linked port, the path ends, are appended to `ends`.
 template <typename K>
 __global__ void __launch_bounds__(256, 8) k_links(unsigned long long const* nb, unsigned long long const* ne,
                                                   K const* __restrict__ n_key, uint8_t const* __restrict__ n_mask,
-                                                  uint32_t k,
-                                                  uint32_t* __restrict__ link) {
+                                                  uint32_t k, uint32_t* __restrict__ link, uint32_t* __restrict__ ends,
+                                                  unsigned long long* nends) {
     const uint64_t n = *nb + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= *ne) return;
-    typedef kmer_ops<K> ops;
-    const K can = n_key[n];
-    const uint32_t m = n_mask[n];
-    const K msk = ops::mask(k);
-    const uint32_t top = 2 * (k - 1);
-    const uint32_t nibr = fwd_nib(m, false), nibl = back_nib(m, false);
-    const K rev = (__popc(nibr) == 1 || __popc(nibl) == 1) ? ops::revcomp(can, k) : can;
-    // R: forward from (can, rc = false)
-    uint32_t lr = NONE32, ll = NONE32;
-    {
-        const uint32_t nib = nibr;
-        if (__popc(nib) == 1) {
-            const uint32_t nt = __ffs(nib) - 1;
+    if (*nb + (uint64_t)blockIdx.x * blockDim.x >= *ne) return;  // whole block
+    bool end = false;
+    if (n < *ne) {
+        typedef kmer_ops<K> ops;
+        const K can = n_key[n];
+        const uint32_t m = n_mask[n];
+        const uint2 only = reinterpret_cast<uint2 const*>(link)[n];
+        const K msk = ops::mask(k);
+        const uint32_t top = 2 * (k - 1);
+        const K rev = only.x != NONE32 || only.y != NONE32 ? ops::revcomp(can, k) : can;
+        uint32_t lr = NONE32, ll = NONE32;
+        // R: forward from (can, rc = false)
+        if (only.y != NONE32) {
+            const uint32_t nt = __ffs(fwd_nib(m, false)) - 1;
             const K nf = ((can << 2) | (K)nt) & msk;
             const K nr = (rev >> 2) | ((K)(3u - nt) << top);
             const bool nrc = !(nf <= nr);
-            const uint32_t nn = link[2 * n + 1];
-            if (nn != NONE32 && __popc(back_nib(n_mask[nn], nrc)) == 1) lr = (nn << 1) | (nrc ? 1u : 0u);
+            if (__popc(back_nib(n_mask[only.y], nrc)) == 1) lr = (only.y << 1) | (nrc ? 1u : 0u);
         }
-    }
-    // L: backward from (can, rc = false) = bstep(can, rc = true) then flip
-    {
-        const uint32_t nib = nibl;
-        if (__popc(nib) == 1) {
-            const uint32_t nt = __ffs(nib) - 1;
+        // L: backward from (can, rc = false) = bstep(can, rc = true) then flip
+        if (only.x != NONE32) {
+            const uint32_t nt = __ffs(back_nib(m, false)) - 1;
             const K nf = ((rev << 2) | (K)nt) & msk;
             const K nr = (can >> 2) | ((K)(3u - nt) << top);
             const bool srcc = !(nf <= nr);
             const bool nrc = !srcc;
-            const uint32_t nn = link[2 * n];
-            if (nn != NONE32 && __popc(fwd_nib(n_mask[nn], nrc)) == 1) ll = (nn << 1) | (nrc ? 1u : 0u);
+            if (__popc(fwd_nib(n_mask[only.x], nrc)) == 1) ll = (only.x << 1) | (nrc ? 1u : 0u);
         }
+        // a port linked to the node itself ends the chain (the reference's walk
+        // meets its own visited k-mer there)
+        if (lr != NONE32 && (lr >> 1) == (uint32_t)n) lr = NONE32;
+        if (ll != NONE32 && (ll >> 1) == (uint32_t)n) ll = NONE32;
+        reinterpret_cast<uint2*>(link)[n] = make_uint2(ll, lr);
+        end = ll == NONE32 || lr == NONE32;
     }
-    // a port linked to the node itself ends the chain (the reference's walk
-    // meets its own visited k-mer there)
-    if (lr != NONE32 && (lr >> 1) == (uint32_t)n) lr = NONE32;
-    if (ll != NONE32 && (ll >> 1) == (uint32_t)n) ll = NONE32;
-    link[2 * n] = ll;
-    link[2 * n + 1] = lr;
+    const unsigned long long at = block_reserve<256>(end ? 1u : 0u, nends);
+    if (end) ends[at] = (uint32_t)n;
 }
 
 // ---- chains ---------------------------------------------------------------
@@ -2019,9 +2023,10 @@ struct chain_ws {
     unsigned long long* ch_ord;
     uint8_t* ch_vis;
     uint32_t* fe;            // fragment elements (node << 1 | walk rc)
+    uint32_t const* n_cid;
     uint32_t* seed_start;    // per seed node: offset into fe
     uint32_t* seed_len;      // per seed node: elements (0 = not a seed)
-    uint8_t* seed_open;
+    uint32_t* seed_info;     // per seed node: color runs << 2 | open right << 1 | open left
     uint8_t* covered;
     unsigned long long* cursor;
     uint64_t D;
@@ -2034,6 +2039,20 @@ __device__ __forceinline__ bool chain_step(uint32_t const* link, uint32_t& c, bo
     c = l >> 1;
     rc = ((l & 1u) != 0) != rc;
     return true;
+}
+
+// Seed s's fragment: fe[start .. start + len), already stored, by this thread.
+__device__ __forceinline__ void put_seed(chain_ws const& W, uint32_t s, uint64_t start, uint32_t len, bool open_l,
+                                         bool open_r) {
+    uint32_t runs = 1, prev = W.n_cid[W.fe[start] >> 1];
+    for (uint32_t j = 1; j < len; ++j) {
+        const uint32_t c = W.n_cid[W.fe[start + j] >> 1];
+        runs += c != prev;
+        prev = c;
+    }
+    W.seed_start[s] = (uint32_t)start;
+    W.seed_len[s] = len;
+    W.seed_info[s] = (runs << 2) | (open_r ? 2u : 0u) | (open_l ? 1u : 0u);
 }
 
 __device__ void heap_sort(unsigned long long* a, uint32_t n) {
@@ -2131,9 +2150,7 @@ __device__ void simulate_chain(chain_ws const& W, uint64_t c0, uint32_t L, bool 
             const bool wrc = (df == 1) ? (crc[q] != 0) : (crc[q] == 0);
             W.fe[fcur + j] = (cn[q] << 1) | (wrc ? 1u : 0u);
         }
-        W.seed_start[s] = (uint32_t)fcur;
-        W.seed_len[s] = flen;
-        W.seed_open[s] = (uint8_t)((open_l ? 1 : 0) | (open_r ? 2 : 0));
+        put_seed(W, s, fcur, flen, open_l, open_r);
         fcur += flen;
     }
 }
@@ -2216,29 +2233,23 @@ __device__ void simulate_chain_small(chain_ws const& W, uint64_t c0, uint32_t L,
             const bool wrc = (df == 1) ? (crc[q] != 0) : (crc[q] == 0);
             W.fe[fcur + j] = (cn[q] << 1) | (wrc ? 1u : 0u);
         }
-        W.seed_start[s] = (uint32_t)fcur;
-        W.seed_len[s] = flen;
-        W.seed_open[s] = (uint8_t)((open_l ? 1 : 0) | (open_r ? 2 : 0));
+        put_seed(W, s, fcur, flen, open_l, open_r);
         fcur += flen;
     }
 }
 
-// Path ends: nodes with at most one linked port, compacted.
-__global__ void __launch_bounds__(256) k_chain_ends(chain_ws W, uint32_t* __restrict__ ends,
-                                                    unsigned long long* __restrict__ nends) {
-    const uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    bool end = false;
-    if (n < W.D) {
-        const uint2 l = reinterpret_cast<uint2 const*>(W.link)[n];
-        end = (l.x == NONE32) || (l.y == NONE32);
-    }
-    const unsigned long long at = block_reserve<256>(end ? 1u : 0u, nends);
-    if (end) ends[at] = (uint32_t)n;
-}
-
-// Each end walks to the other end; the end with the smaller node index leads
-// and reserves the chain's slots [c0, c0 + L).  heads[h] = (node | rc << 31,
-// L, c0 low, c0 high).
+// Each path end walks to the other end; the end with the smaller node index
+// leads and reserves the chain's elements [c0, c0 + L).  Most chains are one
+// fragment: no node inside the chain breaks a contig, and the seed -- the smallest
+// node -- steps to both ends (a seed flagged on the side it would step to does
+// not).  The leader then writes that fragment itself, on a second walk over the
+// links it just read; the other chains go to `heads` (node | rc << 31, L, c0 low,
+// c0 high) for k_chain_paths.
+// Bound: latency of the link reads, mostly cache hits (a chain's nodes are
+// neighbours in node order).  Finding the ends, the leaders, laying out every chain
+// and replaying the seed loop on it, the cycle check, and the run counts from the
+// fragments took 9.8 ms of a 200-genome build; this takes 4.1 and the ends 0.9 more
+// in k_links.
 __global__ void __launch_bounds__(256) k_chain_lead(chain_ws W, uint32_t const* __restrict__ ends,
                                                     unsigned long long const* __restrict__ pends,
                                                     uint4* __restrict__ heads, unsigned long long* __restrict__ nheads,
@@ -2248,164 +2259,309 @@ __global__ void __launch_bounds__(256) k_chain_lead(chain_ws W, uint32_t const* 
     const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint32_t c = 0, L = 0;
     bool rc = false, lead = false;
+    // of the walk: the smallest node with its position, orientation and flags;
+    // the last node; how many nodes before the last, and after the first, break
+    uint32_t seed = 0, seed_at = 0, seed_f = 0, last = 0, last_f = 0, first_f = 0, breaks = 0;
+    bool seed_rc = false, last_rc = false;
     if (i < nends) {
         c = ends[i];
         const uint32_t ll = W.link[2 * (uint64_t)c], lr = W.link[2 * (uint64_t)c + 1];
         rc = (lr == NONE32);  // walk out through the linked port
         L = 1;
         lead = true;
+        seed = last = c;
+        seed_rc = last_rc = rc;
+        seed_f = last_f = first_f = W.meta[c] & 3u;
         if (ll != NONE32 || lr != NONE32) {
             uint32_t cc = c;
             bool r = rc;
             while (chain_step(W.link, cc, r)) {
+                if (L > 1) breaks += last_f == M_LEFT || last_f == M_RIGHT;  // `last` was not the first, nor is it the last
+                last = cc;
+                last_rc = r;
+                last_f = W.meta[cc] & 3u;
+                if (cc < seed) {
+                    seed = cc;
+                    seed_at = L;
+                    seed_rc = r;
+                    seed_f = last_f;
+                }
                 if (++L > W.D) {
                     set_error(err, ERR_CHAIN_LIMIT);
                     lead = false;
                     break;
                 }
             }
-            if (cc < c) lead = false;  // the other end leads
+            if (last < c) lead = false;  // the other end leads
         }
     }
+    // the whole chain from its one seed?
+    const bool inside = seed_at > 0 && seed_at + 1 < L;
+    if (inside) breaks -= seed_f == M_LEFT || seed_f == M_RIGHT;
+    const bool fwd = !seed_rc;  // the walk goes the way of the seed's k-mer
+    const bool before = seed_at > 0, after = seed_at + 1 < L;
+    const bool has_b = fwd ? before : after, has_f = fwd ? after : before;  // nodes behind / ahead of the seed
+    const bool whole = lead && breaks == 0 && !(seed_f == M_LEFT && has_b) && !(seed_f == M_RIGHT && has_f);
     const unsigned long long c0 = block_reserve<256>(lead ? L : 0, W.cursor);
-    const unsigned long long h = block_reserve<256>(lead ? 1 : 0, nheads);
+    const unsigned long long h = block_reserve<256>(lead && !whole ? 1 : 0, nheads);
     if (!lead) return;
     if (c0 + L > W.D) {  // chains partition the nodes; anything else is a bug
         set_error(err, ERR_CAPACITY);
         return;
     }
-    heads[h] = make_uint4(c | (rc ? 0x80000000u : 0u), L, (uint32_t)c0, (uint32_t)(c0 >> 32));
+    if (!whole) {
+        heads[h] = make_uint4(c | (rc ? 0x80000000u : 0u), L, (uint32_t)c0, (uint32_t)(c0 >> 32));
+        return;
+    }
+    // open ends, as the seed loop leaves them: a seed flagged there, or the last
+    // node stepped to when it is flagged
+    auto breaking = [](uint32_t f) { return f == M_LEFT || f == M_RIGHT; };
+    bool open_l = false, open_r = false;
+    if (seed_f == M_LEFT) {
+        open_l = __popc(back_nib(W.mask[seed], false)) <= 1;
+    } else if (has_b) {
+        const uint32_t e = fwd ? c : last, ef = fwd ? first_f : last_f;
+        const bool wrc = fwd ? rc : !last_rc;
+        if (breaking(ef)) open_l = __popc(back_nib(W.mask[e], wrc)) <= 1;
+    }
+    if (seed_f == M_RIGHT) {
+        open_r = __popc(fwd_nib(W.mask[seed], false)) <= 1;
+    } else if (has_f) {
+        const uint32_t e = fwd ? last : c, ef = fwd ? last_f : first_f;
+        const bool wrc = fwd ? last_rc : !rc;
+        if (breaking(ef)) open_r = __popc(fwd_nib(W.mask[e], wrc)) <= 1;
+    }
+    uint32_t cc = c, runs = 1, prev = W.n_cid[c];
+    bool r = rc;
+    for (uint32_t j = 0;;) {
+        W.fe[c0 + (fwd ? j : L - 1 - j)] = (cc << 1) | ((r == fwd) ? 1u : 0u);
+        if (++j == L) break;
+        chain_step(W.link, cc, r);
+        const uint32_t q = W.n_cid[cc];
+        runs += q != prev;
+        prev = q;
+    }
+    W.seed_start[seed] = (uint32_t)c0;
+    W.seed_len[seed] = L;
+    W.seed_info[seed] = (runs << 2) | (open_r ? 2u : 0u) | (open_l ? 1u : 0u);
 }
 
-// One thread per path chain: lay the chain out at c0 and replay the seed loop.
+// The chains of more than one fragment, a thread each: lay the chain out at c0
+// and replay the seed loop.
 __global__ void __launch_bounds__(128) k_chain_paths(chain_ws W, uint4 const* __restrict__ heads,
                                                      unsigned long long const* __restrict__ nheads) {
-    const uint64_t h = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (h >= *nheads) return;
-    const uint4 hd = heads[h];
-    uint32_t cc = hd.x & 0x7fffffffu;
-    bool r = (hd.x >> 31) != 0;
-    const uint32_t L = hd.y;
-    const uint64_t c0 = ((uint64_t)hd.w << 32) | hd.z;
-    W.ch_node[c0] = cc;
-    W.ch_rc[c0] = r ? 1 : 0;
-    W.covered[cc] = 1;
-    for (uint32_t i = 1; i < L && chain_step(W.link, cc, r); ++i) {
-        W.ch_node[c0 + i] = cc;
-        W.ch_rc[c0 + i] = r ? 1 : 0;
-        W.covered[cc] = 1;
+    for (uint64_t h = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; h < *nheads;
+         h += (uint64_t)gridDim.x * blockDim.x) {
+        const uint4 hd = heads[h];
+        uint32_t cc = hd.x & 0x7fffffffu;
+        bool r = (hd.x >> 31) != 0;
+        const uint32_t L = hd.y;
+        const uint64_t c0 = ((uint64_t)hd.w << 32) | hd.z;
+        W.ch_node[c0] = cc;
+        W.ch_rc[c0] = r ? 1 : 0;
+        for (uint32_t i = 1; i < L && chain_step(W.link, cc, r); ++i) {
+            W.ch_node[c0 + i] = cc;
+            W.ch_rc[c0 + i] = r ? 1 : 0;
+        }
+        if (L <= 64)
+            simulate_chain_small(W, c0, L, false);
+        else
+            simulate_chain(W, c0, L, false);
     }
-    if (L <= 64)
-        simulate_chain_small(W, c0, L, false);
-    else
-        simulate_chain(W, c0, L, false);
+}
+
+// The number of nodes on paths; when that is not all there are cycles, and
+// k_chain_cycles needs to know the others.
+__global__ void k_chain_covered(chain_ws W, unsigned long long* __restrict__ paths) {
+    const uint64_t n = *W.cursor;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *paths = n;
+    if (n == W.D) return;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
+        W.covered[W.fe[i] >> 1] = 1;
 }
 
 // Cycles: nodes left uncovered; the smallest node index of a cycle leads.
-__global__ void k_chain_cycles(chain_ws W, uint32_t* err) {
-    uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= W.D || W.covered[n]) return;
-    uint32_t cc = (uint32_t)n;
-    bool r = false;
-    uint32_t L = 1;
-    for (;;) {
-        if (!chain_step(W.link, cc, r)) {
-            set_error(err, ERR_CHAIN_LIMIT);  // an uncovered node must be on a cycle
+// `paths` = the nodes on paths.
+__global__ void k_chain_cycles(chain_ws W, unsigned long long const* __restrict__ paths, uint32_t* err) {
+    if (*paths == W.D) return;
+    for (uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; n < W.D;
+         n += (uint64_t)gridDim.x * blockDim.x) {
+        if (W.covered[n]) continue;
+        uint32_t cc = (uint32_t)n;
+        bool r = false, lead = true;
+        uint32_t L = 1;
+        for (;;) {
+            if (!chain_step(W.link, cc, r)) {
+                set_error(err, ERR_CHAIN_LIMIT);  // an uncovered node must be on a cycle
+                return;
+            }
+            if (cc == n) break;
+            if (cc < n) {
+                lead = false;
+                break;
+            }
+            if (++L > W.D) {
+                set_error(err, ERR_CHAIN_LIMIT);
+                return;
+            }
+        }
+        if (!lead) continue;
+        const uint64_t c0 = atomicAdd(W.cursor, (unsigned long long)L);
+        if (c0 + L > W.D) {
+            set_error(err, ERR_CAPACITY);
             return;
         }
-        if (cc == n) break;
-        if (cc < n) return;
-        if (++L > W.D) {
-            set_error(err, ERR_CHAIN_LIMIT);
-            return;
+        cc = (uint32_t)n;
+        r = false;
+        W.ch_node[c0] = cc;
+        W.ch_rc[c0] = 0;
+        for (uint32_t i = 1; i < L; ++i) {
+            chain_step(W.link, cc, r);
+            W.ch_node[c0 + i] = cc;
+            W.ch_rc[c0 + i] = r ? 1 : 0;
         }
+        if (L <= 64)
+            simulate_chain_small(W, c0, L, true);
+        else
+            simulate_chain(W, c0, L, true);
     }
-    const uint64_t c0 = atomicAdd(W.cursor, (unsigned long long)L);
-    if (c0 + L > W.D) {
-        set_error(err, ERR_CAPACITY);
-        return;
-    }
-    cc = (uint32_t)n;
-    r = false;
-    W.ch_node[c0] = cc;
-    W.ch_rc[c0] = 0;
-    for (uint32_t i = 1; i < L; ++i) {
-        chain_step(W.link, cc, r);
-        W.ch_node[c0 + i] = cc;
-        W.ch_rc[c0 + i] = r ? 1 : 0;
-    }
-    if (L <= 64)
-        simulate_chain_small(W, c0, L, true);
-    else
-        simulate_chain(W, c0, L, true);
 }
 
 // ---- fragments --------------------------------------------------------------
 __device__ __forceinline__ uint32_t frag_cid(uint32_t const* n_cid, uint32_t node) { return n_cid[node]; }
 
-// Seed nodes in node order (= fragment order): seed_of[f] = node of fragment f.
-__global__ void __launch_bounds__(256) k_seed_list(uint64_t D, uint32_t const* __restrict__ seed_len, select_ws ws,
-                                                   uint32_t* __restrict__ seed_of, uint32_t* err) {
+// Fragments in node order of their seeds, in one pass over the nodes: seed_of[f],
+// and off[f], the offset of its record (frag_unitig_writer::write_batch layout);
+// tot[0..2] = fragments, record bytes, sequence bases.
+__global__ void __launch_bounds__(256) k_seed_list(uint64_t D, uint32_t const* __restrict__ seed_len,
+                                                   uint32_t const* __restrict__ seed_info, uint32_t k, select_ws ws,
+                                                   unsigned long long* status_bytes, uint32_t* __restrict__ seed_of,
+                                                   uint64_t* __restrict__ off, unsigned long long* __restrict__ tot,
+                                                   uint32_t* err) {
     __shared__ prim::ordered_select seeds;
+    __shared__ uint64_t wbytes[prim::SEL_ROUNDS * 8], s_bytes;
     const uint64_t tile = prim::select_tile(seeds, ws.counter);
-    uint32_t sel = 0;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint32_t len[prim::SEL_ROUNDS], info[prim::SEL_ROUNDS], sel = 0;
 #pragma unroll
     for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
         const uint64_t n = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
-        if (n < D && seed_len[n]) sel |= 1u << r;
+        len[r] = n < D ? seed_len[n] : 0u;
     }
-    prim::select_rank(seeds, sel, tile, ws.ntiles, ws.status, ws.total, err);
 #pragma unroll
-    for (int r = 0; r < prim::SEL_ROUNDS; ++r)
-        if ((sel >> r) & 1u)
-            seed_of[prim::select_pos(seeds, r)] = (uint32_t)(tile * prim::SEL_TILE + 256u * r + threadIdx.x);
-}
-
-// Thread per fragment: serialized size (frag_unitig_writer::write_batch layout).
-// and, by decoupled look-back over blocks, its offset: off[f], off[F] the total.
-__global__ void __launch_bounds__(256) k_frag_sizes(uint64_t F, uint32_t const* __restrict__ seed_of,
-                                                    uint32_t const* __restrict__ seed_start,
-                                                    uint32_t const* __restrict__ seed_len,
-                                                    uint32_t const* __restrict__ fe,
-                                                    uint32_t const* __restrict__ n_cid, uint32_t k, select_ws ws,
-                                                    uint64_t* __restrict__ off,
-                                                    unsigned long long* __restrict__ seq_total, uint32_t* err) {
-    __shared__ uint64_t sw[256 / 32 + 1], s_tile, s_base;
-    if (threadIdx.x == 0) s_tile = atomicAdd(ws.counter, 1u);
-    __syncthreads();
-    const uint64_t tile = s_tile, f = tile * 256 + threadIdx.x;
-    uint64_t seq = 0, size = 0;
-    if (f < F) {
-        const uint32_t n = seed_of[f];
-        const uint32_t len = seed_len[n], a = seed_start[n];
-        uint32_t runs = 1, prev = frag_cid(n_cid, fe[a] >> 1);
-        for (uint32_t j = 1; j < len; ++j) {
-            const uint32_t c = frag_cid(n_cid, fe[a + j] >> 1);
-            runs += c != prev;
-            prev = c;
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        info[r] = 0;
+        if (len[r]) {
+            info[r] = seed_info[tile * prim::SEL_TILE + 256u * r + threadIdx.x];
+            sel |= 1u << r;
         }
-        seq = (uint64_t)k + len - 1;
-        size = 1 + 4 + 12ull * runs + 4 + seq;
     }
-    uint64_t tot;
-    const uint64_t ex = prim::block_exclusive_scan<uint64_t, 256>(size, sw, tot);
-    if (threadIdx.x < 32) {
+    auto bytes = [&](int r) { return len[r] ? 9 + 12ull * (info[r] >> 2) + k + len[r] - 1 : 0ull; };
+    uint64_t at[prim::SEL_ROUNDS], seq = 0;  // record bytes before this element in its (round, warp)
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t size = bytes(r);
+        // (32-bit sums unless some record is of 64 MiB)
+        if (!__any_sync(0xffffffffu, (size >> 26) != 0)) {
+            const uint32_t incl = prim::warp_inclusive_scan((uint32_t)size);
+            at[r] = incl - (uint32_t)size;
+        } else {
+            at[r] = prim::warp_inclusive_scan(size) - size;
+        }
+        if (lane == 31) wbytes[r * 8 + warp] = at[r] + size;
+        if (len[r]) seq += (uint64_t)k + len[r] - 1;
+    }
+    prim::select_put(seeds, sel);
+    __syncthreads();
+    if (warp == 0) {
+        prim::select_scan(seeds, tile, ws.ntiles, ws.status, tot, err);
+    } else if (warp == 1) {
+        const uint64_t c0 = wbytes[2 * lane], c1 = wbytes[2 * lane + 1];
+        const uint64_t x = prim::warp_inclusive_scan(c0 + c1);
+        const uint64_t sum = __shfl_sync(0xffffffffu, x, 31);
+        wbytes[2 * lane] = x - c0 - c1;
+        wbytes[2 * lane + 1] = x - c1;
         uint64_t excl = 0;
-        const bool ok = prim::lookback_exclusive(ws.status, tile, tot, excl);
-        if (threadIdx.x == 0) {
+        const bool ok = prim::lookback_exclusive(status_bytes, tile, sum, excl);
+        if (lane == 0) {
             if (!ok) set_error(err, ERR_CHAIN_LIMIT);
-            s_base = excl;
+            s_bytes = excl;
+            if (tile == ws.ntiles - 1) tot[1] = excl + sum;
         }
     }
     __syncthreads();
-    if (f < F) off[f] = s_base + ex;
-    if (f == F - 1) off[F] = *ws.total = s_base + ex + size;
-    seq = prim::warp_inclusive_scan(seq);
-    if ((threadIdx.x & 31) == 31 && seq) atomicAdd(seq_total, (unsigned long long)seq);
+#pragma unroll
+    for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
+        const uint64_t n = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        const bool f = (sel >> r) & 1u;
+        if (!f && n != D - 1) continue;
+        const uint64_t at_f = prim::select_pos(seeds, r), o = s_bytes + wbytes[r * 8 + warp] + at[r];
+        if (f) {
+            seed_of[at_f] = (uint32_t)n;
+            off[at_f] = o;
+        }
+        // the total closes the offsets
+        if (n == D - 1) off[at_f + (f ? 1 : 0)] = o + bytes(r);
+    }
+    for (int o = 16; o; o >>= 1) seq += __shfl_xor_sync(0xffffffffu, seq, o);
+    if (lane == 0 && seq) atomicAdd(tot + 2, (unsigned long long)seq);
 }
 
-__device__ __forceinline__ void put_bytes(uint8_t* o, uint64_t v, int n) {
-    for (int i = 0; i < n; ++i) o[i] = (uint8_t)(v >> (8 * i));
+// Bytes one after another at any address (shared or global memory), stored by
+// aligned 4-byte words; the words at the two ends, which hold others' bytes, byte
+// by byte.
+struct byte_writer {
+    uint8_t* p;      // next word (aligned)
+    uint64_t acc;    // bytes not yet stored
+    uint32_t fill;   // of them (< 4), counting the first word's bytes before the start
+    uint32_t skip;   // bytes of the next word before the start
+    __device__ __forceinline__ explicit byte_writer(uint8_t* o) {
+        skip = fill = (uint32_t)(reinterpret_cast<uintptr_t>(o) & 3);
+        p = o - fill;
+        acc = 0;
+    }
+    __device__ __forceinline__ void word() {
+        const uint32_t w = (uint32_t)acc;
+        if (skip == 0) {
+            *reinterpret_cast<uint32_t*>(p) = w;
+        } else {
+            for (uint32_t i = skip; i < 4; ++i) p[i] = (uint8_t)(w >> (8 * i));
+            skip = 0;
+        }
+        p += 4;
+        acc >>= 32;
+    }
+    __device__ __forceinline__ void put4(uint32_t v) {
+        acc |= (uint64_t)v << (8 * fill);
+        word();
+    }
+    __device__ __forceinline__ void put1(uint32_t v) {
+        acc |= (uint64_t)v << (8 * fill);
+        if (++fill == 4) {
+            word();
+            fill = 0;
+        }
+    }
+    __device__ __forceinline__ void end() {
+        for (uint32_t i = skip; i < fill; ++i) p[i] = (uint8_t)(acc >> (8 * i));
+    }
+};
+
+// ASCII of the four 2-bit bases of b, the first in the low bits.
+__device__ __forceinline__ uint32_t ascii4(uint32_t b) {
+    uint32_t s = (b | (b << 4)) & 0x0f0fu;
+    s = (s | (s << 2)) & 0x3333u;
+    return __byte_perm(0x54474341u, 0u, s);  // byte i = "ACGT"[nibble i]
+}
+// Bases of a k-mer, base i at bits 2i.
+__device__ __forceinline__ void bases_of(uint64_t w, uint32_t k, uint64_t& lo, uint64_t& hi) {
+    lo = rev2_64(w) >> (64 - 2 * k);
+    hi = 0;
+}
+__device__ __forceinline__ void bases_of(u128 w, uint32_t k, uint64_t& lo, uint64_t& hi) {
+    const u128 x = kmer_ops<u128>::rev2_128(w) >> (128 - 2 * k);
+    lo = (uint64_t)x;
+    hi = (uint64_t)(x >> 64);
 }
 
 // One fragment record (unitig_spill.hpp:491-522 layout) at `o` (shared or
@@ -2415,48 +2571,64 @@ __device__ __forceinline__ void put_bytes(uint8_t* o, uint64_t v, int n) {
 template <typename K>
 __device__ __forceinline__ void emit_fragment(uint8_t* o, uint32_t n, uint32_t const* __restrict__ seed_start,
                                               uint32_t const* __restrict__ seed_len,
-                                              uint8_t const* __restrict__ seed_open, uint32_t const* __restrict__ fe,
+                                              uint32_t const* __restrict__ seed_info, uint32_t const* __restrict__ fe,
                                               uint32_t const* __restrict__ n_cid, K const* __restrict__ n_key,
                                               uint32_t k) {
     typedef kmer_ops<K> ops;
-    const uint32_t len = seed_len[n];
-    const uint32_t a = seed_start[n];
-    o[0] = seed_open[n];
-    uint32_t runs = 0;
-    uint8_t* rp = o + 5;
-    uint32_t prev = frag_cid(n_cid, fe[a] >> 1), cnt = 1;
-    for (uint32_t j = 1; j <= len; ++j) {
-        const uint32_t c = j < len ? frag_cid(n_cid, fe[a + j] >> 1) : ~prev;
-        if (j < len && c == prev) {
-            ++cnt;
-            continue;
-        }
-        const uint64_t cid64 = prev == NONE32 ? ~0ull : (uint64_t)prev;
-        put_bytes(rp, cid64, 8);
-        put_bytes(rp + 8, cnt, 4);
-        rp += 12;
-        ++runs;
-        prev = c;
+    const uint32_t len = seed_len[n], info = seed_info[n];
+    uint32_t const* el = fe + seed_start[n];
+    byte_writer w(o);
+    w.put1(info & 3u);
+    w.put4(info >> 2);
+    auto run = [&](uint32_t cid, uint32_t cnt) {
+        w.put4(cid);
+        w.put4(cid == NONE32 ? 0xffffffffu : 0u);
+        w.put4(cnt);
+    };
+    uint32_t prev = n_cid[el[0] >> 1], cnt = len;
+    if ((info >> 2) > 1) {
         cnt = 1;
+        for (uint32_t j = 1; j < len; ++j) {
+            const uint32_t c = n_cid[el[j] >> 1];
+            if (c != prev) {
+                run(prev, cnt);
+                prev = c;
+                cnt = 0;
+            }
+            ++cnt;
+        }
     }
-    put_bytes(o + 1, runs, 4);
-    const uint32_t seq_len = k + len - 1;
-    put_bytes(rp, seq_len, 4);
-    uint8_t* sp = rp + 4;
-    const char acgt[4] = {'A', 'C', 'G', 'T'};
+    run(prev, cnt);
+    w.put4(k + len - 1);
+    uint64_t lo, hi;
     {
-        const uint32_t e = fe[a];
-        K w = n_key[e >> 1];
-        if (e & 1u) w = ops::revcomp(w, k);
-        for (uint32_t i = 0; i < k; ++i) sp[k - 1 - i] = acgt[ops::low2(w >> (2 * i))];
+        const uint32_t e = el[0];
+        K x = n_key[e >> 1];
+        if (e & 1u) x = ops::revcomp(x, k);
+        bases_of(x, k, lo, hi);
     }
+    uint32_t left = k;
+    for (; left >= 4; left -= 4) {
+        w.put4(ascii4((uint32_t)lo & 0xffu));
+        lo >>= 8;
+        if constexpr (sizeof(K) == 16) {
+            lo |= hi << 56;
+            hi >>= 8;
+        }
+    }
+    uint32_t b = (uint32_t)lo;  // `left` < 4 bases not yet written
     const uint32_t top = 2 * (k - 1);
     for (uint32_t j = 1; j < len; ++j) {
-        const uint32_t e = fe[a + j];
-        const K w = n_key[e >> 1];
-        const uint32_t b = (e & 1u) ? 3u - ops::low2(w >> top) : ops::low2(w);
-        sp[k - 1 + j] = acgt[b];
+        const uint32_t e = el[j];
+        const K x = n_key[e >> 1];
+        b |= ((e & 1u) ? 3u - ops::low2(x >> top) : ops::low2(x)) << (2 * left);
+        if (++left == 4) {
+            w.put4(ascii4(b));
+            b = left = 0;
+        }
     }
+    for (uint32_t x = ascii4(b); left; --left, x >>= 8) w.put1(x & 0xffu);
+    w.end();
 }
 
 // Fragments [f0, f0 + FW_THREADS) of a block occupy one contiguous byte range
@@ -2464,13 +2636,17 @@ __device__ __forceinline__ void emit_fragment(uint8_t* o, uint32_t n, uint32_t c
 // 16-byte phase and stored with aligned 16-byte writes (bytes at the two
 // ragged ends one by one), instead of a few dozen scattered byte stores per
 // fragment.  A block whose range does not fit writes directly.
+// Bound: the gathers of a fragment's elements (its keys and color sets).  With the
+// records put together byte by byte 5.7 ms for 2.3 GB of a 200-genome build, by
+// words 3.9 (0.6 TB/s), with 24 KB of buffer and 64 registers for 8 blocks per SM
+// (32 KB and 76: 6) 3.4.
 constexpr int FW_THREADS = 128;
-constexpr int FW_BYTES = 32 * 1024;
+constexpr int FW_BYTES = 24 * 1024;
 
 template <typename K>
-__global__ void __launch_bounds__(FW_THREADS)
+__global__ void __launch_bounds__(FW_THREADS, 8)
     k_frag_write(uint64_t F, uint32_t const* __restrict__ seed_of, uint32_t const* __restrict__ seed_start,
-                 uint32_t const* __restrict__ seed_len, uint8_t const* __restrict__ seed_open,
+                 uint32_t const* __restrict__ seed_len, uint32_t const* __restrict__ seed_info,
                  uint32_t const* __restrict__ fe, uint32_t const* __restrict__ n_cid, K const* __restrict__ n_key,
                  uint32_t k, uint64_t const* __restrict__ off, uint64_t base, uint8_t* __restrict__ out) {
     __shared__ __align__(16) uint8_t buf[FW_BYTES];
@@ -2480,11 +2656,11 @@ __global__ void __launch_bounds__(FW_THREADS)
     const uint32_t phase = (uint32_t)(g0 & 15);
     const uint64_t f = f0 + threadIdx.x;
     if (g1 - g0 + phase > (uint64_t)FW_BYTES) {  // block-uniform
-        if (f < F) emit_fragment<K>(out + base + off[f], seed_of[f], seed_start, seed_len, seed_open, fe, n_cid, n_key, k);
+        if (f < F) emit_fragment<K>(out + base + off[f], seed_of[f], seed_start, seed_len, seed_info, fe, n_cid, n_key, k);
         return;
     }
     if (f < F)
-        emit_fragment<K>(buf + phase + (base + off[f] - g0), seed_of[f], seed_start, seed_len, seed_open, fe, n_cid, n_key,
+        emit_fragment<K>(buf + phase + (base + off[f] - g0), seed_of[f], seed_start, seed_len, seed_info, fe, n_cid, n_key,
                          k);
     __syncthreads();
     const uint64_t a0 = (g0 + 15) & ~uint64_t(15);  // first aligned byte inside the range
@@ -2728,10 +2904,13 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     }
     // zeroed together: look-back status, the node and pair counts so far
     // (alternating by group), tile counters
-    unsigned long long* nb_status = A.alloc<unsigned long long>(gtile[ng] + 4 + (ng + 1) / 2 + 1);
+    // and the number of path ends
+    uint32_t* ends = A.alloc<uint32_t>(nocc);
+    unsigned long long* nb_status = A.alloc<unsigned long long>(gtile[ng] + 5 + (ng + 1) / 2 + 1);
     unsigned long long* ncnt = nb_status + gtile[ng];
-    uint32_t* nb_counter = reinterpret_cast<uint32_t*>(ncnt + 4);
-    CDBG_CUDA(cudaMemsetAsync(nb_status, 0, 8 * (gtile[ng] + 4 + (ng + 1) / 2 + 1), st));
+    unsigned long long* nends = ncnt + 4;
+    uint32_t* nb_counter = reinterpret_cast<uint32_t*>(ncnt + 5);
+    CDBG_CUDA(cudaMemsetAsync(nb_status, 0, 8 * (gtile[ng] + 5 + (ng + 1) / 2 + 1), st));
     for (size_t g = 0; g < ng; ++g) {
         const uint32_t g0 = gb[g], g1 = gb[g + 1];
         const uint64_t t0 = bocc[b0 + g0] - O0, tn = bocc[b0 + g1] - bocc[b0 + g0];
@@ -2790,20 +2969,21 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         CDBG_CHECK_LAUNCH();
         {
             CDBG_PROF("k_links", st);
-            k_links<K><<<grid(tn, 256), 256, 0, st>>>(nbase, nnext, n_key, n_mask, k, link);
+            k_links<K><<<grid(tn, 256), 256, 0, st>>>(nbase, nnext, n_key, n_mask, k, link, ends, nends);
         }
         CDBG_CHECK_LAUNCH();
     }
     uint64_t counts[2];  // nodes, pairs
+    uint64_t n_ends = 0;
     uint32_t derr = 0;
-    mail_reader(st).add(counts, ncnt + 2 * (ng & 1), 16).add(&derr, d_err).wait();
+    mail_reader(st).add(counts, ncnt + 2 * (ng & 1), 16).add(&n_ends, nends).add(&derr, d_err).wait();
     const uint64_t D = counts[0], npairs = counts[1];
     if (D >= (1ull << 31)) throw std::runtime_error("too many distinct k-mers in one bucket batch");
     if (derr) check_device_error_word(d_err, st, "k-mer table insert");
     // zeroed together: selections over the pairs, records, nodes and fragments,
     // heavy-record flags, the chains' seed lengths and covered flags, counts
-    zero_block Z(3 * zero_block::select_words(npairs) + zero_block::select_words(nrec) + zero_block::select_words(D) +
-                     zero_block::select_words(D, 256) + nrec / 2 + D / 2 + D / 8 + 16,
+    zero_block Z(3 * zero_block::select_words(npairs) + zero_block::select_words(nrec) +
+                     2 * zero_block::select_words(D) + nrec / 2 + D / 2 + D / 8 + 16,
                  A, st);
     // ---- multi-record k-mers, from their (node, record) pairs
     uint64_t M = 0;
@@ -3120,61 +3300,48 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     W.fe = A.alloc<uint32_t>(D);
     W.seed_start = A.alloc<uint32_t>(D);
     W.seed_len = Z.take<uint32_t>(D);
-    W.seed_open = A.alloc<uint8_t>(D);
+    W.seed_info = A.alloc<uint32_t>(D);
     W.covered = Z.take<uint8_t>(D);
+    W.n_cid = n_cid;
     W.cursor = Z.take<unsigned long long>(1);
     W.D = D;
     {
-        uint32_t* ends = A.alloc<uint32_t>(D);
-        unsigned long long* cnt2 = Z.take<unsigned long long>(2);
-        {
-            CDBG_PROF("k_chain_ends", st);
-            k_chain_ends<<<grid(D, 256), 256, 0, st>>>(W, ends, cnt2);
-        }
-        CDBG_CHECK_LAUNCH();
-        // grids and the heads sized for D ends when that is cheaper than the waits
-        // for their number (about 10 us each)
-        const bool wait = D > (1ull << 21);
-        const uint64_t nends = wait ? read_dev(cnt2, st) : D;
-        uint4* heads = A.alloc<uint4>(nends + 1);
-        if (nends) {
+        uint4* heads = A.alloc<uint4>(n_ends + 1);
+        unsigned long long* cnt2 = Z.take<unsigned long long>(2);  // heads, nodes on paths
+        if (n_ends) {
             CDBG_PROF("k_chain_lead", st);
-            k_chain_lead<<<grid(nends, 256), 256, 0, st>>>(W, ends, cnt2, heads, cnt2 + 1, d_err);
+            k_chain_lead<<<grid(n_ends, 256), 256, 0, st>>>(W, ends, nends, heads, cnt2, d_err);
         }
         CDBG_CHECK_LAUNCH();
-        const uint64_t nheads = wait ? read_dev(cnt2 + 1, st) : nends;
-        if (nheads) {
+        {
             CDBG_PROF("k_chain_paths", st);
-            k_chain_paths<<<grid(nheads, 128), 128, 0, st>>>(W, heads, cnt2 + 1);
+            k_chain_paths<<<(unsigned)std::min<uint64_t>(grid(n_ends + 1, 128), 148 * 16), 128, 0, st>>>(W, heads, cnt2);
+        }
+        CDBG_CHECK_LAUNCH();
+        {
+            CDBG_PROF("k_chain_cycles", st);
+            const unsigned blocks = (unsigned)std::min<uint64_t>(grid(D, 128), 148 * 16);
+            k_chain_covered<<<blocks, 128, 0, st>>>(W, cnt2 + 1);
+            CDBG_CHECK_LAUNCH();
+            k_chain_cycles<<<blocks, 128, 0, st>>>(W, cnt2 + 1, d_err);
         }
         CDBG_CHECK_LAUNCH();
     }
-    {
-        CDBG_PROF("k_chain_cycles", st);
-        k_chain_cycles<<<grid(D, 128), 128, 0, st>>>(W, d_err);
-    }
-    CDBG_CHECK_LAUNCH();
-    // ---- fragments, in seed order
+    // ---- fragments, in seed order (offsets and seeds sized for D of them)
     uint32_t* seed_of = A.alloc<uint32_t>(D);
-    select_ws wseed = Z.select(D), wfrag = Z.select(D, 256);
+    uint64_t* foff = A.alloc<uint64_t>(D + 1);
+    select_ws wseed = Z.select(D), wbytes = Z.select(D);
+    unsigned long long* ftot = Z.take<unsigned long long>(3);
     {
         CDBG_PROF("k_seed_list", st);
-        k_seed_list<<<(unsigned)wseed.ntiles, 256, 0, st>>>(D, W.seed_len, wseed, seed_of, d_err);
+        k_seed_list<<<(unsigned)wseed.ntiles, 256, 0, st>>>(D, W.seed_len, W.seed_info, k, wseed, wbytes.status, seed_of,
+                                                            foff, ftot, d_err);
     }
     CDBG_CHECK_LAUNCH();
-    uint64_t nfr = 0;
-    mail_reader(st).add(&nfr, wseed.total).add(&derr, d_err).wait();
+    uint64_t ft[3], new_ints = 0;
+    mail_reader(st).add(ft, ftot, 24).add(&new_ints, ints).add(&derr, d_err).wait();
     if (derr) check_device_error_word(d_err, st, "unitig walk");
-    uint64_t* foff = A.alloc<uint64_t>(nfr + 1);
-    unsigned long long* seqt = Z.take<unsigned long long>(1);
-    if (nfr) {
-        CDBG_PROF("k_frag_sizes", st);
-        k_frag_sizes<<<grid(nfr, 256), 256, 0, st>>>(nfr, seed_of, W.seed_start, W.seed_len, W.fe, n_cid, k, wfrag, foff,
-                                                     seqt, d_err);
-    }
-    CDBG_CHECK_LAUNCH();
-    uint64_t fbytes = 0, seq_total = 0, new_ints = 0;
-    mail_reader(st).add(&fbytes, wfrag.total).add(&seq_total, seqt).add(&new_ints, ints).wait();
+    const uint64_t nfr = ft[0], fbytes = ft[1], seq_total = ft[2];
     dict.total_integers += new_ints;
     const uint64_t frag_old = dfrag.n;
     uint8_t* fb = nullptr;  // the fragments: scratch on their way to the host, or where the output stays
@@ -3192,7 +3359,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     if (nfr) {
         CDBG_PROF("k_frag_write", st);
         k_frag_write<K><<<grid(nfr, FW_THREADS), FW_THREADS, 0, st>>>(nfr, seed_of, W.seed_start, W.seed_len,
-                                                                       W.seed_open, W.fe, n_cid, n_key, k, foff,
+                                                                       W.seed_info, W.fe, n_cid, n_key, k, foff,
                                                                        p.to_host ? 0 : frag_old, fb);
     }
     CDBG_CHECK_LAUNCH();

@@ -109,14 +109,17 @@ __device__ __forceinline__ bool lookback_exclusive(unsigned long long* status, u
     return ok;
 }
 
-// Positions of the selected elements of a tile of SEL_TILE = 4 rounds x 256
+// Positions of the selected elements of a tile of SEL_TILE = 8 rounds x 256
 // threads among all selected ones, in element order: element tile * SEL_TILE +
-// round * 256 + thread.  Every thread of the 256 calls all three.
-constexpr int SEL_ROUNDS = 4;
+// round * 256 + thread.  Every thread of the 256 calls select_tile, select_put
+// and (after a barrier, one warp select_scan, and another barrier) select_pos; a
+// kernel with two selections gives each its own warp, so their look-backs wait
+// side by side.
+constexpr int SEL_ROUNDS = 8;
 constexpr int SEL_TILE = SEL_ROUNDS * 256;
 struct ordered_select {
-    uint32_t bal[32];   // selected lanes of (round, warp)
-    uint32_t cnt[32];   // selected before (round, warp) in the tile
+    uint32_t bal[SEL_ROUNDS * 8];  // selected lanes of (round, warp)
+    uint32_t cnt[SEL_ROUNDS * 8];  // selected before (round, warp) in the tile
     uint64_t tile, base;
 };
 __device__ __forceinline__ uint64_t select_tile(ordered_select& s, uint32_t* tile_counter) {
@@ -124,30 +127,39 @@ __device__ __forceinline__ uint64_t select_tile(ordered_select& s, uint32_t* til
     __syncthreads();
     return s.tile;
 }
-// Bit r of `sel`: this thread's element of round r is selected.  The last tile
-// stores the total.
-__device__ __forceinline__ void select_rank(ordered_select& s, uint32_t sel, uint64_t tile, uint64_t ntiles,
-                                            unsigned long long* status, unsigned long long* total, uint32_t* err) {
+// Bit r of `sel`: this thread's element of round r is selected.
+__device__ __forceinline__ void select_put(ordered_select& s, uint32_t sel) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int r = 0; r < SEL_ROUNDS; ++r) {
         const uint32_t b = __ballot_sync(0xffffffffu, (sel >> r) & 1u);
         if (lane == 0) s.bal[r * 8 + warp] = b;
     }
-    __syncthreads();
-    if (warp == 0) {
-        const uint32_t c = __popc(s.bal[lane]);
-        const uint32_t x = warp_inclusive_scan(c);
-        const uint32_t tot = __shfl_sync(0xffffffffu, x, 31);
-        s.cnt[lane] = x - c;
-        uint64_t excl = 0;
-        const bool ok = lookback_exclusive(status, tile, tot, excl);
-        if (lane == 0) {
-            if (!ok) set_error(err, ERR_CHAIN_LIMIT);
-            s.base = excl;
-            if (tile == ntiles - 1) *total = excl + tot;
-        }
+}
+// By one whole warp; the last tile stores the total.
+__device__ __forceinline__ void select_scan(ordered_select& s, uint64_t tile, uint64_t ntiles,
+                                            unsigned long long* status, unsigned long long* total, uint32_t* err) {
+    static_assert(SEL_ROUNDS * 8 == 64, "two counts per lane");
+    const int lane = threadIdx.x & 31;
+    const uint32_t c0 = __popc(s.bal[2 * lane]), c1 = __popc(s.bal[2 * lane + 1]);
+    const uint32_t x = warp_inclusive_scan(c0 + c1);
+    const uint32_t tot = __shfl_sync(0xffffffffu, x, 31);
+    s.cnt[2 * lane] = x - c0 - c1;
+    s.cnt[2 * lane + 1] = x - c1;
+    uint64_t excl = 0;
+    const bool ok = lookback_exclusive(status, tile, tot, excl);
+    if (lane == 0) {
+        if (!ok) set_error(err, ERR_CHAIN_LIMIT);
+        s.base = excl;
+        if (tile == ntiles - 1) *total = excl + tot;
     }
+}
+// All of it for a kernel with one selection.
+__device__ __forceinline__ void select_rank(ordered_select& s, uint32_t sel, uint64_t tile, uint64_t ntiles,
+                                            unsigned long long* status, unsigned long long* total, uint32_t* err) {
+    select_put(s, sel);
+    __syncthreads();
+    if (threadIdx.x < 32) select_scan(s, tile, ntiles, status, total, err);
     __syncthreads();
 }
 // Selected elements before this thread's element of round r.

@@ -100,3 +100,19 @@ def test_device_input_alignment(oracle, engine, tmp_path, shift, tail):
     want = native.result_frag_bytes(want)
     assert native.result_frag_bytes(engine.build(b, k, B, 2)) == want
     _check(oracle, engine, tmp_path, [s[:2], s[2:]], k, B)
+
+
+@pytest.mark.parametrize("k", [31, 63])
+@pytest.mark.parametrize("unit", [33, 64, 65, 131, 700])
+def test_cycles_and_broken_chains(oracle, engine, tmp_path, k, unit):
+    """Chains that are cycles, of up to 64 k-mers and more, chains broken by
+    contig ends inside a bucket, and chains that are one fragment."""
+    rng = np.random.default_rng(unit + k)
+    u, a, b = _dna(rng, unit), _dna(rng, 500), _dna(rng, 900)
+    g0 = [u * (3 + 2 * k // unit), a, b[:400]]
+    g1 = [a[100:300], b[300:], b[200:260 + k]]
+    g2 = [a[:k], a[-k:], a[200:200 + k + 1], u + u[: k + 2]]
+    for B in (1, 5):
+        d = tmp_path / str(B)
+        d.mkdir()
+        _check(oracle, engine, d, [g0, g1, g2], k, B)
