@@ -43,6 +43,7 @@
 #include <cstddef>
 #include <cstdlib>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "device_kmer.cuh"
@@ -1179,94 +1180,128 @@ __device__ __forceinline__ void or_bits(uint64_t* w, uint64_t pos, uint64_t val,
     atomicOr((unsigned long long*)&w[i], (unsigned long long)(val << s));
     if (s && s + len > 64) atomicOr((unsigned long long*)&w[i + 1], (unsigned long long)(val >> (64 - s)));
 }
-__device__ __forceinline__ uint64_t put_delta(uint64_t* w, uint64_t pos, uint64_t x) {
+// Delta code of x < 2^32: its bits (at most 43), `len` of them.
+__device__ __forceinline__ uint64_t delta_code(uint64_t x, uint32_t& len) {
     const uint64_t y = x + 1;
     const uint32_t l = msb64(y);
-    const uint64_t L1 = l + 1;
-    const uint32_t ll = msb64(L1);
-    // gamma(L1): ll zeros, a one, the low ll bits of L1
-    const uint64_t g = (1ull << ll) | ((L1 & ((1ull << ll) - 1)) << (ll + 1));
-    or_bits(w, pos, g, 2 * ll + 1);
-    pos += 2 * ll + 1;
-    if (l) or_bits(w, pos, y, l);
-    return pos + l;
+    const uint32_t L1 = l + 1, ll = msb64(L1);
+    // gamma(L1): ll zeros, a one, the low ll bits of L1; then the low l bits of y
+    const uint64_t g = (1ull << ll) | ((uint64_t)(L1 & ((1u << ll) - 1u)) << (ll + 1));
+    len = 2 * ll + 1 + l;
+    return g | ((y & ((1ull << l) - 1)) << (2 * ll + 1));
 }
+__device__ __forceinline__ uint64_t put_delta(uint64_t* w, uint64_t pos, uint64_t x) {
+    uint32_t len;
+    const uint64_t c = delta_code(x, len);
+    or_bits(w, pos, c, len);
+    return pos + len;
+}
+// Codes one after another from bit `pos` on, stored a word at a time: the words
+// in between are this writer's alone, the first and last are shared.
+struct code_writer {
+    uint64_t* w;
+    uint64_t acc;
+    uint32_t fill;
+    bool shared;  // the current word holds others' bits
+    __device__ __forceinline__ code_writer(uint64_t* words, uint64_t pos)
+        : w(words + (pos >> 6)), acc(0), fill((uint32_t)(pos & 63)), shared(true) {}
+    __device__ __forceinline__ void put(uint64_t c, uint32_t len) {
+        acc |= c << fill;
+        if (fill + len >= 64) {
+            if (shared)
+                atomicOr((unsigned long long*)w, (unsigned long long)acc);
+            else
+                *w = acc;
+            ++w;
+            shared = false;
+            acc = fill ? c >> (64 - fill) : 0;
+            fill = fill + len - 64;
+        } else {
+            fill += len;
+        }
+    }
+    __device__ __forceinline__ void end() {
+        if (acc) atomicOr((unsigned long long*)w, (unsigned long long)acc);
+    }
+};
 
-// One candidate class by the whole warp (bm: the warp's C-bit shared bitmap).
-// Pass 0 (ENC = false): encoded size -> nbits[j].  Pass 1: write at bit
-// offset pos0 of `words` (zeroed).
-template <bool ENC>
-__device__ __forceinline__ void encode_one(cand_set const& cs, uint64_t j, uint64_t pos0, uint32_t C, uint32_t nw,
-                                           uint32_t* bm, int lane, uint64_t* __restrict__ nbits,
+// One candidate class by a group of GW consecutive lanes (a power of two; gl: the
+// lane in the group; bm: the group's C-bit shared bitmap).  Groups of a warp run
+// together, a group without a candidate with an empty set.  Pass 0 (ENC =
+// false): encoded size -> nbits[j].  Pass 1: write at bit offset pos0 of `words`
+// (zeroed).
+template <int GW, typename T>
+__device__ __forceinline__ T group_excl_scan(T v, T& total) {
+    const int gl = threadIdx.x & (GW - 1);
+    T x = v;
+#pragma unroll
+    for (int o = 1; o < GW; o <<= 1) {
+        const T y = __shfl_up_sync(0xffffffffu, x, o, GW);
+        if (gl >= o) x += y;
+    }
+    total = __shfl_sync(0xffffffffu, x, GW - 1, GW);
+    return x - v;
+}
+template <bool ENC, int GW>
+__device__ __forceinline__ void encode_one(cand_set const& cs, bool on, uint64_t j, uint64_t pos0, uint32_t C,
+                                           uint32_t nw, uint32_t* bm, uint64_t* __restrict__ nbits,
                                            uint64_t* __restrict__ words) {
-    const uint64_t N = cs.n;
+    const int gl = threadIdx.x & (GW - 1);
+    const uint64_t N = on ? cs.n : 0;
     const uint64_t sparse_t = (uint64_t)(0.25 * (double)C);
     const uint64_t dense_t = (uint64_t)(0.75 * (double)C);
     const uint32_t hdr = delta_bits(N);
-    if (!ENC) {
-        // sizes that need no bitmap: the plain-bitmap range has a fixed size,
-        // and a sparse set held as an ascending list has its gaps in the list
-        if (N >= sparse_t && N < dense_t) {
-            if (lane == 0) nbits[j] = hdr + C;
-            return;
-        }
-        if (cs.list && N < sparse_t) {
-            uint64_t acc = 0;
-            for (uint64_t base = 0; base < N; base += 32) {
-                const uint64_t i = base + lane;
-                const uint32_t v = i < N ? cs.list[i] : 0u;
-                uint32_t pv = __shfl_up_sync(0xffffffffu, v, 1);
-                if (lane == 0 && base) pv = cs.list[base - 1];
-                if (i < N) acc += delta_bits(i == 0 ? (uint64_t)v : (uint64_t)(v - pv - 1));
-            }
-            acc = warp_sum64(acc);
-            if (lane == 0) nbits[j] = hdr + acc;
-            return;
-        }
-    }
-    if (ENC && cs.list && N < sparse_t) {
-        // a sparse set held as an ascending list: its gap codes straight
-        // from the list, 32 at a time at offsets from a warp scan of their
-        // lengths (the codes the bitmap walk below would write)
-        if (lane == 0) put_delta(words, pos0, N);
-        uint64_t p = pos0 + hdr;
-        for (uint64_t base = 0; base < N; base += 32) {
-            const uint64_t i = base + lane;
-            const uint32_t v = i < N ? cs.list[i] : 0u;
-            uint32_t pv = __shfl_up_sync(0xffffffffu, v, 1);
-            if (lane == 0 && base) pv = cs.list[base - 1];
+    const bool plain = N >= sparse_t && N < dense_t;       // a C-bit bitmap
+    const bool gaps = !plain && cs.list && N < sparse_t;   // gap codes straight from the ascending list
+    const bool walk = on && !plain && !gaps;               // gap codes of the bitmap or its complement
+    if (ENC && on && gl == 0) put_delta(words, pos0, N);
+    // gap codes from the list, GW at a time
+    {
+        uint64_t acc = 0, p = pos0 + hdr;
+        const uint64_t n = on && gaps ? N : 0;
+        for (uint64_t base = 0; __any_sync(0xffffffffu, base < n); base += GW) {
+            const uint64_t i = base + gl;
+            const uint32_t v = i < n ? cs.list[i] : 0u;
+            uint32_t pv = __shfl_up_sync(0xffffffffu, v, 1, GW);
+            if (gl == 0 && base && base < n) pv = cs.list[base - 1];
             const uint64_t gap = i == 0 ? (uint64_t)v : (uint64_t)(v - pv - 1);
-            uint64_t total;
-            const uint64_t ex = warp_excl_scan64(i < N ? delta_bits(gap) : 0u, total);
-            if (i < N) put_delta(words, p + ex, gap);
-            p += total;
-        }
-        return;
-    }
-    if (cs.bm) {
-        for (uint32_t w = lane; w < nw; w += 32) bm[w] = cs.bm[w];
-    } else {
-        for (uint32_t w = lane; w < nw; w += 32) bm[w] = 0;
-        __syncwarp();
-        warp_or_list(bm, cs.list, 0, N, nw, lane);
-    }
-    __syncwarp();
-    uint64_t pos = pos0;
-    if (ENC && lane == 0) put_delta(words, pos, N);
-    pos += hdr;
-    if (N >= sparse_t && N < dense_t) {
-        // plain C-bit bitmap
-        if (ENC)
-            for (uint32_t w = lane; w < nw; w += 32) {
-                const uint32_t len = min(32u, C - w * 32);
-                or_bits(words, pos + (uint64_t)w * 32, bm[w], len);
+            if (ENC) {
+                uint32_t len = 0, total;
+                const uint64_t c = i < n ? delta_code(gap, len) : 0;
+                const uint32_t ex = group_excl_scan<GW>(len, total);
+                if (i < n) or_bits(words, p + ex, c, len);
+                p += total;
+            } else if (i < n) {
+                acc += delta_bits(gap);
             }
-        if (!ENC && lane == 0) nbits[j] = hdr + C;
-        return;
+        }
+        if (!ENC && on && gaps) {
+            // (only this group's lanes are here: its own mask)
+            const uint32_t gm = GW == 32 ? 0xffffffffu : ((1u << GW) - 1u) << ((threadIdx.x & 31) & ~(GW - 1));
+#pragma unroll
+            for (int o = GW / 2; o; o >>= 1) acc += __shfl_xor_sync(gm, acc, o, GW);
+            if (gl == 0) nbits[j] = hdr + acc;
+        }
     }
+    if (!ENC && on && plain && gl == 0) nbits[j] = hdr + C;
+    // the others through the bitmap
+    const bool need_bm = walk || (ENC && on && plain);
+    if (!__any_sync(0xffffffffu, need_bm)) return;
+    if (need_bm)
+        for (uint32_t w = gl; w < nw; w += GW) bm[w] = cs.bm ? cs.bm[w] : 0u;
+    __syncwarp();
+    if (need_bm && !cs.bm)
+        for (uint64_t c = gl; c < N; c += GW) {
+            const uint32_t v = cs.list[c];
+            atomicOr(&bm[v >> 5], 1u << (v & 31));
+        }
+    __syncwarp();
+    if (ENC && on && plain)
+        for (uint32_t w = gl; w < nw; w += GW)
+            or_bits(words, pos0 + hdr + (uint64_t)w * 32, bm[w], min(32u, C - w * 32));
     const bool want_ones = N < sparse_t;  // else complement: values not in the set
-    const uint32_t per = (nw + 31) / 32;
-    const uint32_t w0 = lane * per, w1 = min(w0 + per, nw);
+    const uint32_t per = (nw + GW - 1) / GW;
+    const uint32_t w0 = walk ? gl * per : 0u, w1 = walk ? min(w0 + per, nw) : 0u;
     auto word_bits = [&](uint32_t w) -> uint32_t {
         uint32_t x = want_ones ? bm[w] : ~bm[w];
         const uint32_t valid = C - w * 32;
@@ -1282,12 +1317,13 @@ __device__ __forceinline__ void encode_one(cand_set const& cs, uint64_t j, uint6
     int32_t prev;
     {
         int32_t x = last;
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t y = __shfl_up_sync(0xffffffffu, x, o);
-            if (lane >= o) x = max(x, y);
+#pragma unroll
+        for (int o = 1; o < GW; o <<= 1) {
+            const int32_t y = __shfl_up_sync(0xffffffffu, x, o, GW);
+            if (gl >= o) x = max(x, y);
         }
-        prev = __shfl_up_sync(0xffffffffu, x, 1);
-        if (lane == 0) prev = -1;
+        prev = __shfl_up_sync(0xffffffffu, x, 1, GW);
+        if (gl == 0) prev = -1;
     }
     uint64_t mybits = 0;
     {
@@ -1304,12 +1340,12 @@ __device__ __forceinline__ void encode_one(cand_set const& cs, uint64_t j, uint6
         }
     }
     uint64_t total;
-    const uint64_t ex = warp_excl_scan64(mybits, total);
+    const uint64_t ex = group_excl_scan<GW>(mybits, total);
     if (!ENC) {
-        if (lane == 0) nbits[j] = hdr + total;
+        if (walk && gl == 0) nbits[j] = hdr + total;
         return;
     }
-    uint64_t p = pos + ex;
+    code_writer out(words, pos0 + hdr + ex);
     int32_t pv = prev;
     for (uint32_t w = w0; w < w1; ++w) {
         uint32_t x = word_bits(w);
@@ -1317,37 +1353,48 @@ __device__ __forceinline__ void encode_one(cand_set const& cs, uint64_t j, uint6
             const uint32_t b = __ffs(x) - 1;
             x &= x - 1;
             const int32_t v = (int32_t)(w * 32 + b);
-            p = put_delta(words, p, pv < 0 ? (uint64_t)v : (uint64_t)(v - pv - 1));
+            uint32_t len;
+            const uint64_t c = delta_code(pv < 0 ? (uint64_t)v : (uint64_t)(v - pv - 1), len);
+            out.put(c, len);
             pv = v;
         }
     }
+    out.end();
 }
 
-// Warp per 32 candidate classes: the lanes fetch the 32 candidates' sets
-// (and pass-1 offsets) at once, then the warp encodes them one by one, so the
-// dependent metadata loads are paid once per 32 candidates.
-template <bool ENC>
-__global__ void k_encode(uint64_t nc, cand_view cv, list_src L, uint32_t C, uint64_t* __restrict__ nbits,
-                         uint64_t const* __restrict__ boff, uint64_t* __restrict__ words) {
+// Warp per 32 candidate classes (class j = candidate order[j], or j): the lanes
+// fetch the 32 candidates' sets (and pass-1 offsets) at once, then groups of GW lanes encode one each, 32 / GW
+// at a time, so the dependent metadata loads are paid once per 32 candidates and a
+// set of few words does not leave most of a warp idle.
+// Bound: latency of the list and bitmap reads, then the bit ORs.  200 genomes (7
+// bitmap words, 4.9e6 classes): whole warps 5.1 ms, groups of 8 1.8 ms;
+// the first batch's classes are encoded where they stay (appending them took 0.5 ms
+// more a batch).
+template <bool ENC, int GW>
+__global__ void k_encode(uint64_t nc, uint32_t const* __restrict__ order, cand_view cv, list_src L, uint32_t C,
+                         uint64_t* __restrict__ nbits, uint64_t const* __restrict__ boff,
+                         uint64_t* __restrict__ words) {
     extern __shared__ uint32_t smem_bm[];
     const uint32_t nw = (C + 31) / 32;
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    uint32_t* bm = smem_bm + (size_t)wib * nw;
+    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5, grp = lane / GW;
+    constexpr int GROUPS = 32 / GW;
+    uint32_t* bm = smem_bm + ((size_t)wib * GROUPS + grp) * nw;
     const uint64_t j0 = ((uint64_t)blockIdx.x * (blockDim.x >> 5) + wib) * 32;
     if (j0 >= nc) return;
     const uint64_t jl = j0 + lane;
     cand_set mine{nullptr, nullptr, 0};
     uint64_t pos = 0;
     if (jl < nc) {
-        mine = cand_get(L, cv.kind_id[jl]);
+        mine = cand_get(L, cv.kind_id[order ? order[jl] : jl]);
         if (ENC) pos = boff[jl];
     }
     const uint32_t cnt = nc - j0 < 32 ? (uint32_t)(nc - j0) : 32u;
-    for (uint32_t q = 0; q < cnt; ++q) {
-        const cand_set cs = shfl_set(mine, (int)q);
-        const uint64_t p = __shfl_sync(0xffffffffu, pos, (int)q);
-        encode_one<ENC>(cs, j0 + q, p, C, nw, bm, lane, nbits, words);
-        __syncwarp();  // the next candidate reuses the bitmap
+    for (uint32_t q0 = 0; q0 < cnt; q0 += GROUPS) {
+        const uint32_t q = q0 + grp;
+        const cand_set cs = shfl_set(mine, (int)(q & 31));
+        const uint64_t p = __shfl_sync(0xffffffffu, pos, (int)(q & 31));
+        encode_one<ENC, GW>(cs, q < cnt, j0 + q, p, C, nw, bm, nbits, words);
+        __syncwarp();  // the next candidates reuse the bitmaps
     }
 }
 
@@ -1410,13 +1457,6 @@ __global__ void __launch_bounds__(256) k_hash_runs(uint64_t n, uint64_t const* _
         if (h) run_start[q] = (uint32_t)i;
         rep_first[i] = NONE32;
     }
-}
-
-// New class j (in first-appearance order) = candidate rcand[j]; cid base+j.
-__global__ void k_assign_new(uint64_t nnew, uint32_t const* __restrict__ rcand, uint64_t base,
-                             uint32_t* __restrict__ cid) {
-    uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (j < nnew) cid[rcand[j]] = (uint32_t)(base + j);
 }
 
 // Set comparison split by length.  A set of at most SHORT_SET words is
@@ -1652,19 +1692,22 @@ __global__ void k_cand_cid(uint64_t nc, uint32_t const* __restrict__ rep, uint32
     if (c < nc) cid[c] = rcid[rep_index[rep[c]]];
 }
 
-// Per new class: encoded length, hash and color count (summed per warp,
-// one atomic per warp on the shared counter).
-__global__ void k_new_sizes(uint64_t nnew, uint32_t const* __restrict__ rcand, cand_view cv, list_src L,
-                            uint64_t const* __restrict__ cb, uint64_t* __restrict__ nbits,
-                            uint64_t* __restrict__ hashes, unsigned long long* __restrict__ ints) {
+// New class j (in first-appearance order) = candidate rcand[j]: its id base + j,
+// hash, color count (summed per warp, one atomic per warp on the shared counter)
+// and, with the candidates' bit offsets cb, its encoded length.
+__global__ void k_new_classes(uint64_t nnew, uint32_t const* __restrict__ rcand, cand_view cv, list_src L,
+                              uint64_t const* __restrict__ cb, uint64_t* __restrict__ nbits,
+                              uint64_t* __restrict__ hashes, uint64_t base, uint32_t* __restrict__ cid,
+                              unsigned long long* __restrict__ ints) {
     const uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     uint64_t n = 0;
     if (j < nnew) {
         const uint32_t c = rcand[j];
         uint32_t const* p;
         cand_list(L, cv.kind_id[c], p, n);
-        nbits[j] = cb[c + 1] - cb[c];
+        if (cb) nbits[j] = cb[c + 1] - cb[c];
         hashes[j] = cv.hash[c];
+        cid[c] = (uint32_t)(base + j);
     }
     const uint64_t sum = warp_sum64(n);
     if ((threadIdx.x & 31) == 0 && sum) atomicAdd(ints, (unsigned long long)sum);
@@ -3194,89 +3237,107 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
             compact_reps(wp2);
             nr = read_dev(wp2.total, st);
         }
-        int wpb = (int)std::max<uint64_t>(1, std::min<uint64_t>(8, (96 * 1024) / (4ull * nw)));
-        const size_t shm = (size_t)wpb * nw * 4;
-        if (shm > 48 * 1024) {
-            CDBG_CUDA(cudaFuncSetAttribute(k_encode<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-            CDBG_CUDA(cudaFuncSetAttribute(k_encode<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-        }
         uint64_t* cbits = A.alloc<uint64_t>(nr);
-        uint64_t* cb = A.alloc<uint64_t>(nr + 1);
-        {
-            CDBG_PROF("k_encode", st);
-            k_encode<false><<<grid(ceil_div(nr, 32), wpb), wpb * 32, shm, st>>>(nr, rv, L, C, cbits, nullptr, nullptr);
-        }
-        CDBG_CHECK_LAUNCH();
-        prim::exclusive_scan<uint64_t, uint64_t>(cbits, cb, nr, A, st, cb + nr);
-        const uint64_t ctot = read_dev(cb + nr, st);
-        const uint64_t cwn = ctot / 64 + 4;
-        uint64_t* cw = A.alloc<uint64_t>(cwn);
-        CDBG_CUDA(cudaMemsetAsync(cw, 0, 8 * cwn, st));
-        {
-            CDBG_PROF("k_encode", st);
-            k_encode<true><<<grid(ceil_div(nr, 32), wpb), wpb * 32, shm, st>>>(nr, rv, L, C, nullptr, cb, cw);
-        }
-        CDBG_CHECK_LAUNCH();
-        // 3. new classes in order of first appearance.  An empty dictionary (the
-        // first batch) holds none of them.
+        // lanes per candidate: one per bitmap word, 8 at least
+        auto encode = [&](auto enc, uint32_t const* order, uint64_t* nbits, uint64_t const* boff, uint64_t* words) {
+            constexpr bool ENC = decltype(enc)::value;
+            auto launch = [&](auto kern, int groups) {
+                const uint64_t wbytes = 4ull * nw * groups;  // bitmaps of a warp
+                const int wpb = (int)std::max<uint64_t>(1, std::min<uint64_t>(8, (96 * 1024) / wbytes));
+                const size_t shm = wpb * wbytes;
+                if (shm > 48 * 1024)
+                    CDBG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
+                CDBG_PROF("k_encode", st);
+                kern<<<grid(ceil_div(nr, 32), wpb), wpb * 32, shm, st>>>(nr, order, rv, L, C, nbits, boff, words);
+                CDBG_CHECK_LAUNCH();
+            };
+            if (nw <= 8)
+                launch(k_encode<ENC, 8>, 4);
+            else if (nw <= 16)
+                launch(k_encode<ENC, 16>, 2);
+            else
+                launch(k_encode<ENC, 32>, 1);
+        };
         uint32_t* rcid = A.alloc<uint32_t>(nr + 1);
-        const bool all_new = dict.n == 0;
-        uint64_t nnew = nr;
-        uint32_t* rkey = rv.first;
         uint32_t* rcand = A.alloc<uint32_t>(nr);
-        if (!all_new) {
+        const int node_bits = D > 1 ? 64 - __builtin_clzll(D - 1) : 1;
+        const uint64_t base = dict.n;
+        uint64_t nnew = nr, badd = 0;
+        auto room = [&](uint64_t classes, uint64_t words) {
+            if (p.copy_st && (dict.bit_off.cap < classes + 1 || dict.words.cap < words)) {
+                // growing frees the old arrays: after the host copies that read them
+                CDBG_CUDA(cudaEventRecord(p.copy_ev, p.copy_st));
+                CDBG_CUDA(cudaStreamWaitEvent(st, p.copy_ev, 0));
+            }
+            dict.cls_hash.reserve(classes, st);
+            dict.bit_off.reserve(classes + 1, st);
+            dict.words.reserve(words, st, true);
+        };
+        auto new_classes = [&](uint64_t const* cb, uint64_t* nbits) {
+            CDBG_PROF("k_new_classes", st);
+            k_new_classes<<<grid(nnew, 256), 256, 0, st>>>(nnew, rcand, rv, L, cb, nbits, dict.cls_hash.p + base, base,
+                                                           rcid, ints);
+            CDBG_CHECK_LAUNCH();
+        };
+        if (base == 0) {
+            // an empty dictionary (the first batch): every representative is a new
+            // class, encoded where it stays, in order of first appearance
+            prim::radix_sort_pairs<uint32_t, uint32_t>(rv.first, rcand, nr, 0, node_bits, A, st, d_err, true);
+            room(nr, 0);
+            new_classes(nullptr, nullptr);
+            encode(std::false_type{}, rcand, cbits, nullptr, nullptr);
+            prim::exclusive_scan<uint64_t, uint64_t>(cbits, dict.bit_off.p, nr, A, st, dict.bit_off.p + nr);
+            badd = read_dev(dict.bit_off.p + nr, st);
+            room(nr, (badd + 63) / 64 + 4);
+            encode(std::true_type{}, rcand, nullptr, dict.bit_off.p, dict.words.p);
+        } else {
+            // 3. the dictionary is asked by encoding; the classes it does not hold
+            // are new, in order of first appearance
+            uint64_t* cb = A.alloc<uint64_t>(nr + 1);
+            encode(std::false_type{}, nullptr, cbits, nullptr, nullptr);
+            prim::exclusive_scan<uint64_t, uint64_t>(cbits, cb, nr, A, st, cb + nr);
+            const uint64_t ctot = read_dev(cb + nr, st);
+            const uint64_t cwn = ctot / 64 + 4;
+            uint64_t* cw = A.alloc<uint64_t>(cwn);
+            CDBG_CUDA(cudaMemsetAsync(cw, 0, 8 * cwn, st));
+            encode(std::true_type{}, nullptr, nullptr, cb, cw);
             dict.ensure_table(st, d_err);
             {
                 CDBG_PROF("k_dict_lookup", st);
                 k_dict_lookup<<<grid(nr, 256), 256, 0, st>>>(nr, rv, cw, cb, dict.view(), rcid);
             }
             CDBG_CHECK_LAUNCH();
-            rkey = A.alloc<uint32_t>(nr);
+            uint32_t* rkey = A.alloc<uint32_t>(nr);
+            wn.ntiles = zero_block::tiles(nr, prim::SEL_TILE);
             {
                 CDBG_PROF("k_new_reps", st);
-                k_new_reps<<<(unsigned)zero_block::tiles(nr, prim::SEL_TILE), 256, 0, st>>>(
-                    nr, rcid, select_ws{wn.status, wn.total, wn.counter, zero_block::tiles(nr, prim::SEL_TILE)}, rv, rkey,
-                    rcand, d_err);
+                k_new_reps<<<(unsigned)wn.ntiles, 256, 0, st>>>(nr, rcid, wn, rv, rkey, rcand, d_err);
             }
             CDBG_CHECK_LAUNCH();
             nnew = read_dev(wn.total, st);
-        }
-        if (nnew) {
-            const int node_bits = D > 1 ? 64 - __builtin_clzll(D - 1) : 1;
-            prim::radix_sort_pairs<uint32_t, uint32_t>(rkey, rcand, nnew, 0, node_bits, A, st, d_err, all_new);
-            const uint64_t base = dict.n;
-            k_assign_new<<<grid(nnew, 256), 256, 0, st>>>(nnew, rcand, base, rcid);
-            CDBG_CHECK_LAUNCH();
-            uint64_t* nbits = A.alloc<uint64_t>(nnew);
-            uint64_t* nh = A.alloc<uint64_t>(nnew);
-            uint64_t* boff = A.alloc<uint64_t>(nnew + 1);
-            k_new_sizes<<<grid(nnew, 256), 256, 0, st>>>(nnew, rcand, rv, L, cb, nbits, nh, ints);
-            CDBG_CHECK_LAUNCH();
-            prim::exclusive_scan<uint64_t, uint64_t>(nbits, boff, nnew, A, st, boff + nnew);
-            const uint64_t badd = all_new ? ctot : read_dev(boff + nnew, st);
-            add_offsets(boff, nnew + 1, dict.nbits, boff, st);  // absolute bit offsets
-            if (p.copy_st && (dict.bit_off.cap < base + nnew + 1 ||
-                              dict.words.cap < (dict.nbits + badd + 63) / 64 + 4)) {
-                // growing frees the old arrays: after the host copies that read them
-                CDBG_CUDA(cudaEventRecord(p.copy_ev, p.copy_st));
-                CDBG_CUDA(cudaStreamWaitEvent(st, p.copy_ev, 0));
+            if (nnew) {
+                prim::radix_sort_pairs<uint32_t, uint32_t>(rkey, rcand, nnew, 0, node_bits, A, st, d_err);
+                uint64_t* nbits = A.alloc<uint64_t>(nnew);
+                uint64_t* boff = A.alloc<uint64_t>(nnew + 1);
+                room(base + nnew, 0);
+                new_classes(cb, nbits);
+                prim::exclusive_scan<uint64_t, uint64_t>(nbits, boff, nnew, A, st, boff + nnew);
+                badd = read_dev(boff + nnew, st);
+                add_offsets(boff, nnew + 1, dict.nbits, boff, st);  // absolute bit offsets
+                room(base + nnew, (dict.nbits + badd + 63) / 64 + 4);
+                CDBG_CUDA(cudaMemcpyAsync(dict.bit_off.p + base, boff, 8 * (nnew + 1), cudaMemcpyDeviceToDevice, st));
+                {
+                    CDBG_PROF("k_append_bits", st);
+                    k_append_bits<<<grid(nnew, 8), 256, 0, st>>>(nnew, rcand, cw, cb, boff, dict.words.p);
+                }
+                CDBG_CHECK_LAUNCH();
             }
-            dict.cls_hash.reserve(base + nnew, st);
-            dict.bit_off.reserve(base + nnew + 1, st);
-            CDBG_CUDA(cudaMemcpyAsync(dict.cls_hash.p + base, nh, 8 * nnew, cudaMemcpyDeviceToDevice, st));
-            CDBG_CUDA(cudaMemcpyAsync(dict.bit_off.p + base, boff, 8 * (nnew + 1), cudaMemcpyDeviceToDevice, st));
-            dict.words.reserve((dict.nbits + badd + 63) / 64 + 4, st, true);
-            {
-                CDBG_PROF("k_append_bits", st);
-                k_append_bits<<<grid(nnew, 8), 256, 0, st>>>(nnew, rcand, cw, cb, boff, dict.words.p);
-            }
-            CDBG_CHECK_LAUNCH();
-            dict.n = base + nnew;
-            dict.cls_hash.n = dict.n;
-            dict.bit_off.n = dict.n + 1;
-            dict.nbits += badd;
-            dict.words.n = (dict.nbits + 63) / 64;
         }
+        dict.n = base + nnew;
+        dict.cls_hash.n = dict.n;
+        dict.bit_off.n = dict.n + 1;
+        dict.nbits += badd;
+        dict.words.n = (dict.nbits + 63) / 64;
         // 4. every candidate takes its representative's class id
         k_cand_cid<<<grid(nc, 256), 256, 0, st>>>(nc, rep, rep_index, rcid, cid);
         CDBG_CHECK_LAUNCH();

@@ -116,3 +116,25 @@ def test_cycles_and_broken_chains(oracle, engine, tmp_path, k, unit):
         d = tmp_path / str(B)
         d.mkdir()
         _check(oracle, engine, d, [g0, g1, g2], k, B)
+
+
+@pytest.mark.parametrize("colors", [1, 2, 3, 31, 255, 256, 257, 512, 513, 1100])
+def test_color_set_encoding(oracle, engine, tmp_path, colors):
+    """Color sets of every form (sparse, plain bitmap, complement, all) at the
+    widths where the encoder's lane groups change, some classes new in a later
+    batch."""
+    k, B = 31, 8
+    rng = np.random.default_rng(colors)
+    blocks = [_dna(rng, 90 + 7 * i) for i in range(9)]
+    share = [1.0, 0.95, 0.8, 0.74, 0.5, 0.26, 0.2, 0.05, 0.0]
+    genomes = [[b for b, p in zip(blocks, share) if rng.random() < p] + [_dna(rng, 40)] for _ in range(colors)]
+    genomes[-1].append(blocks[-1])
+    _check(oracle, engine, tmp_path, genomes, k, B)
+    flat = [(s, g) for g, seqs in enumerate(genomes) for s in seqs]
+    hb = native.host_batch([s for s, _ in flat], [g for _, g in flat])
+
+    def out(**kw):
+        r = engine.build(hb, k, B, colors, **kw)
+        return native.result_frag_bytes(r), native.result_class_words(r).tobytes(), native.result_class_offsets(r).tobytes()
+
+    assert out(batch_occ=64) == out()
