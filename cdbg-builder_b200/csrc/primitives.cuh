@@ -311,14 +311,18 @@ constexpr int RS_WARPS = RS_THREADS / 32;
 // *err and publishes what it has, so no successor waits on it, and its
 // successors' positions can only come out smaller than the true ones, which
 // keeps every write inside the output.
+// Bound: latency of the ranking (matches and counter updates; 27% issue, 24 warps
+// per SM by registers).  All matches before the counter updates, values after the
+// keys through the same buffer: 9.8 -> 9.3 ms of a 200-genome build; 4 blocks per SM
+// (64 registers, spilling) 9.6, 5 blocks 10.8.
 constexpr unsigned long long RS_AGG = 1ull << 62, RS_INC = 2ull << 62, RS_VALMASK = (1ull << 58) - 1;
 
 template <int BITS, int ITEMS, typename K, typename V>
 struct rs_smem {
     static constexpr int BINS = 1 << BITS;
     static constexpr int TILE = RS_THREADS * ITEMS;
-    K sk[TILE];
-    V sv[TILE];
+    static_assert(sizeof(V) <= sizeof(K), "keys and values share the buffer");
+    K sk[TILE];                     // keys in digit order, then values
     uint32_t wcnt[RS_WARPS][BINS];  // per-warp digit counts, then prefixes
     uint32_t dstart[BINS];          // tile-local start of each digit
     uint64_t gbase[BINS];           // global start of each digit for this tile
@@ -346,30 +350,28 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
     const uint64_t base = tile * TILE;
     const uint32_t tile_n = (uint32_t)((n - base) < (uint64_t)TILE ? (n - base) : TILE);
     K k[ITEMS];
-    V v[ITEMS];
     uint32_t rk[ITEMS];
+    const uint32_t p0 = (uint32_t)warp * (ITEMS * 32) + lane;  // round r: position p0 + 32 r
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) k[r] = p0 + 32u * r < tile_n ? keys_in[base + p0 + 32u * r] : ~K(0);
+    // the lanes of each round with the same digit (positions past the end have a
+    // digit of their own): all rounds' matches first, they do not depend on each
+    // other; then the warp's counters round by round
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r)
+        rk[r] = __match_any_sync(0xffffffffu, p0 + 32u * r < tile_n ? (uint32_t)(k[r] >> shift) & (BINS - 1) : BINS);
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
-        const uint32_t pos = (uint32_t)warp * (ITEMS * 32) + (uint32_t)r * 32 + lane;
-        const bool ok = pos < tile_n;
-        k[r] = ok ? keys_in[base + pos] : ~K(0);
-        v[r] = !ok ? V(0) : vals_in ? vals_in[base + pos] : (V)(base + pos);
-    }
-#pragma unroll
-    for (int r = 0; r < ITEMS; ++r) {
-        const uint32_t pos = (uint32_t)warp * (ITEMS * 32) + (uint32_t)r * 32 + lane;
-        const bool ok = pos < tile_n;
-        const uint32_t d = ok ? (uint32_t)((k[r] >> shift) & (BINS - 1)) : BINS;  // sentinel
-        const uint32_t active = __ballot_sync(0xffffffffu, ok);
-        const uint32_t peers = __match_any_sync(0xffffffffu, d) & active;
+        const bool ok = p0 + 32u * r < tile_n;
+        const uint32_t peers = rk[r];
+        const int leader = __ffs(peers) - 1;
         uint32_t old = 0;
-        const int leader = peers ? __ffs(peers) - 1 : 0;
         if (ok && lane == leader) {
+            const uint32_t d = (uint32_t)(k[r] >> shift) & (BINS - 1);
             old = sm.wcnt[warp][d];
             sm.wcnt[warp][d] = old + __popc(peers);
         }
-        old = __shfl_sync(0xffffffffu, old, leader);
-        rk[r] = ok ? old + __popc(peers & lanemask_lt()) : 0;
+        rk[r] = __shfl_sync(0xffffffffu, old, leader) + __popc(peers & lanemask_lt());
     }
     __syncthreads();
     // per digit: exclusive prefix over warps and the tile's count
@@ -439,26 +441,46 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
         }
     }
     __syncthreads();
+    // keys, then values, through the same buffer in digit order
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
-        const uint32_t pos = (uint32_t)warp * (ITEMS * 32) + (uint32_t)r * 32 + lane;
-        if (pos < tile_n) {
-            const uint32_t d = (uint32_t)((k[r] >> shift) & (BINS - 1));
-            const uint32_t lp = sm.dstart[d] + sm.wcnt[warp][d] + rk[r];
-            sm.sk[lp] = k[r];
-            sm.sv[lp] = v[r];
+        if (p0 + 32u * r < tile_n) {
+            const uint32_t d = (uint32_t)(k[r] >> shift) & (BINS - 1);
+            rk[r] += sm.dstart[d] + sm.wcnt[warp][d];
+            sm.sk[rk[r]] = k[r];
+        }
+    }
+    V v[ITEMS];
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r) {
+        const uint32_t p = p0 + 32u * r;
+        v[r] = p >= tile_n ? V(0) : vals_in ? vals_in[base + p] : (V)(base + p);
+    }
+    __syncthreads();
+    uint32_t dst[ITEMS];  // (n < 2^32)
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t p = threadIdx.x + i * RS_THREADS;
+        dst[i] = 0xffffffffu;
+        if (p < tile_n) {
+            const K key = sm.sk[p];
+            const uint32_t d = (uint32_t)((key >> shift) & (BINS - 1));
+            const uint64_t o = sm.gbase[d] + (p - sm.dstart[d]);
+            if (o < n) {
+                dst[i] = (uint32_t)o;
+                keys_out[o] = key;
+            }
         }
     }
     __syncthreads();
-    for (uint32_t p = threadIdx.x; p < tile_n; p += RS_THREADS) {
-        const K key = sm.sk[p];
-        const uint32_t d = (uint32_t)((key >> shift) & (BINS - 1));
-        const uint64_t dst = sm.gbase[d] + (p - sm.dstart[d]);
-        if (dst < n) {
-            keys_out[dst] = key;
-            vals_out[dst] = sm.sv[p];
-        }
-    }
+    V* sv = reinterpret_cast<V*>(sm.sk);
+#pragma unroll
+    for (int r = 0; r < ITEMS; ++r)
+        if (p0 + 32u * r < tile_n) sv[rk[r]] = v[r];
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+        if (dst[i] != 0xffffffffu) vals_out[dst[i]] = sv[threadIdx.x + i * RS_THREADS];
 }
 
 // Up to RS_SMALL pairs: the whole LSD sort by one block in shared memory, in one
