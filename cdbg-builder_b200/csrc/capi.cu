@@ -702,6 +702,42 @@ int cdbg_gpu_phase1(cdbg_engine* e, const cdbg_phase1_args* a, cdbg_phase1_stats
     }
 }
 
+namespace {
+// Device bytes src[0, n) to a file at `off` through the pinned buffer `buf`: the
+// copy goes in pieces and each is written by the host threads while the next ones
+// still copy.
+void write_from_device(cdbg_engine* e, uint8_t const* src, uint8_t* buf, uint64_t n, cdbg::io::range_file& f,
+                       uint64_t off, uint32_t threads) {
+    if (n == 0) return;
+    const uint64_t piece = std::max<uint64_t>(16ull << 20, cdbg::ceil_div(n, 8));
+    const size_t np = (size_t)cdbg::ceil_div(n, piece);
+    struct events {
+        std::vector<cudaEvent_t> v;
+        ~events() {
+            for (auto x : v) cudaEventDestroy(x);
+        }
+    } ev;
+    for (size_t i = 0; i < np; ++i) {
+        const uint64_t x = i * piece, c = std::min(piece, n - x);
+        CDBG_CUDA(cudaMemcpyAsync(buf + x, src + x, c, cudaMemcpyDeviceToHost, e->st));
+        cudaEvent_t v;
+        CDBG_CUDA(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
+        ev.v.push_back(v);
+        CDBG_CUDA(cudaEventRecord(v, e->st));
+    }
+    try {
+        for (size_t i = 0; i < np; ++i) {
+            const uint64_t x = i * piece, c = std::min(piece, n - x);
+            CDBG_CUDA(cudaEventSynchronize(ev.v[i]));
+            f.write(buf + x, off + x, c, threads);
+        }
+    } catch (...) {
+        cudaStreamSynchronize(e->st);  // the buffer's copies are done before the caller goes on
+        throw;
+    }
+}
+}  // namespace
+
 int cdbg_gpu_phase2(cdbg_engine* e, const cdbg_phase2_args* a, cdbg_phase2_stats* s) {
     if (!e) {
         g_last_error = "null engine";
@@ -763,14 +799,17 @@ int cdbg_gpu_phase2(cdbg_engine* e, const cdbg_phase2_args* a, cdbg_phase2_stats
                 rerr = std::current_exception();
             }
         };
-        std::FILE* ff = std::fopen(a->frag_path, "wb");
-        if (!ff) throw std::runtime_error(std::string("cannot open frag spill: ") + a->frag_path);
-        struct file_closer {
-            std::FILE*& f;
-            ~file_closer() {
-                if (f) std::fclose(f);
-            }
-        } fc{ff};
+        std::unique_ptr<cdbg::io::range_file> ff;
+        try {
+            ff.reset(new cdbg::io::range_file(a->frag_path));
+        } catch (std::exception const&) {
+            throw std::runtime_error(std::string("cannot open frag spill: ") + a->frag_path);
+        }
+        uint64_t written = 0;
+        // the fragments stay on the device until their range is done and come
+        // through pinned memory (an engine with a memory cap keeps them in scratch,
+        // which its cap covers, and returns them batch by batch)
+        const bool resident = e->mem_limit == 0;
         cdbg_phase2_stats st{};
         cdbg::phase2_result res;
         double dev_s = 0;
@@ -801,30 +840,42 @@ int cdbg_gpu_phase2(cdbg_engine* e, const cdbg_phase2_args* a, cdbg_phase2_stats
             pp.table_slots_q = e->tune.table_slots_q;
             pp.union_bitmaps = e->tune.union_lists == 0;
             pp.group_bytes = e->tune.table_group_mb ? (uint64_t)e->tune.table_group_mb << 20 : ~0ull;
-            pp.to_host = true;
+            pp.to_host = !resident;
             pp.keep_dict = i > 0;
             pp.copy_dict = i + 1 == nr;
             res.state = &e->p2;
             cdbg::run_phase2(rs, pp, e->A, e->st, e->d_err, res);
             dev_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - td).count();
             // this range's fragments, then (only then) its bucket files go
-            if (!res.frag.empty() && std::fwrite(res.frag.data(), 1, res.frag.size(), ff) != res.frag.size())
-                throw std::runtime_error(std::string("short write to ") + a->frag_path);
-            if (a->delete_consumed) {
-                if (std::fflush(ff) != 0) throw std::runtime_error(std::string("short write to ") + a->frag_path);
-                cdbg::io::delete_bucket_files(dir, rb[i], rb[i + 1]);
-            }
+            if (resident)
+                write_from_device(e, res.d_frag, (uint8_t*)e->h_frag.ensure(res.frag_nbytes + 8), res.frag_nbytes, *ff,
+                                  written, T);
+            else
+                ff->write(res.frag.data(), written, res.frag.size(), T);
+            written += res.frag_nbytes;
+            if (a->delete_consumed) cdbg::io::delete_bucket_files(dir, rb[i], rb[i + 1]);
             st.n_records += rs.n;
             st.n_kmers += res.n_occ;
             st.n_distinct += res.n_distinct;
             st.n_fragments += res.n_fragments;
             st.total_seq_bytes += res.total_seq_bytes;
         }
-        if (std::fclose(ff) != 0) {
-            ff = nullptr;
-            throw std::runtime_error(std::string("short write to ") + a->frag_path);
+        ff->finish(written);
+        const uint64_t nwords = (res.nbits + 63) / 64;
+        uint64_t const* words = res.words.data();
+        if (resident && (a->color_sets_path || a->on_class)) {
+            uint64_t* hw = (uint64_t*)e->h_words.ensure(8 * nwords + 8);
+            if (nwords) CDBG_CUDA(cudaMemcpyAsync(hw, res.d_words, 8 * nwords, cudaMemcpyDeviceToHost, e->st));
+            if (a->on_class) {
+                res.offsets.resize(res.n_classes);
+                if (res.n_classes)
+                    CDBG_CUDA(cudaMemcpyAsync(res.offsets.data(), res.d_offsets, 8 * res.n_classes,
+                                              cudaMemcpyDeviceToHost, e->st));
+            }
+            CDBG_CUDA(cudaStreamSynchronize(e->st));
+            if (a->on_class) res.words.assign(hw, hw + nwords);
+            words = hw;
         }
-        ff = nullptr;
         if (a->color_sets_path) {
             // the Elias-Fano finalize of the class offsets runs on the device,
             // over the offsets the dictionary holds there
@@ -838,7 +889,7 @@ int cdbg_gpu_phase2(cdbg_engine* e, const cdbg_phase2_args* a, cdbg_phase2_stats
                 CDBG_CUDA(cudaMemcpyAsync(lh.data() + ef.low_words, ef.high, 8 * ef.high_words,
                                           cudaMemcpyDeviceToHost, e->st));
             CDBG_CUDA(cudaStreamSynchronize(e->st));
-            cdbg::io::write_color_sets_ef(a->color_sets_path, a->num_colors, res.words.data(), res.nbits, ef.n,
+            cdbg::io::write_color_sets_ef(a->color_sets_path, a->num_colors, words, res.nbits, ef.n,
                                           ef.l, lh.data(), lh.data() + ef.low_words, ef.high_bits);
         }
         if (a->on_class) {
@@ -1600,7 +1651,8 @@ int cdbg_gpu_build_files(cdbg_engine* e, const cdbg_build_files_args* a, cdbg_bu
             uint64_t* hw = (uint64_t*)e->h_words.ensure(8 * nwords + 8);
             uint64_t* hl = (uint64_t*)e->h_offsets.ensure(
                 a->color_sets_path ? 8 * (ef.low_words + ef.high_words) + 16 : 8 * r->n_color_sets + 8);
-            if (frag_out && r->frag_nbytes > have)
+            // (with a frag file, the rest goes to it piece by piece below)
+            if (frag_out && !fw && r->frag_nbytes > have)
                 CDBG_CUDA(cudaMemcpyAsync(hf + have, r->frag_bytes + have, r->frag_nbytes - have,
                                           cudaMemcpyDeviceToHost, e->st));
             if (!a->color_sets_path) {
@@ -1638,7 +1690,13 @@ int cdbg_gpu_build_files(cdbg_engine* e, const cdbg_build_files_args* a, cdbg_bu
             if (fw) {
                 try {
                     fw->drain();  // the streamed ranges are in the file
-                    fw->file.write(hf + streamed, streamed, r->frag_nbytes - streamed, th);
+                    // (a buffer that just moved takes them again, for the result)
+                    if (have < streamed)
+                        CDBG_CUDA(cudaMemcpyAsync(hf + have, r->frag_bytes + have, streamed - have,
+                                                  cudaMemcpyDeviceToHost, e->st));
+                    write_from_device(e, r->frag_bytes + streamed, hf + streamed, r->frag_nbytes - streamed, fw->file,
+                                      streamed, th);
+                    CDBG_CUDA(cudaStreamSynchronize(e->st));
                     fw->file.finish(r->frag_nbytes);
                 } catch (...) {
                     if (cs_writer.joinable()) cs_writer.join();

@@ -335,13 +335,14 @@ range_file::~range_file() {
 
 void range_file::write(uint8_t const* data, uint64_t off, uint64_t n, uint32_t threads) {
     if (n == 0) return;
-    const uint64_t piece = std::max<uint64_t>(32ull << 20, (n + threads - 1) / std::max<uint32_t>(threads, 1));
+    const uint64_t piece = std::max<uint64_t>(4ull << 20, (n + threads - 1) / std::max<uint32_t>(threads, 1));
     const size_t np = (size_t)((n + piece - 1) / piece);
     std::atomic<bool> bad{false};
     void* map = MAP_FAILED;
     const uint64_t pg = (uint64_t)::sysconf(_SC_PAGESIZE);
     const uint64_t a = off & ~(pg - 1);
-    if (m_tmpfs && ::fallocate(m_fd, 0, (off_t)off, (off_t)n) == 0)
+    // (one piece gains nothing from a mapping)
+    if (m_tmpfs && np > 1 && ::fallocate(m_fd, 0, (off_t)off, (off_t)n) == 0)
         map = ::mmap(nullptr, (size_t)(off + n - a), PROT_WRITE, MAP_SHARED, m_fd, (off_t)a);
     if (map != MAP_FAILED) {
         uint8_t* dst = (uint8_t*)map + (off - a);
