@@ -912,87 +912,136 @@ __global__ void k_heavy_bitmaps(uint64_t nrec, uint32_t const* __restrict__ flag
     }
 }
 
-// Warp per multi-record node: OR of its records' color sets (bitmap words for
+// A group of GW lanes per union: OR of its records' color sets (bitmap words for
 // heavy records, per-color bits for the rest) -> mbits, size, set hash.
-// The records' metadata is fetched 32 at a time, one record per lane; heavy
-// records' bitmap words are ORed into registers (lane owns words lane + 32u,
+// The records' metadata is fetched GW at a time, one record per lane; heavy
+// records' bitmap words are ORed into registers (lane owns words lane + GW u,
 // u < WPL), four records' lines in flight at a time; the rest have their
-// colors spread over the lanes and set bits in the warp's shared bitmap.
-template <int WPL>
-__global__ void __launch_bounds__(256) k_union_bm(
+// colors spread over the lanes and set bits in the group's shared bitmap.
+// Groups of a warp go through the loops together, and a union of more than
+// 4 GW records has its remaining ones spread over the whole warp (90 genomes
+// in skewed buckets: 3.1 ms, 4.3 with a group alone on its union).
+// Bound: issue, at 32 registers so that all warps fit (40: 1.5 ms).  200
+// genomes, 7 words, a handful of records per union: whole warps 2.9 ms, groups
+// of 16 2.3, of 8 1.25.
+template <int WPL, int GW>
+__global__ void __launch_bounds__(256, WPL == 1 ? 8 : 1) k_union_bm(
     uint64_t M, uint64_t const* __restrict__ mbeg, uint64_t const* __restrict__ mend,
     uint32_t const* __restrict__ urec, uint64_t const* __restrict__ col_off, uint32_t const* __restrict__ colors,
     uint32_t R0, uint32_t const* __restrict__ hflag, uint64_t const* __restrict__ hpos,
     uint32_t const* __restrict__ rbits, uint32_t nw, uint32_t* __restrict__ mbits, uint32_t* __restrict__ msize,
     uint64_t* __restrict__ mhash) {
     extern __shared__ uint32_t smem_bm[];
-    const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
-    uint32_t* bm = smem_bm + (size_t)wib * nw;
-    const uint64_t m = (uint64_t)blockIdx.x * (blockDim.x >> 5) + wib;
-    if (m >= M) return;
-    for (uint32_t w = lane; w < nw; w += 32) bm[w] = 0;
+    constexpr uint32_t FULL = 0xffffffffu;
+    constexpr uint32_t GMASK = GW == 32 ? FULL : (1u << (GW & 31)) - 1u;
+    const int lane = threadIdx.x & 31, gl = lane & (GW - 1), gs = lane & ~(GW - 1);
+    const uint32_t grp = threadIdx.x / GW;
+    uint32_t* bm = smem_bm + (size_t)grp * nw;
+    const uint64_t m = (uint64_t)blockIdx.x * (blockDim.x / GW) + grp;
+    if (__all_sync(FULL, m >= M)) return;
+    const bool on = m < M;
+    for (uint32_t w = gl; w < nw; w += GW) bm[w] = 0;
     __syncwarp();
     uint32_t acc[WPL];
 #pragma unroll
     for (int u = 0; u < WPL; ++u) acc[u] = 0;
-    const uint64_t pend = mend[m];
-    for (uint64_t p0 = mbeg[m]; p0 < pend; p0 += 32) {
-        const uint64_t p = p0 + lane;
-        bool heavy = false, light = false;
-        uint64_t src = 0, c0 = 0, c1 = 0;
-        if (p < pend) {
-            const uint32_t r = urec[p];
-            heavy = hflag && hflag[r - R0] != 0;
-            light = !heavy;
-            if (heavy) {
-                src = hpos[r - R0] * (uint64_t)nw;
-            } else {
-                c0 = col_off[r];
-                c1 = col_off[r + 1];
+    // [p0, pend): the records a group goes through, GW of them every `stride`,
+    // into its registers and the bitmap `to`: first its own union's, then, one
+    // long union of the warp after another, its share of that one's rest
+    const uint64_t pe = on ? mend[m] : 0;
+    uint64_t p0 = on ? mbeg[m] : 0, pend = pe, rest = pe;
+    uint32_t stride = GW, longs = 0;
+    uint32_t* to = bm;
+    if constexpr (GW < 32) {
+        if (p0 + 4 * GW < pe) rest = pend = p0 + 4 * GW;
+        longs = __ballot_sync(FULL, gl == 0 && rest < pe);
+    }
+    int own = gs;          // the first lane of the group whose union the records belong to
+    uint32_t keep[WPL];    // the words of a group's own union while it helps another's
+    for (;;) {
+        for (; __any_sync(FULL, p0 < pend); p0 += stride) {
+            const uint64_t p = p0 + gl;
+            bool heavy = false, light = false;
+            uint64_t src = 0, c0 = 0, c1 = 0;
+            if (p < pend) {
+                const uint32_t r = urec[p];
+                heavy = hflag && hflag[r - R0] != 0;
+                light = !heavy;
+                if (heavy) {
+                    src = hpos[r - R0] * (uint64_t)nw;
+                } else {
+                    c0 = col_off[r];
+                    c1 = col_off[r + 1];
+                }
+            }
+            uint32_t hm = (__ballot_sync(FULL, heavy) >> gs) & GMASK;
+            while (__any_sync(FULL, hm != 0)) {
+                // four records' lines in flight (a record repeats when fewer remain)
+                const bool any = hm != 0;
+                int q[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    q[j] = hm ? __ffs(hm) - 1 : j ? q[0] : 0;
+                    if (hm) hm &= hm - 1;
+                }
+                uint64_t s[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) s[j] = __shfl_sync(FULL, src, q[j], GW);
+#pragma unroll
+                for (int u = 0; u < WPL; ++u) {
+                    const uint32_t w = gl + GW * u;
+                    if (any && w < nw) acc[u] |= rbits[s[0] + w] | rbits[s[1] + w] | rbits[s[2] + w] | rbits[s[3] + w];
+                }
+            }
+            // light records: their colors laid end to end over the group, GW at a
+            // time (a lane finds its record by a search over the length prefix)
+            const uint32_t len = light ? (uint32_t)(c1 - c0) : 0u;  // < 8192 colors in bitmap mode
+            uint32_t incl = len;
+#pragma unroll
+            for (int o = 1; o < GW; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, incl, o, GW);
+                if (gl >= o) incl += y;
+            }
+            const uint32_t excl = incl - len;
+            const uint32_t total = __shfl_sync(FULL, incl, GW - 1, GW);
+            for (uint32_t e0 = 0; __any_sync(FULL, e0 < total); e0 += GW) {
+                const uint32_t e = e0 + gl;
+                int q = 0;  // the last lane whose range starts at or before e
+#pragma unroll
+                for (int step = GW / 2; step; step >>= 1) {
+                    const uint32_t ex = __shfl_sync(FULL, excl, (q + step) & (GW - 1), GW);
+                    if (q + step < GW && ex <= e) q += step;
+                }
+                const uint64_t cq = __shfl_sync(FULL, c0, q, GW);
+                const uint32_t xq = __shfl_sync(FULL, excl, q, GW);
+                if (e < total) {
+                    const uint32_t v = colors[cq + (e - xq)];
+                    atomicOr(&to[v >> 5], 1u << (v & 31));
+                }
             }
         }
-        uint32_t hm = __ballot_sync(0xffffffffu, heavy);
-        while (hm) {
-            // four records' lines in flight (a record repeats when fewer remain)
-            int q[4];
+        if constexpr (GW == 32) {
+            break;
+        } else {
+            if (stride == 32) {
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                q[j] = hm ? __ffs(hm) - 1 : q[0];
-                if (hm) hm &= hm - 1;
+                for (int u = 0; u < WPL; ++u) {
+#pragma unroll
+                    for (int o = GW; o < 32; o <<= 1) acc[u] |= __shfl_xor_sync(FULL, acc[u], o);
+                    if (gs != own) acc[u] = keep[u];
+                }
             }
-            uint64_t s[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) s[j] = __shfl_sync(0xffffffffu, src, q[j]);
+            if (!longs) break;
+            own = __ffs(longs) - 1;
+            longs &= longs - 1;
+            stride = 32;
+            p0 = __shfl_sync(FULL, rest, own) + gs;
+            pend = __shfl_sync(FULL, pe, own);
+            to = smem_bm + (size_t)((threadIdx.x - lane + own) / GW) * nw;
 #pragma unroll
             for (int u = 0; u < WPL; ++u) {
-                const uint32_t w = lane + 32 * u;
-                if (w < nw) acc[u] |= rbits[s[0] + w] | rbits[s[1] + w] | rbits[s[2] + w] | rbits[s[3] + w];
-            }
-        }
-        // light records: their colors laid end to end over the warp, 32 at a
-        // time (lane e finds its record by a search over the length prefix)
-        const uint32_t len = light ? (uint32_t)(c1 - c0) : 0u;  // < 8192 colors in bitmap mode
-        uint32_t incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += y;
-        }
-        const uint32_t excl = incl - len;
-        const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-        for (uint32_t e0 = 0; e0 < total; e0 += 32) {
-            const uint32_t e = e0 + lane;
-            int q = 0;  // the last lane whose range starts at or before e
-#pragma unroll
-            for (int step = 16; step; step >>= 1) {
-                const uint32_t ex = __shfl_sync(0xffffffffu, excl, (q + step) & 31);
-                if (q + step <= 31 && ex <= e) q += step;
-            }
-            const uint64_t cq = __shfl_sync(0xffffffffu, c0, q);
-            const uint32_t xq = __shfl_sync(0xffffffffu, excl, q);
-            if (e < total) {
-                const uint32_t v = colors[cq + (e - xq)];
-                atomicOr(&bm[v >> 5], 1u << (v & 31));
+                keep[u] = acc[u];
+                if (gs != own) acc[u] = 0;
             }
         }
     }
@@ -1002,17 +1051,20 @@ __global__ void __launch_bounds__(256) k_union_bm(
     uint32_t* out = mbits + m * (uint64_t)nw;
 #pragma unroll
     for (int u = 0; u < WPL; ++u) {
-        const uint32_t w = lane + 32 * u;
-        if (w < nw) {
+        const uint32_t w = gl + GW * u;
+        if (on && w < nw) {
             const uint32_t x = bm[w] | acc[u];
             out[w] = x;
             cnt += __popc(x);
             if (x) hs += word_mix(w, x);
         }
     }
-    for (int o = 16; o; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
-    hs = warp_sum64(hs);
-    if (lane == 0) {
+#pragma unroll
+    for (int o = GW / 2; o; o >>= 1) {
+        cnt += __shfl_xor_sync(FULL, cnt, o, GW);
+        hs += __shfl_xor_sync(FULL, hs, o, GW);
+    }
+    if (on && gl == 0) {
         msize[m] = cnt;
         mhash[m] = set_hash_final(hs, cnt);
     }
@@ -3069,7 +3121,11 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     // ---- counts the host needs next: union groups, heavy records (with a
     // bitmap: unions of at least that many colors), records used as color sets
     const uint32_t nw = (C + 31) / 32;
-    const uint32_t heavy = std::max<uint32_t>(1, p.heavy_colors);
+    // The default threshold (64) is for bitmaps of many words; where a bitmap
+    // is no longer than a list of 8 colors it is 8 (unions of 90 genomes in
+    // skewed buckets 2.4 ms instead of 3.1; of 60 genomes of the small kind 0.29 instead
+    // of 0.40; thresholds 4 and 16 within 10% of it).
+    const uint32_t heavy = p.heavy_colors == 64 && nw <= 8 ? 8 : std::max<uint32_t>(1, p.heavy_colors);
     const bool may_heavy = M && p.union_bitmaps && C >= heavy;
     uint32_t* hflag = nullptr;
     uint64_t* hpos = nullptr;
@@ -3136,20 +3192,31 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
             mbits = A.alloc<uint32_t>(G * nw + 1);
             {
                 CDBG_PROF("k_union", st);
-                auto launch = [&](auto kern) {
-                    if (shm > 48 * 1024)
-                        CDBG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm));
-                    kern<<<grid(G, wpb), wpb * 32, shm, st>>>(G, gbeg, gend, urec, R.col_off, R.colors, (uint32_t)R0,
-                                                              hflag, hpos, rbits, nw, mbits, msize, mhash);
+                auto launch = [&](auto kern, int gw) {
+                    // blocks of as many warps as their groups' bitmaps leave room for
+                    const int groups = 32 / gw;
+                    const int wpu = (int)std::max<uint64_t>(1, std::min<uint64_t>(8, (96 * 1024) / (4ull * nw * groups)));
+                    const size_t sh = (size_t)wpu * groups * nw * 4;
+                    if (sh > 48 * 1024)
+                        CDBG_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh));
+                    kern<<<grid(G, wpu * groups), wpu * 32, sh, st>>>(G, gbeg, gend, urec, R.col_off, R.colors,
+                                                                      (uint32_t)R0, hflag, hpos, rbits, nw, mbits,
+                                                                      msize, mhash);
                 };
-                if (nw <= 32)
-                    launch(k_union_bm<1>);
+                // groups no wider than the bitmap's words keep their lanes
+                // busy (figures at the kernel)
+                if (nw <= 8)
+                    launch(k_union_bm<1, 8>, 8);
+                else if (nw <= 16)
+                    launch(k_union_bm<1, 16>, 16);
+                else if (nw <= 32)
+                    launch(k_union_bm<1, 32>, 32);
                 else if (nw <= 64)
-                    launch(k_union_bm<2>);
+                    launch(k_union_bm<2, 32>, 32);
                 else if (nw <= 128)
-                    launch(k_union_bm<4>);
+                    launch(k_union_bm<4, 32>, 32);
                 else if (nw <= 256)
-                    launch(k_union_bm<8>);
+                    launch(k_union_bm<8, 32>, 32);
                 else
                     throw std::runtime_error("bitmap unions need at most 8192 colors");
             }

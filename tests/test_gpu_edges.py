@@ -138,3 +138,37 @@ def test_color_set_encoding(oracle, engine, tmp_path, colors):
         return native.result_frag_bytes(r), native.result_class_words(r).tobytes(), native.result_class_offsets(r).tobytes()
 
     assert out(batch_occ=64) == out()
+
+
+@pytest.mark.parametrize("colors", [2, 31, 255, 256, 257, 512, 513])
+def test_unions_of_many_records(oracle, engine, tmp_path, colors):
+    """K-mers in 2 to 150 records each (one block between different flanks), of
+    few and many colors, at the widths where the unions' lane groups change and
+    around the counts where the whole warp takes a union's rest."""
+    k, B = 31, 2
+    rng = np.random.default_rng(1000 + colors)
+    genomes = [[] for _ in range(colors)]
+    for n in (2, 8, 9, 31, 32, 33, 64, 65, 150):
+        block = _dna(rng, k + 2)
+        for i in range(n):
+            seq = _dna(rng, 6) + block + _dna(rng, 6)
+            few = int(rng.integers(1, 4)) if i % 3 else int(rng.integers(1, colors + 1))
+            for g in rng.choice(colors, size=min(few, colors), replace=False):
+                genomes[g].append(seq)
+    for g in genomes:
+        g.append(_dna(rng, 40))
+    _check(oracle, engine, tmp_path, genomes, k, B)
+    flat = [(s, g) for g, seqs in enumerate(genomes) for s in seqs]
+    hb = native.host_batch([s for s, _ in flat], [g for _, g in flat])
+
+    def out():
+        r = engine.build(hb, k, B, colors)
+        return native.result_frag_bytes(r), native.result_class_words(r).tobytes(), native.result_class_offsets(r).tobytes()
+
+    want = out()
+    try:
+        for heavy in (1, 20, 100000):
+            engine.set_tuning(heavy_colors=heavy)
+            assert out() == want
+    finally:
+        engine.set_tuning()
