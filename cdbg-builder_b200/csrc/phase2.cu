@@ -1070,14 +1070,37 @@ __global__ void __launch_bounds__(256, WPL == 1 ? 8 : 1) k_union_bm(
     }
 }
 
+// Four consecutive nodes' words from n0 (a multiple of 4; n_rec starts on 16
+// bytes); NONE32 past D.
+__device__ __forceinline__ void load_nodes4(uint32_t const* __restrict__ w, uint64_t n0, uint64_t D, uint32_t (&r)[4]) {
+    if (n0 + 4 <= D) {
+        const uint4 v = *reinterpret_cast<uint4 const*>(w + n0);
+        r[0] = v.x;
+        r[1] = v.y;
+        r[2] = v.z;
+        r[3] = v.w;
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[j] = n0 + j < D ? w[n0 + j] : NONE32;
+    }
+}
+
 // rec_first[r] = smallest node index whose color set is record r's list.
-__global__ void k_rec_first(uint64_t D, uint32_t const* __restrict__ n_rec, uint32_t R0,
-                            uint32_t* __restrict__ rec_first) {
-    uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= D) return;
-    const uint32_t r = n_rec[n];
-    if (r == NONE32 || (r & MULTI_TAG)) return;
-    atomicMin(&rec_first[r - R0], (uint32_t)n);
+// Neighbouring nodes mostly come from one record, so a thread takes four and
+// only the first of consecutive nodes with the same record sends a minimum
+// (200 genomes: 1.0 ms with one for every node, 0.26 so).
+__global__ void __launch_bounds__(256) k_rec_first(uint64_t D, uint32_t const* __restrict__ n_rec, uint32_t R0,
+                                                   uint32_t* __restrict__ rec_first) {
+    const uint64_t n0 = 4 * ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    uint32_t r[4];
+    load_nodes4(n_rec, n0, D, r);
+    uint32_t prev = __shfl_up_sync(0xffffffffu, r[3], 1);
+    if ((threadIdx.x & 31) == 0) prev = NONE32;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        if (r[j] != NONE32 && !(r[j] & MULTI_TAG) && r[j] != prev) atomicMin(&rec_first[r[j] - R0], (uint32_t)(n0 + j));
+        prev = r[j];
+    }
 }
 
 // Candidate class sources: used records then multi nodes.
@@ -1780,15 +1803,28 @@ __global__ void k_append_bits(uint64_t nnew, uint32_t const* __restrict__ rcand,
     }
 }
 
-__global__ void k_node_cid(uint64_t D, uint32_t const* __restrict__ n_rec, uint32_t R0,
-                           uint32_t const* __restrict__ rec_cand, uint64_t mbase, uint32_t const* __restrict__ mgrp,
-                           uint32_t const* __restrict__ cid, uint32_t* __restrict__ n_cid) {
-    uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= D) return;
-    const uint32_t r = n_rec[n];
-    uint32_t c = NONE32;
-    if (r != NONE32) c = (r & MULTI_TAG) ? cid[mbase + mgrp[r & ~MULTI_TAG]] : cid[rec_cand[r - R0]];
-    n_cid[n] = c;
+// Bound: latency of two dependent lookups, so four nodes per thread (200 genomes:
+// 1.35 ms with one, 0.53 so).
+__global__ void __launch_bounds__(256) k_node_cid(uint64_t D, uint32_t const* __restrict__ n_rec, uint32_t R0,
+                                                  uint32_t const* __restrict__ rec_cand, uint64_t mbase,
+                                                  uint32_t const* __restrict__ mgrp, uint32_t const* __restrict__ cid,
+                                                  uint32_t* __restrict__ n_cid) {
+    const uint64_t n0 = 4 * ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x);
+    uint32_t r[4], c[4];
+    load_nodes4(n_rec, n0, D, r);
+    uint64_t at[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+        at[j] = r[j] == NONE32 ? 0 : (r[j] & MULTI_TAG) ? mbase + mgrp[r[j] & ~MULTI_TAG] : rec_cand[r[j] - R0];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) c[j] = r[j] == NONE32 ? NONE32 : cid[at[j]];
+    if (n0 + 4 <= D) {
+        *reinterpret_cast<uint4*>(n_cid + n0) = make_uint4(c[0], c[1], c[2], c[3]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            if (n0 + j < D) n_cid[n0 + j] = c[j];
+    }
 }
 
 // ---- extension masks and clean links -------------------------------------
@@ -1822,6 +1858,21 @@ __device__ __forceinline__ uint32_t node_probe(slot_t<u128> const* t, uint32_t c
         p = p + 1 == cap ? 0u : p + 1;
     }
     return NONE32;
+}
+
+// The state (node << 1) | rc reached over a side from the node of canonical
+// k-mer `can` (reverse complement `rev`), whose only neighbour there, by base
+// nt, is `node`.
+template <typename K>
+__device__ __forceinline__ uint32_t right_state(K can, K rev, uint32_t nt, uint32_t k, uint32_t node) {
+    const K nf = ((can << 2) | (K)nt) & kmer_ops<K>::mask(k);
+    const K nr = (rev >> 2) | ((K)(3u - nt) << (2 * (k - 1)));
+    return (node << 1) | (nf <= nr ? 0u : 1u);
+}
+// backward from (can, rc = false) = forward from (can, rc = true), then flipped
+template <typename K>
+__device__ __forceinline__ uint32_t left_state(K can, K rev, uint32_t nt, uint32_t k, uint32_t node) {
+    return right_state<K>(rev, can, nt, k, node) ^ 1u;
 }
 
 // One bucket of k_ext_mask / k_ext_flat: blocks from `block` on share its
@@ -1883,16 +1934,17 @@ constexpr uint32_t EXT_FILTER_OCC = 1u << 18;
 constexpr uint32_t EXT_ITEM_OCC = 16384;  // least occurrences worth reading the bucket's keys again
 
 // Extension masks: which of a node's 8 possible neighbours are nodes of its
-// bucket, and per side the neighbour's node when it is the side's only one
-// (link[2n] left, link[2n + 1] right, NONE32 otherwise), so k_links needs no
-// probe.  A neighbour is first compared with the nodes before and after (nodes
+// bucket, and per side the state over to the neighbour when it is the side's
+// only one (link[2n] left, link[2n + 1] right, NONE32 otherwise), so k_links
+// needs neither k-mers nor probes.  A neighbour is first compared with the nodes before and after (nodes
 // are in insertion order: most neighbours along a record are there), then
 // looked up in a bitmap of the bucket's keys in shared memory, two bits of one
 // word per key, and only what passes is probed in the table, a warp's lookups packed over its
 // lanes.
 // Bound: instruction issue (70% of the ALU pipe), then the table's random sectors.
 // 200 genomes, k = 31: 13.4 -> 7.4 ms, 60 genomes, k = 63: 11.6 -> 5.9 ms against
-// all 8 neighbours probed; with one filter bit per key 8.9 / 6.1.
+// all 8 neighbours probed; with one filter bit per key 8.9 / 6.1.  (The states
+// for k_links add 0.4 and 0.6 ms.)
 template <typename K>
 __global__ void __launch_bounds__(ext_cfg<K>::THREADS, 2)
     k_ext_mask(ext_item const* __restrict__ items, uint32_t nitems, uint32_t t1, unsigned long long const* ne,
@@ -2004,8 +2056,8 @@ __global__ void __launch_bounds__(ext_cfg<K>::THREADS, 2)
             n_mask[n] = (uint8_t)out;
             auto node = [&](uint32_t v) { return (v & NODE_TAG) ? v & ~NODE_TAG : node_of(fw, v); };
             uint2 l;
-            l.x = __popc(out >> 4) == 1 ? node(side[1]) : NONE32;
-            l.y = __popc(out & 0xfu) == 1 ? node(side[0]) : NONE32;
+            l.x = __popc(out >> 4) == 1 ? left_state<K>(can, rev, __ffs(out >> 4) - 1, k, node(side[1])) : NONE32;
+            l.y = __popc(out & 0xfu) == 1 ? right_state<K>(can, rev, __ffs(out & 0xfu) - 1, k, node(side[0])) : NONE32;
             reinterpret_cast<uint2*>(link)[n] = l;
         }
     }
@@ -2050,8 +2102,8 @@ __global__ void __launch_bounds__(256, 8)
         }
         n_mask[n] = (uint8_t)out;
         uint2 l;
-        l.x = __popc(out >> 4) == 1 ? node_of(fw, left) : NONE32;
-        l.y = __popc(out & 0xfu) == 1 ? node_of(fw, right) : NONE32;
+        l.x = __popc(out >> 4) == 1 ? left_state<K>(can, rev, __ffs(out >> 4) - 1, k, node_of(fw, left)) : NONE32;
+        l.y = __popc(out & 0xfu) == 1 ? right_state<K>(can, rev, __ffs(out & 0xfu) - 1, k, node_of(fw, right)) : NONE32;
         reinterpret_cast<uint2*>(link)[n] = l;
     }
 }
@@ -2060,52 +2112,50 @@ __device__ __forceinline__ uint32_t fwd_nib(uint32_t m, bool rc) { return (rc ? 
 __device__ __forceinline__ uint32_t back_nib(uint32_t m, bool rc) { return (rc ? m : (m >> 4)) & 0xfu; }
 
 // link[2n] = L port, link[2n+1] = R port: (node << 1) | rc of the state
-// reached, NONE32 when the step is not clean.  On entry link holds the
-// sides' only neighbours as k_ext_mask found them.  Nodes with at most one
-// linked port, the path ends, are appended to `ends`.
-template <typename K>
+// reached, NONE32 when the step is not clean.  On entry link holds the sides'
+// only neighbours as k_ext_mask found them; a neighbour with more than one way
+// back, or the node itself (the reference's walk meets its own visited k-mer
+// there), ends the chain and leaves NONE32.  Nodes with at most one port are
+// the chain ends, listed in any order.
+// Bound: latency of the neighbours' masks, so four nodes per thread.  200
+// genomes: 2.9 ms with one and the states taken from the k-mers here, 0.90 so
+// (and 0.4 more in k_ext_mask, which has the k-mers at hand).
+constexpr int LINKS_PER = 4;
 __global__ void __launch_bounds__(256, 8) k_links(unsigned long long const* nb, unsigned long long const* ne,
-                                                  K const* __restrict__ n_key, uint8_t const* __restrict__ n_mask,
-                                                  uint32_t k, uint32_t* __restrict__ link, uint32_t* __restrict__ ends,
-                                                  unsigned long long* nends) {
-    const uint64_t n = *nb + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (*nb + (uint64_t)blockIdx.x * blockDim.x >= *ne) return;  // whole block
-    bool end = false;
-    if (n < *ne) {
-        typedef kmer_ops<K> ops;
-        const K can = n_key[n];
-        const uint32_t m = n_mask[n];
-        const uint2 only = reinterpret_cast<uint2 const*>(link)[n];
-        const K msk = ops::mask(k);
-        const uint32_t top = 2 * (k - 1);
-        const K rev = only.x != NONE32 || only.y != NONE32 ? ops::revcomp(can, k) : can;
-        uint32_t lr = NONE32, ll = NONE32;
-        // R: forward from (can, rc = false)
-        if (only.y != NONE32) {
-            const uint32_t nt = __ffs(fwd_nib(m, false)) - 1;
-            const K nf = ((can << 2) | (K)nt) & msk;
-            const K nr = (rev >> 2) | ((K)(3u - nt) << top);
-            const bool nrc = !(nf <= nr);
-            if (__popc(back_nib(n_mask[only.y], nrc)) == 1) lr = (only.y << 1) | (nrc ? 1u : 0u);
+                                                  uint8_t const* __restrict__ n_mask, uint32_t* __restrict__ link,
+                                                  uint32_t* __restrict__ ends, unsigned long long* nends) {
+    const uint64_t lo = *nb, hi = *ne;
+    for (uint64_t n0 = lo + (uint64_t)blockIdx.x * (256 * LINKS_PER); n0 < hi;
+         n0 += (uint64_t)gridDim.x * (256 * LINKS_PER)) {
+        uint2 l[LINKS_PER];
+        uint32_t ml[LINKS_PER], mr[LINKS_PER];
+#pragma unroll
+        for (int j = 0; j < LINKS_PER; ++j) {
+            const uint64_t n = n0 + 256 * j + threadIdx.x;
+            l[j] = n < hi ? reinterpret_cast<uint2 const*>(link)[n] : make_uint2(0, 0);
         }
-        // L: backward from (can, rc = false) = bstep(can, rc = true) then flip
-        if (only.x != NONE32) {
-            const uint32_t nt = __ffs(back_nib(m, false)) - 1;
-            const K nf = ((rev << 2) | (K)nt) & msk;
-            const K nr = (can >> 2) | ((K)(3u - nt) << top);
-            const bool srcc = !(nf <= nr);
-            const bool nrc = !srcc;
-            if (__popc(fwd_nib(n_mask[only.x], nrc)) == 1) ll = (only.x << 1) | (nrc ? 1u : 0u);
+#pragma unroll
+        for (int j = 0; j < LINKS_PER; ++j) {
+            const uint64_t n = n0 + 256 * j + threadIdx.x;
+            ml[j] = n < hi && l[j].x != NONE32 ? n_mask[l[j].x >> 1] : 0u;
+            mr[j] = n < hi && l[j].y != NONE32 ? n_mask[l[j].y >> 1] : 0u;
         }
-        // a port linked to the node itself ends the chain (the reference's walk
-        // meets its own visited k-mer there)
-        if (lr != NONE32 && (lr >> 1) == (uint32_t)n) lr = NONE32;
-        if (ll != NONE32 && (ll >> 1) == (uint32_t)n) ll = NONE32;
-        reinterpret_cast<uint2*>(link)[n] = make_uint2(ll, lr);
-        end = ll == NONE32 || lr == NONE32;
+        uint32_t end = 0;
+#pragma unroll
+        for (int j = 0; j < LINKS_PER; ++j) {
+            const uint64_t n = n0 + 256 * j + threadIdx.x;
+            if (n >= hi) continue;
+            uint2 t = l[j];
+            if (t.x != NONE32 && (__popc(fwd_nib(ml[j], t.x & 1u)) != 1 || (t.x >> 1) == (uint32_t)n)) t.x = NONE32;
+            if (t.y != NONE32 && (__popc(back_nib(mr[j], t.y & 1u)) != 1 || (t.y >> 1) == (uint32_t)n)) t.y = NONE32;
+            if (t.x != l[j].x || t.y != l[j].y) reinterpret_cast<uint2*>(link)[n] = t;
+            end |= (t.x == NONE32 || t.y == NONE32 ? 1u : 0u) << j;
+        }
+        unsigned long long at = block_reserve<256>(__popc(end), nends);
+#pragma unroll
+        for (int j = 0; j < LINKS_PER; ++j)
+            if ((end >> j) & 1u) ends[at++] = (uint32_t)(n0 + 256 * j + threadIdx.x);
     }
-    const unsigned long long at = block_reserve<256>(end ? 1u : 0u, nends);
-    if (end) ends[at] = (uint32_t)n;
 }
 
 // ---- chains ---------------------------------------------------------------
@@ -3064,7 +3114,8 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         CDBG_CHECK_LAUNCH();
         {
             CDBG_PROF("k_links", st);
-            k_links<K><<<grid(tn, 256), 256, 0, st>>>(nbase, nnext, n_key, n_mask, k, link, ends, nends);
+            k_links<<<(unsigned)std::min<uint64_t>(grid(tn, 256 * LINKS_PER), 148 * 16), 256, 0, st>>>(
+                nbase, nnext, n_mask, link, ends, nends);
         }
         CDBG_CHECK_LAUNCH();
     }
@@ -3150,7 +3201,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     CDBG_CUDA(cudaMemsetAsync(rec_first, 0xff, 4 * nrec, st));
     {
         CDBG_PROF("k_rec_first", st);
-        k_rec_first<<<grid(D, 256), 256, 0, st>>>(D, n_rec, (uint32_t)R0, rec_first);
+        k_rec_first<<<grid(D, 1024), 256, 0, st>>>(D, n_rec, (uint32_t)R0, rec_first);
     }
     CDBG_CHECK_LAUNCH();
     // candidates: used records, then union groups
@@ -3413,7 +3464,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     uint32_t* n_cid = A.alloc<uint32_t>(D);
     {
         CDBG_PROF("k_node_cid", st);
-        k_node_cid<<<grid(D, 256), 256, 0, st>>>(D, n_rec, (uint32_t)R0, rec_cand, nrc, mgrp, cid, n_cid);
+        k_node_cid<<<grid(D, 1024), 256, 0, st>>>(D, n_rec, (uint32_t)R0, rec_cand, nrc, mgrp, cid, n_cid);
     }
     CDBG_CHECK_LAUNCH();
     // ---- chains (extension masks and links were made with the tables)
