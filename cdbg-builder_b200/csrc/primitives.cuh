@@ -301,7 +301,7 @@ constexpr int RS_WARPS = RS_THREADS / 32;
 // digit).  Tiles take their indices in launch order from *tile_counter, so
 // every predecessor of a tile is running or done.  A tile ranks its keys
 // stably (warp w owns positions [w*ITEMS*32, (w+1)*ITEMS*32), processed in
-// rounds of 32 with warp match-any), publishes its per-digit counts in
+// rounds of 32 matched by ballots), publishes its per-digit counts in
 // status[tile][d], walks back over its predecessors' entries of the same digit
 // until an inclusive prefix (one thread per digit), publishes its own
 // inclusive prefix, stages the tile in shared memory in digit order and writes
@@ -311,10 +311,14 @@ constexpr int RS_WARPS = RS_THREADS / 32;
 // *err and publishes what it has, so no successor waits on it, and its
 // successors' positions can only come out smaller than the true ones, which
 // keeps every write inside the output.
-// Bound: latency of the ranking (matches and counter updates; 27% issue, 24 warps
-// per SM by registers).  All matches before the counter updates, values after the
-// keys through the same buffer: 9.8 -> 9.3 ms of a 200-genome build; 4 blocks per SM
-// (64 registers, spilling) 9.6, 5 blocks 10.8.
+// Bound: the ranking's instructions and their latency (52% issue, 59% of the ALU
+// pipe at 24 warps per SM).  A 200-genome build's passes: 9.8 ms; all matches
+// before the counter updates and values after the keys through the same buffer
+// 9.3; matches by ballots instead of match.any 9.05; no bounds checks between the
+// loads and the stores (positions past the end rank last), one lookup per key for
+// its place 8.5; digits kept instead of destinations, for 4 blocks per SM, 8.2.
+// 12 or 20 keys per thread 8.8 and 8.9, a look-back over four predecessors at a
+// time 0.7 slower.
 constexpr unsigned long long RS_AGG = 1ull << 62, RS_INC = 2ull << 62, RS_VALMASK = (1ull << 58) - 1;
 
 template <int BITS, int ITEMS, typename K, typename V>
@@ -323,15 +327,27 @@ struct rs_smem {
     static constexpr int TILE = RS_THREADS * ITEMS;
     static_assert(sizeof(V) <= sizeof(K), "keys and values share the buffer");
     K sk[TILE];                     // keys in digit order, then values
-    uint32_t wcnt[RS_WARPS][BINS];  // per-warp digit counts, then prefixes
-    uint32_t dstart[BINS];          // tile-local start of each digit
-    uint64_t gbase[BINS];           // global start of each digit for this tile
+    uint32_t wcnt[RS_WARPS][BINS];  // per-warp digit counts, then tile-local starts
+    uint32_t goff[BINS];            // a digit's output position less its tile-local one
     uint64_t sw[RS_WARPS + 1];
     uint32_t tile;
 };
 
+// The lanes of the warp with this lane's low BITS bits of `d`.
+template <int BITS>
+__device__ __forceinline__ uint32_t match_digit(uint32_t d) {
+    uint32_t peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b < BITS; ++b) {
+        const bool one = (d >> b) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, one);
+        peers &= one ? m : ~m;
+    }
+    return peers;
+}
+
 template <int BITS, int ITEMS, typename K, typename V>
-__global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restrict__ keys_in,
+__global__ void __launch_bounds__(RS_THREADS, 4) k_rs_onesweep(K const* __restrict__ keys_in,
                                                             V const* __restrict__ vals_in,
                                                             K* __restrict__ keys_out, V* __restrict__ vals_out,
                                                             uint64_t n, int shift, uint32_t* tile_counter,
@@ -354,24 +370,24 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
     const uint32_t p0 = (uint32_t)warp * (ITEMS * 32) + lane;  // round r: position p0 + 32 r
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) k[r] = p0 + 32u * r < tile_n ? keys_in[base + p0 + 32u * r] : ~K(0);
-    // the lanes of each round with the same digit (positions past the end have a
-    // digit of their own): all rounds' matches first, they do not depend on each
-    // other; then the warp's counters round by round
+    auto digit = [&](K key) { return (uint32_t)(key >> shift) & (BINS - 1); };
+    // the lanes of each round with the same digit: all rounds' matches first,
+    // they do not depend on each other; then the warp's counters round by round.
+    // Positions past the end hold the largest key: they rank after every pair,
+    // and their digit's count leaves them out.
 #pragma unroll
-    for (int r = 0; r < ITEMS; ++r)
-        rk[r] = __match_any_sync(0xffffffffu, p0 + 32u * r < tile_n ? (uint32_t)(k[r] >> shift) & (BINS - 1) : BINS);
+    for (int r = 0; r < ITEMS; ++r) rk[r] = match_digit<BITS>((uint32_t)(k[r] >> shift));
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
-        const bool ok = p0 + 32u * r < tile_n;
         const uint32_t peers = rk[r];
-        const int leader = __ffs(peers) - 1;
+        const uint32_t below = __popc(peers & lanemask_lt());
         uint32_t old = 0;
-        if (ok && lane == leader) {
-            const uint32_t d = (uint32_t)(k[r] >> shift) & (BINS - 1);
+        if (below == 0) {
+            const uint32_t d = digit(k[r]);
             old = sm.wcnt[warp][d];
             sm.wcnt[warp][d] = old + __popc(peers);
         }
-        rk[r] = __shfl_sync(0xffffffffu, old, leader) + __popc(peers & lanemask_lt());
+        rk[r] = __shfl_sync(0xffffffffu, old, __ffs(peers) - 1) + below;
     }
     __syncthreads();
     // per digit: exclusive prefix over warps and the tile's count
@@ -387,15 +403,18 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
                 sm.wcnt[w][d] = run;
                 run += c;
             }
+            if ((uint32_t)d == digit(~K(0))) run -= TILE - tile_n;
             const unsigned long long ep = (unsigned long long)epoch << 58;
             *(volatile unsigned long long*)&status[tile * BINS + d] = (tile == 0 ? RS_INC : RS_AGG) | ep | run;
         }
         cnt[j] = run;
     }
     // look-back, one thread per digit
+    uint32_t before[DPT];
 #pragma unroll
     for (int j = 0; j < DPT; ++j) {
         const int d = threadIdx.x + j * RS_THREADS;
+        before[j] = 0;
         if (d >= BINS) continue;
         uint64_t excl = 0;
         if (tile > 0) {
@@ -418,7 +437,7 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
             const unsigned long long ep = (unsigned long long)epoch << 58;
             *(volatile unsigned long long*)&status[tile * BINS + d] = RS_INC | ep | ((excl + cnt[j]) & RS_VALMASK);
         }
-        sm.gbase[d] = excl;
+        before[j] = (uint32_t)excl;
     }
     // digit starts (exclusive scans over digits): tile-local ones of the counts,
     // global ones of the pass's histogram
@@ -434,8 +453,10 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
             uint64_t tot;
             const uint64_t ex = carry + block_exclusive_scan<uint64_t, RS_THREADS>(both, sm.sw, tot);
             if (d < BINS) {
-                sm.dstart[d] = (uint32_t)(ex & 0xffffu);
-                sm.gbase[d] += ex >> 16;
+                const uint32_t ds = (uint32_t)(ex & 0xffffu);
+#pragma unroll
+                for (int w = 0; w < RS_WARPS; ++w) sm.wcnt[w][d] += ds;
+                sm.goff[d] = (uint32_t)(ex >> 16) + before[j] - ds;
             }
             carry += tot;
         }
@@ -444,11 +465,8 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
     // keys, then values, through the same buffer in digit order
 #pragma unroll
     for (int r = 0; r < ITEMS; ++r) {
-        if (p0 + 32u * r < tile_n) {
-            const uint32_t d = (uint32_t)(k[r] >> shift) & (BINS - 1);
-            rk[r] += sm.dstart[d] + sm.wcnt[warp][d];
-            sm.sk[rk[r]] = k[r];
-        }
+        rk[r] += sm.wcnt[warp][digit(k[r])];
+        sm.sk[rk[r]] = k[r];
     }
     V v[ITEMS];
 #pragma unroll
@@ -457,30 +475,28 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_onesweep(K const* __restri
         v[r] = p >= tile_n ? V(0) : vals_in ? vals_in[base + p] : (V)(base + p);
     }
     __syncthreads();
-    uint32_t dst[ITEMS];  // (n < 2^32)
+    // (the digits of the positions written are kept, packed, for the values)
+    constexpr int PACK = BITS <= 8 ? 4 : 2;
+    uint32_t dg[(ITEMS + PACK - 1) / PACK] = {};
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         const uint32_t p = threadIdx.x + i * RS_THREADS;
-        dst[i] = 0xffffffffu;
-        if (p < tile_n) {
-            const K key = sm.sk[p];
-            const uint32_t d = (uint32_t)((key >> shift) & (BINS - 1));
-            const uint64_t o = sm.gbase[d] + (p - sm.dstart[d]);
-            if (o < n) {
-                dst[i] = (uint32_t)o;
-                keys_out[o] = key;
-            }
-        }
+        const K key = sm.sk[p];
+        const uint32_t d = digit(key), o = sm.goff[d] + p;  // (n < 2^32)
+        dg[i / PACK] |= d << (32 / PACK * (i % PACK));
+        if (p < tile_n && o < n) keys_out[o] = key;
     }
     __syncthreads();
     V* sv = reinterpret_cast<V*>(sm.sk);
 #pragma unroll
-    for (int r = 0; r < ITEMS; ++r)
-        if (p0 + 32u * r < tile_n) sv[rk[r]] = v[r];
+    for (int r = 0; r < ITEMS; ++r) sv[rk[r]] = v[r];
     __syncthreads();
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i)
-        if (dst[i] != 0xffffffffu) vals_out[dst[i]] = sv[threadIdx.x + i * RS_THREADS];
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t p = threadIdx.x + i * RS_THREADS;
+        const uint32_t o = sm.goff[(dg[i / PACK] >> (32 / PACK * (i % PACK))) & (BINS - 1)] + p;
+        if (p < tile_n && o < n) vals_out[o] = sv[p];
+    }
 }
 
 // Up to RS_SMALL pairs: the whole LSD sort by one block in shared memory, in one

@@ -24,3 +24,29 @@ def test_sort_edges(engine, n, kind):
     order = np.argsort(k, kind="stable")
     assert np.array_equal(vals.cpu().numpy().view(np.uint32), order.astype(np.uint32))
     assert np.array_equal(keys.cpu().numpy().view(np.uint64), k[order])
+
+
+@pytest.mark.parametrize("bits", [8, 11])
+@pytest.mark.parametrize("n", [8193, 8223, 12287, 12289, 40_001])
+def test_largest_keys_in_partial_tiles(engine, n, bits):
+    """Keys equal to what fills a tile past the end, beside ones that share some
+    of its digits."""
+    import torch
+    rng = np.random.default_rng(n)
+    k = rng.integers(0, 1 << 63, n, dtype=np.uint64) * np.uint64(2)
+    k[rng.random(n) < 0.3] = np.uint64(2 ** 64 - 1)
+    top = rng.random(n) < 0.3
+    k[top] |= np.uint64(0xffffffff00000000)
+    k[-40:] = np.uint64(2 ** 64 - 1)
+    keys = torch.from_numpy(k.view(np.int64)).cuda()
+    vals = torch.arange(n, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    try:
+        engine.set_tuning(radix_bits=bits)
+        engine.sort_pairs_u64(keys.data_ptr(), vals.data_ptr(), n)
+    finally:
+        engine.set_tuning()
+    torch.cuda.synchronize()
+    order = np.argsort(k, kind="stable")
+    assert np.array_equal(vals.cpu().numpy().view(np.uint32), order.astype(np.uint32))
+    assert np.array_equal(keys.cpu().numpy().view(np.uint64), k[order])
