@@ -628,9 +628,9 @@ def _per_unit(w):
         # one (k-mer, record) read per occurrence + one table entry per distinct k-mer
         "k_insert": None,
         "k_number": ("occ", 4 + w + 8),           # occurrence slot + its k-mer's table slot
-        "k_ext_mask": ("distinct", w + 4 + 1),    # key + bucket read, mask written
-        "k_links": ("distinct", w + 1 + 8 + 8),   # key + mask + recorded neighbours read, two links written
-        "k_chain_paths": ("distinct", 8 + 1 + 1 + 4),  # links + flags + mask read, fragment element written
+        "k_ext_mask": ("distinct", w + 1 + 8),    # key read, mask and two neighbour states written
+        "k_links": ("distinct", 8 + 2),           # two states and their nodes' masks read
+        "k_chain_lead": ("distinct", 8 + 1 + 1 + 4),  # links + flags + mask read, fragment element written
         "k_frag_write": ("frag_bytes", 1),        # fragment records written
     }
 
@@ -673,15 +673,15 @@ def path_algorithmic_bytes(r, w, record_bytes):
 # DRAM bytes per algorithmic byte of kernels whose launch sites declare their
 # algorithmic bytes (one capture; the ratio carries to other sizes).
 TRAFFIC_RATIO = {
-    # first phase-1 pass at 40 genomes: 20,646,311 pairs, 495.5 MB algorithmic, 463.8 MB DRAM
-    "k_rs_onesweep": (463810560 / 495511464, "profiles/phase12_top_kernels_pangenome40.md"),
+    # a phase-1 pass at 40 genomes: 20,646,311 pairs, 495.5 MB algorithmic, 431.1 MB DRAM
+    "k_rs_onesweep": (431.1e6 / 495511464, "profiles/phase12_top_kernels_pangenome40.md"),
 }
 
 TRAFFIC_PER_UNIT = {
-    "k_minimizers": (1.691, "profiles/phase12_top_kernels_pangenome40.md"),   # per base
-    "k_insert": (61.321, "profiles/phase12_top_kernels_pangenome40.md"),      # per occurrence
-    "k_ext_mask": (55.196, "profiles/phase12_top_kernels_pangenome40.md"),    # per distinct k-mer
-    "k_frag_write": (3.688, "profiles/phase12_top_kernels_pangenome40.md"),   # per fragment byte
+    "k_minimizers": (1.667, "profiles/phase12_top_kernels_pangenome40.md"),   # per base
+    "k_insert": (60.95, "profiles/phase12_top_kernels_pangenome40.md"),      # per occurrence
+    "k_ext_mask": (50.64, "profiles/phase12_top_kernels_pangenome40.md"),    # per distinct k-mer
+    "k_frag_write": (4.006, "profiles/phase12_top_kernels_pangenome40.md"),   # per fragment byte
 }
 
 

@@ -1631,7 +1631,7 @@ struct noalloc_scratch {
 // cudaGetSymbolAddress (noalloc_scratch_ptr below).
 static __device__ __align__(256) noalloc_scratch g_noalloc_scratch;
 
-// Tiles per run like k_run_tiles, for caller-supplied runs: a run shorter
+// Tiles per run as in the run table, for caller-supplied runs: a run shorter
 // than k has no k-mer and would make the tile arithmetic wrap, so it counts
 // zero tiles and sets `err` (the host reads it before any tile kernel runs).
 __global__ void k_noalloc_run_tiles(uint32_t nruns, uint32_t const* __restrict__ len, uint32_t k, uint32_t tt,
