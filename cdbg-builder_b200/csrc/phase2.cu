@@ -1933,6 +1933,12 @@ constexpr uint32_t EXT_FILTER_WORDS = 102 * 1024 / 4;
 // 31: 63 K 28.8 / 50, 111 K 36 / 50, 189 K (about 2^18 occurrences) 54 / 50, 473 K
 // 133 / 50; k = 63: 77 K 52 / 92, 139 K 66 / 93, 348 K 148 / 94.
 constexpr uint32_t EXT_FILTER_OCC = 1u << 18;
+// 128-bit k-mers' buckets above that, up to 7 * 2^16 occurrences, take twice the
+// filter in one block of twice the threads per SM (the same warps): us per million
+// k-mers, wide / k_ext_flat, at 272 K occurrences per bucket 68 / 96, 340 K 77 / 96,
+// 504 K 109 / 100.  64-bit ones would lose half their warps: 480 K 52 / 51.
+template <typename K>
+constexpr uint32_t EXT_WIDE_OCC = sizeof(K) == 16 ? 7u << 16 : EXT_FILTER_OCC;
 constexpr uint32_t EXT_ITEM_OCC = 16384;  // least occurrences worth reading the bucket's keys again
 
 // Extension masks: which of a node's 8 possible neighbours are nodes of its
@@ -1947,13 +1953,14 @@ constexpr uint32_t EXT_ITEM_OCC = 16384;  // least occurrences worth reading the
 // 200 genomes, k = 31: 13.4 -> 7.4 ms, 60 genomes, k = 63: 11.6 -> 5.9 ms against
 // all 8 neighbours probed; with one filter bit per key 8.9 / 6.1.  (The states
 // for k_links add 0.4 and 0.6 ms.)
-template <typename K>
-__global__ void __launch_bounds__(ext_cfg<K>::THREADS, 2)
+template <typename K, bool WIDE>
+__global__ void __launch_bounds__(WIDE ? 1024 : ext_cfg<K>::THREADS, WIDE ? 1 : 2)
     k_ext_mask(ext_item const* __restrict__ items, uint32_t nitems, uint32_t t1, unsigned long long const* ne,
                tables<K> T, K const* __restrict__ n_key, uint32_t k, uint2 const* __restrict__ fw, uint8_t* __restrict__ n_mask,
                uint32_t* __restrict__ link) {
     typedef kmer_ops<K> ops;
-    constexpr uint32_t THREADS = ext_cfg<K>::THREADS;
+    constexpr uint32_t THREADS = WIDE ? 1024 : ext_cfg<K>::THREADS;
+    constexpr uint32_t WORDS = WIDE ? 2 * EXT_FILTER_WORDS : EXT_FILTER_WORDS;
     extern __shared__ __align__(16) uint32_t ext_filter[];
     __shared__ uint8_t queue[THREADS / 32][256];
     const ext_share it = find_share(items, nitems);
@@ -1961,7 +1968,7 @@ __global__ void __launch_bounds__(ext_cfg<K>::THREADS, 2)
     const uint32_t na = nodes_before(it.oa), nz = nodes_before(it.ob);
     if (na == nz) return;
     const uint32_t ba = nodes_before(it.ba), bb = nodes_before(it.bb);
-    const uint32_t words = min(EXT_FILTER_WORDS, ((bb - ba) / 2 + 4) & ~3u);  // 16 bits per key if they fit
+    const uint32_t words = min(WORDS, ((bb - ba) / 2 + 4) & ~3u);  // 16 bits per key if they fit
     for (uint32_t i = threadIdx.x; i < words / 4; i += THREADS)
         reinterpret_cast<uint4*>(ext_filter)[i] = make_uint4(0, 0, 0, 0);
     __syncthreads();
@@ -2392,7 +2399,8 @@ __device__ void simulate_chain_small(chain_ws const& W, uint64_t c0, uint32_t L,
 // not).  The leader then writes that fragment itself, on a second walk over the
 // links it just read; the other chains go to `heads` (node | rc << 31, L, c0 low,
 // c0 high) for k_chain_paths.
-// Bound: latency of the link reads, mostly cache hits (a chain's nodes are
+// Bound: issue (72%; half the lanes walk a chain the other end leads), then the
+// latency of the link reads, mostly cache hits (a chain's nodes are
 // neighbours in node order).  Finding the ends, the leaders, laying out every chain
 // and replaying the seed loop on it, the cycle check, and the run counts from the
 // fragments took 9.8 ms of a 200-genome build; this takes 4.1 and the ends 0.9 more
@@ -2992,21 +3000,24 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     uint64_t Tmax = 0;
     for (size_t g = 0; g < ng; ++g) Tmax = std::max<uint64_t>(Tmax, toff[gb[g + 1]] - toff[gb[g]]);
     uint32_t* occ_slot = A.alloc<uint32_t>(nocc);
-    // the buckets of k_ext_mask and of k_ext_flat, per group, with their blocks.
+    // the buckets of k_ext_mask, of its wide form and of k_ext_flat, per group, with
+    // their blocks.
     // A k_ext_mask bucket is split so that there are about four blocks per
     // resident one (the last ones leave few SMs idle), but into no smaller parts
     // than are worth reading the bucket's keys again for its filter.
     std::vector<ext_item> items;
-    std::vector<uint32_t> gitem(2 * ng + 1, 0), gblocks(2 * ng, 0);
+    std::vector<uint32_t> gitem(3 * ng + 1, 0), gblocks(3 * ng, 0);
     {
         const uint64_t share = std::max<uint64_t>(EXT_ITEM_OCC, nocc / (148 * 8));
-        for (size_t g = 0; g < 2 * ng; ++g) {  // group g / 2, flat when odd
+        for (size_t g = 0; g < 3 * ng; ++g) {  // group g / 3: filter, wide filter, flat
             uint32_t blocks = 0;
-            for (uint32_t b = gb[g / 2]; b < gb[g / 2 + 1]; ++b) {
+            for (uint32_t b = gb[g / 3]; b < gb[g / 3 + 1]; ++b) {
                 const uint64_t ba = bocc[b0 + b] - O0, n = bocc[b0 + b + 1] - O0 - ba;
-                if (n == 0 || (n > EXT_FILTER_OCC) != (g & 1)) continue;
-                items.push_back(ext_item{b - gb[g / 2], blocks, (uint32_t)ba, (uint32_t)(ba + n)});
-                blocks += (uint32_t)((g & 1) ? ceil_div(n, (uint64_t)ext_cfg<K>::FLAT_OCC) : n > share + share / 2 ? ceil_div(n, share) : 1);
+                if (n == 0 || (n > EXT_FILTER_OCC) + (n > EXT_WIDE_OCC<K>) != (int)(g % 3)) continue;
+                items.push_back(ext_item{b - gb[g / 3], blocks, (uint32_t)ba, (uint32_t)(ba + n)});
+                blocks += (uint32_t)(g % 3 == 2                ? ceil_div(n, (uint64_t)ext_cfg<K>::FLAT_OCC)
+                                     : n > share + share / 2 ? ceil_div(n, share)
+                                                             : 1);
             }
             items.push_back(ext_item{0, blocks, 0, 0});
             gblocks[g] = blocks;
@@ -3103,15 +3114,18 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         {
             CDBG_PROF("k_ext_mask", st);
             constexpr int smem = EXT_FILTER_WORDS * 4;
-            CDBG_CUDA(cudaFuncSetAttribute(k_ext_mask<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-            if (gblocks[2 * g])
-                k_ext_mask<K><<<gblocks[2 * g], ext_cfg<K>::THREADS, smem, st>>>(
-                    d_items + gitem[2 * g], gitem[2 * g + 1] - gitem[2 * g] - 1, (uint32_t)(t0 + tn), nnext, TG, n_key, k,
-                    fw, n_mask, link);
-            if (gblocks[2 * g + 1])
-                k_ext_flat<K><<<gblocks[2 * g + 1], 256, 0, st>>>(
-                    d_items + gitem[2 * g + 1], gitem[2 * g + 2] - gitem[2 * g + 1] - 1, (uint32_t)(t0 + tn), nnext, TG,
-                    n_key, k, fw, n_mask, link);
+            CDBG_CUDA(cudaFuncSetAttribute(k_ext_mask<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+            if constexpr (sizeof(K) == 16)
+                CDBG_CUDA(cudaFuncSetAttribute(k_ext_mask<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * smem));
+            const uint32_t t1 = (uint32_t)(t0 + tn);
+            auto launch = [&](auto kern, int c, int threads, int sm) {
+                const uint32_t a = gitem[3 * g + c], n = gitem[3 * g + c + 1] - a - 1;
+                if (gblocks[3 * g + c])
+                    kern<<<gblocks[3 * g + c], threads, sm, st>>>(d_items + a, n, t1, nnext, TG, n_key, k, fw, n_mask, link);
+            };
+            launch(k_ext_mask<K, false>, 0, ext_cfg<K>::THREADS, smem);
+            if constexpr (sizeof(K) == 16) launch(k_ext_mask<K, true>, 1, 1024, 2 * smem);
+            launch(k_ext_flat<K>, 2, 256, 0);
         }
         CDBG_CHECK_LAUNCH();
         {

@@ -172,3 +172,16 @@ def test_unions_of_many_records(oracle, engine, tmp_path, colors):
             assert out() == want
     finally:
         engine.set_tuning()
+
+
+@pytest.mark.parametrize("n", [440_000, 470_000, 600_000])
+def test_neighbour_lookups_of_large_buckets_of_long_kmers(oracle, engine, tmp_path, n):
+    """128-bit k-mers on both sides of the largest bucket that gets the wide
+    presence filter (7 * 2^16 occurrences)."""
+    k = 63
+    rng = np.random.default_rng(n)
+    a = _dna(rng, n)
+    b = bytearray(a[:6000])
+    for i in rng.integers(0, len(b), 90).tolist():
+        b[i] = b"ACGT"[int(rng.integers(0, 4))]
+    _check(oracle, engine, tmp_path, [[a, b"A" * (2 * k), b"ACGT" * k], [bytes(b), a[-2 * k:] + a[:2 * k]]], k, 1)
