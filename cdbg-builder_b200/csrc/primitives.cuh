@@ -387,6 +387,7 @@ __global__ void __launch_bounds__(RS_THREADS, 4) k_rs_onesweep(K const* __restri
             old = sm.wcnt[warp][d];
             sm.wcnt[warp][d] = old + __popc(peers);
         }
+        __syncwarp();  // the next round's reader of a counter may be another lane
         rk[r] = __shfl_sync(0xffffffffu, old, __ffs(peers) - 1) + below;
     }
     __syncthreads();
@@ -548,6 +549,7 @@ __global__ void __launch_bounds__(RSS_THREADS) k_rs_small(K* __restrict__ keys, 
                 old = sm.wcnt[warp][d];
                 sm.wcnt[warp][d] = (uint16_t)(old + __popc(peers));
             }
+            __syncwarp();  // (as in k_rs_onesweep)
             rk[r] = __shfl_sync(0xffffffffu, old, leader) + __popc(peers & lanemask_lt());
         }
         __syncthreads();
