@@ -195,59 +195,107 @@ __global__ void __launch_bounds__(EV_THREADS)
     ev_write(E, St, p0, s_excl + ex, cap, events);
 }
 
-// Pair events into runs.  size[i] = (1 << 32) + stream words of a run of at
-// least k bases, tiles[i] its minimizer tiles of tt (k-1)-mers, both 0 for a
-// shorter one; acc[0..1] += k-mers and bases of the runs kept.
-__global__ void k_runs_from_events(uint64_t const* __restrict__ ev, uint64_t nruns,
-                                   uint64_t const* __restrict__ seq_off, uint32_t num_seqs,
-                                   uint32_t const* __restrict__ seq_color, uint32_t k, uint32_t tt,
-                                   uint64_t* __restrict__ src, uint32_t* __restrict__ len,
-                                   uint32_t* __restrict__ color, uint64_t* __restrict__ size,
-                                   uint64_t* __restrict__ tiles, unsigned long long* __restrict__ acc, uint32_t* err) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
+// The run table from the events, in one pass: the runs of at least k bases in
+// order, with the exclusive sums of their stream words (soff, in bases, from word
+// `base` on) and of their minimizer tiles of tt (k-1)-mers (tstart), each closed
+// by its total.  Runs, words and tiles have a look-back of their own (tot[0..2],
+// status[0 .. 3 ntiles)): every sum keeps the full width, whatever the number of
+// runs.  acc[0..1] += k-mers and bases of the runs kept.
+// Bound: latency.  Sizes, two scans and a compaction took four launches where
+// this takes one and a memset, and 52 bytes of scratch a run.
+__global__ void __launch_bounds__(256)
+    k_run_table(uint64_t const* __restrict__ ev, uint64_t nruns, uint64_t const* __restrict__ seq_off,
+                uint32_t num_seqs, uint32_t const* __restrict__ seq_color, uint32_t k, uint32_t tt, uint64_t base,
+                uint64_t ntiles, uint32_t* tile_counter, unsigned long long* status,
+                unsigned long long* __restrict__ tot, uint64_t* __restrict__ osrc, uint32_t* __restrict__ olen,
+                uint32_t* __restrict__ ocolor, uint64_t* __restrict__ soff, uint64_t* __restrict__ tstart,
+                unsigned long long* __restrict__ acc, uint32_t* err) {
+    constexpr int R = prim::SEL_ROUNDS;
+    static_assert(MAX_RAW_RUNS * ((MAX_RUN_BASES + 31) / 32) < prim::LB_VAL, "sums of runs, words and tiles fit");
+    __shared__ prim::ordered_select keep;
+    __shared__ uint64_t part[2][R * 8], before[2];  // words, tiles: of (round, warp), then before it; before the tile
+    const uint64_t tile = prim::select_tile(keep, tile_counter);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t src[R], at_w[R], at_t[R];  // (words and tiles before this run in its (round, warp))
+    uint32_t len[R], sel = 0;
     unsigned long long kmers = 0, bases = 0;
-    if (i < nruns) {
-        const uint64_t a = ev[2 * i] >> 1, b = ev[2 * i + 1] >> 1;
-        const uint64_t l = b - a;
-        if (l >= 0xffffffffull) set_error(err, ERR_FIELD_OVERFLOW);
-        src[i] = a;
-        len[i] = (uint32_t)l;
-        const uint32_t s = upper_bound_u64(seq_off, num_seqs + 1, a) - 1;
-        color[i] = seq_color[s];
-        const bool keep = l >= k;
-        size[i] = keep ? (1ull << 32) + (l + 31) / 32 : 0;
-        tiles[i] = keep ? (l - k + 2 + tt - 1) / tt : 0;
-        kmers = keep ? l - k + 1 : 0;
-        bases = keep ? l : 0;
+    bool over = false;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint64_t i = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        uint64_t l = 0;
+        src[r] = 0;
+        if (i < nruns) {
+            src[r] = ev[2 * i] >> 1;
+            l = (ev[2 * i + 1] >> 1) - src[r];
+        }
+        over |= l > MAX_RUN_BASES;
+        len[r] = (uint32_t)l;
+        const run_sums a = run_adds(l, k, tt);
+        if (a.runs) {
+            sel |= 1u << r;
+            kmers += l - k + 1;
+            bases += l;
+        }
+        const uint64_t w = prim::warp_inclusive_scan(a.words), t = prim::warp_inclusive_scan(a.tiles);
+        at_w[r] = w - a.words;
+        at_t[r] = t - a.tiles;
+        if (lane == 31) {
+            part[0][r * 8 + warp] = w;
+            part[1][r * 8 + warp] = t;
+        }
     }
+    if (over) set_error(err, ERR_FIELD_OVERFLOW);
 #pragma unroll
     for (int o = 16; o; o >>= 1) {
         kmers += __shfl_down_sync(0xffffffffu, kmers, o);
         bases += __shfl_down_sync(0xffffffffu, bases, o);
     }
-    if ((threadIdx.x & 31) == 0 && bases) {
+    if (lane == 0 && bases) {
         atomicAdd(acc, kmers);
         atomicAdd(acc + 1, bases);
     }
-}
-
-// Runs of at least k bases in order: pos[i] and tpos[i] are the exclusive sums of
-// size and tiles (their totals at nruns).  Stream offsets start at word `base`.
-__global__ void k_runs_compact(uint64_t nruns, uint64_t const* __restrict__ size, uint64_t const* __restrict__ pos,
-                               uint64_t const* __restrict__ tpos, uint64_t const* __restrict__ src,
-                               uint32_t const* __restrict__ len, uint32_t const* __restrict__ color, uint64_t base,
-                               uint64_t* __restrict__ osrc, uint32_t* __restrict__ olen,
-                               uint32_t* __restrict__ ocolor, uint64_t* __restrict__ soff,
-                               uint64_t* __restrict__ tstart) {
-    const uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i > nruns || (i < nruns && !size[i])) return;
-    const uint64_t o = pos[i] >> 32;
-    soff[o] = ((pos[i] & 0xffffffffu) + base) * 32;
-    tstart[o] = tpos[i];
-    if (i == nruns) return;
-    osrc[o] = src[i];
-    olen[o] = len[i];
-    ocolor[o] = color[i];
+    prim::select_put(keep, sel);
+    __syncthreads();
+    if (warp == 0) {
+        prim::select_scan(keep, tile, ntiles, status, tot, err);
+    } else if (warp < 3) {
+        uint64_t* p = part[warp - 1];
+        const uint64_t c0 = p[2 * lane], c1 = p[2 * lane + 1];
+        const uint64_t x = prim::warp_inclusive_scan(c0 + c1);
+        const uint64_t sum = __shfl_sync(0xffffffffu, x, 31);
+        p[2 * lane] = x - c0 - c1;
+        p[2 * lane + 1] = x - c1;
+        uint64_t excl = 0;
+        const bool ok = prim::lookback_exclusive(status + warp * ntiles, tile, sum, excl);
+        if (lane == 0) {
+            if (!ok) set_error(err, ERR_CHAIN_LIMIT);
+            before[warp - 1] = excl;
+            if (tile == ntiles - 1) tot[warp] = excl + sum;
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        const uint64_t i = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
+        const bool on = (sel >> r) & 1u;
+        if (i >= nruns || (!on && i != nruns - 1)) continue;
+        const uint64_t o = prim::select_pos(keep, r);
+        const uint64_t w = base + before[0] + part[0][r * 8 + warp] + at_w[r];
+        const uint64_t t = before[1] + part[1][r * 8 + warp] + at_t[r];
+        if (on) {
+            osrc[o] = src[r];
+            olen[o] = len[r];
+            ocolor[o] = seq_color[upper_bound_u64(seq_off, num_seqs + 1, src[r]) - 1];
+            soff[o] = w * 32;
+            tstart[o] = t;
+        }
+        if (i == nruns - 1) {  // the totals close the sums
+            const run_sums a = run_adds(len[r], k, tt);
+            soff[o + a.runs] = (w + a.words) * 32;
+            tstart[o + a.runs] = t + a.tiles;
+        }
+    }
 }
 
 // 2-bit codes of four ACGT bytes (either case), byte i at bits 2i: bits 1-2 of
@@ -1147,7 +1195,7 @@ void build_runs(seq_input const& in, uint32_t k, dev_arena& A, cudaStream_t st, 
     // zeroed together: sequence-start bitmap (bit p: a sequence starts at p, or p
     // = nbytes), look-back status, tile counter, and the counts the host reads
     const uint64_t nsw = ((in.nbytes >> 5) + 2 + 1) / 2;  // in 8-byte words
-    enum { C_EVENTS, C_RUNS, C_TILES, C_KMERS, C_BASES, C_ERR, C_COUNTER, NCOUNTS };
+    enum { C_EVENTS, C_KMERS, C_BASES, C_ERR, C_COUNTER, NCOUNTS };
     unsigned long long* zero = A.alloc<unsigned long long>(NCOUNTS + tiles + nsw);
     unsigned long long* counts = zero;
     unsigned long long* status = zero + NCOUNTS;
@@ -1192,38 +1240,32 @@ void build_runs(seq_input const& in, uint32_t k, dev_arena& A, cudaStream_t st, 
     }
     const uint64_t nraw = nev / 2;
     if (nraw == 0) return;
-    if (nraw >= 0xffffffffull) throw std::runtime_error("too many ACGT runs");
-    uint64_t* src = A.alloc<uint64_t>(nraw);
-    uint32_t* len = A.alloc<uint32_t>(nraw);
-    uint32_t* color = A.alloc<uint32_t>(nraw);
-    uint64_t* size = A.alloc<uint64_t>(nraw);
-    uint64_t* ntl = A.alloc<uint64_t>(nraw);
-    uint64_t* pos = A.alloc<uint64_t>(nraw + 1);
-    uint64_t* tpos = A.alloc<uint64_t>(nraw + 1);
+    if (nraw > MAX_RAW_RUNS) throw std::runtime_error("too many ACGT runs");
     rt.src = A.alloc<uint64_t>(nraw);
     rt.len = A.alloc<uint32_t>(nraw);
     rt.color = A.alloc<uint32_t>(nraw);
     rt.soff = A.alloc<uint64_t>(nraw + 1);
     rt.tstart = A.alloc<uint64_t>(nraw + 1);
-    k_runs_from_events<<<grid(nraw, 256), 256, 0, st>>>(ev, nraw, in.seq_off, in.num_seqs, in.seq_color, k, rt.tile,
-                                                         src, len, color, size, ntl, counts + C_KMERS, err);
+    const uint64_t rtiles = ceil_div(nraw, (uint64_t)prim::SEL_TILE);
+    unsigned long long* rws = A.alloc<unsigned long long>(3 * rtiles + 4);  // three look-backs, totals, tile counter
+    unsigned long long* tot = rws + 3 * rtiles;
+    CDBG_CUDA(cudaMemsetAsync(rws, 0, 8 * (3 * rtiles + 4), st));
+    k_run_table<<<(unsigned)rtiles, 256, 0, st>>>(ev, nraw, in.seq_off, in.num_seqs, in.seq_color, k, rt.tile, word_base,
+                                                  rtiles, reinterpret_cast<uint32_t*>(tot + 3), rws, tot, rt.src, rt.len,
+                                                  rt.color, rt.soff, rt.tstart, counts + C_KMERS, err);
     CDBG_CHECK_LAUNCH();
-    // (runs in the high 32 bits, stream words in the low: an input on the device
-    // has fewer than 2^32 words of 32 bases)
-    prim::exclusive_scan<uint64_t, uint64_t>(size, pos, nraw, A, st, pos + nraw);
-    prim::exclusive_scan<uint64_t, uint64_t>(ntl, tpos, nraw, A, st, tpos + nraw);
-    k_runs_compact<<<grid(nraw + 1, 256), 256, 0, st>>>(nraw, size, pos, tpos, src, len, color, word_base, rt.src,
-                                                         rt.len, rt.color, rt.soff, rt.tstart);
-    CDBG_CHECK_LAUNCH();
-    uint64_t total = 0;
-    mail_reader(st).add(h, counts, sizeof(h)).add(&total, pos + nraw).add(&rt.ntiles, tpos + nraw).wait();
-    if ((uint32_t)h[C_ERR]) throw std::runtime_error("run length exceeds 2^32 bases");
-    const uint64_t nruns = total >> 32;
+    uint64_t sums[3];
+    mail_reader(st).add(h, counts, sizeof(h)).add(sums, tot, sizeof(sums)).wait();
+    const uint32_t re = (uint32_t)h[C_ERR];
+    if (re == ERR_CHAIN_LIMIT) throw std::runtime_error("run table: look-back wait limit reached");
+    if (re) throw std::runtime_error("run length exceeds 2^32 bases");
+    const uint64_t nruns = sums[0];
     if (nruns == 0) return;
     rt.n = (uint32_t)nruns;
+    rt.ntiles = sums[2];
     rt.n_kmers = h[C_KMERS];
     rt.n_bases = h[C_BASES];
-    const uint64_t nwd = total & 0xffffffffu;
+    const uint64_t nwd = sums[1];
     uint64_t* dst;
     if (words_out) {
         // this batch's runs go at word `word_base` of a shared stream

@@ -17,6 +17,7 @@
 
 #include "arena.cuh"
 #include "common.cuh"
+#include "run_sums.hpp"
 
 namespace cdbg {
 namespace prim {
@@ -70,7 +71,9 @@ __device__ __forceinline__ U block_exclusive_scan(U v, U* smem_warp, U& total) {
 // predecessor took its index earlier, so it is running or done; every wait is
 // still bounded, and on a timeout the tile publishes what it has (so its
 // successors never wait on it) and returns false.
-constexpr unsigned long long LB_AGG = 1ull << 62, LB_INC = 2ull << 62, LB_VAL = (1ull << 62) - 1;
+constexpr unsigned long long LB_AGG = 1ull << LOOKBACK_SUM_BITS, LB_INC = 2ull << LOOKBACK_SUM_BITS,
+                             LB_VAL = (1ull << LOOKBACK_SUM_BITS) - 1;
+static_assert(LOOKBACK_SUM_BITS == 62, "two flag bits above the sum");
 __device__ __forceinline__ bool lookback_exclusive(unsigned long long* status, uint64_t tile, uint64_t tot,
                                                    uint64_t& excl) {
     const int lane = threadIdx.x & 31;
