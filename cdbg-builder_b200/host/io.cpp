@@ -15,6 +15,7 @@
 
 #include <fcntl.h>
 #include <sys/mman.h>
+#include <sys/stat.h>
 #include <sys/vfs.h>
 #include <unistd.h>
 
@@ -322,11 +323,22 @@ bool read_files_into(std::vector<std::string> const& files, size_t first, size_t
 }
 
 range_file::range_file(std::string const& path) : m_path(path) {
-    m_fd = ::open(path.c_str(), O_RDWR | O_CREAT | O_TRUNC, 0644);
+    // A mapping needs a readable descriptor; a file that may only be written, and
+    // what is no regular file (a FIFO would not wait for its reader), are opened
+    // for writing.
+    struct stat sb;
+    const bool regular = ::stat(path.c_str(), &sb) != 0 || S_ISREG(sb.st_mode);
+    constexpr int kNew = O_CREAT | O_TRUNC;
+    if (regular) {
+        m_fd = ::open(path.c_str(), O_RDWR | kNew, 0666);
+        m_map = m_fd >= 0;
+    }
+    if (m_fd < 0 && (!regular || errno == EACCES)) m_fd = ::open(path.c_str(), O_WRONLY | kNew, 0666);
     if (m_fd < 0) throw std::runtime_error("cannot open output file: " + path + ": " + std::strerror(errno));
+    m_regular = ::fstat(m_fd, &sb) == 0 && S_ISREG(sb.st_mode);
     struct statfs fs;
     constexpr long kTmpfsMagic = 0x01021994;
-    m_tmpfs = ::fstatfs(m_fd, &fs) == 0 && (long)fs.f_type == kTmpfsMagic;
+    m_map = m_map && m_regular && ::fstatfs(m_fd, &fs) == 0 && (long)fs.f_type == kTmpfsMagic;
 }
 
 range_file::~range_file() {
@@ -335,6 +347,17 @@ range_file::~range_file() {
 
 void range_file::write(uint8_t const* data, uint64_t off, uint64_t n, uint32_t threads) {
     if (n == 0) return;
+    if (!m_regular) {
+        if (off != m_at) throw std::runtime_error("output is no regular file and takes bytes in order only: " + m_path);
+        for (uint64_t x = 0; x < n;) {
+            const ssize_t w = ::write(m_fd, data + x, (size_t)std::min<uint64_t>(n - x, 1ull << 30));
+            if (w < 0 && errno == EINTR) continue;
+            if (w <= 0) throw std::runtime_error("short write to " + m_path);
+            x += (uint64_t)w;
+        }
+        m_at += n;
+        return;
+    }
     const uint64_t piece = std::max<uint64_t>(4ull << 20, (n + threads - 1) / std::max<uint32_t>(threads, 1));
     const size_t np = (size_t)((n + piece - 1) / piece);
     std::atomic<bool> bad{false};
@@ -342,7 +365,7 @@ void range_file::write(uint8_t const* data, uint64_t off, uint64_t n, uint32_t t
     const uint64_t pg = (uint64_t)::sysconf(_SC_PAGESIZE);
     const uint64_t a = off & ~(pg - 1);
     // (one piece gains nothing from a mapping)
-    if (m_tmpfs && np > 1 && ::fallocate(m_fd, 0, (off_t)off, (off_t)n) == 0)
+    if (m_map && np > 1 && ::fallocate(m_fd, 0, (off_t)off, (off_t)n) == 0)
         map = ::mmap(nullptr, (size_t)(off + n - a), PROT_WRITE, MAP_SHARED, m_fd, (off_t)a);
     if (map != MAP_FAILED) {
         uint8_t* dst = (uint8_t*)map + (off - a);
@@ -372,7 +395,7 @@ void range_file::write(uint8_t const* data, uint64_t off, uint64_t n, uint32_t t
 void range_file::finish(uint64_t total) {
     const int fd = m_fd;
     m_fd = -1;
-    const bool ok = ::ftruncate(fd, (off_t)total) == 0;
+    const bool ok = !m_regular || ::ftruncate(fd, (off_t)total) == 0;
     if (::close(fd) != 0 || !ok) throw std::runtime_error("cannot finish output file " + m_path);
 }
 

@@ -67,7 +67,9 @@ void write_file_parallel(std::string const& path, uint8_t const* data, uint64_t 
 // threads: on a RAM-backed file system (tmpfs), where writes to one file take
 // its lock one call at a time, through shared mappings of the range filled in
 // parallel (the space reserved first, so a full file system is an error, not
-// a fault); elsewhere by positional writes of disjoint pieces.
+// a fault); elsewhere by positional writes of disjoint pieces.  What is no
+// regular file (a FIFO, a device) takes its ranges in ascending order, each by
+// the calling thread.
 class range_file {
 public:
     explicit range_file(std::string const& path);
@@ -75,13 +77,15 @@ public:
     range_file(range_file const&) = delete;
     range_file& operator=(range_file const&) = delete;
     void write(uint8_t const* data, uint64_t off, uint64_t n, uint32_t threads);
-    // sets the file's size and closes it
+    // sets a regular file's size and closes it
     void finish(uint64_t total);
 
 private:
     std::string m_path;
     int m_fd = -1;
-    bool m_tmpfs = false;
+    bool m_regular = false;  // positions and a size of its own
+    bool m_map = false;      // on tmpfs, written through mappings
+    uint64_t m_at = 0;       // bytes written, of what is no regular file
 };
 
 // ---- bucket files (bucket_io.hpp:19-40) ------------------------------------
