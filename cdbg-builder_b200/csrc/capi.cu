@@ -702,14 +702,16 @@ int cdbg_gpu_phase1(cdbg_engine* e, const cdbg_phase1_args* a, cdbg_phase1_stats
     }
 }
 
+extern "C++" {  // (templates have no C linkage)
 namespace {
-// Device bytes src[0, n) to a file at `off` through the pinned buffer `buf`: the
-// copy goes in pieces and each is written by the host threads while the next ones
-// still copy.
-void write_from_device(cdbg_engine* e, uint8_t const* src, uint8_t* buf, uint64_t n, cdbg::io::range_file& f,
-                       uint64_t off, uint32_t threads) {
-    if (n == 0) return;
-    const uint64_t piece = std::max<uint64_t>(16ull << 20, cdbg::ceil_div(n, 8));
+constexpr uint64_t WRITE_PIECE = 16ull << 20;
+
+// Device bytes src[0, n) through the pinned buffer `buf` of `slots` pieces:
+// `put(data, at, bytes)` takes each piece while the next ones still copy, and its
+// slot then takes the piece `slots` further on.
+template <typename Put>
+void write_from_device(cdbg_engine* e, uint8_t const* src, uint8_t* buf, uint64_t piece, size_t slots, uint64_t n,
+                       Put const& put) {
     const size_t np = (size_t)cdbg::ceil_div(n, piece);
     struct events {
         std::vector<cudaEvent_t> v;
@@ -717,26 +719,74 @@ void write_from_device(cdbg_engine* e, uint8_t const* src, uint8_t* buf, uint64_
             for (auto x : v) cudaEventDestroy(x);
         }
     } ev;
-    for (size_t i = 0; i < np; ++i) {
-        const uint64_t x = i * piece, c = std::min(piece, n - x);
-        CDBG_CUDA(cudaMemcpyAsync(buf + x, src + x, c, cudaMemcpyDeviceToHost, e->st));
-        cudaEvent_t v;
-        CDBG_CUDA(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
-        ev.v.push_back(v);
-        CDBG_CUDA(cudaEventRecord(v, e->st));
-    }
+    auto len = [&](size_t i) { return std::min(piece, n - i * piece); };
+    auto copy = [&](size_t i) {
+        CDBG_CUDA(cudaMemcpyAsync(buf + i % slots * piece, src + i * piece, len(i), cudaMemcpyDeviceToHost, e->st));
+        CDBG_CUDA(cudaEventRecord(ev.v[i % slots], e->st));
+    };
     try {
+        for (size_t i = 0; i < np && i < slots; ++i) {
+            cudaEvent_t v;
+            CDBG_CUDA(cudaEventCreateWithFlags(&v, cudaEventDisableTiming));
+            ev.v.push_back(v);
+            copy(i);
+        }
         for (size_t i = 0; i < np; ++i) {
-            const uint64_t x = i * piece, c = std::min(piece, n - x);
-            CDBG_CUDA(cudaEventSynchronize(ev.v[i]));
-            f.write(buf + x, off + x, c, threads);
+            CDBG_CUDA(cudaEventSynchronize(ev.v[i % slots]));
+            put(buf + i % slots * piece, i * piece, len(i));
+            if (i + slots < np) copy(i + slots);
         }
     } catch (...) {
         cudaStreamSynchronize(e->st);  // the buffer's copies are done before the caller goes on
         throw;
     }
 }
+
+// Device bytes through a few pinned pieces (in h_frag), or pageable ones where no
+// more memory can be page-locked.  Pieces of up to 64 MB, as each pays for its
+// writing threads and its reserved pages: phase 2 of 60 genomes, with 807 MB of
+// fragments, takes 263 ms (261 through one buffer of all of them), with pieces of 32
+// MB 18 ms more; an engine's first call 0.62 s (1.2 s).
+constexpr size_t SPILL_SLOTS = 3;
+template <typename Put>
+void spill_from_device(cdbg_engine* e, uint8_t const* src, uint64_t n, Put const& put) {
+    if (n == 0) return;
+    const uint64_t piece = std::min(n, std::clamp(cdbg::ceil_div(n, (uint64_t)8), WRITE_PIECE, 4 * WRITE_PIECE));
+    size_t slots = std::min<size_t>(SPILL_SLOTS, (size_t)cdbg::ceil_div(n, piece));
+    std::vector<uint8_t> pageable;
+    uint8_t* buf;
+    try {
+        buf = (uint8_t*)e->h_frag.ensure(slots * piece);
+    } catch (std::exception const&) {
+        cudaGetLastError();
+        pageable.resize(piece);
+        buf = pageable.data();
+        slots = 1;
+    }
+    write_from_device(e, src, buf, piece, slots, n, put);
+}
+
+// The fragments of drop-in phase 2 on their way to their file, batch by batch,
+// from the batch's scratch: neither the device nor the host holds more of them.
+struct frag_spill {
+    cdbg_engine* e;
+    cdbg::io::range_file& file;
+    uint32_t threads;
+    uint64_t written = 0;
+    double seconds = 0;
+
+    static void take(void* ctx, uint8_t const* src, uint64_t n) {
+        auto& w = *static_cast<frag_spill*>(ctx);
+        const auto t = std::chrono::steady_clock::now();
+        spill_from_device(w.e, src, n, [&](uint8_t const* data, uint64_t at, uint64_t c) {
+            w.file.write(data, w.written + at, c, w.threads);
+        });
+        w.written += n;
+        w.seconds += std::chrono::duration<double>(std::chrono::steady_clock::now() - t).count();
+    }
+};
 }  // namespace
+}
 
 int cdbg_gpu_phase2(cdbg_engine* e, const cdbg_phase2_args* a, cdbg_phase2_stats* s) {
     if (!e) {
@@ -805,11 +855,7 @@ int cdbg_gpu_phase2(cdbg_engine* e, const cdbg_phase2_args* a, cdbg_phase2_stats
         } catch (std::exception const&) {
             throw std::runtime_error(std::string("cannot open frag spill: ") + a->frag_path);
         }
-        uint64_t written = 0;
-        // the fragments stay on the device until their range is done and come
-        // through pinned memory (an engine with a memory cap keeps them in scratch,
-        // which its cap covers, and returns them batch by batch)
-        const bool resident = e->mem_limit == 0;
+        frag_spill spill{e, *ff, T};
         cdbg_phase2_stats st{};
         cdbg::phase2_result res;
         double dev_s = 0;
@@ -840,19 +886,15 @@ int cdbg_gpu_phase2(cdbg_engine* e, const cdbg_phase2_args* a, cdbg_phase2_stats
             pp.table_slots_q = e->tune.table_slots_q;
             pp.union_bitmaps = e->tune.union_lists == 0;
             pp.group_bytes = e->tune.table_group_mb ? (uint64_t)e->tune.table_group_mb << 20 : ~0ull;
-            pp.to_host = !resident;
+            pp.take_frag = &frag_spill::take;
+            pp.take_frag_ctx = &spill;
             pp.keep_dict = i > 0;
-            pp.copy_dict = i + 1 == nr;
+            pp.copy_dict = i + 1 == nr && a->on_class;
             res.state = &e->p2;
+            const double ws = spill.seconds;
             cdbg::run_phase2(rs, pp, e->A, e->st, e->d_err, res);
-            dev_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - td).count();
-            // this range's fragments, then (only then) its bucket files go
-            if (resident)
-                write_from_device(e, res.d_frag, (uint8_t*)e->h_frag.ensure(res.frag_nbytes + 8), res.frag_nbytes, *ff,
-                                  written, T);
-            else
-                ff->write(res.frag.data(), written, res.frag.size(), T);
-            written += res.frag_nbytes;
+            dev_s += std::chrono::duration<double>(std::chrono::steady_clock::now() - td).count() - (spill.seconds - ws);
+            // (this range's fragments are in the file)
             if (a->delete_consumed) cdbg::io::delete_bucket_files(dir, rb[i], rb[i + 1]);
             st.n_records += rs.n;
             st.n_kmers += res.n_occ;
@@ -860,22 +902,7 @@ int cdbg_gpu_phase2(cdbg_engine* e, const cdbg_phase2_args* a, cdbg_phase2_stats
             st.n_fragments += res.n_fragments;
             st.total_seq_bytes += res.total_seq_bytes;
         }
-        ff->finish(written);
-        const uint64_t nwords = (res.nbits + 63) / 64;
-        uint64_t const* words = res.words.data();
-        if (resident && (a->color_sets_path || a->on_class)) {
-            uint64_t* hw = (uint64_t*)e->h_words.ensure(8 * nwords + 8);
-            if (nwords) CDBG_CUDA(cudaMemcpyAsync(hw, res.d_words, 8 * nwords, cudaMemcpyDeviceToHost, e->st));
-            if (a->on_class) {
-                res.offsets.resize(res.n_classes);
-                if (res.n_classes)
-                    CDBG_CUDA(cudaMemcpyAsync(res.offsets.data(), res.d_offsets, 8 * res.n_classes,
-                                              cudaMemcpyDeviceToHost, e->st));
-            }
-            CDBG_CUDA(cudaStreamSynchronize(e->st));
-            if (a->on_class) res.words.assign(hw, hw + nwords);
-            words = hw;
-        }
+        ff->finish(spill.written);
         if (a->color_sets_path) {
             // the Elias-Fano finalize of the class offsets runs on the device,
             // over the offsets the dictionary holds there
@@ -889,8 +916,11 @@ int cdbg_gpu_phase2(cdbg_engine* e, const cdbg_phase2_args* a, cdbg_phase2_stats
                 CDBG_CUDA(cudaMemcpyAsync(lh.data() + ef.low_words, ef.high, 8 * ef.high_words,
                                           cudaMemcpyDeviceToHost, e->st));
             CDBG_CUDA(cudaStreamSynchronize(e->st));
-            cdbg::io::write_color_sets_ef(a->color_sets_path, a->num_colors, words, res.nbits, ef.n,
-                                          ef.l, lh.data(), lh.data() + ef.low_words, ef.high_bits);
+            auto words = [&](cdbg::io::byte_sink const& put) {
+                spill_from_device(e, (uint8_t const*)e->p2.words.p, 8 * ((res.nbits + 63) / 64),
+                                  [&](uint8_t const* data, uint64_t, uint64_t c) { put(data, c); });
+            };
+            cdbg::io::write_color_sets_ef(a->color_sets_path, a->num_colors, words, res.nbits, ef.n, ef.l, lh.data(), lh.data() + ef.low_words, ef.high_bits);
         }
         if (a->on_class) {
             std::vector<uint32_t> cls;
@@ -1357,7 +1387,6 @@ int build_core(cdbg_engine* e, const cdbg_build_params* p, phase1_fn const& phas
         pp.table_slots_q = e->tune.table_slots_q;
         pp.union_bitmaps = e->tune.union_lists == 0;
         pp.group_bytes = e->tune.table_group_mb ? (uint64_t)e->tune.table_group_mb << 20 : ~0ull;
-        pp.to_host = false;  // outputs accumulate in HBM
         pp.keep_frag_offsets = e->keep_frag_offsets && !p->outputs_to_host;
         e->frag_sink.streamed = 0;
         if (!p->outputs_to_host && e->frag_sink.fn && e->h_frag.p && e->h_frag.cap) {
@@ -1681,7 +1710,8 @@ int cdbg_gpu_build_files(cdbg_engine* e, const cdbg_build_files_args* a, cdbg_bu
             if (a->color_sets_path)
                 cs_writer = std::thread([&] {
                     try {
-                        cdbg::io::write_color_sets_ef(a->color_sets_path, a->num_files, hw, r->class_bits,
+                        auto words = [&](cdbg::io::byte_sink const& put) { put((uint8_t const*)hw, 8 * nwords); };
+                        cdbg::io::write_color_sets_ef(a->color_sets_path, a->num_files, words, r->class_bits,
                                                       ef.n, ef.l, hl, hl + ef.low_words, ef.high_bits);
                     } catch (...) {
                         cs_err = std::current_exception();
@@ -1694,8 +1724,14 @@ int cdbg_gpu_build_files(cdbg_engine* e, const cdbg_build_files_args* a, cdbg_bu
                     if (have < streamed)
                         CDBG_CUDA(cudaMemcpyAsync(hf + have, r->frag_bytes + have, streamed - have,
                                                   cudaMemcpyDeviceToHost, e->st));
-                    write_from_device(e, r->frag_bytes + streamed, hf + streamed, r->frag_nbytes - streamed, fw->file,
-                                      streamed, th);
+                    // (every piece stays where it lands: the result points there)
+                    const uint64_t rest = r->frag_nbytes - streamed;
+                    const uint64_t piece = std::max(WRITE_PIECE, cdbg::ceil_div(rest, (uint64_t)8));
+                    write_from_device(e, r->frag_bytes + streamed, hf + streamed, piece,
+                                      (size_t)cdbg::ceil_div(rest, piece), rest,
+                                      [&](uint8_t const* data, uint64_t at, uint64_t c) {
+                                          fw->file.write(data, streamed + at, c, th);
+                                      });
                     CDBG_CUDA(cudaStreamSynchronize(e->st));
                     fw->file.finish(r->frag_nbytes);
                 } catch (...) {

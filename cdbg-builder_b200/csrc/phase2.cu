@@ -3540,7 +3540,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     dict.total_integers += new_ints;
     const uint64_t frag_old = dfrag.n;
     uint8_t* fb = nullptr;  // the fragments: scratch on their way to the host, or where the output stays
-    if (p.to_host) {
+    if (p.take_frag) {
         fb = A.alloc<uint8_t>(fbytes + 16);
     } else {
         if (p.copy_st && dfrag.n + fbytes + 16 > dfrag.cap) {
@@ -3555,17 +3555,16 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         CDBG_PROF("k_frag_write", st);
         k_frag_write<K><<<grid(nfr, FW_THREADS), FW_THREADS, 0, st>>>(nfr, seed_of, W.seed_start, W.seed_len,
                                                                        W.seed_info, W.fe, n_cid, n_key, k, foff,
-                                                                       p.to_host ? 0 : frag_old, fb);
+                                                                       p.take_frag ? 0 : frag_old, fb);
     }
     CDBG_CHECK_LAUNCH();
     out.n_fragments += nfr;
     out.total_seq_bytes += seq_total;
     out.n_occ += nocc;
     out.n_distinct += D;
-    if (p.to_host) {
-        const size_t o = out.frag.size();
-        out.frag.resize(o + fbytes);
-        CDBG_CUDA(cudaMemcpyAsync(out.frag.data() + o, fb, fbytes, cudaMemcpyDeviceToHost, st));
+    if (p.take_frag) {
+        check_device_error_word(d_err, st, "phase-2 batch");
+        if (fbytes) p.take_frag(p.take_frag_ctx, fb, fbytes);
     } else {
         const uint64_t old_n = frag_old;
         dfrag.n += fbytes;
@@ -3584,7 +3583,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
             if (p.on_frag) p.on_frag(p.on_frag_ctx, old_n, fbytes);
         }
     }
-    if (!p.to_host && p.copy_st) {
+    if (!p.take_frag && p.copy_st) {
         // completed class words (all but the one later classes still fill) and
         // class offsets go to the host while the next batch runs
         const uint64_t wdone = dict.nbits / 64;
@@ -3605,9 +3604,8 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
             out.offs_host_copied = dict.n;
         }
     }
-    if (p.to_host) CDBG_CUDA(cudaStreamSynchronize(st));
     out.frag_nbytes += fbytes;
-    check_device_error_word(d_err, st, "phase-2 batch");
+    if (!p.take_frag) check_device_error_word(d_err, st, "phase-2 batch");
     A.release(mark);
 }
 
@@ -3693,7 +3691,7 @@ void run_all(record_set const& rs, phase2_params const& p, dev_arena& A, cudaStr
     out.nbits = dict.nbits;
     out.total_integers = dict.total_integers;
     const uint64_t nwords = (dict.nbits + 63) / 64;
-    if (p.to_host && p.copy_dict) {
+    if (p.take_frag && p.copy_dict) {
         out.words.resize(nwords);
         out.offsets.resize(dict.n);
         if (nwords)
@@ -3703,7 +3701,7 @@ void run_all(record_set const& rs, phase2_params const& p, dev_arena& A, cudaStr
     }
     CDBG_CUDA(cudaStreamSynchronize(st));
     A.release(mark);
-    if (!p.to_host) {
+    if (!p.take_frag) {
         // outputs stay in the persistent state
         out.d_frag = S.frag.p;
         out.d_words = S.words.p;
@@ -3720,7 +3718,7 @@ void run_phase2(record_set const& rs, phase2_params const& p, dev_arena& A, cuda
         out = phase2_result();
         out.state = S;
     }
-    if (!p.to_host && !out.state) throw std::runtime_error("device-resident phase-2 outputs need persistent storage");
+    if (!p.take_frag && !out.state) throw std::runtime_error("device-resident phase-2 outputs need persistent storage");
     if (p.k < 2 || p.k > 63) throw std::runtime_error("k must be in [2, 63]");
     if (p.num_colors == 0) throw std::runtime_error("num_colors must be > 0");
     if (rs.n >= (1ull << 31)) throw std::runtime_error("more than 2^31 bucket records in one build");

@@ -54,18 +54,17 @@ struct phase2_result {
     uint64_t offs_host_copied = 0;  // leading class offsets queued to params.offs_host
     // frag_unitigs.bin bytes (unitig_spill.hpp:642-665 record layout), in
     // bucket order and, per bucket, in seed order.
-    std::vector<uint8_t> frag;          // host copy (when to_host)
-    uint8_t* d_frag = nullptr;          // device copy (when !to_host), arena memory
+    uint8_t* d_frag = nullptr;          // device copy (without take_frag), persistent state
     uint64_t frag_nbytes = 0;
     // color classes in global cid order
     std::vector<uint64_t> words;        // encoded .color_sets bit vector
     std::vector<uint64_t> offsets;      // bit offset of each class
-    uint64_t* d_words = nullptr;        // device copies (when !to_host)
+    uint64_t* d_words = nullptr;        // device copies (without take_frag)
     uint64_t* d_offsets = nullptr;
     uint64_t nbits = 0;
     uint64_t n_classes = 0;
     uint64_t total_integers = 0;
-    // persistent storage to use (required when !to_host: the device
+    // persistent storage to use (required without take_frag: the device
     // outputs live in it); null = temporary storage for this call
     phase2_state* state = nullptr;
     // counters
@@ -78,7 +77,11 @@ struct phase2_params {
     uint32_t k = 31;
     uint32_t num_colors = 0;
     uint64_t batch_occ = 0;   // k-mer occurrences per batch (0 = auto)
-    bool to_host = true;      // copy outputs to host vectors
+    // Given: each batch's fragment bytes are handed over on the device as the
+    // batch finishes (scratch, the caller's until it returns) and the dictionary
+    // goes to host vectors.  Null: all outputs stay on the device.
+    void (*take_frag)(void* ctx, uint8_t const* d_bytes, uint64_t n) = nullptr;
+    void* take_frag_ctx = nullptr;
     // multi-record color unions as C-bit bitmaps (else as lists; bitmaps cost
     // C/8 bytes per such k-mer, so very large color counts use lists)
     bool union_bitmaps = true;
@@ -91,7 +94,7 @@ struct phase2_params {
     // (bucket ranges of one build processed call by call) instead of
     // starting it empty
     bool keep_dict = false;
-    // with to_host: copy the dictionary's words and offsets to the host
+    // with take_frag: copy the dictionary's words and offsets to the host
     // (the last call of a range-by-range build only)
     bool copy_dict = true;
     // table bytes of one bucket group: the buckets of a batch are processed in

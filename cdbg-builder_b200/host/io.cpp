@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstring>
 #include <filesystem>
+#include <memory>
 #include <stdexcept>
 #include <thread>
 
@@ -812,24 +813,26 @@ void read_bucket_range(std::string const& dir, uint32_t B, uint32_t b_lo, uint32
     });
 }
 
-void write_color_sets_ef(std::string const& path, uint32_t C, uint64_t const* words, uint64_t nbits,
+void write_color_sets_ef(std::string const& path, uint32_t C,
+                         std::function<void(byte_sink const&)> const& words, uint64_t nbits,
                          uint64_t nvalues, uint64_t l, uint64_t const* low, uint64_t const* high,
                          uint64_t high_bits) {
     std::FILE* f = std::fopen(path.c_str(), "wb");
     if (!f) throw std::runtime_error("cannot open color-set output: " + path);
+    std::unique_ptr<std::FILE, int (*)(std::FILE*)> guard(f, &std::fclose);  // (`words` may throw)
     const uint32_t st = (uint32_t)(0.25 * C), dt = (uint32_t)(0.75 * C);
     const uint64_t nwords = (nbits + 63) / 64;
     bool ok = std::fwrite(&C, 4, 1, f) == 1 && std::fwrite(&st, 4, 1, f) == 1 &&
               std::fwrite(&dt, 4, 1, f) == 1 && std::fwrite(&nbits, 8, 1, f) == 1 &&
               std::fwrite(&nwords, 8, 1, f) == 1;
-    if (ok && nwords) ok = std::fwrite(words, 8, nwords, f) == nwords;
+    if (ok && nwords) words([&](uint8_t const* p, uint64_t n) { ok = ok && std::fwrite(p, 1, n, f) == n; });
     const uint64_t U = nbits, lbits = nvalues * l, lw = (lbits + 63) / 64, hw = (high_bits + 63) / 64;
     ok = ok && std::fwrite(&U, 8, 1, f) == 1 && std::fwrite(&nvalues, 8, 1, f) == 1 && std::fwrite(&l, 8, 1, f) == 1;
     ok = ok && std::fwrite(&lbits, 8, 1, f) == 1 && std::fwrite(&lw, 8, 1, f) == 1;
     if (ok && lw) ok = std::fwrite(low, 8, lw, f) == lw;
     ok = ok && std::fwrite(&high_bits, 8, 1, f) == 1 && std::fwrite(&hw, 8, 1, f) == 1;
     if (ok && hw) ok = std::fwrite(high, 8, hw, f) == hw;
-    std::fclose(f);
+    guard.reset();
     if (!ok) throw std::runtime_error("short write to " + path);
 }
 

@@ -184,8 +184,11 @@ void delete_bucket_files(std::string const& dir, uint32_t b_lo, uint32_t b_hi);
 // layout of this project's `bits` stand-in (u64 universe, u64 n, u64 l, then
 // the low and high bit vectors each as [u64 num_bits][u64 num_words][words]),
 // the encoding made on the device (ef_encode): l low bits per value, the low
-// and high bit vectors as words.
-void write_color_sets_ef(std::string const& path, uint32_t C, uint64_t const* words, uint64_t nbits,
+// and high bit vectors as words.  `words` hands the (nbits + 63) / 64 words to the
+// sink it is given, piece by piece, in order.
+using byte_sink = std::function<void(uint8_t const*, uint64_t)>;
+void write_color_sets_ef(std::string const& path, uint32_t C,
+                         std::function<void(byte_sink const&)> const& words, uint64_t nbits,
                          uint64_t nvalues, uint64_t l, uint64_t const* low, uint64_t const* high,
                          uint64_t high_bits);
 
