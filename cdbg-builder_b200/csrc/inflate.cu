@@ -19,9 +19,10 @@
 // boundaries after a few symbols, and threads whose guess was wrong decode
 // again from their predecessor's exit until all agree (3 rounds for gzip -1
 // genomes, 5 for gzip -6).  The threads then write their symbols at their
-// output positions, one literal or match distance per output byte, and every
-// byte of the window finds its literal by following distances, independent of
-// the others; a source before the window is read from HBM.  A literal/length
+// output positions, one literal or distance per output byte -- every byte of a
+// match that overlaps itself points before the match -- and every byte of the
+// window finds its literal by following distances, independent of the others; a
+// source before the window is read from HBM.  A literal/length
 // lookup of 11 bits yields up to three literals at once, or a whole match
 // length; a distance lookup of 11 bits a whole distance (gzip -1 writes DNA as
 // matches of about 4 bytes at a few hundred bytes' distance, whose codes and
@@ -31,6 +32,12 @@
 // Bound: the latency of one thread's dependent lookups, about 60 symbols per
 // window of 14 KB.  130 gzip -1 files of 2.4 MB (one per SM): 14.2 ms; symbol by
 // symbol with one warp per file 228 ms, windows of one warp per file 58.6 ms.
+// Runs (N gaps on one line, short tandem repeats) would follow one match's bytes
+// one by one.  Eight files of 2.4 MB, ms at gzip -1 / -6, 1 MB of each one run 12.3 /
+// 11.0, all of it 10.1 / 12.0; with the bytes of a match pointing a distance back
+// each 36.6 / 480 and 61 / 1263; without the stop at the window's last byte (guesses
+// between equal symbols stay out of step) 36.3 / 17.6 and 61 / 32; with a match
+// written by its thread alone 12.7 / 17.5 and 11.4 / 32.
 
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -57,6 +64,10 @@ static_assert(IF_THREADS * WIN_LANE_BITS + 63 + 48 + 96 <= 64 * WIN_STAGE, "a wi
 // takes at least 2 bits), so every window makes progress.
 constexpr uint32_t WIN_OUT = 24576;
 static_assert((WIN_LANE_BITS / 2 + 1) * 258 <= WIN_OUT, "one thread's symbols fit the window");
+// Matches of at least this many bytes are written by the whole CTA: in a long run
+// one thread has all of a window's bytes.
+constexpr uint32_t LONG_MATCH = 192;
+static_assert(WIN_OUT / LONG_MATCH * 2 <= IF_THREADS, "a window's long matches fit cta_state::exits");
 
 // RFC 1951 3.2.5: length codes 257..285 and distance codes 0..29
 __constant__ uint16_t c_len_base[29] = {3,  4,  5,  6,  7,  8,  9,  10, 11,  13,  15,  17,  19,  23, 27,
@@ -115,11 +126,12 @@ struct __align__(16) cta_state {
     code_aux la, da, ca;
     uint32_t hist[2][16];
     uint8_t lens[320];
-    uint32_t exits[IF_THREADS];  // bit after each thread's symbols
+    uint32_t exits[IF_THREADS];  // bit after each thread's symbols; then the long matches (start | length << 16, distance)
     uint32_t warp_sum[IF_WARPS];
     uint32_t stop[2];
     uint32_t total, end;  // of a window: bytes, bit after the last symbol
     uint32_t ok[2];
+    uint32_t nlong;       // long matches of the window
     block_ctl ctl;
 };
 
@@ -440,7 +452,23 @@ __device__ __forceinline__ uint32_t lane_symbols(cta_state& w, uint32_t& pos, ui
                 st = LANE_BAD;
                 break;
             }
-            for (uint32_t i = 0; i < L; ++i) w.ent[o + n + i] = (uint16_t)(d - 1);
+            if (L >= LONG_MATCH) {  // by the CTA, after the window's symbols
+                const uint32_t at = 2 * atomicAdd(&w.nlong, 1u);
+                w.exits[at] = (o + n) | (L << 16);
+                w.exits[at + 1] = d;
+            } else if (d >= L) {
+                for (uint32_t i = 0; i < L; ++i) w.ent[o + n + i] = (uint16_t)(d - 1);
+            } else {
+                // an overlapping match: all its bytes point before it, byte i at its
+                // period's distance (d < 258 here, so at most 514)
+                for (uint32_t i = 0, c = 0, q = d; i < L; ++i) {
+                    w.ent[o + n + i] = (uint16_t)(q - 1);
+                    if (++c == d) {
+                        c = 0;
+                        q += d;
+                    }
+                }
+            }
         }
         n += L;
     }
@@ -466,6 +494,7 @@ __device__ __forceinline__ uint32_t window_decode(cta_state& w, uint8_t const* i
         w.stage[i] = a < end + 16 ? __ldg(reinterpret_cast<unsigned long long const*>(in + a)) : 0ull;
     }
     if (t < 2) w.stop[t] = IF_THREADS - 1;
+    if (t == 2) w.total = w.nlong = 0;
     __syncthreads();
     // bits of the stream left from a0 on (a window past them is refused)
     const uint64_t left = end > a0 ? (end - a0) * 8 : 0;
@@ -477,11 +506,19 @@ __device__ __forceinline__ uint32_t window_decode(cta_state& w, uint8_t const* i
     // Thread 0 started right; each round every thread up to the first that
     // stopped takes its predecessor's exit as its start, so after r rounds
     // threads 0..r are right whatever the guesses were: the loop ends by itself
-    // within IF_THREADS rounds.
+    // within IF_THREADS rounds.  Thread r adds its bytes when it is known to be
+    // right, and the first one past the window's bytes stops the rest: in long
+    // runs a few threads fill the window, while guesses between symbols that
+    // repeat do not fall into step.
     uint32_t stop = 0;
+    bool full = false;
     for (int r = 0; r <= IF_THREADS; ++r) {
         w.exits[t] = pos;
-        if (st != LANE_MORE) atomicMin(&w.stop[r & 1], t);
+        if ((int)t == r) {
+            w.total += n;
+            full = w.total > WIN_OUT;
+        }
+        if (st != LANE_MORE || full) atomicMin(&w.stop[r & 1], t);
         __syncthreads();
         stop = w.stop[r & 1];
         const uint32_t want = t ? w.exits[t - 1] : start;
@@ -517,6 +554,15 @@ __device__ __forceinline__ uint32_t window_decode(cta_state& w, uint8_t const* i
         wst = lane_symbols<true>(w, p, limit, bits_end, m, incl - n, op - member0);
     }
     if (__syncthreads_or(wst == LANE_BAD)) return WIN_BAD;  // a distance before the member's first byte
+    const uint32_t nlong = w.nlong;
+    if (nlong) {
+        for (uint32_t m = warp; m < nlong; m += IF_WARPS) {
+            const uint32_t x = w.exits[2 * m], d = w.exits[2 * m + 1], L = x >> 16;
+            uint16_t* en = w.ent + (x & 0xffffu);
+            for (uint32_t i = lane; i < L; i += 32) en[i] = (uint16_t)((d >= L ? d : i - i % d + d) - 1);
+        }
+        __syncthreads();
+    }
     const uint32_t total = w.total;
     const bool done = w.ok[0] != 0;
     if ((uint64_t)op + total > cap) return WIN_OVERFLOW;

@@ -1,0 +1,83 @@
+"""GPU: the device inflater on long and short-period runs -- whole windows of
+overlapping matches, one thread's worth of symbols filling a window (24,576
+bytes), matches on both sides of the length from which the whole CTA writes them
+(192), distances of 1 to 32,768 -- against zlib's bytes, and in a time that does
+not grow with the square of a run."""
+import time
+import zlib
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _dna(rng, n):
+    return rng.choice(np.frombuffer(b"ACGT", dtype=np.uint8), size=n).tobytes()
+
+
+def _gz(data, level, strategy=zlib.Z_DEFAULT_STRATEGY):
+    c = zlib.compressobj(level, zlib.DEFLATED, 31, 9, strategy)
+    return c.compress(data) + c.flush()
+
+
+def _check(engine, datas, strategy=zlib.Z_DEFAULT_STRATEGY):
+    streams, want = [], []
+    for d in datas:
+        for level in (1, 6, 9):
+            streams.append(_gz(d, level, strategy))
+            want.append(d)
+    for i, ((st, out), w) in enumerate(zip(engine.gunzip(streams, [len(w) for w in want]), want)):
+        assert st == 0 and out == w, i
+
+
+@pytest.mark.parametrize("period", [1, 2, 3, 5, 16, 64, 129, 191, 192, 193, 256, 257, 258, 259, 700])
+def test_periods(engine, period):
+    rng = np.random.default_rng(period)
+    u = _dna(rng, period)
+    out = []
+    for n in (3, 190, 191, 192, 193, 194, 257, 258, 259, 260, 517, 5000, 24_575, 24_576, 24_577, 70_000):
+        run = (u * (n // period + 2))[: period + n]
+        out.append(_dna(rng, 50) + run + _dna(rng, 33))
+    _check(engine, out + [b"".join(out)])
+    _check(engine, [b"".join(out)], zlib.Z_FIXED)
+
+
+@pytest.mark.parametrize("distance", [1, 2, 257, 258, 259, 24_575, 24_576, 24_577, 32_505, 32_506])
+def test_distances(engine, distance):
+    """Copies from before the window and inside it, at and around the window's
+    bytes and the largest distance."""
+    rng = np.random.default_rng(distance)
+    base = _dna(rng, distance)
+    _check(engine, [base + base[:n] + b"".join(_dna(rng, int(g)) + base[int(o):int(o) + 300] for g, o in
+                                               zip(rng.integers(0, 40, 60), rng.integers(0, max(1, distance - 300), 60)))
+                    for n in (200, 258, 600)])
+
+
+def test_rle_and_huffman_only_streams(engine):
+    rng = np.random.default_rng(9)
+    d = b"".join(bytes([int(b)]) * int(n) for b, n in zip(rng.integers(0, 6, 300), rng.integers(1, 900, 300)))
+    _check(engine, [d], zlib.Z_RLE)
+    _check(engine, [d], zlib.Z_HUFFMAN_ONLY)
+
+
+def test_runs_take_no_longer_than_sequence(engine):
+    """Eight files of 2.4 MB: with the bytes of a run followed one match's byte at
+    a time the run files take 30 to 90 times as long as the others; they take at
+    most three times as long (1.3 measured)."""
+    rng = np.random.default_rng(4)
+    n = 2_400_000
+    dna = _dna(rng, n)
+    kinds = {"dna": dna, "half": dna[: n // 2] + b"N" * (n // 2), "all": b"N" * n}
+    best = {}
+    for name, d in kinds.items():
+        z = [_gz(d, 6)] * 8
+        engine.gunzip(z, [n] * 8)
+        t = []
+        for _ in range(3):
+            t0 = time.perf_counter()
+            got = engine.gunzip(z, [n] * 8)
+            t.append(time.perf_counter() - t0)
+        assert all(st == 0 and out == d for st, out in got)
+        best[name] = min(t)
+    assert best["half"] < 3 * best["dna"] and best["all"] < 3 * best["dna"], best
