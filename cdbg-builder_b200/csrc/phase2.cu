@@ -47,6 +47,7 @@
 #include <vector>
 
 #include "device_kmer.cuh"
+#include "ext_plan.hpp"
 #include "phase2.cuh"
 #include "primitives.cuh"
 
@@ -1917,29 +1918,13 @@ __device__ __forceinline__ uint32_t strand_hash(u128 v) {
     const uint32_t a = (uint32_t)v, b = (uint32_t)((uint64_t)v >> 32);
     return ((a ^ (a >> 15)) * 0x85ebca6bu ^ b) * 0x9e3779b1u;
 }
-// Threads of a block: two blocks per SM, with 32 registers a thread (64 for
-// 128-bit k-mers).  FLAT_OCC: occurrences of a k_ext_flat block, for four or two
-// rounds of its threads: fewer leave threads idle, more put the tables of too many
-// buckets in flight for L2 (k = 31: 57 / 54 / 50 / 56 / 88 us per million k-mers
-// at 256 / 512 / 1024 / 2048 / 4096; k = 63: 98 / 93 / 98 / 120 / 156).
+// Threads of a filter block: two blocks per SM, with 32 registers a thread (64 for
+// 128-bit k-mers).
 template <typename K>
 struct ext_cfg {
     static constexpr int THREADS = sizeof(K) == 8 ? 1024 : 512;
-    static constexpr uint32_t FLAT_OCC = sizeof(K) == 8 ? 1024 : 512;
 };
 constexpr uint32_t EXT_FILTER_WORDS = 102 * 1024 / 4;
-// Buckets of more occurrences go to k_ext_flat: their keys fill the filter.  us
-// per million k-mers by distinct k-mers per bucket, k_ext_mask / k_ext_flat: k =
-// 31: 63 K 28.8 / 50, 111 K 36 / 50, 189 K (about 2^18 occurrences) 54 / 50, 473 K
-// 133 / 50; k = 63: 77 K 52 / 92, 139 K 66 / 93, 348 K 148 / 94.
-constexpr uint32_t EXT_FILTER_OCC = 1u << 18;
-// 128-bit k-mers' buckets above that, up to 7 * 2^16 occurrences, take twice the
-// filter in one block of twice the threads per SM (the same warps): us per million
-// k-mers, wide / k_ext_flat, at 272 K occurrences per bucket 68 / 96, 340 K 77 / 96,
-// 504 K 109 / 100.  64-bit ones would lose half their warps: 480 K 52 / 51.
-template <typename K>
-constexpr uint32_t EXT_WIDE_OCC = sizeof(K) == 16 ? 7u << 16 : EXT_FILTER_OCC;
-constexpr uint32_t EXT_ITEM_OCC = 16384;  // least occurrences worth reading the bucket's keys again
 
 // Extension masks: which of a node's 8 possible neighbours are nodes of its
 // bucket, and per side the state over to the neighbour when it is the side's
@@ -2072,8 +2057,9 @@ __global__ void __launch_bounds__(WIDE ? 1024 : ext_cfg<K>::THREADS, WIDE ? 1 : 
     }
 }
 
-// The same without a filter, for buckets of more keys than one is good for:
-// small blocks in bucket order, so the buckets in flight stay in L2.
+// The same without a filter, for buckets of more keys than one is good for and for
+// groups of too few buckets to fill the chip with filter blocks (ext_plan): small
+// blocks in bucket order, so the buckets in flight stay in L2.
 template <typename K>
 __global__ void __launch_bounds__(256, 8)
     k_ext_flat(ext_item const* __restrict__ items, uint32_t nitems, uint32_t t1, unsigned long long const* ne,
@@ -3001,27 +2987,25 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     for (size_t g = 0; g < ng; ++g) Tmax = std::max<uint64_t>(Tmax, toff[gb[g + 1]] - toff[gb[g]]);
     uint32_t* occ_slot = A.alloc<uint32_t>(nocc);
     // the buckets of k_ext_mask, of its wide form and of k_ext_flat, per group, with
-    // their blocks.
-    // A k_ext_mask bucket is split so that there are about four blocks per
-    // resident one (the last ones leave few SMs idle), but into no smaller parts
-    // than are worth reading the bucket's keys again for its filter.
+    // their blocks
     std::vector<ext_item> items;
     std::vector<uint32_t> gitem(3 * ng + 1, 0), gblocks(3 * ng, 0);
-    {
-        const uint64_t share = std::max<uint64_t>(EXT_ITEM_OCC, nocc / (148 * 8));
-        for (size_t g = 0; g < 3 * ng; ++g) {  // group g / 3: filter, wide filter, flat
+    const ext_plan plan(sizeof(K) == 16, nocc);
+    for (size_t g = 0; g < ng; ++g) {
+        uint64_t const* off = bocc.data() + b0 + gb[g];
+        const uint32_t gn = gb[g + 1] - gb[g];
+        const uint64_t cut = plan.cut(off, gn), tn = off[gn] - off[0];
+        for (int f = 0; f < 3; ++f) {
             uint32_t blocks = 0;
-            for (uint32_t b = gb[g / 3]; b < gb[g / 3 + 1]; ++b) {
-                const uint64_t ba = bocc[b0 + b] - O0, n = bocc[b0 + b + 1] - O0 - ba;
-                if (n == 0 || (n > EXT_FILTER_OCC) + (n > EXT_WIDE_OCC<K>) != (int)(g % 3)) continue;
-                items.push_back(ext_item{b - gb[g / 3], blocks, (uint32_t)ba, (uint32_t)(ba + n)});
-                blocks += (uint32_t)(g % 3 == 2                ? ceil_div(n, (uint64_t)ext_cfg<K>::FLAT_OCC)
-                                     : n > share + share / 2 ? ceil_div(n, share)
-                                                             : 1);
+            for (uint32_t b = 0; b < gn; ++b) {
+                const uint64_t ba = off[b] - O0, n = off[b + 1] - off[b];
+                if (n == 0 || plan.form(n, cut) != f) continue;
+                items.push_back(ext_item{b, blocks, (uint32_t)ba, (uint32_t)(ba + n)});
+                blocks += (uint32_t)plan.blocks(n, f, tn);
             }
             items.push_back(ext_item{0, blocks, 0, 0});
-            gblocks[g] = blocks;
-            gitem[g + 1] = (uint32_t)items.size();
+            gblocks[3 * g + f] = blocks;
+            gitem[3 * g + f + 1] = (uint32_t)items.size();
         }
     }
     // one upload: table offsets, capacities, items
@@ -3112,7 +3096,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         }
         CDBG_CHECK_LAUNCH();
         {
-            CDBG_PROF("k_ext_mask", st);
+            CDBG_PROF("k_ext_mask", st);  // (its three forms)
             constexpr int smem = EXT_FILTER_WORDS * 4;
             CDBG_CUDA(cudaFuncSetAttribute(k_ext_mask<K, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
             if constexpr (sizeof(K) == 16)
@@ -3123,9 +3107,9 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
                 if (gblocks[3 * g + c])
                     kern<<<gblocks[3 * g + c], threads, sm, st>>>(d_items + a, n, t1, nnext, TG, n_key, k, fw, n_mask, link);
             };
-            launch(k_ext_mask<K, false>, 0, ext_cfg<K>::THREADS, smem);
-            if constexpr (sizeof(K) == 16) launch(k_ext_mask<K, true>, 1, 1024, 2 * smem);
-            launch(k_ext_flat<K>, 2, 256, 0);
+            launch(k_ext_mask<K, false>, EXT_FILTER, ext_cfg<K>::THREADS, smem);
+            if constexpr (sizeof(K) == 16) launch(k_ext_mask<K, true>, EXT_WIDE, 1024, 2 * smem);
+            launch(k_ext_flat<K>, EXT_FLAT, 256, 0);
         }
         CDBG_CHECK_LAUNCH();
         {
