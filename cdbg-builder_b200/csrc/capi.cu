@@ -2039,7 +2039,6 @@ int cdbg_engine_set_tuning(cdbg_engine* e, const cdbg_tuning* t) {
     }
     cdbg_tuning v = *t;
     if (v.minimizer_tile == 0) v.minimizer_tile = 4096;
-    if (v.heavy_colors == 0) v.heavy_colors = 64;
     if (v.table_slots_q == 0) v.table_slots_q = 8;
     if (v.minimizer_tile != 1024 && v.minimizer_tile != 2048 && v.minimizer_tile != 4096) {
         g_last_error = "minimizer_tile must be 1024, 2048 or 4096";
@@ -2099,7 +2098,6 @@ int cdbg_engine_autotune(cdbg_engine* e, const cdbg_seq_batch* b, const cdbg_bui
         };
         cdbg_tuning cur = e->tune;
         if (cur.minimizer_tile == 0) cur.minimizer_tile = 4096;
-        if (cur.heavy_colors == 0) cur.heavy_colors = 64;
         if (cur.table_slots_q == 0) cur.table_slots_q = 8;
         if (cur.radix_bits == 0) cur.radix_bits = 8;
         measure(cur);  // warm-up: allocations reach their working sizes
@@ -2121,7 +2119,7 @@ int cdbg_engine_autotune(cdbg_engine* e, const cdbg_seq_batch* b, const cdbg_bui
             t.minimizer_tile = v;
             if (t.minimizer_tile != cur.minimizer_tile) consider(t);
         }
-        for (uint32_t v : {16u, 32u, 64u, 128u, 256u}) {
+        for (uint32_t v : {0u, 8u, 16u, 32u, 64u, 128u, 256u}) {
             cdbg_tuning t = cur;
             t.heavy_colors = v;
             if (t.heavy_colors != cur.heavy_colors) consider(t);

@@ -3172,11 +3172,11 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     // ---- counts the host needs next: union groups, heavy records (with a
     // bitmap: unions of at least that many colors), records used as color sets
     const uint32_t nw = (C + 31) / 32;
-    // The default threshold (64) is for bitmaps of many words; where a bitmap
-    // is no longer than a list of 8 colors it is 8 (unions of 90 genomes in
-    // skewed buckets 2.4 ms instead of 3.1; of 60 genomes of the small kind 0.29 instead
-    // of 0.40; thresholds 4 and 16 within 10% of it).
-    const uint32_t heavy = p.heavy_colors == 64 && nw <= 8 ? 8 : std::max<uint32_t>(1, p.heavy_colors);
+    // Unless the caller names a threshold: 64 colors; where a bitmap is no longer
+    // than a list of 8 colors, 8 (unions of 90 genomes in skewed buckets 2.4 ms
+    // instead of 3.1; of 60 genomes of the small kind 0.29 instead of 0.40;
+    // thresholds 4 and 16 within 10% of it).
+    const uint32_t heavy = p.heavy_colors ? p.heavy_colors : nw <= 8 ? 8 : 64;
     const bool may_heavy = M && p.union_bitmaps && C >= heavy;
     uint32_t* hflag = nullptr;
     uint64_t* hpos = nullptr;

@@ -86,8 +86,8 @@ struct phase2_params {
     // C/8 bytes per such k-mer, so very large color counts use lists)
     bool union_bitmaps = true;
     // records with at least this many colors get a precomputed bitmap in
-    // multi-record unions (performance only)
-    uint32_t heavy_colors = 64;
+    // multi-record unions (performance only); 0: by the number of colors
+    uint32_t heavy_colors = 0;
     // k-mer table slots per 4 occurrences of a bucket, 5..16 (performance only)
     uint32_t table_slots_q = 8;
     // continue the class dictionary of the previous call on the same state

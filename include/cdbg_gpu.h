@@ -63,8 +63,9 @@ typedef struct cdbg_tuning {
     uint32_t minimizer_tile;   /* (k-1)-mers per minimizer tile: 1024, 2048 or
                                   4096 (default 4096) */
     uint32_t heavy_colors;     /* records with >= this many colors get a bitmap
-                                  in multi-record unions (default 64, taken as 8
-                                  up to 256 colors) */
+                                  in multi-record unions (0, the default: 8
+                                  up to 256 colors, 64 above; any other value
+                                  as given) */
     uint32_t table_slots_q;    /* k-mer table slots per 4 occurrences of a
                                   bucket, 5..16 (default 8: a load factor of at
                                   most 1/2 over occurrences; fewer slots move
