@@ -185,12 +185,6 @@ struct bit_reader {
     }
 };
 
-__device__ __forceinline__ uint32_t lanemask_lt_() {
-    uint32_t m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
-}
-
 // The canonical code with lengths lens[0, n) by length: counts, first codes and
 // symbols in order.  Returns false for an over-subscribed set, and for an
 // incomplete one unless it is a single code of one bit or no code at all (with

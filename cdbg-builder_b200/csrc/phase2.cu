@@ -787,16 +787,6 @@ __device__ __forceinline__ uint32_t warp_excl_scan32(uint32_t v, uint32_t& total
     total = __shfl_sync(0xffffffffu, x, 31);
     return x - v;
 }
-__device__ __forceinline__ uint64_t warp_excl_scan64(uint64_t v, uint64_t& total) {
-    const int lane = threadIdx.x & 31;
-    uint64_t x = v;
-    for (int o = 1; o < 32; o <<= 1) {
-        uint64_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= o) x += y;
-    }
-    total = __shfl_sync(0xffffffffu, x, 31);
-    return x - v;
-}
 
 // OR the ascending list [c0, c1) of `list` into the shared bitmap `bm` of
 // `nw` words (all 32 lanes call it).  A dense list (at least one element per
@@ -2569,8 +2559,6 @@ __global__ void k_chain_cycles(chain_ws W, unsigned long long const* __restrict_
 }
 
 // ---- fragments --------------------------------------------------------------
-__device__ __forceinline__ uint32_t frag_cid(uint32_t const* n_cid, uint32_t node) { return n_cid[node]; }
-
 // Fragments in node order of their seeds, in one pass over the nodes: seed_of[f],
 // and off[f], the offset of its record (frag_unitig_writer::write_batch layout);
 // tot[0..2] = fragments, record bytes, sequence bases.
@@ -3129,7 +3117,7 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     // zeroed together: selections over the pairs, records, nodes and fragments,
     // heavy-record flags, the chains' seed lengths and covered flags, counts
     zero_block Z(3 * zero_block::select_words(npairs) + zero_block::select_words(nrec) +
-                     2 * zero_block::select_words(D) + nrec / 2 + D / 2 + D / 8 + 16,
+                     zero_block::select_words(D) + zero_block::tiles(D, prim::SEL_TILE) + nrec / 2 + D / 2 + D / 8 + 16,
                  A, st);
     // ---- multi-record k-mers, from their (node, record) pairs
     uint64_t M = 0;
@@ -3509,11 +3497,12 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     // ---- fragments, in seed order (offsets and seeds sized for D of them)
     uint32_t* seed_of = A.alloc<uint32_t>(D);
     uint64_t* foff = A.alloc<uint64_t>(D + 1);
-    select_ws wseed = Z.select(D), wbytes = Z.select(D);
+    select_ws wseed = Z.select(D);
+    unsigned long long* byte_status = Z.take<unsigned long long>(wseed.ntiles);
     unsigned long long* ftot = Z.take<unsigned long long>(3);
     {
         CDBG_PROF("k_seed_list", st);
-        k_seed_list<<<(unsigned)wseed.ntiles, 256, 0, st>>>(D, W.seed_len, W.seed_info, k, wseed, wbytes.status, seed_of,
+        k_seed_list<<<(unsigned)wseed.ntiles, 256, 0, st>>>(D, W.seed_len, W.seed_info, k, wseed, byte_status, seed_of,
                                                             foff, ftot, d_err);
     }
     CDBG_CHECK_LAUNCH();
