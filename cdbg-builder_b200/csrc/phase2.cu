@@ -2983,16 +2983,18 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         uint64_t const* off = bocc.data() + b0 + gb[g];
         const uint32_t gn = gb[g + 1] - gb[g];
         const uint64_t cut = plan.cut(off, gn), tn = off[gn] - off[0];
+        std::vector<ext_item> of[3];
+        uint32_t* blocks = &gblocks[3 * g];
+        for (uint32_t b = 0; b < gn; ++b) {
+            const uint64_t ba = off[b] - O0, n = off[b + 1] - off[b];
+            if (n == 0) continue;
+            const int f = plan.form(n, cut);
+            of[f].push_back(ext_item{b, blocks[f], (uint32_t)ba, (uint32_t)(ba + n)});
+            blocks[f] += (uint32_t)plan.blocks(n, f, tn);
+        }
         for (int f = 0; f < 3; ++f) {
-            uint32_t blocks = 0;
-            for (uint32_t b = 0; b < gn; ++b) {
-                const uint64_t ba = off[b] - O0, n = off[b + 1] - off[b];
-                if (n == 0 || plan.form(n, cut) != f) continue;
-                items.push_back(ext_item{b, blocks, (uint32_t)ba, (uint32_t)(ba + n)});
-                blocks += (uint32_t)plan.blocks(n, f, tn);
-            }
-            items.push_back(ext_item{0, blocks, 0, 0});
-            gblocks[3 * g + f] = blocks;
+            items.insert(items.end(), of[f].begin(), of[f].end());
+            items.push_back(ext_item{0, blocks[f], 0, 0});
             gitem[3 * g + f + 1] = (uint32_t)items.size();
         }
     }
