@@ -210,7 +210,9 @@ typedef struct cdbg_phase2_args {
     uint32_t num_buckets;
     uint32_t k;
     uint32_t num_colors;
-    const char* frag_path;       /* frag_unitigs.bin (unitig_spill.hpp:642-665 layout) */
+    const char* frag_path;       /* frag_unitigs.bin (unitig_spill.hpp:642-665 layout):
+                                    a file, or anything that can be written in
+                                    order (a FIFO, a device) */
     const char* color_sets_path; /* finalized .color_sets, or NULL */
     cdbg_class_cb on_class;      /* may be NULL */
     void* ctx;
