@@ -727,10 +727,54 @@ __global__ void __launch_bounds__(256, 8) k_multi_index(uint64_t n, uint32_t con
 
 // Multi-record nodes in node order whose owning-record list equals the
 // previous one's (the k-mers of a stretch shared by the same records) share
-// one union: group g has its first node and its record range, every multi
+// one union.  Bit m % 32 of same[m / 32]: node m's list is node m - 1's.  A lane
+// compares lists of up to SHORT_LIST records itself, the warp the longer ones.
+// A pass of its own, without order: repeats have stretches of k-mers in thousands
+// of records, and a tile of those would hold up every later tile's look-back (300
+// genomes with shared and tandem repeats, k = 63: 7.8 ms with the comparison inside
+// k_multi_groups, 1.4 for the two).
+constexpr uint64_t SHORT_LIST = 8;
+__global__ void __launch_bounds__(256) k_multi_same(uint64_t M, uint64_t const* __restrict__ moff,
+                                                    uint32_t const* __restrict__ urec, uint32_t* __restrict__ same) {
+    const uint64_t m = (uint64_t)blockIdx.x * 256 + threadIdx.x;
+    const int lane = threadIdx.x & 31;
+    if (m - lane >= M) return;
+    uint64_t a0 = 0, a1 = 0;
+    bool eq = false;
+    if (m > 0 && m < M) {
+        a0 = moff[m - 1];
+        a1 = moff[m];
+        eq = a1 - a0 == moff[m + 1] - a1;
+    }
+    const uint64_t n = a1 - a0;
+    uint32_t todo = __ballot_sync(0xffffffffu, eq && n > SHORT_LIST);
+    if (eq && n <= SHORT_LIST)
+        for (uint64_t i = 0; i < n && eq; ++i) eq = urec[a0 + i] == urec[a1 + i];
+    __syncwarp();
+    while (todo) {
+        const int src = __ffs(todo) - 1;
+        todo &= todo - 1;
+        const uint64_t x = __shfl_sync(0xffffffffu, a0, src), y = __shfl_sync(0xffffffffu, a1, src);
+        bool bad = false;
+        for (uint64_t base = 0; base < y - x && !bad; base += 128) {  // (the same trips for all lanes)
+            bool b = false;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint64_t i = base + 32 * q + lane;
+                b |= i < y - x && urec[x + i] != urec[y + i];
+            }
+            bad = __any_sync(0xffffffffu, b);
+        }
+        if (lane == src) eq = !bad;
+    }
+    const uint32_t w = __ballot_sync(0xffffffffu, eq);
+    if (lane == 0) same[m >> 5] = w;
+}
+
+// Group g of the nodes above has its first node and its record range, every multi
 // node its group.
-__global__ void __launch_bounds__(256) k_multi_groups(uint64_t M, uint64_t const* __restrict__ moff,
-                                                      uint32_t const* __restrict__ urec,
+__global__ void __launch_bounds__(256) k_multi_groups(uint64_t M, uint32_t const* __restrict__ same,
+                                                      uint64_t const* __restrict__ moff,
                                                       uint32_t const* __restrict__ mnode, select_ws ws,
                                                       uint32_t* __restrict__ gnode, uint64_t* __restrict__ gbeg,
                                                       uint64_t* __restrict__ gend, uint32_t* __restrict__ mgrp,
@@ -741,20 +785,7 @@ __global__ void __launch_bounds__(256) k_multi_groups(uint64_t M, uint64_t const
 #pragma unroll
     for (int r = 0; r < prim::SEL_ROUNDS; ++r) {
         const uint64_t m = tile * prim::SEL_TILE + 256u * r + threadIdx.x;
-        if (m >= M) continue;
-        bool same = false;
-        if (m > 0) {
-            const uint64_t a0 = moff[m - 1], a1 = moff[m], b1 = moff[m + 1];
-            if (a1 - a0 == b1 - a1) {
-                same = true;
-                for (uint64_t i = 0; i < a1 - a0; ++i)
-                    if (urec[a0 + i] != urec[a1 + i]) {
-                        same = false;
-                        break;
-                    }
-            }
-        }
-        if (!same) sel |= 1u << r;
+        if (m < M && !((same[m >> 5] >> (m & 31)) & 1u)) sel |= 1u << r;
     }
     prim::select_rank(head, sel, tile, ws.ntiles, ws.status, ws.total, err);
 #pragma unroll
@@ -3174,8 +3205,11 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     if (M) {
         wg = Z.select(M);
         {
-            CDBG_PROF("k_multi_groups", st);
-            k_multi_groups<<<(unsigned)wg.ntiles, 256, 0, st>>>(M, moff, urec, mnode, wg, gnode, gbeg, gend, mgrp,
+            uint32_t* same = A.alloc<uint32_t>(ceil_div(M, (uint64_t)32));
+            CDBG_PROF("k_multi_groups", st);  // (both)
+            k_multi_same<<<grid(M, 256), 256, 0, st>>>(M, moff, urec, same);
+            CDBG_CHECK_LAUNCH();
+            k_multi_groups<<<(unsigned)wg.ntiles, 256, 0, st>>>(M, same, moff, mnode, wg, gnode, gbeg, gend, mgrp,
                                                                 d_err);
         }
         CDBG_CHECK_LAUNCH();
