@@ -1899,31 +1899,39 @@ __device__ __forceinline__ uint32_t left_state(K can, K rev, uint32_t nt, uint32
     return right_state<K>(rev, can, nt, k, node) ^ 1u;
 }
 
-// One bucket of k_ext_mask / k_ext_flat: blocks from `block` on share its
-// occurrences [ba, bb) (batch-relative) evenly, a block taking the k-mers first
-// inserted by its share.  An item past the last holds the grid's size.
+// One bucket of k_ext_mask or k_ext_flat, its occurrences [ba, bb)
+// (batch-relative): blocks from `first` on share them evenly, a block taking the
+// k-mers first inserted by its share.  In k_ext_flat's packed form `first` = the
+// occurrences of the list's buckets before it, and its blocks take equal stretches
+// of all of them.  An item past the last holds the grid's size or the sum.
 struct ext_item {
-    uint32_t bucket, block, ba, bb;
+    uint32_t bucket, first, ba, bb;
 };
-struct ext_share {
-    uint32_t bucket, oa, ob, ba, bb;
-};
-// The calling block's share: 32-way search over the n items (whole warps call).
-__device__ __forceinline__ ext_share find_share(ext_item const* __restrict__ items, uint32_t n) {
+// The last of the n items whose `first` is at most x (whole warps call; the first
+// item's is 0): 32-way search.
+__device__ __forceinline__ uint32_t find_item(ext_item const* __restrict__ items, uint32_t n, uint32_t x) {
     const uint32_t lane = threadIdx.x & 31;
     uint32_t lo = 0, hi = n;  // the item is in [lo, hi)
     while (hi - lo > 1) {
         const uint32_t step = (hi - lo + 31) / 32;
         const uint32_t i = lo + lane * step;
-        const bool le = i < hi && items[i].block <= blockIdx.x;
+        const bool le = i < hi && items[i].first <= x;
         const uint32_t m = __ballot_sync(0xffffffffu, le);  // a prefix of the lanes, lane 0 among them
         const uint32_t at = 31 - __clz(m);
         const uint32_t l = lo + at * step;
         hi = min(l + step, hi);
         lo = l;
     }
-    const ext_item it = items[lo];
-    const uint32_t parts = items[lo + 1].block - it.block, c = blockIdx.x - it.block;
+    return lo;
+}
+struct ext_share {
+    uint32_t bucket, oa, ob, ba, bb;
+};
+// The calling block's share (not packed).
+__device__ __forceinline__ ext_share find_share(ext_item const* __restrict__ items, uint32_t n) {
+    const uint32_t at = find_item(items, n, blockIdx.x);
+    const ext_item it = items[at];
+    const uint32_t parts = items[at + 1].first - it.first, c = blockIdx.x - it.first;
     const uint64_t len = it.bb - it.ba;
     return ext_share{it.bucket, it.ba + (uint32_t)(len * c / parts), it.ba + (uint32_t)(len * (c + 1) / parts), it.ba,
                      it.bb};
@@ -2078,49 +2086,97 @@ __global__ void __launch_bounds__(WIDE ? 1024 : ext_cfg<K>::THREADS, WIDE ? 1 : 
     }
 }
 
-// The same without a filter, for buckets of more keys than one is good for and for
-// groups of too few buckets to fill the chip with filter blocks (ext_plan): small
-// blocks in bucket order, so the buckets in flight stay in L2.
+// Node n's mask and states with all eight neighbours probed in its bucket's table.
 template <typename K>
-__global__ void __launch_bounds__(256, 8)
-    k_ext_flat(ext_item const* __restrict__ items, uint32_t nitems, uint32_t t1, unsigned long long const* ne,
-               tables<K> T, K const* __restrict__ n_key, uint32_t k, uint2 const* __restrict__ fw,
-               uint8_t* __restrict__ n_mask, uint32_t* __restrict__ link) {
+__device__ __forceinline__ void probe_neighbours(uint32_t n, slot_t<K> const* t, uint32_t cap,
+                                                 K const* __restrict__ n_key, uint32_t k,
+                                                 uint2 const* __restrict__ fw, uint8_t* __restrict__ n_mask,
+                                                 uint32_t* __restrict__ link) {
     typedef kmer_ops<K> ops;
-    const ext_share it = find_share(items, nitems);
-    auto nodes_before = [&](uint32_t o) { return o < t1 ? node_of(fw, o) : (uint32_t)*ne; };
-    const uint32_t na = nodes_before(it.oa), nz = nodes_before(it.ob);
     const K msk = ops::mask(k);
     const uint32_t top = 2 * (k - 1);
-    const uint32_t cap = (uint32_t)T.tab_cap[it.bucket];
-    slot_t<K> const* t = T.slots + (T.tab_off[it.bucket] - T.off0);
-    for (uint32_t n = na + threadIdx.x; n < nz; n += 256) {
-        const K can = n_key[n];
-        const K rev = ops::revcomp(can, k);
-        uint32_t out = 0, right = NONE32, left = NONE32;
+    const K can = n_key[n];
+    const K rev = ops::revcomp(can, k);
+    uint32_t out = 0, right = NONE32, left = NONE32;
 #pragma unroll
-        for (uint32_t nt = 0; nt < 4; ++nt) {
-            const K hi = (K)(3u - nt) << top;
-            const K f = ((can << 2) | (K)nt) & msk;
-            const K fr = (rev >> 2) | hi;
-            const uint32_t a = node_probe(t, cap, f <= fr ? f : fr);
-            if (a != NONE32) {
-                out |= 1u << nt;
-                right = a;
-            }
-            const K r = ((rev << 2) | (K)nt) & msk;
-            const K rr = (can >> 2) | hi;
-            const uint32_t b = node_probe(t, cap, r <= rr ? r : rr);
-            if (b != NONE32) {
-                out |= 1u << (4 + nt);
-                left = b;
-            }
+    for (uint32_t nt = 0; nt < 4; ++nt) {
+        const K hi = (K)(3u - nt) << top;
+        const K f = ((can << 2) | (K)nt) & msk;
+        const K fr = (rev >> 2) | hi;
+        const uint32_t a = node_probe(t, cap, f <= fr ? f : fr);
+        if (a != NONE32) {
+            out |= 1u << nt;
+            right = a;
         }
-        n_mask[n] = (uint8_t)out;
-        uint2 l;
-        l.x = __popc(out >> 4) == 1 ? left_state<K>(can, rev, __ffs(out >> 4) - 1, k, node_of(fw, left)) : NONE32;
-        l.y = __popc(out & 0xfu) == 1 ? right_state<K>(can, rev, __ffs(out & 0xfu) - 1, k, node_of(fw, right)) : NONE32;
-        reinterpret_cast<uint2*>(link)[n] = l;
+        const K r = ((rev << 2) | (K)nt) & msk;
+        const K rr = (can >> 2) | hi;
+        const uint32_t b = node_probe(t, cap, r <= rr ? r : rr);
+        if (b != NONE32) {
+            out |= 1u << (4 + nt);
+            left = b;
+        }
+    }
+    n_mask[n] = (uint8_t)out;
+    uint2 l;
+    l.x = __popc(out >> 4) == 1 ? left_state<K>(can, rev, __ffs(out >> 4) - 1, k, node_of(fw, left)) : NONE32;
+    l.y = __popc(out & 0xfu) == 1 ? right_state<K>(can, rev, __ffs(out & 0xfu) - 1, k, node_of(fw, right)) : NONE32;
+    reinterpret_cast<uint2*>(link)[n] = l;
+}
+
+// The same without a filter, for buckets of more keys than one is good for and for
+// groups of too few or too small buckets to fill the chip with filter blocks
+// (ext_plan): small blocks in bucket order, so the buckets in flight stay in L2.
+// PACKED: blocks of `share` occurrences of the list's buckets laid end to end, for
+// buckets of less than a few blocks.
+constexpr uint32_t FLAT_MOST = 1024;  // largest share
+template <typename K, bool PACKED>
+__global__ void __launch_bounds__(256, 8)
+    k_ext_flat(ext_item const* __restrict__ items, uint32_t nitems, uint32_t share, uint32_t t1,
+               unsigned long long const* ne, tables<K> T, K const* __restrict__ n_key, uint32_t k,
+               uint2 const* __restrict__ fw, uint8_t* __restrict__ n_mask, uint32_t* __restrict__ link) {
+    auto nodes_before = [&](uint32_t o) { return o < t1 ? node_of(fw, o) : (uint32_t)*ne; };
+    if constexpr (!PACKED) {
+        const ext_share it = find_share(items, nitems);
+        const uint32_t na = nodes_before(it.oa), nz = nodes_before(it.ob);
+        const uint32_t cap = (uint32_t)T.tab_cap[it.bucket];
+        slot_t<K> const* t = T.slots + (T.tab_off[it.bucket] - T.off0);
+        for (uint32_t n = na + threadIdx.x; n < nz; n += 256) probe_neighbours<K>(n, t, cap, n_key, k, fw, n_mask, link);
+    } else {
+        // of the block's buckets: its first node, and the block's nodes before it
+        __shared__ uint32_t s_node[FLAT_MOST], s_at[FLAT_MOST], sw[256 / 32 + 1];
+        const uint32_t v0 = blockIdx.x * share, v1 = min(v0 + share, items[nitems].first);
+        const uint32_t lo = find_item(items, nitems, v0);
+        const uint32_t cnt = find_item(items, nitems, v1 - 1) + 1 - lo;  // at most `share`: an item has an occurrence
+        uint32_t total = 0;
+        for (uint32_t i0 = 0; i0 < cnt; i0 += 256) {
+            const uint32_t i = i0 + threadIdx.x;
+            uint32_t a = 0, c = 0, all;
+            if (i < cnt) {
+                const ext_item it = items[lo + i];
+                a = nodes_before(it.ba + (v0 > it.first ? v0 - it.first : 0u));
+                c = nodes_before(it.ba + min(it.bb - it.ba, v1 - it.first)) - a;
+            }
+            const uint32_t at = total + prim::block_exclusive_scan<uint32_t, 256>(c, sw, all);
+            if (i < cnt) {
+                s_node[i] = a;
+                s_at[i] = at;
+            }
+            total += all;
+        }
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < total; j += 256) {
+            uint32_t q = 0;  // the node's bucket: the last that starts at or before it
+            for (uint32_t h = cnt; h - q > 1;) {
+                const uint32_t mid = (q + h) >> 1;
+                if (s_at[mid] <= j)
+                    q = mid;
+                else
+                    h = mid;
+            }
+            const uint32_t bucket = items[lo + q].bucket;
+            probe_neighbours<K>(s_node[q] + (j - s_at[q]), T.slots + (T.tab_off[bucket] - T.off0),
+                                (uint32_t)T.tab_cap[bucket], n_key, k, fw, n_mask, link);
+        }
     }
 }
 
@@ -3008,26 +3064,39 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
     // the buckets of k_ext_mask, of its wide form and of k_ext_flat, per group, with
     // their blocks
     std::vector<ext_item> items;
-    std::vector<uint32_t> gitem(3 * ng + 1, 0), gblocks(3 * ng, 0);
+    std::vector<uint32_t> gitem(3 * ng + 1, 0), gblocks(3 * ng, 0), gshare(ng, 0);  // (share 0: not packed)
     const ext_plan plan(sizeof(K) == 16, nocc);
     for (size_t g = 0; g < ng; ++g) {
         uint64_t const* off = bocc.data() + b0 + gb[g];
         const uint32_t gn = gb[g + 1] - gb[g];
-        const uint64_t cut = plan.cut(off, gn), tn = off[gn] - off[0];
+        const uint64_t cut = plan.cut(off, gn);
+        const uint64_t tn = off[gn] - off[0];
         std::vector<ext_item> of[3];
-        uint32_t* blocks = &gblocks[3 * g];
+        uint32_t first[3] = {0, 0, 0};
         for (uint32_t b = 0; b < gn; ++b) {
             const uint64_t ba = off[b] - O0, n = off[b + 1] - off[b];
             if (n == 0) continue;
             const int f = plan.form(n, cut);
-            of[f].push_back(ext_item{b, blocks[f], (uint32_t)ba, (uint32_t)(ba + n)});
-            blocks[f] += (uint32_t)plan.blocks(n, f, tn);
+            of[f].push_back(ext_item{b, first[f], (uint32_t)ba, (uint32_t)(ba + n)});
+            first[f] += (uint32_t)(f == EXT_FLAT ? n : plan.parts(n));
+        }
+        const uint32_t share = plan.flat_occ(tn);
+        const bool packed = plan.packed(first[EXT_FLAT], of[EXT_FLAT].size(), tn);
+        if (!packed) {
+            first[EXT_FLAT] = 0;
+            for (ext_item& it : of[EXT_FLAT]) {
+                it.first = first[EXT_FLAT];
+                first[EXT_FLAT] += (it.bb - it.ba + share - 1) / share;
+            }
         }
         for (int f = 0; f < 3; ++f) {
             items.insert(items.end(), of[f].begin(), of[f].end());
-            items.push_back(ext_item{0, blocks[f], 0, 0});
+            items.push_back(ext_item{0, first[f], 0, 0});
             gitem[3 * g + f + 1] = (uint32_t)items.size();
+            gblocks[3 * g + f] = first[f];
         }
+        gshare[g] = packed ? share : 0;
+        if (packed) gblocks[3 * g + EXT_FLAT] = (uint32_t)ceil_div((uint64_t)first[EXT_FLAT], (uint64_t)share);
     }
     // one upload: table offsets, capacities, items
     const size_t items_at = 8 * (2 * (size_t)nb + 1), up_bytes = items_at + items.size() * sizeof(ext_item);
@@ -3123,14 +3192,18 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
             if constexpr (sizeof(K) == 16)
                 CDBG_CUDA(cudaFuncSetAttribute(k_ext_mask<K, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * smem));
             const uint32_t t1 = (uint32_t)(t0 + tn);
-            auto launch = [&](auto kern, int c, int threads, int sm) {
+            auto launch = [&](auto kern, int c, int threads, int sm, auto... share) {
                 const uint32_t a = gitem[3 * g + c], n = gitem[3 * g + c + 1] - a - 1;
                 if (gblocks[3 * g + c])
-                    kern<<<gblocks[3 * g + c], threads, sm, st>>>(d_items + a, n, t1, nnext, TG, n_key, k, fw, n_mask, link);
+                    kern<<<gblocks[3 * g + c], threads, sm, st>>>(d_items + a, n, share..., t1, nnext, TG, n_key, k, fw,
+                                                                  n_mask, link);
             };
             launch(k_ext_mask<K, false>, EXT_FILTER, ext_cfg<K>::THREADS, smem);
             if constexpr (sizeof(K) == 16) launch(k_ext_mask<K, true>, EXT_WIDE, 1024, 2 * smem);
-            launch(k_ext_flat<K>, EXT_FLAT, 256, 0);
+            if (gshare[g])
+                launch(k_ext_flat<K, true>, EXT_FLAT, 256, 0, gshare[g]);
+            else
+                launch(k_ext_flat<K, false>, EXT_FLAT, 256, 0, 0u);
         }
         CDBG_CHECK_LAUNCH();
         {

@@ -18,7 +18,8 @@ DRIVER = r'''
 #include <vector>
 #include "ext_plan.hpp"
 using namespace cdbg;
-// wide keys, then "count size" pairs; prints buckets and blocks per form
+// wide keys, then "count size" pairs; prints buckets per form, blocks of the filters
+// and occurrences of a flat block
 int main(int argc, char** v) {
     std::vector<uint64_t> off{12345};
     for (int i = 2; i + 1 < argc; i += 2)
@@ -26,19 +27,19 @@ int main(int argc, char** v) {
     const uint64_t tn = off.back() - off[0];
     const ext_plan p(v[1][0] == '1', tn);
     const uint64_t cut = p.cut(off.data(), off.size() - 1);
-    uint64_t nb[3] = {}, bl[3] = {};
+    uint64_t nb[3] = {}, bl[2] = {};
     for (size_t b = 0; b + 1 < off.size(); ++b) {
         const uint64_t n = off[b + 1] - off[b];
         if (!n) continue;
         const int f = p.form(n, cut);
         nb[f]++;
-        bl[f] += p.blocks(n, f, tn);
-        if (!p.blocks(n, f, tn)) return 1;
+        if (f != EXT_FLAT) bl[f] += p.parts(n);
+        if (!p.parts(n)) return 1;
         if (f != EXT_FLAT && n > p.wide_occ) return 2;
         if (f == EXT_WIDE && v[1][0] == '0') return 3;
     }
     std::printf("%llu %llu %llu %llu %llu %llu\n", (unsigned long long)nb[0], (unsigned long long)nb[1],
-                (unsigned long long)nb[2], (unsigned long long)bl[0], (unsigned long long)bl[1], (unsigned long long)bl[2]);
+                (unsigned long long)nb[2], (unsigned long long)bl[0], (unsigned long long)bl[1], (unsigned long long)p.flat_occ(tn));
     return 0;
 }
 '''
@@ -63,8 +64,8 @@ def plan(tmp_path_factory):
 
 @pytest.mark.parametrize("wide", [False, True])
 def test_forms_by_group(plan, wide):
-    assert plan(wide) == [0] * 6
-    assert plan(wide, 5, 0) == [0] * 6
+    assert plan(wide) == [0] * 5 + [256]
+    assert plan(wide, 5, 0) == [0] * 5 + [256]
     assert plan(wide, 64, 600)[:3] == [64, 0, 0]           # a toy build: one launch, no probes to spare
     assert plan(wide, 1024, 49_000)[:3] == [1024, 0, 0]    # full groups
     assert plan(wide, 4096, 200_000)[:3] == [4096, 0, 0]
@@ -76,8 +77,30 @@ def test_forms_by_group(plan, wide):
         assert plan(wide, 1, max(n, 50_000))[2] == 1
         assert plan(wide, 4, max(n, 50_000))[2] == 4
     assert plan(wide, 4096, 100_000, 3, 5_000_000)[:3] == [4096, 0, 3]
-    # blocks of one round of 256 where the chip is idle
-    assert plan(wide, 1, 60_000)[5] == (60_000 + 255) // 256
+    for n in (1, 30, 120):                                 # blocks cost more than what small buckets hold
+        assert plan(wide, 16_384, n)[2] == 16_384
+    assert plan(wide, 60_000, 40, 900, 60_000)[:3] in ([900, 0, 60_000], [60_900, 0, 0])
+    # flat blocks of one round of 256 where the chip is idle, never more than the kernel's lists hold
+    assert plan(wide, 1, 60_000)[5] == 256
+    assert plan(wide, 4096, 1_000_000)[5] == (512 if wide else 1024)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [31, 63])
+@pytest.mark.parametrize("bases,buckets", [(900, 7), (40_000, 1), (40_000, 1500), (60_000, 20_000), (1_500_000, 30_000),
+                                           (1_500_000, 400)])
+def test_small_buckets(oracle, engine, tmp_path, k, bases, buckets):
+    """Flat blocks over many small buckets, empty ones among them, and large ones
+    beside them, against the CPU oracle."""
+    from test_gpu_edges import _check
+    rng = np.random.default_rng(bases + buckets + k)
+    dna = lambda n: rng.choice(np.frombuffer(b"ACGT", dtype=np.uint8), size=n).tobytes()  # noqa: E731
+    a = dna(bases)
+    b = bytearray(a[: bases // 2])
+    for i in rng.integers(0, len(b), len(b) // 70).tolist():
+        b[i] = b"ACGT"[int(rng.integers(0, 4))]
+    low = b"A" * (bases // 8) + b"AC" * (bases // 16) + dna(50)  # a few buckets hold an eighth of all
+    _check(oracle, engine, tmp_path, [[a, low], [bytes(b), a[-2 * k:] + a[: 2 * k]]], k, buckets)
 
 
 @pytest.mark.gpu
