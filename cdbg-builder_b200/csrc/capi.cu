@@ -1082,12 +1082,7 @@ bool phase1_device_reader(cdbg_engine* e, std::vector<std::string> const& files,
     }
     const uint64_t tot_in = ioff[nf], tot_out = ooff[nf];
     if (!any_gz) return false;
-    // A CTA inflates ~170 MB/s and all files at once, T host threads ~T x 200
-    // MB/s together: the device reader wins while no file holds more than about
-    // 1/T of the input.  Phase 1 with the reading, device / host reader, gzip -1
-    // genomes: T = 16, 2.4 Mbp files: 12 files 20.2 / 16.5 ms, 16 files 21.3 /
-    // 24.9, 64 files 25.5 / 72; T = 4: 4 files 18.3 / 11.2, 6 files 18.6 / 21.3.
-    if (e->tune.gpu_inflate == 0 && (double)max_out * 1.25 * threads > (double)tot_out) return false;
+    if (e->tune.gpu_inflate == 0 && !cdbg::io::device_reader_pays(max_out, tot_out, tot_in, threads)) return false;
     cudaStream_t st = e->st;
     char* h = (char*)e->h_in.ensure(tot_in + 64);
     cdbg::io::read_raw_files(files, threads, h, ioff.data());

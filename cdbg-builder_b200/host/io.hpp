@@ -3,6 +3,7 @@
 // zlib and the system LZ4 block library.
 #pragma once
 
+#include <algorithm>
 #include <cstdint>
 #include <functional>
 #include <string>
@@ -49,6 +50,21 @@ struct file_probe {
 };
 file_probe probe_file(std::string const& path);
 void probe_files(std::vector<std::string> const& files, uint32_t threads, std::vector<file_probe>& out);
+
+// Whether the device reader is the faster one for files of at most max_out bytes
+// inflated, tot_out together, tot_in as stored.  A CTA inflates ~200 MB/s whatever
+// the bytes are, all files at once; T host threads ~T x 62 MB/s of stored bytes
+// together (200 MB/s of sequence, several times that of runs): the device wins while
+// no file holds more than about 1/T of the input, counted as sequence that deflates
+// to 0.31 where it deflates further.  Phase 1 with the reading, files of 2.4 MB,
+// device / host reader, ms: gzip -1 genomes T = 16, 16 files 20.0 / 27.1, 40 files
+// 22.0 / 36.0, T = 4, 5 files 18.1 / 19.3 (4 files 18.3 / 11.2); gzip -6, T = 16, 16
+// files 17.1 / 16.9, 32 files 18.8 / 28.5; half of each N, gzip -6, T = 16, 20 files
+// 18.1 / 14.3, 40 files 19.4 / 19.5, T = 4, 8 files 16.7 / 10.0, 12 files 17.0 / 15.3.
+inline bool device_reader_pays(uint64_t max_out, uint64_t tot_out, uint64_t tot_in, uint32_t threads) {
+    const double seq = std::min((double)tot_out, (double)tot_in / 0.31);
+    return 1.25 * threads * (double)max_out <= seq;
+}
 
 // Reads files[i] whole (as stored on disk) into dst + off[i], in parallel;
 // off has files.size() + 1 entries, off[i + 1] - off[i] the file's size.
