@@ -2193,6 +2193,7 @@ __device__ __forceinline__ uint32_t back_nib(uint32_t m, bool rc) { return (rc ?
 // genomes: 2.9 ms with one and the states taken from the k-mers here, 0.90 so
 // (and 0.4 more in k_ext_mask, which has the k-mers at hand).
 constexpr int LINKS_PER = 4;
+template <bool EVEN_K>
 __global__ void __launch_bounds__(256, 8) k_links(unsigned long long const* nb, unsigned long long const* ne,
                                                   uint8_t const* __restrict__ n_mask, uint32_t* __restrict__ link,
                                                   uint32_t* __restrict__ ends, unsigned long long* nends) {
@@ -2220,6 +2221,10 @@ __global__ void __launch_bounds__(256, 8) k_links(unsigned long long const* nb, 
             uint2 t = l[j];
             if (t.x != NONE32 && (__popc(fwd_nib(ml[j], t.x & 1u)) != 1 || (t.x >> 1) == (uint32_t)n)) t.x = NONE32;
             if (t.y != NONE32 && (__popc(back_nib(mr[j], t.y & 1u)) != 1 || (t.y >> 1) == (uint32_t)n)) t.y = NONE32;
+            // a k-mer that is its own reverse complement (k even) has the same
+            // neighbour on both sides, at one port of it: the walk ends there (it is
+            // entered with rc = false, whose way on is the R port)
+            if (EVEN_K && t.x != NONE32 && t.x == (t.y ^ 1u)) t.y = NONE32;
             if (t.x != l[j].x || t.y != l[j].y) reinterpret_cast<uint2*>(link)[n] = t;
             end |= (t.x == NONE32 || t.y == NONE32 ? 1u : 0u) << j;
         }
@@ -2523,8 +2528,11 @@ __global__ void __launch_bounds__(256) k_chain_lead(chain_ws W, uint32_t const* 
     const unsigned long long c0 = block_reserve<256>(lead ? L : 0, W.cursor);
     const unsigned long long h = block_reserve<256>(lead && !whole ? 1 : 0, nheads);
     if (!lead) return;
-    if (c0 + L > W.D) {  // chains partition the nodes; anything else is a bug
+    if (c0 + L > W.D) {
+        // (chains partition the nodes, anything else is a bug: an error, and no
+        // chain is left half described)
         set_error(err, ERR_CAPACITY);
+        if (!whole) heads[h] = make_uint4(0, 0, 0, 0);
         return;
     }
     if (!whole) {
@@ -2575,6 +2583,7 @@ __global__ void __launch_bounds__(128) k_chain_paths(chain_ws W, uint4 const* __
         bool r = (hd.x >> 31) != 0;
         const uint32_t L = hd.y;
         const uint64_t c0 = ((uint64_t)hd.w << 32) | hd.z;
+        if (L == 0) continue;
         W.ch_node[c0] = cc;
         W.ch_rc[c0] = r ? 1 : 0;
         for (uint32_t i = 1; i < L && chain_step(W.link, cc, r); ++i) {
@@ -2589,11 +2598,12 @@ __global__ void __launch_bounds__(128) k_chain_paths(chain_ws W, uint4 const* __
 }
 
 // The number of nodes on paths; when that is not all there are cycles, and
-// k_chain_cycles needs to know the others.
+// k_chain_cycles needs to know the others.  (More than all: an error is set, and not
+// every fragment element is written.)
 __global__ void k_chain_covered(chain_ws W, unsigned long long* __restrict__ paths) {
     const uint64_t n = *W.cursor;
     if (blockIdx.x == 0 && threadIdx.x == 0) *paths = n;
-    if (n == W.D) return;
+    if (n >= W.D) return;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
         W.covered[W.fe[i] >> 1] = 1;
 }
@@ -2601,7 +2611,7 @@ __global__ void k_chain_covered(chain_ws W, unsigned long long* __restrict__ pat
 // Cycles: nodes left uncovered; the smallest node index of a cycle leads.
 // `paths` = the nodes on paths.
 __global__ void k_chain_cycles(chain_ws W, unsigned long long const* __restrict__ paths, uint32_t* err) {
-    if (*paths == W.D) return;
+    if (*paths >= W.D) return;
     for (uint64_t n = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; n < W.D;
          n += (uint64_t)gridDim.x * blockDim.x) {
         if (W.covered[n]) continue;
@@ -3208,8 +3218,11 @@ void run_batch(record_set const& rs, rec_view const& R, phase2_params const& p, 
         CDBG_CHECK_LAUNCH();
         {
             CDBG_PROF("k_links", st);
-            k_links<<<(unsigned)std::min<uint64_t>(grid(tn, 256 * LINKS_PER), 148 * 16), 256, 0, st>>>(
-                nbase, nnext, n_mask, link, ends, nends);
+            const unsigned blocks = (unsigned)std::min<uint64_t>(grid(tn, 256 * LINKS_PER), 148 * 16);
+            if (k & 1u)
+                k_links<false><<<blocks, 256, 0, st>>>(nbase, nnext, n_mask, link, ends, nends);
+            else
+                k_links<true><<<blocks, 256, 0, st>>>(nbase, nnext, n_mask, link, ends, nends);
         }
         CDBG_CHECK_LAUNCH();
     }
